@@ -1,13 +1,15 @@
 // Plain matrix product on the CUDA cores: out[t, n] = sum_k x[t, k] * w[n, k] (+ bias[n]).
 // Every product and sum is an fp32 FMA (no tensor cores, no TF32, no reduced-precision staging),
-// and each output accumulates over k in ascending order whatever the number of rows, so a row's
-// result does not depend on what else is in the batch.  This is the matrix product of the 32-bit
-// path, and the checked fallback for shapes the tensor-core kernel refuses.
+// and each output is summed in one order whatever the number of rows (even and odd k's ascending within
+// runs, the runs within parts and the parts in ascending order: gemm_f32.cuh), so a row's result does not depend on what else is in the batch.
+// This is the checked fallback for shapes that the tensor-core kernels refuse, and for 32-bit rows that the
+// kernels of gemm_f32.cu do not take (K or strides that are no multiples of four); it sums in the order of theirs.
 //
 // The weight keeps the layout of the model folder, [out features, in features]; the reference
 // transposes at load and computes out[n] += x[k] * W[k, n] over ascending k
 // (crates/ferrisinfer-kernel/src/cpu/matmul.rs:437-446), which is the same sum.
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 namespace {
 
@@ -26,12 +28,13 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TIn* x, const TIn*
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tr = tid / 16, tc = tid % 16;  // this thread's 4x4 patch: rows tr*4.., cols tc*4..
     const int lrow = tid / 4, lk = (tid % 4) * 4;
-    float acc[TM][TN];
+    float acc[2][TM][TN], part[TM][TN], total[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+        for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = part[i][j] = total[i][j] = 0.0f;
 
+    const int part_k = f32_runs_per_part((K + F32_CHUNK - 1) / F32_CHUNK) * F32_CHUNK;
     for (int k0 = 0; k0 < K; k0 += BK) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -51,9 +54,24 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TIn* x, const TIn*
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
         }
         __syncthreads();
+        const bool last = k0 + BK >= K;
+        if (last || (k0 + BK) % F32_CHUNK == 0) {  // a run ends, and with it perhaps a part
+            const bool ends = last || (k0 + BK) % part_k == 0;
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    part[i][j] += acc[0][i][j] + acc[1][i][j];
+                    acc[0][i][j] = acc[1][i][j] = 0.0f;
+                    if (ends) {
+                        total[i][j] += part[i][j];
+                        part[i][j] = 0.0f;
+                    }
+                }
+        }
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -63,7 +81,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TIn* x, const TIn*
         for (int j = 0; j < TN; ++j) {
             const int n = n0 + tc * TN + j;
             if (n >= N) continue;
-            float v = acc[i][j];
+            float v = total[i][j];
             if (bias) v += bias[n];
             TOut* o = out + (size_t)m * ldo + n;
             if (MODE == 1)
@@ -100,6 +118,11 @@ FERRIS_API int ferris_gemm_simt(const void* x, const void* w, const float* bias,
     if (accumulate && out_dtype != FERRIS_F32) FERRIS_REFUSE("gemm: accumulation needs an fp32 output");
     if ((M + BM - 1) / BM > 65535) FERRIS_REFUSE("gemm: %d rows are more than one launch takes", M);
     cudaStream_t s = (cudaStream_t)stream;
+    if (in_dtype == FERRIS_F32 && out_dtype == FERRIS_F32 && ferris_gemm_f32_takes(x, w, out, K, ldx, ldw)) {
+        bool taken;
+        const int rc = ferris_gemm_f32((const float*)x, (const float*)w, bias, (float*)out, M, N, K, ldx, ldw, ldo, accumulate, s, &taken);
+        if (taken) return rc;
+    }
     if (in_dtype == FERRIS_F32 && out_dtype == FERRIS_F32)
         return launch<float, float>(x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, s);
     if (in_dtype == FERRIS_BF16 && out_dtype == FERRIS_F32)

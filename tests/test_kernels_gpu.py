@@ -100,6 +100,36 @@ def test_gemm_rows_do_not_depend_on_the_batch(device):
     assert torch.equal(one[0], full[41])
 
 
+@pytest.mark.parametrize("N, K", [(8, 4), (150, 132), (75, 1020), (896, 896), (67, 1028), (64, 2052), (40, 9220)])
+def test_gemm_fp32_sums_in_one_order_in_every_form(N, K, device):
+    """The 32-bit products for few rows, for many rows and for rows that are not aligned (runs of 128 k's within at most
+    eight parts of K, at their edges) give one row the same bits; against 64 bits within the bound of the longest chain of sums."""
+    from ferrisinfer_b200.kernels import ops
+
+    w, bias = rnd((N, K), F32, device, 20), rnd((N,), F32, device, 21)
+    x = rnd((137, K), F32, device, 22)
+    acc0 = rnd((137, N), F32, device, 23)
+    odd_x, odd_w = torch.empty(137, K + 1, device=device), torch.empty(N, K + 1, device=device)
+    odd_x[:, 1:], odd_w[:, 1:] = x, w
+    want = x.double() @ w.double().t() + bias.double()
+    # |error| <= (rounds on an element's way through run, part, parts, bias) 2^-24 sum |x w|
+    bound = (128 + K / 1024 + 8 + 3) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t() + bias.double().abs())
+    first = None
+    for M in (137, 65, 33, 32, 17, 9, 8, 5, 4, 3, 2, 1):
+        out = torch.full((M, N), 7.0, device=device)
+        ops.gemm_simt(x[:M], w, bias, out)
+        assert ((out.double() - want[:M]).abs() <= bound[:M]).all()
+        first = out if first is None else first
+        assert torch.equal(out, first[:M]), M
+        acc = acc0[:M].clone()
+        ops.gemm_simt(x[:M], w, bias, acc, accumulate=True)
+        assert torch.equal(acc, acc0[:M] + first[:M]), M
+    out = torch.empty(137, N, device=device)
+    ops.gemm_simt(odd_x[:, 1:], odd_w[:, 1:], bias, out)
+    assert torch.equal(out, first)
+    assert ops.kernel_status() == 0
+
+
 # ------------------------------------------------------------------------- tensor-core gemm
 TC_SHAPES = [(1, 1152, 896), (8, 1152, 896), (64, 896, 4864), (5, 130, 72), (16, 128, 64), (17, 300, 1000),
              (300, 256, 128), (2048, 384, 256), (33, 1000, 80), (257, 129, 200),
