@@ -1,11 +1,15 @@
 // The general attention over a bf16 cache on tensor cores, with the softmax's weights in 32-bit: head sizes of any multiple
 // of eight up to 256 (the values' may differ, or lie in the keys), any page size, any grouping of heads, a window, a chunk or
-// every key, pooled keys before the window or first tokens that it keeps, a soft cap, a sink, gates.  The formulas and arguments are those of attention_simt.cu.
+// every key, pooled keys before the window or first tokens that it keeps, a soft cap, distance penalties, a sink, gates.  The formulas and arguments are those of attention_simt.cu.
 //
 // q . k is a product of bf16 numbers with fp32 sums, as exact as FMAs on the widened numbers.  The second product, weights
 // times values, must not round the weights to bf16: a weight p is cut into three bf16 parts, p1 = bf16(p), p2 = bf16(p - p1),
 // p3 = bf16(p - p1 - p2), whose sum is p to the last of its 24 bits, and the three products with the values meet in one fp32
 // accumulator.  Scores, maximum, exponentials and sums are fp32 (powers of two: the scale carries log2 e).
+//
+// A distance penalty (TERMS) is one fp32 FMA, or a logarithm, on every score beside the 12 instructions that a score costs
+// anyway; it is a form of its own so that the plain one keeps its registers.  A prompt of 2,048 tokens, 16 heads of 128 over 4, a
+// window of 1,024 and slopes: 167 us on tensor cores (bound by their products, three for one), 929 us on CUDA cores.
 //
 // Two kernels.  Portions of prompts: a block takes 64 rows, the g query heads of one kv head for floor(64 / g) consecutive
 // tokens, and walks the keys in tiles that asynchronous copies bring into shared memory one tile ahead; each of its four
@@ -73,7 +77,22 @@ struct AttentionArgs {
     const bf16* gate;  // the heads' gates, rows ldgate apart (null: none)
     int ldgate;
     int values_in_keys;  // a value is the first dv elements of its key: the keys' tile serves both products, v is not read
+    const float* slopes;  // distance penalties per query head (null: none): linear,
+    const float* log_r1;  // or with the logarithm of the distance
+    const float* log_r2;
 };
+// The distance penalty of a head in powers of two, and a scaled score with it taken off.
+struct Penalty {
+    float a, b;
+    bool log;
+};
+__device__ __forceinline__ Penalty penalty_of(const AttentionArgs& p, int h) {
+    if (p.log_r1) return {p.log_r1[h] * LOG2E, p.log_r2[h], true};
+    return {p.slopes[h] * LOG2E, 0.0f, false};
+}
+__device__ __forceinline__ float penalised(float s, const Penalty& t, int distance) {
+    return t.log ? s - t.a * log1pf(t.b * (float)distance) : fmaf(-t.a, (float)distance, s);
+}
 // sigmoid of the gate of head h at token t
 __device__ __forceinline__ float gate_of(const AttentionArgs& p, int t, int h) {
     return p.gate ? 1.0f / (1.0f + expf(-to_float(p.gate[(size_t)t * p.ldgate + h]))) : 1.0f;
@@ -154,7 +173,7 @@ __device__ __forceinline__ void weights_times_values(float (&o)[DT][4], const fl
 // ------------------------------------------------------------------------------------------ portions of prompts
 // D: columns held for a head (64, 128, 256; d, dv <= D).  KT: keys to a tile.  The query fragments stay in registers up to
 // D = 128 and come from shared memory beyond.
-template <int D, int KT, bool POOL>
+template <int D, int KT, bool POOL, bool TERMS>
 __global__ void __launch_bounds__(AR_THREADS, D <= 128 ? 3 : 2) attention_rows_kernel(const AttentionArgs p) {
     constexpr int KS = D / 16, DT = D / 8, NT = KT / 8;
     constexpr bool QREG = D <= 128;
@@ -180,9 +199,11 @@ __global__ void __launch_bounds__(AR_THREADS, D <= 128 ? 3 : 2) attention_rows_k
     }
     int rt[2], rpos[2], rseq[2];
     const bf16* qrow[2];
+    Penalty pen[2];
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
         const int r = 16 * warp + gq + 8 * a;
+        if constexpr (TERMS) pen[a] = penalty_of(p, hk * g + r % g);
         rt[a] = r < qt * g ? t_first + r / g : p.tokens;
         const bool ok = rt[a] < t_end;
         rpos[a] = ok ? p.positions[rt[a]] : -1;
@@ -305,7 +326,19 @@ __global__ void __launch_bounds__(AR_THREADS, D <= 128 ? 3 : 2) attention_rows_k
                 to[a] = (run ? seen_runs[a] - 1 : hi[a]) - j0;
             }
             const bool whole = from[0] <= 0 && from[1] <= 0 && to[0] >= KT - 1 && to[1] >= KT - 1;
-            if (__all_sync(0xffffffffu, whole)) {
+            if constexpr (TERMS) {  // (rows ahead of the window are kept tokens here: they lie at their positions)
+                const int far0 = hi[0] - j0 - 2 * tq, far1 = hi[1] - j0 - 2 * tq;
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int c = 8 * n + 2 * tq + (e & 1);
+                        // (a key beyond the token is not seen, and its distance would leave the logarithm's domain)
+                        const int far = max(0, (e >> 1 ? far1 : far0) - 8 * n - (e & 1));
+                        const float x = penalised(s[n][e] * p.scale2, pen[e >> 1], far);
+                        s[n][e] = c >= from[e >> 1] && c <= to[e >> 1] ? x : -INFINITY;
+                    }
+            } else if (__all_sync(0xffffffffu, whole)) {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -363,7 +396,7 @@ struct SingleStages {
     static constexpr int value = D <= 64 ? 4 : (D <= 128 ? 3 : 2);
 };
 
-template <int D, bool POOL, bool FAST>
+template <int D, bool POOL, bool FAST, bool TERMS>
 __global__ void __launch_bounds__(AR_THREADS) attention_single_rows_kernel(const AttentionArgs p, int row_groups, int splits) {
     constexpr int KS = D / 16, MT = D / 16, STAGES = SingleStages<D>::value;
     constexpr int PITCH = (D + 8) * 2;
@@ -403,6 +436,11 @@ __global__ void __launch_bounds__(AR_THREADS) attention_single_rows_kernel(const
             qf[ks][0] = gq < rows && c < d ? *reinterpret_cast<const uint32_t*>(row + c) : 0u;
             qf[ks][1] = gq < rows && c + 8 < d ? *reinterpret_cast<const uint32_t*>(row + c + 8) : 0u;
         }
+    }
+    Penalty pen[2];
+    if constexpr (TERMS) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a) pen[a] = penalty_of(p, hk * g + r0 + min(2 * tq + a, rows - 1));
     }
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
     float o[MT][4];
@@ -480,7 +518,9 @@ __global__ void __launch_bounds__(AR_THREADS) attention_single_rows_kernel(const
             const int at = gq + (e >> 1) * 8;
             float x = s[0][e] + s[1][e];
             if (p.scale_cap > 0.0f) x = tanhf(x * p.scale_cap);
-            w[e] = at >= from && at <= to ? x * p.scale2 : -INFINITY;
+            x *= p.scale2;
+            if constexpr (TERMS) x = penalised(x, pen[e & 1], max(0, P - first_of(c) - at));
+            w[e] = at >= from && at <= to ? x : -INFINITY;
         }
         float alpha[2];
         bool moved = false;
@@ -616,36 +656,43 @@ int device_sms() {
     return sms;
 }
 
-template <int D, bool POOL>
-int launch_rows(const AttentionArgs& p, cudaStream_t s) {
+template <int D, bool POOL, bool TERMS>
+int launch_rows_form(const AttentionArgs& p, cudaStream_t s) {
     const int qt = AR_ROWS / (p.nh / p.nkv);
     constexpr int KT = rows_keys<D>();
     constexpr size_t smem = rows_smem<D>();
-    int rc = ferris_allow_dynamic_smem((const void*)attention_rows_kernel<D, KT, POOL>, smem);
+    int rc = ferris_allow_dynamic_smem((const void*)attention_rows_kernel<D, KT, POOL, TERMS>, smem);
     if (rc != FERRIS_OK) return rc;
-    ferris_launch(attention_rows_kernel<D, KT, POOL>, dim3((p.tokens + qt - 1) / qt, p.nkv), dim3(AR_THREADS), smem, s, p);
+    ferris_launch(attention_rows_kernel<D, KT, POOL, TERMS>, dim3((p.tokens + qt - 1) / qt, p.nkv), dim3(AR_THREADS), smem, s, p);
     FERRIS_LAUNCH_CHECK();
 }
 
-template <int D, bool POOL, bool FAST>
+template <int D, bool POOL>
+int launch_rows(const AttentionArgs& p, cudaStream_t s) {
+    return p.slopes || p.log_r1 ? launch_rows_form<D, POOL, true>(p, s) : launch_rows_form<D, POOL, false>(p, s);
+}
+
+template <int D, bool POOL, bool FAST, bool TERMS>
 int launch_single_form(const AttentionArgs& p, int splits, cudaStream_t s) {
     const int groups = (p.nh / p.nkv + AS_ROWS - 1) / AS_ROWS;
     constexpr size_t smem = single_smem<D>();
     static_assert((size_t)(AR_WARPS + 1) * AS_ROWS * (D + 2) * sizeof(float) <= smem, "the warps meet in the ring's memory");
-    int rc = ferris_allow_dynamic_smem((const void*)attention_single_rows_kernel<D, POOL, FAST>, smem);
+    int rc = ferris_allow_dynamic_smem((const void*)attention_single_rows_kernel<D, POOL, FAST, TERMS>, smem);
     if (rc != FERRIS_OK) return rc;
     const dim3 grid(p.tokens, p.nkv * groups, splits);
     if (splits > 1)
-        ferris_launch_cluster(attention_single_rows_kernel<D, POOL, FAST>, grid, dim3(AR_THREADS), smem, s, (unsigned)splits, p, groups, splits);
+        ferris_launch_cluster(attention_single_rows_kernel<D, POOL, FAST, TERMS>, grid, dim3(AR_THREADS), smem, s, (unsigned)splits, p, groups, splits);
     else
-        ferris_launch(attention_single_rows_kernel<D, POOL, FAST>, grid, dim3(AR_THREADS), smem, s, p, groups, splits);
+        ferris_launch(attention_single_rows_kernel<D, POOL, FAST, TERMS>, grid, dim3(AR_THREADS), smem, s, p, groups, splits);
     FERRIS_LAUNCH_CHECK();
 }
 
 template <int D, bool POOL>
 int launch_single(const AttentionArgs& p, int splits, cudaStream_t s) {
     const bool fast = !p.values_in_keys && p.d == D && p.dv == D && p.page_size % AS_KEYS == 0;
-    return fast ? launch_single_form<D, POOL, true>(p, splits, s) : launch_single_form<D, POOL, false>(p, splits, s);
+    if (p.slopes || p.log_r1)
+        return fast ? launch_single_form<D, POOL, true, true>(p, splits, s) : launch_single_form<D, POOL, false, true>(p, splits, s);
+    return fast ? launch_single_form<D, POOL, true, false>(p, splits, s) : launch_single_form<D, POOL, false, false>(p, splits, s);
 }
 
 }  // namespace
@@ -657,14 +704,14 @@ FERRIS_API int ferris_attention_rows_takes(int nh, int nkv, int d, int dv, int p
     return portions ? nh / nkv <= AR_ROWS : 1;
 }
 
-// Arguments as ferris_paged_attention_simt, bf16 throughout, no distance penalty; v_stride is 0 (values in rows of their own)
+// Arguments as ferris_paged_attention_simt, bf16 throughout; v_stride is 0 (values in rows of their own)
 // or d, with v_cache the key cache (a value is the first dv elements of its key).  portions:
 // requests bring several tokens each (the kernel of 64-row blocks); else kv_span is the most keys a token sees (0: unknown),
 // by which they are cut into shares.
 FERRIS_API int ferris_attention_rows(const void* q, int ldq, void* out, int ldo, const void* k_cache, const void* v_cache,
                                      const int* block_tables, int max_blocks, const int* token_seq, const int* positions,
                                      int tokens, int nh, int nkv, int d, int dv, int page_size, int window, float scale,
-                                     const float* sink, int v_stride, const void* pool_k, const void* pool_v, const int* pool_tables,
+                                     const float* slopes, const float* log_r1, const float* log_r2, const float* sink, int v_stride, const void* pool_k, const void* pool_v, const int* pool_tables,
                                      int pool_max_blocks, int pool_every, int keep, float softcap, const void* gate, int ldgate,
                                      int portions, int kv_span, void* stream) {
     if (tokens <= 0) return FERRIS_OK;
@@ -673,16 +720,17 @@ FERRIS_API int ferris_attention_rows(const void* q, int ldq, void* out, int ldo,
     if (page_size <= 0 || max_blocks <= 0) FERRIS_REFUSE("attention: page_size=%d max_blocks=%d", page_size, max_blocks);
     if (v_stride != 0 && (v_stride != d || dv > d || v_cache != k_cache))
         FERRIS_REFUSE("attention rows: values %d elements apart in keys of %d", v_stride, d);
-    const ScoreTerms st = {nullptr, nullptr, nullptr, sink, v_stride, softcap, gate, ldgate};
+    const ScoreTerms st = {slopes, log_r1, log_r2, sink, v_stride, softcap, gate, ldgate};
     const PooledKeys pk = keys_beside(pool_k, pool_v, pool_tables, pool_max_blocks, pool_every, keep, k_cache, v_cache, block_tables, max_blocks);
     if (int rc = check_pooled(pk, window, st)) return rc;
+    if ((log_r1 != nullptr) != (log_r2 != nullptr)) FERRIS_REFUSE("attention rows: half of a logarithmic penalty");
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)pool_k | (uintptr_t)pool_v) & 15) != 0 || ldq % 8 ||
         ((uintptr_t)out & 3) || (ldo & 1))
         FERRIS_REFUSE("attention rows: rows must start on 16 bytes");
     const AttentionArgs p = {(const bf16*)q, (bf16*)out, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, token_seq,
                              positions, sink, pk, ldq, ldo, max_blocks, tokens, nh, nkv, d, dv, page_size, window,
                              (softcap > 0.0f ? softcap : scale) * LOG2E, softcap > 0.0f ? scale / softcap : 0.0f,
-                             (const bf16*)gate, ldgate, v_stride > 0 ? 1 : 0};
+                             (const bf16*)gate, ldgate, v_stride > 0 ? 1 : 0, slopes, log_r1, log_r2};
     cudaStream_t s = (cudaStream_t)stream;
     const bool pool = pk.every > 0 || pk.keep > 0;
     const int bucket = rows_bucket(d, dv);

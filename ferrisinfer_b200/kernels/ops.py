@@ -832,7 +832,7 @@ def paged_attention_simt(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Te
     window's tokens the query sees one row of ``pooled`` for every run of positions that lies wholly before the window.
     ``keep_first`` (with a window, without ``pooled``): beside the window's tokens the query sees the request's first
     ``keep_first`` tokens.
-    bf16 without a distance penalty runs on tensor cores where the geometry allows it (``set_attention_rows``); everything else on CUDA cores."""
+    bf16 runs on tensor cores where the geometry allows it (``set_attention_rows``); everything else on CUDA cores."""
     dv = int(v_head_dim or head_dim)
     if chunk:
         if window or chunk < 0:
@@ -890,16 +890,17 @@ def paged_attention_simt(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Te
     if pooled is not None:
         span += max_kv_len // pooled.every
     single = max_q_len <= 1 and max_kv_len > 0 and workspace is not None
-    # bf16 without a distance penalty: on tensor cores, with the weights' 24 bits kept (the tiled kernel switched off, the
-    # CUDA-core form of single tokens is asked for)
-    if (_attention_rows and qkv.dtype == torch.bfloat16 and terms.slopes is None and terms.log_r1 is None
-            and (max_q_len <= 1 or _attention_tiled) and ldq % 8 == 0 and ldo % 2 == 0 and qkv.data_ptr() % 16 == 0
+    # bf16: on tensor cores, with the weights' 24 bits kept (the tiled kernel switched off, the CUDA-core form of single
+    # tokens is asked for)
+    if (_attention_rows and qkv.dtype == torch.bfloat16 and (max_q_len <= 1 or _attention_tiled) and ldq % 8 == 0
+            and ldo % 2 == 0 and (qkv.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0 and out.data_ptr() % 4 == 0
             and _lib().ferris_attention_rows_takes(num_heads, num_kv_heads, head_dim, dv, 1 if max_q_len > 1 else 0)):
         _check(_lib().ferris_attention_rows(
             _ptr(qkv), _c_int(ldq), _ptr(out), _c_int(ldo), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
             _c_int(block_tables.shape[1]), _ptr(token_seq), _ptr(positions), _c_int(T), _c_int(num_heads),
             _c_int(num_kv_heads), _c_int(head_dim), _c_int(dv), _c_int(k_cache.shape[2]),
-            _c_int(-chunk if chunk else (window or 0)), _c_float(scale), _ptr(terms.sink), _c_int(v_stride), *pool_args,
+            _c_int(-chunk if chunk else (window or 0)), _c_float(scale), _ptr(score_slopes), _ptr(terms.log_r1),
+            _ptr(terms.log_r2), _ptr(terms.sink), _c_int(v_stride), *pool_args,
             _c_int(1 if max_q_len > 1 else 0), _c_int(span if single else 0), _stream()), "attention rows")
         return
     fn = _lib().ferris_paged_attention_simt

@@ -363,6 +363,59 @@ def test_unit_norm_temperature_slopes_window_attention(device, nh, nkv, d, dv, w
             pos += n
 
 
+@pytest.mark.parametrize("kind", ["linear", "logarithmic"])
+@pytest.mark.parametrize("nh,nkv,d,dv", [(4, 1, 128, 128), (7, 1, 64, 64), (3, 3, 40, 24), (20, 2, 96, 200), (2, 1, 256, 256)])
+def test_distance_penalties_on_tensor_cores(device, nh, nkv, d, dv, kind):
+    """bf16 attention with a distance penalty: two requests' portions, and single tokens in one share and in several, with
+    every key, a window, a chunk, a window with kept tokens; tiles of 64 keys end inside, at and after what a token sees.
+    Against 64 bits: the output's own rounding (a bf16 has eight bits: up to 2^-8 of it), and scores of up to 2^7 that an fp32 sum leaves 2^-17 off."""
+    ops = _ops()
+    from ferrisinfer_b200.engine.workspace import Workspace
+
+    torch.manual_seed(nh + d)
+    lengths, starts, ps = [129, 66], [63, 0], 16
+    blocks = [-(-(a + n) // ps) for a, n in zip(starts, lengths)]
+    order = torch.randperm(sum(blocks))
+    table = torch.full((2, max(blocks)), -1, dtype=torch.int32)
+    table[0, :blocks[0]], table[1, :blocks[1]] = order[:blocks[0]].int(), order[blocks[0]:].int()
+    k = torch.randn(sum(blocks), nkv, ps, d).to(BF16)
+    v = torch.randn(sum(blocks), nkv, ps, dv).to(BF16)
+    q = torch.randn(sum(lengths), nh * d).to(BF16)
+    a, b = 0.02 + torch.rand(nh), 0.1 + torch.rand(nh)
+    a[0] = 0.0
+    terms = ops.ScoreTerms(slopes=a.to(device)) if kind == "linear" else ops.ScoreTerms(log_r1=a.to(device), log_r2=b.to(device))
+    scale, of = 2.0 / math.sqrt(d), torch.arange(nh) // (nh // nkv)
+    kd, vd, td = k.to(device), v.to(device), table.to(device)
+    for window, chunk, keep in ((0, 0, 0), (37, 0, 0), (64, 0, 0), (0, 50, 0), (30, 0, 9)):
+        want = torch.zeros(sum(lengths), nh, dv, dtype=F64)
+        for r, (n, p0) in enumerate(zip(lengths, starts)):
+            rows = table[r, :blocks[r]].long()
+            keys = k[rows].double().transpose(1, 2).reshape(-1, nkv, d)[:p0 + n]
+            values = v[rows].double().transpose(1, 2).reshape(-1, nkv, dv)[:p0 + n]
+            P, j = torch.arange(p0, p0 + n)[:, None], torch.arange(p0 + n)[None]
+            seen = j <= P
+            if window:
+                seen &= (P - j < window) | (j < keep)
+            if chunk:
+                seen &= j // chunk == P // chunk
+            far = (P - j).clamp_min(0).double()[None]
+            pen = a.double()[:, None, None] * (far if kind == "linear" else torch.log1p(b.double()[:, None, None] * far))
+            at = sum(lengths[:r])
+            s = torch.einsum("thd,shd->hts", q[at:at + n].double().view(n, nh, d), keys[:, of]) * scale - pen
+            wgt = torch.softmax(s.masked_fill(~seen, -math.inf), -1)
+            want[at:at + n] = torch.einsum("hts,shv->thv", wgt, values[:, of])
+        bound = 2.0 ** -8 * want.abs() + 2.0 ** -14 * vd.abs().max().item()
+        for form in ("portions", "single", "shares"):
+            ctx = fake_ctx(device, lengths, starts, [0, 1])
+            out = torch.empty(sum(lengths), nh * dv, dtype=BF16, device=device)
+            extra = dict(max_kv_len=max(p + n for p, n in zip(starts, lengths)), workspace=Workspace(device)) if form == "shares" else {}
+            ops.paged_attention_simt(q.to(device), out, kd, vd, td, ctx.token_seq, ctx.positions, nh, nkv, d, window, scale,
+                                     score_slopes=terms, v_head_dim=dv, max_q_len=max(lengths) if form == "portions" else 1,
+                                     chunk=chunk, keep_first=keep, **extra)
+            err = (out.cpu().double().view(-1, nh, dv) - want).abs()
+            assert (err <= bound).all(), (form, window, chunk, keep, (err / bound).max())
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("nh,nkv,d,dv", [(8, 2, 64, 64), (4, 2, 96, 32), (6, 1, 16, 16)])
 def test_attention_of_single_tokens_in_shares_of_keys(device, nh, nkv, d, dv, dtype):
