@@ -13,9 +13,8 @@
 // transposed in memory, [slot, head, vdim, dim], so that a warp reads and writes whole rows of it.
 // q, k, v may be passed through SiLU on the way in (`silu`), in fp32 whatever the storage type; q and k may be
 // rotated by their positions there, and k scaled (RotaryArgs): what enters the recurrence is then fp32 throughout.
-#include <math.h>
-
 #include "common.cuh"
+#include "linear_attention.cuh"
 
 namespace {
 
@@ -23,19 +22,6 @@ constexpr int LA_COLS = 8;
 constexpr int LA_WARPS = 4;
 constexpr int LA_STAGE = 8;      // tokens whose q, k, v stand in shared memory at a time
 constexpr int LA_MAX_DIM = 256;  // largest head size
-
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-
-// Rotary positions on q and k on their way in (positions null: none), and a factor on k after them.  The first
-// `rotary` elements of a head are rotated by the token's position: the pair (u, v), elements (i, i + rotary / 2)
-// or, `interleaved`, (2i, 2i + 1), becomes (u c - v s, v c + u s) with c = mag cos(pos * freq[i]), s = mag sin(same);
-// position x frequency is one fp32 product, sine and cosine are in full precision.
-struct RotaryArgs {
-    const int* positions;
-    const float* freq;
-    int rotary, interleaved;
-    float mag, k_scale;
-};
 
 // Eight sums over the warp's lanes with nine shuffles instead of forty: at each of the first three steps a lane
 // hands half of its partial sums to its partner and keeps the other half.  Every lane returns the sum of column
@@ -72,7 +58,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32) linear_attention_scan_kernel(
     const T* qkv, int ld, int q_off, int k_off, int v_off, float* __restrict__ out, int ldo, float* state,
     float* scratch, const float* __restrict__ decay, const int* __restrict__ seq_q_start,
     const int* __restrict__ seq_state_slot, int heads, int dim, int vdim, int silu, int write_state, int seg_len,
-    int segs_max, const RotaryArgs rot) {
+    int segs_max, int most, const RotaryArgs rot) {
     pdl_wait();
     pdl_launch_dependents();
     // q, k and this block's 32 columns of v of LA_STAGE tokens at a time, activation applied once, for all four warps
@@ -86,6 +72,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32) linear_attention_scan_kernel(
     const bool mine_cols = col0 < vdim;  // a warp beyond the last column only helps to stage
     int row0 = seq_q_start[seq];
     int row1 = seq_q_start[seq + 1];
+    if (MODE == 0 && row1 - row0 > most) return;
     bool last = true;
     if (MODE != 0) {
         row0 += seg * seg_len;
@@ -247,14 +234,14 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const float* o, int 
 template <typename T, int MODE>
 void launch_scan_mode(const void* qkv, int ld, int q_off, int k_off, int v_off, float* out, int ldo, float* state,
                       float* scratch, const float* decay, const int* seq_q_start, const int* seq_state_slot, int seqs,
-                      int heads, int dim, int vdim, int silu, int write_state, int seg_len, int segs_max, const RotaryArgs rot,
+                      int heads, int dim, int vdim, int silu, int write_state, int seg_len, int segs_max, int most, const RotaryArgs rot,
                       cudaStream_t s) {
     const dim3 grid(MODE == 0 ? seqs : seqs * segs_max, heads, (vdim + LA_COLS * LA_WARPS - 1) / (LA_COLS * LA_WARPS));
     const dim3 block(LA_WARPS * 32);
 #define FERRIS_LA_LAUNCH(RPL)                                                                                       \
     ferris_launch(linear_attention_scan_kernel<T, RPL, MODE>, grid, block, 0, s, (const T*)qkv, ld, q_off, k_off,   \
                   v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, heads, dim, vdim, silu,       \
-                  write_state, seg_len, segs_max, rot)
+                  write_state, seg_len, segs_max, most, rot)
     if (dim <= 32)
         FERRIS_LA_LAUNCH(1);
     else if (dim <= 64)
@@ -269,20 +256,20 @@ void launch_scan_mode(const void* qkv, int ld, int q_off, int k_off, int v_off, 
 template <typename T>
 int launch_scan(const void* qkv, int ld, int q_off, int k_off, int v_off, float* out, int ldo, float* state,
                 float* scratch, const float* decay, const int* seq_q_start, const int* seq_state_slot, int seqs,
-                int heads, int dim, int vdim, int silu, int write_state, int seg_len, int segs_max, const RotaryArgs rot,
+                int heads, int dim, int vdim, int silu, int write_state, int seg_len, int segs_max, int most, const RotaryArgs rot,
                 cudaStream_t s) {
     if (segs_max <= 1) {
         launch_scan_mode<T, 0>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot,
-                               seqs, heads, dim, vdim, silu, write_state, seg_len, 1, rot, s);
+                               seqs, heads, dim, vdim, silu, write_state, seg_len, 1, most, rot, s);
         FERRIS_LAUNCH_CHECK();
     }
     launch_scan_mode<T, 1>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, seqs,
-                           heads, dim, vdim, silu, write_state, seg_len, segs_max, rot, s);
+                           heads, dim, vdim, silu, write_state, seg_len, segs_max, most, rot, s);
     const size_t per_state = (size_t)heads * vdim * dim;
     ferris_launch(linear_attention_combine_kernel, dim3((unsigned)((per_state + 255) / 256), seqs), dim3(256), 0, s,
                   (const float*)state, scratch, decay, seq_q_start, seq_state_slot, heads, dim, vdim, seg_len);
     launch_scan_mode<T, 2>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, seqs,
-                           heads, dim, vdim, silu, write_state, seg_len, segs_max, rot, s);
+                           heads, dim, vdim, silu, write_state, seg_len, segs_max, most, rot, s);
     FERRIS_LAUNCH_CHECK();
 }
 
@@ -292,13 +279,14 @@ int launch_scan(const void* qkv, int ld, int q_off, int k_off, int v_off, float*
 // (heads x vdim), head by head; out: fp32 [tokens, heads x vdim] rows ldo apart; state: fp32 [slots, heads, vdim, dim];
 // decay: fp32 [heads].  The rows of request s are seq_q_start[s] .. seq_q_start[s + 1] - 1, in order.
 // segs_max > 1: no request brings more than segs_max * seg_len tokens, and they run as segments of seg_len side by
-// side through `scratch`, fp32 [tokens / seg_len + seqs + 1, heads, vdim, dim].
+// side through `scratch`, fp32 [tokens / seg_len + seqs + 1, heads, vdim, dim].  most: without segments, requests that bring
+// more tokens are left alone (the chunks of linear_chunks.cu are theirs).
 FERRIS_API int ferris_linear_attention(const void* qkv, int ld, int q_off, int k_off, int v_off, int dtype, float* out,
                                        int ldo, float* state, const float* decay, const int* seq_q_start,
                                        const int* seq_state_slot, int seqs, int heads, int dim, int vdim, int silu,
                                        int write_state, int seg_len, int segs_max, float* scratch,
                                        const int* positions, const float* freq, int rotary, int interleaved, float mag,
-                                       float k_scale, void* stream) {
+                                       float k_scale, int most, void* stream) {
     if (seqs <= 0) return FERRIS_OK;
     if (positions && (rotary < 0 || rotary > dim || (rotary & 1) || (rotary > 0 && !freq)))
         FERRIS_REFUSE("linear attention: %d rotated elements of heads of %d", rotary, dim);
@@ -310,9 +298,9 @@ FERRIS_API int ferris_linear_attention(const void* qkv, int ld, int q_off, int k
     if (!state || !decay) FERRIS_REFUSE("linear attention: no state or no decay");
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == FERRIS_F32)
-        return launch_scan<float>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, seqs, heads, dim, vdim, silu, write_state, seg_len, segs_max, rot, s);
+        return launch_scan<float>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, seqs, heads, dim, vdim, silu, write_state, seg_len, segs_max, most, rot, s);
     if (dtype == FERRIS_BF16)
-        return launch_scan<bf16>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, seqs, heads, dim, vdim, silu, write_state, seg_len, segs_max, rot, s);
+        return launch_scan<bf16>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot, seqs, heads, dim, vdim, silu, write_state, seg_len, segs_max, most, rot, s);
     FERRIS_REFUSE("linear attention: unknown dtype %d", dtype);
 }
 

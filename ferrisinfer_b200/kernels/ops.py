@@ -1135,6 +1135,15 @@ def short_conv(y: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, state: 
 
 
 LINEAR_ATTENTION_SEGMENT = 128
+LINEAR_ATTENTION_CHUNK = 64  # tokens of a chunk of the tensor-core form (linear_chunks.cu)
+LINEAR_ATTENTION_WALK_MAX = 32  # requests of at most so many tokens are walked token by token
+
+
+def _linear_scratch(ctx, floats: int, device) -> torch.Tensor:
+    ws = getattr(ctx, "workspace", None)
+    if ws is not None:
+        return ws.get("linear_attn_segments", (floats,), torch.float32)
+    return torch.empty(floats, dtype=torch.float32, device=device)
 
 
 def linear_attention(qkv: torch.Tensor, offsets: tuple, out: torch.Tensor, state: torch.Tensor, decay: torch.Tensor,
@@ -1147,7 +1156,9 @@ def linear_attention(qkv: torch.Tensor, offsets: tuple, out: torch.Tensor, state
     than ``segment`` tokens (128 by default) runs as segments side by side: a pass that sums each segment alone, one
     that carries the state from segment to segment, one that forms the outputs (scratch from the step's workspace).
     ``rotary``: q and k are rotated by the tokens' positions (``ctx.positions``) on their way in; ``k_scale``: k is then
-    multiplied by it.  Both in fp32, so what enters the recurrence is never rounded."""
+    multiplied by it.  Both in fp32, so what enters the recurrence is never rounded.
+    bf16 rows of steps with longer portions run as chunks of 64 tokens on tensor cores where the geometry allows it and no
+    ``segment`` is asked for; their products keep 21 bits and more."""
     T, width, ld = _rows(qkv, "linear attention input")
     T2, n, ldo = _rows(out, "linear attention output")
     _need(state, "linear attention state", torch.float32)
@@ -1156,22 +1167,47 @@ def linear_attention(qkv: torch.Tensor, offsets: tuple, out: torch.Tensor, state
     if (T2 != T or out.dtype != torch.float32 or n != heads * vdim or state.shape[1:] != (heads, vdim, dim)
             or decay.numel() != heads or max(q_off, k_off) + heads * dim > width or v_off + heads * vdim > width):
         raise KernelError(f"linear attention: qkv {tuple(qkv.shape)}, out {tuple(out.shape)}, state {tuple(state.shape)}")
-    seg = int(segment or LINEAR_ATTENTION_SEGMENT)
     longest = int(getattr(ctx, "max_q_len", 0) or T)
+    if (segment is None and longest > LINEAR_ATTENTION_WALK_MAX and qkv.dtype == torch.bfloat16
+            and _lib().ferris_linear_attention_chunks_takes(
+                _ptr(qkv), _c_int(ld), _c_int(q_off), _c_int(k_off), _c_int(v_off), _ptr(out), _c_int(ldo), _ptr(state),
+                _c_int(ctx.num_seqs), _c_int(longest), _c_int(heads), _c_int(dim), _c_int(vdim))):
+        states = (T // LINEAR_ATTENTION_CHUNK + ctx.num_seqs + 1) * heads * vdim * dim  # (a multiple of 64 floats)
+        scratch = _linear_scratch(ctx, states + T * heads * (2 * dim + vdim), qkv.device)
+        turn = (*_rotary_args(rotary, ctx, dim, qkv.device), _c_float(k_scale))
+        if ctx.num_seqs > 1:  # short requests beside the long ones
+            _check(
+                _lib().ferris_linear_attention(_ptr(qkv), _c_int(ld), _c_int(q_off), _c_int(k_off), _c_int(v_off),
+                                               _c_int(_dt(qkv, "linear attention")), _ptr(out), _c_int(ldo), _ptr(state),
+                                               _ptr(decay), _ptr(ctx.seq_q_start), _ptr(ctx.seq_state_slot), _c_int(ctx.num_seqs),
+                                               _c_int(heads), _c_int(dim), _c_int(vdim), _c_int(1 if silu else 0),
+                                               _c_int(1 if write_state else 0), _c_int(1), _c_int(1), _ptr(None), *turn,
+                                               _c_int(LINEAR_ATTENTION_WALK_MAX), _stream()),
+                "linear attention",
+            )
+        _check(
+            _lib().ferris_linear_attention_chunks(
+                _ptr(qkv), _c_int(ld), _c_int(q_off), _c_int(k_off), _c_int(v_off), _ptr(out), _c_int(ldo), _ptr(state),
+                _ptr(decay), _ptr(ctx.seq_q_start), _ptr(ctx.seq_state_slot), _c_int(T), _c_int(ctx.num_seqs),
+                _c_int(longest), _c_int(LINEAR_ATTENTION_WALK_MAX if ctx.num_seqs > 1 else 0), _c_int(heads), _c_int(dim), _c_int(vdim),
+                _c_int(1 if silu else 0), _c_int(1 if write_state else 0), _ptr(scratch), _ptr(scratch[states:]), *turn, _stream()),
+            "linear attention", 4,
+        )
+        return
+    seg = int(segment or LINEAR_ATTENTION_SEGMENT)
     segs_max = max(1, -(-longest // seg))
     scratch = None
     if segs_max > 1:
         floats = (T // seg + ctx.num_seqs + 1) * heads * vdim * dim
-        ws = getattr(ctx, "workspace", None)
-        scratch = ws.get("linear_attn_segments", (floats,), torch.float32) if ws is not None else \
-            torch.empty(floats, dtype=torch.float32, device=qkv.device)
+        scratch = _linear_scratch(ctx, floats, qkv.device)
     _check(
         _lib().ferris_linear_attention(_ptr(qkv), _c_int(ld), _c_int(q_off), _c_int(k_off), _c_int(v_off),
                                        _c_int(_dt(qkv, "linear attention")), _ptr(out), _c_int(ldo), _ptr(state),
                                        _ptr(decay), _ptr(ctx.seq_q_start), _ptr(ctx.seq_state_slot), _c_int(ctx.num_seqs),
                                        _c_int(heads), _c_int(dim), _c_int(vdim), _c_int(1 if silu else 0),
                                        _c_int(1 if write_state else 0), _c_int(seg), _c_int(segs_max), _ptr(scratch),
-                                       *_rotary_args(rotary, ctx, dim, qkv.device), _c_float(k_scale), _stream()),
+                                       *_rotary_args(rotary, ctx, dim, qkv.device), _c_float(k_scale), _c_int(0x7FFFFFFF),
+                                       _stream()),
         "linear attention", 1 if segs_max == 1 else 3,
     )
 

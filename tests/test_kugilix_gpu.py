@@ -228,6 +228,89 @@ def test_linear_attention_segments_of_several_requests(device):
     assert torch.equal(together[1], start[1])  # a slot that no request of the step holds
 
 
+def _decayed(q, k, v, S, decay):
+    """The recurrence in 64 bits: q, k [T, heads, dim], v [T, heads, vdim], S [heads, vdim, dim]; (outputs, last state)."""
+    out = []
+    for t in range(q.shape[0]):
+        S = decay[:, None, None] * S + v[t][:, :, None] * k[t][:, None, :]
+        out.append((S @ q[t][:, :, None])[..., 0])
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("heads,dim,vdim,silu,turn", [(2, 128, 128, True, None), (3, 64, 72, False, "halves"), (1, 8, 8, True, None),
+                                                      (2, 120, 64, False, "pairs"), (2, 40, 200, True, "halves")])
+def test_linear_attention_chunks_on_tensor_cores(device, heads, dim, vdim, silu, turn):
+    """bf16 portions that end at, before and after a chunk's edge beside short requests (which are walked), each from a state of its own, in turn
+    with and without the state moving on.  Bound: three cuts of 2^-22 on either product and fp32 sums over up to 64 tokens, 128
+    channels and five chunks, each 2^-24 of the sum of the terms' absolute values."""
+    ops = _ops()
+    torch.manual_seed(dim)
+    lens, starts, slots = [64, 1, 129, 63, 300, 32, 33], [7, 40, 0, 1000, 3, 9, 5], [4, 0, 5, 2, 1, 6, 7]
+    T, width, pad = sum(lens), 2 * heads * dim + heads * vdim, 8
+    proj = (torch.randn(T, width + pad) * 0.7).to(BF16)
+    decay = torch.tensor([0.98, 1.0, 0.0][:heads] if heads > 1 else [0.9])
+    start = torch.randn(8, heads, vdim, dim)
+    rotary, positions = None, torch.cat([torch.arange(a, a + n) for a, n in zip(starts, lens)]).float()
+    p = proj[:, :width].double()
+    q, k, v = p[:, :heads * dim].view(T, heads, dim), p[:, heads * dim:2 * heads * dim].view(T, heads, dim), p[:, 2 * heads * dim:].view(T, heads, vdim)
+    if silu:
+        q, k, v = plain.silu(q), plain.silu(k), plain.silu(v)
+    if turn:
+        R = dim // 2 - dim // 2 % 2
+        freq = 100.0 ** (-torch.arange(R // 2) / R)
+        rotary = ops.RotaryTable(freq.to(device), R, turn == "pairs", 1.25)
+        ang = (positions[:, None] * freq).double()[:, None]  # the product is one of 32 bits
+        c, s_ = 1.25 * torch.cos(ang), 1.25 * torch.sin(ang)
+        at = (slice(0, R, 2), slice(1, R, 2)) if turn == "pairs" else (slice(0, R // 2), slice(R // 2, R))
+
+        def turned(x):
+            y = x.clone()
+            y[..., at[0]], y[..., at[1]] = x[..., at[0]] * c - x[..., at[1]] * s_, x[..., at[1]] * c + x[..., at[0]] * s_
+            return y
+        q, k = turned(q), turned(k) * 0.3
+    else:
+        k = k * 0.3
+    ctx = fake_ctx(device, lens, starts, slots)
+    for write in (True, False):
+        state = start.clone().to(device)
+        out = torch.empty(T, heads * vdim, device=device)
+        before = ops.launch_count()
+        ops.linear_attention(proj.to(device), (0, heads * dim, 2 * heads * dim), out, state, decay.to(device), ctx, heads, dim, vdim,
+                             silu=silu, write_state=write, rotary=rotary, k_scale=0.3)
+        assert ops.launch_count() - before == 5
+        row = 0
+        for n, slot in zip(lens, slots):
+            args = [x[row:row + n] for x in (q, k, v)] + [start[slot].double()]
+            want, last = _decayed(*args, decay.double())
+            size, last_size = _decayed(*[x.abs() for x in args], decay.double())
+            got = out[row:row + n].cpu().double().view(n, heads, vdim)
+            rel = (6 * 2.0 ** -22 + (64 + 128 + 5) * 2.0 ** -24)
+            assert ((got - want).abs() <= rel * size + 1e-30).all(), (n, write)
+            if write:
+                assert ((state[slot].cpu().double() - last).abs() <= rel * last_size + 1e-30).all(), n
+            row += n
+        assert torch.equal(state[3].cpu(), start[3])
+        if not write:
+            assert torch.equal(state.cpu(), start)
+
+
+def test_linear_attention_chunks_keep_an_infinity_from_earlier_tokens(device):
+    """An infinite value spoils the tokens from its own on, none before it."""
+    ops = _ops()
+    torch.manual_seed(0)
+    heads, dim, vdim, T = 1, 64, 64, 100
+    proj = torch.randn(T, 3 * 64).to(BF16)
+    ctx = fake_ctx(device, [T], [0], [0])
+    outs = []
+    for value in (1.0, math.inf):
+        proj[75, 128 + 5] = value
+        out = torch.empty(T, vdim, device=device)
+        ops.linear_attention(proj.to(device), (0, 64, 128), out, torch.zeros(1, 1, vdim, dim, device=device),
+                             torch.tensor([0.9], device=device), ctx, heads, dim, vdim)
+        outs.append(out.cpu())
+    assert torch.allclose(outs[0][:75], outs[1][:75], atol=1e-4) and not bool(torch.isfinite(outs[1][75:, 5]).any())
+
+
 def test_linear_attention_keeps_a_key_from_hundreds_of_tokens_ago(device):
     """With a decay of one, a key that matches the last query, 600 tokens back among keys that do not, comes through
     with its value: one wrong state row or a lost update shows at full size."""
