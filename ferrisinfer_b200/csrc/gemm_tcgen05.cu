@@ -768,91 +768,134 @@ __device__ __forceinline__ void pt_epilogue_qkv_rope(const PTParams& p, uint32_t
     }
 }
 
+// The activations of a chunk of 32 accumulators (of a gate's and an up product's), the kind known to the compiler.
+template <int KIND>
+__device__ __forceinline__ void pt_gated(const uint32_t (&g)[32], const uint32_t (&u)[32], float scale, float limit,
+                                         uint32_t (&packed)[16]) {
+#pragma unroll
+    for (int c = 0; c < 32; c += 2)
+        packed[c >> 1] = pack_bf16(
+            ferris_gated_act(scale * __uint_as_float(g[c]), scale * __uint_as_float(u[c]), KIND, limit),
+            ferris_gated_act(scale * __uint_as_float(g[c + 1]), scale * __uint_as_float(u[c + 1]), KIND, limit));
+}
+template <int KIND>
+__device__ __forceinline__ void pt_activated(uint32_t (&z)[32], float scale, const FerrisEpilogueAct& act) {
+    const FerrisEpilogueAct known = {KIND, act.a, act.b};
+#pragma unroll
+    for (int c = 0; c < 32; ++c) z[c] = __float_as_uint(ferris_epilogue_act(scale * __uint_as_float(z[c]), known));
+}
+
 // The epilogue of one token-major tile for one warp: its 32 tokens (TMEM lanes, lane = token t) and every second
 // 32-column chunk of the accumulator buffer at d0 (gate columns first, up columns p.bn further in SwiGLU mode).
-template <int MODE>
+// ACT: an activation of the product's own, or a factor per row (p.act, p.row_scale).  A form of its own, with the kind tested once
+// per chunk: the code of every kind in the plain SwiGLU's loop, tested for each pair of columns, kept the epilogue from hiding behind
+// the MMAs (gate/up on pairs, us, before / now: 2,048 tokens x 9,728 x 896 70 / 37, 512 x 17,920 x 1,536 45 / 27, 2,345 x the same
+// 138 / 105, 2,048 x 37,888 x 3,584 396 / 371).
+template <int MODE, bool ACT>
+__device__ __forceinline__ float pt_row_scale(const PTParams& p, int t) {
+    return ACT && p.row_scale && t < p.T ? *(reinterpret_cast<const volatile float*>(p.row_scale) + t) : 1.0f;
+}
+// One chunk: columns n .. n + 31 of the output, of which the tile holds `width` (a multiple of 16).
+template <int MODE, bool ACT>
+__device__ __forceinline__ void pt_epilogue_chunk(const PTParams& p, const CUtensorMap& map_out, uint32_t (&ra)[32],
+                                                  const uint32_t (&rb)[32], int n, int width, int rows0, int lane, int t,
+                                                  float row_scale, uint8_t* out_stage) {
+    if (MODE == STORE_F32 || MODE == ACCUM_F32) {
+        // the warp's 32 x 32 block goes to shared memory (lane = row, 16-byte chunks swizzled as the
+        // tensor map expects) and from there to global memory by one TMA store / add-reduction,
+        // which also clips rows >= T and columns >= N
+        if (n >= p.N || rows0 >= p.T) return;  // warp-uniform
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+            float4 r;
+            r.x = __uint_as_float(ra[4 * v]) + ((p.bias && n + 4 * v < p.N) ? __ldg(p.bias + n + 4 * v) : 0.0f);
+            r.y = __uint_as_float(ra[4 * v + 1]) + ((p.bias && n + 4 * v + 1 < p.N) ? __ldg(p.bias + n + 4 * v + 1) : 0.0f);
+            r.z = __uint_as_float(ra[4 * v + 2]) + ((p.bias && n + 4 * v + 2 < p.N) ? __ldg(p.bias + n + 4 * v + 2) : 0.0f);
+            r.w = __uint_as_float(ra[4 * v + 3]) + ((p.bias && n + 4 * v + 3 < p.N) ? __ldg(p.bias + n + 4 * v + 3) : 0.0f);
+            *reinterpret_cast<float4*>(out_stage + swizzle128(lane, v)) = r;
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+            if (MODE == ACCUM_F32)
+                tma_reduce_add_2d(&map_out, out_stage, n, rows0);
+            else
+                tma_store_2d(&map_out, out_stage, n, rows0);
+            tma_store_commit();
+        }
+        return;
+    }
+    if (t >= p.T || n >= p.N) return;
+    if (MODE == STORE_BF16 || MODE == SWIGLU_BF16) {
+        bf16* o = reinterpret_cast<bf16*>(p.out) + (size_t)t * p.ldo + n;
+        uint32_t packed[16];
+        if constexpr (MODE == SWIGLU_BF16) {
+            if constexpr (!ACT) {
+#pragma unroll
+                for (int c = 0; c < 32; c += 2)
+                    packed[c >> 1] = pack_bf16(silu_mul(__uint_as_float(ra[c]), __uint_as_float(rb[c])),
+                                               silu_mul(__uint_as_float(ra[c + 1]), __uint_as_float(rb[c + 1])));
+            } else {
+                const int kind = p.act.kind ? p.act.kind - FERRIS_EPILOGUE_GATED : FERRIS_GATED_SILU;
+                if (kind == FERRIS_GATED_GELU_TANH)
+                    pt_gated<FERRIS_GATED_GELU_TANH>(ra, rb, row_scale, p.act.a, packed);
+                else if (kind == FERRIS_GATED_CLAMPED_SWISH)
+                    pt_gated<FERRIS_GATED_CLAMPED_SWISH>(ra, rb, row_scale, p.act.a, packed);
+                else
+                    pt_gated<FERRIS_GATED_SILU>(ra, rb, row_scale, p.act.a, packed);
+            }
+        } else {
+            if (p.bias) {
+#pragma unroll
+                for (int c = 0; c < 32; ++c)
+                    ra[c] = __float_as_uint(__uint_as_float(ra[c]) + (n + c < p.N ? __ldg(p.bias + n + c) : 0.0f));
+            }
+            if constexpr (ACT) {
+                if (p.act.kind == 1)
+                    pt_activated<1>(ra, row_scale, p.act);
+                else if (p.act.kind == 2)
+                    pt_activated<2>(ra, row_scale, p.act);
+                else if (p.act.kind == 3)
+                    pt_activated<3>(ra, row_scale, p.act);
+                else
+                    pt_activated<0>(ra, row_scale, p.act);
+            }
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) packed[c >> 1] = pack_bf16(__uint_as_float(ra[c]), __uint_as_float(ra[c + 1]));
+        }
+        if (n + width <= p.N) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                if (8 * v < width)
+                    reinterpret_cast<uint4*>(o)[v] = make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+                if (c < width && n + c < p.N)
+                    o[c] = __ushort_as_bfloat16(
+                        (unsigned short)((c & 1) ? (packed[c >> 1] >> 16) : (packed[c >> 1] & 0xffffu)));
+        }
+    }
+}
+template <int MODE, bool ACT>
 __device__ __forceinline__ void pt_epilogue_tile(const PTParams& p, const CUtensorMap& map_out, uint32_t d0, int m0, int n0,
                                                  int quarter, int half, int lane, int t, uint8_t* out_stage) {
     constexpr int ACCS = MODE == SWIGLU_BF16 ? 2 : 1;
     const int cols = p.bn;  // output columns of this tile
-    float row_scale = 1.0f;
-    if ((MODE == SWIGLU_BF16 || MODE == STORE_BF16) && p.row_scale && t < p.T) row_scale = *(reinterpret_cast<const volatile float*>(p.row_scale) + t);
+    const float row_scale = pt_row_scale<MODE, ACT>(p, t);
     for (int c0 = half * 32; c0 < cols; c0 += 64) {
         uint32_t ra[32], rb[32];
         tmem_load_32x32(d0 + c0, ra);
         if (ACCS == 2) tmem_load_32x32(d0 + p.bn + c0, rb);
         tmem_load_wait();
-        const int n = n0 + c0;
-        if (MODE == STORE_F32 || MODE == ACCUM_F32) {
-            // the warp's 32 x 32 block goes to shared memory (lane = row, 16-byte chunks swizzled as the
-            // tensor map expects) and from there to global memory by one TMA store / add-reduction,
-            // which also clips rows >= T and columns >= N
-            if (n >= p.N || m0 + quarter * 32 >= p.T) continue;  // warp-uniform
-            if (lane == 0) tma_store_wait_read();
-            __syncwarp();
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                float4 r;
-                r.x = __uint_as_float(ra[4 * v]) + ((p.bias && n + 4 * v < p.N) ? __ldg(p.bias + n + 4 * v) : 0.0f);
-                r.y = __uint_as_float(ra[4 * v + 1]) + ((p.bias && n + 4 * v + 1 < p.N) ? __ldg(p.bias + n + 4 * v + 1) : 0.0f);
-                r.z = __uint_as_float(ra[4 * v + 2]) + ((p.bias && n + 4 * v + 2 < p.N) ? __ldg(p.bias + n + 4 * v + 2) : 0.0f);
-                r.w = __uint_as_float(ra[4 * v + 3]) + ((p.bias && n + 4 * v + 3 < p.N) ? __ldg(p.bias + n + 4 * v + 3) : 0.0f);
-                *reinterpret_cast<float4*>(out_stage + swizzle128(lane, v)) = r;
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-                if (MODE == ACCUM_F32)
-                    tma_reduce_add_2d(&map_out, out_stage, n, m0 + quarter * 32);
-                else
-                    tma_store_2d(&map_out, out_stage, n, m0 + quarter * 32);
-                tma_store_commit();
-            }
-            continue;
-        }
-        if (t >= p.T || n >= p.N) continue;
-        const bool whole = n + 32 <= p.N;
-        if (MODE == STORE_BF16 || MODE == SWIGLU_BF16) {
-            bf16* o = reinterpret_cast<bf16*>(p.out) + (size_t)t * p.ldo + n;
-            uint32_t packed[16];
-#pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-                float v0, v1;
-                if (MODE == SWIGLU_BF16) {
-                    if (p.row_scale) {
-                        const int kind = p.act.kind ? p.act.kind - FERRIS_EPILOGUE_GATED : FERRIS_GATED_SILU;
-                        v0 = ferris_gated_act(row_scale * __uint_as_float(ra[c]), row_scale * __uint_as_float(rb[c]), kind, p.act.a);
-                        v1 = ferris_gated_act(row_scale * __uint_as_float(ra[c + 1]), row_scale * __uint_as_float(rb[c + 1]), kind, p.act.a);
-                    } else if (p.act.kind) {  // another gated activation than SiLU
-                        v0 = ferris_gated_act(__uint_as_float(ra[c]), __uint_as_float(rb[c]), p.act.kind - FERRIS_EPILOGUE_GATED, p.act.a);
-                        v1 = ferris_gated_act(__uint_as_float(ra[c + 1]), __uint_as_float(rb[c + 1]), p.act.kind - FERRIS_EPILOGUE_GATED, p.act.a);
-                    } else {
-                        v0 = silu_mul(__uint_as_float(ra[c]), __uint_as_float(rb[c]));
-                        v1 = silu_mul(__uint_as_float(ra[c + 1]), __uint_as_float(rb[c + 1]));
-                    }
-                } else {
-                    v0 = __uint_as_float(ra[c]) + ((p.bias && n + c < p.N) ? __ldg(p.bias + n + c) : 0.0f);
-                    v1 = __uint_as_float(ra[c + 1]) + ((p.bias && n + c + 1 < p.N) ? __ldg(p.bias + n + c + 1) : 0.0f);
-                    if (p.act.kind) v0 = ferris_epilogue_act(row_scale * v0, p.act), v1 = ferris_epilogue_act(row_scale * v1, p.act);
-                }
-                packed[c >> 1] = pack_bf16(v0, v1);
-            }
-            if (whole) {
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    reinterpret_cast<uint4*>(o)[v] = make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-            } else {
-#pragma unroll
-                for (int c = 0; c < 32; ++c)
-                    if (n + c < p.N)
-                        o[c] = __ushort_as_bfloat16(
-                            (unsigned short)((c & 1) ? (packed[c >> 1] >> 16) : (packed[c >> 1] & 0xffffu)));
-            }
-        }
+        pt_epilogue_chunk<MODE, ACT>(p, map_out, ra, rb, n0 + c0, min(32, cols - c0), m0 + quarter * 32, lane, t, row_scale,
+                                     out_stage);
     }
 }
 
-template <int MODE>
+template <int MODE, bool ACT>
 __global__ void __launch_bounds__(PT_THREADS)
     gemm_tokens_m_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          const __grid_constant__ CUtensorMap map_out, const PTParams p) {
@@ -969,7 +1012,7 @@ __global__ void __launch_bounds__(PT_THREADS)
             if constexpr (MODE == QKV_ROPE_BF16)
                 pt_epilogue_qkv_rope(p, d0, n0, half, t);
             else
-                pt_epilogue_tile<MODE>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
+                pt_epilogue_tile<MODE, ACT>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
             // this warp has read its part of the buffer: the MMA warp may overwrite it
             tcgen05_fence_before();
             __syncwarp();
@@ -997,7 +1040,7 @@ __global__ void __launch_bounds__(PT_THREADS)
 // =============================================================================================
 constexpr int PP_STAGES = 6;
 
-template <int MODE>
+template <int MODE, bool ACT>
 __global__ void __launch_bounds__(PT_THREADS)
     gemm_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                             const __grid_constant__ CUtensorMap map_out, const PTParams p) {
@@ -1116,7 +1159,7 @@ __global__ void __launch_bounds__(PT_THREADS)
             if (!mbar_wait(&tmem_full[buf], (local >> 1) & 1, p.status, 33)) break;
             tcgen05_fence_after();
             const uint32_t d0 = lane_addr + buf * n_mma;
-            pt_epilogue_tile<MODE>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
+            pt_epilogue_tile<MODE, ACT>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[buf]), 0));
@@ -1263,10 +1306,10 @@ bool ferris_gemm_pair_enabled(int mode, int T) {
     return g_pair == 2 && mode == SWIGLU_BF16 && (m128 % 2 == 0 || m128 >= 9);
 }
 
-template <int MODE>
+template <int MODE, bool ACT = false>
 int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const PTParams& p, int pairs,
                 size_t smem, cudaStream_t s) {
-    int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_pair_kernel<MODE>, smem);
+    int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_pair_kernel<MODE, ACT>, smem);
     if (rc != FERRIS_OK) return rc;
     cudaError_t e = cudaSuccess;
     {
@@ -1284,7 +1327,7 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap&
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = ferris_pdl_enabled() ? 2 : 1;
-        e = cudaLaunchKernelEx(&cfg, gemm_tokens_pair_kernel<MODE>, mx, mw, mo, p);
+        e = cudaLaunchKernelEx(&cfg, gemm_tokens_pair_kernel<MODE, ACT>, mx, mw, mo, p);
     }
     if (e != cudaSuccess) {
         ferris_set_error("gemm: %s", cudaGetErrorString(e));
@@ -1342,12 +1385,12 @@ int active_clusters(int size) {
     return clusters;
 }
 
-template <int MODE>
+template <int MODE, bool ACT = false>
 int launch_pt(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const PTParams& p, int ctas,
               size_t smem, cudaStream_t s) {
-    int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_m_kernel<MODE>, smem);
+    int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_m_kernel<MODE, ACT>, smem);
     if (rc != FERRIS_OK) return rc;
-    cudaError_t e = ferris_launch(gemm_tokens_m_kernel<MODE>, dim3(ctas), dim3(PT_THREADS), smem, s, mx, mw, mo, p);
+    cudaError_t e = ferris_launch(gemm_tokens_m_kernel<MODE, ACT>, dim3(ctas), dim3(PT_THREADS), smem, s, mx, mw, mo, p);
     if (e != cudaSuccess) {
         ferris_set_error("gemm: %s", cudaGetErrorString(e));
         return (int)e;
@@ -1619,10 +1662,14 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
     int ctas = q.m_tiles * q.n_tiles;
     if (ctas > g_sms) ctas = g_sms;
     switch (mode) {
-        case STORE_BF16: return launch_pt<STORE_BF16>(mx, mw, mo, q, ctas, smem, s);
+        case STORE_BF16:
+            if (q.act.kind) return launch_pt<STORE_BF16, true>(mx, mw, mo, q, ctas, smem, s);
+            return launch_pt<STORE_BF16>(mx, mw, mo, q, ctas, smem, s);
         case STORE_F32: return launch_pt<STORE_F32>(mx, mw, mo, q, ctas, smem, s);
         case ACCUM_F32: return launch_pt<ACCUM_F32>(mx, mw, mo, q, ctas, smem, s);
-        case SWIGLU_BF16: return launch_pt<SWIGLU_BF16>(mx, mw, mo, q, ctas, smem, s);
+        case SWIGLU_BF16:
+            if (q.act.kind || q.row_scale) return launch_pt<SWIGLU_BF16, true>(mx, mw, mo, q, ctas, smem, s);
+            return launch_pt<SWIGLU_BF16>(mx, mw, mo, q, ctas, smem, s);
         default: return launch_pt<QKV_ROPE_BF16>(mx, mw, mo, q, ctas, smem, s);
     }
 }
@@ -1716,10 +1763,14 @@ static int gemm_tcgen05_impl(const void* x, const void* w, const float* bias, vo
         int pairs = q.m_tiles * q.n_tiles;
         if (pairs > pairs_all) pairs = pairs_all;
         switch (mode) {
-            case STORE_BF16: return launch_pair<STORE_BF16>(mx, mw, mo, q, pairs, smem, s);
+            case STORE_BF16:
+                if (q.act.kind) return launch_pair<STORE_BF16, true>(mx, mw, mo, q, pairs, smem, s);
+                return launch_pair<STORE_BF16>(mx, mw, mo, q, pairs, smem, s);
             case STORE_F32: return launch_pair<STORE_F32>(mx, mw, mo, q, pairs, smem, s);
             case ACCUM_F32: return launch_pair<ACCUM_F32>(mx, mw, mo, q, pairs, smem, s);
-            default: return launch_pair<SWIGLU_BF16>(mx, mw, mo, q, pairs, smem, s);
+            default:
+                if (q.act.kind || q.row_scale) return launch_pair<SWIGLU_BF16, true>(mx, mw, mo, q, pairs, smem, s);
+                return launch_pair<SWIGLU_BF16>(mx, mw, mo, q, pairs, smem, s);
         }
     }
     if (long_step)
