@@ -681,6 +681,7 @@ struct PTParams {
     int m_tiles, n_tiles;
     int up_row_offset;
     int* status;
+    int splits, kb_per;  // CTA pairs only: pairs that share a tile's K slices, and the slices of each but the last
     RopeEpilogue rope;  // mode QKV_ROPE_BF16 only
     FerrisEpilogueAct act;  // applied by the bf16 store (mode STORE_BF16)
     // A product per group of token tiles (a mixture of experts whose rows lie sorted by expert, every expert's rows
@@ -932,6 +933,21 @@ __global__ void __launch_bounds__(PT_THREADS)
     tcgen05_fence_after();
     const uint32_t tmem = tmem_base;
     pdl_launch_dependents();
+    // The weights of the first tile's first slices are requested ahead of the wait (no launch writes them, unless the tile's
+    // expert says which they are), the tokens after it: a weight's first slices come from HBM while the launch before ends (us a
+    // product in a row of them: 9,728 x 896 at 256 to 2,048 tokens 14.0 / 19.1 / 25.3 / 36.8 -> 13.5 / 18.1 / 24.3 / 35.7)
+    int early = 0;
+    auto load_weights = [&](int it, int kb, int row) {
+        uint8_t* st = smem + (size_t)(it % PT_STAGES) * stage_bytes;
+        uint64_t* bar = &full[it % PT_STAGES];
+        mbar_expect_tx(bar, stage_bytes);
+        tma_load_2d(st + a_bytes, &map_w, kb * BLOCK_K, row, bar);
+        if (ACCS == 2) tma_load_2d(st + a_bytes + b_bytes, &map_w, kb * BLOCK_K, p.up_row_offset + row, bar);
+    };
+    if (threadIdx.x == 0 && !p.tile_expert) {
+        early = min(PT_STAGES, p.kblocks);
+        for (int kb = 0; kb < early; ++kb) load_weights(kb, kb, ((int)blockIdx.x / p.m_tiles) * p.bn);
+    }
     pdl_wait();
     FERRIS_TL_BEGIN();
 
@@ -949,12 +965,8 @@ __global__ void __launch_bounds__(PT_THREADS)
                         ok = false;
                         break;
                     }
-                    uint8_t* st = smem + (size_t)s * stage_bytes;
-                    mbar_expect_tx(&full[s], stage_bytes);
-                    tma_load_2d(st, &map_x, kb * BLOCK_K, m0, &full[s]);
-                    tma_load_2d(st + a_bytes, &map_w, kb * BLOCK_K, wrow + n0, &full[s]);
-                    if (ACCS == 2)
-                        tma_load_2d(st + a_bytes + b_bytes, &map_w, kb * BLOCK_K, wrow + p.up_row_offset + n0, &full[s]);
+                    if (it >= early) load_weights(it, kb, wrow + n0);
+                    tma_load_2d(smem + (size_t)s * stage_bytes, &map_x, kb * BLOCK_K, m0, &full[s]);
                 }
             }
         }
@@ -1036,9 +1048,19 @@ __global__ void __launch_bounds__(PT_THREADS)
 // work, and L2-to-SM traffic is what bounds the single-CTA kernel at these sizes.  The even CTA issues the MMAs;
 // both CTAs' TMA loads count on its `full` barrier; tcgen05.commit arrives on `empty` / `tmem_full` of both;
 // the epilogue warps of both arrive on its `tmem_empty`.  In SwiGLU mode CTA 0 holds the gate rows and CTA 1 the
-// up rows of the tile: accumulator columns [0, 128) are gate, [128, 256) up, as in the single-CTA kernel.
+// up rows of the tile: accumulator columns [0, bn) are gate, [bn, 2 bn) up, as in the single-CTA kernel.
+//
+// K SPLITS (one accumulator, p.splits > 1): a cluster of `splits` pairs takes one tile, pair s the s-th run of K slices.  When
+// all of them are done (their rings are free), every CTA sends each run of columns of its 128 rows to the ring of the
+// CTA that owns it, and the owners add the runs up in the order of the splits and store: a fixed order, no memory
+// beside the CTAs' own.  For products whose tiles are few and whose K is long, which are bound by the bytes on their way to the
+// few SMs that have one (us, single CTAs / pairs with splits, the residual's product: 512 x 1,536 x 8,960 48 / 22 in four, 700 tokens
+// 49 / 25 in three, 1,024 52 / 32 in two; 1,000 x 896 x 4,864 29 / 18 in three, 2,048 tokens 30 / 22 in two; 256 x 3,584 x 18,944
+// 103 / 39 in four, 512 tokens 100 / 60 in two).  The exchange and its two barriers cost 4 to 6 us.
 // =============================================================================================
 constexpr int PP_STAGES = 6;
+constexpr int PP_MAX_SPLITS = 4;  // pairs of a cluster of at most eight CTAs
+constexpr int PP_CHUNK_BYTES = PT_BLOCK_M * 32 * 4;  // 128 rows x 32 columns of partial sums
 
 template <int MODE, bool ACT>
 __global__ void __launch_bounds__(PT_THREADS)
@@ -1051,8 +1073,12 @@ __global__ void __launch_bounds__(PT_THREADS)
     __shared__ uint32_t tmem_base;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank();  // 0: the leader
-    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const uint32_t cta = cluster_ctarank(), rank = cta & 1, leader = cta & ~1u;  // rank 0: the leader of its pair
+    const int splits = ACCS == 1 ? p.splits : 1, split = ACCS == 1 ? (int)(cta >> 1) : 0;
+    const int pair = ACCS == 1 ? (int)blockIdx.x / (2 * splits) : blockIdx.x >> 1;  // (with splits: the cluster)
+    const int pairs = ACCS == 1 ? (int)gridDim.x / (2 * splits) : gridDim.x >> 1;
+    const int kb0 = split * p.kb_per, kb1 = min(p.kblocks, kb0 + p.kb_per);
+    const uint16_t both = (uint16_t)(3u << leader);
     const int n_mma = ACCS * p.bn;            // columns of the pair's MMA and of one accumulator buffer
     const int half_rows = n_mma / 2;          // weight rows this CTA holds per K slice
     const int a_bytes = PT_BLOCK_M * BLOCK_K * 2, b_bytes = half_rows * BLOCK_K * 2;
@@ -1080,29 +1106,40 @@ __global__ void __launch_bounds__(PT_THREADS)
     tcgen05_fence_after();
     const uint32_t tmem = tmem_base;
     pdl_launch_dependents();
+    const uint32_t leader_full = map_to_cta(smem_u32(&full[0]), leader);
+    // this CTA's weight rows of a tile.  SwiGLU: the leader holds the gate rows, its peer the up rows; else each one half
+    auto weight_row = [&](int tile) {
+        const int n0 = (tile / p.m_tiles) * p.bn;
+        return ACCS == 2 ? (rank == 0 ? n0 : p.up_row_offset + n0) : n0 + (int)rank * half_rows;
+    };
+    auto load_weights = [&](int it, int kb, int row) {
+        const int s = it % PP_STAGES;
+        if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);  // both CTAs' bytes
+        tma_load_2d_pair(smem + (size_t)s * stage_bytes + a_bytes, &map_w, kb * BLOCK_K, row, leader_full + 8u * s);
+    };
+    int early = 0;  // slices whose weights are requested ahead of the wait, as above
+    if (threadIdx.x == 0) {
+        early = min(PP_STAGES, kb1 - kb0);
+        for (int i = 0; i < early; ++i) load_weights(i, kb0 + i, weight_row(pair));
+    }
     pdl_wait();
     FERRIS_TL_BEGIN();
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t leader_full = map_to_cta(smem_u32(&full[0]), 0);
             int it = 0;
             bool ok = true;
             for (int tile = pair; tile < tiles && ok; tile += pairs) {
                 const int m0 = (tile % p.m_tiles) * (2 * PT_BLOCK_M) + (int)rank * PT_BLOCK_M;
-                const int n0 = (tile / p.m_tiles) * p.bn;
-                // SwiGLU: the leader holds the gate rows, its peer the up rows; else each holds one half of the rows
-                const int w_row = ACCS == 2 ? (rank == 0 ? n0 : p.up_row_offset + n0) : n0 + (int)rank * half_rows;
-                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+                const int w_row = weight_row(tile);
+                for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % PP_STAGES;
                     if (it >= PP_STAGES && !mbar_wait(&empty[s], ((it / PP_STAGES) - 1) & 1, p.status, 30)) {
                         ok = false;
                         break;
                     }
-                    uint8_t* st = smem + (size_t)s * stage_bytes;
-                    if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);  // both CTAs' bytes
-                    tma_load_2d_pair(st, &map_x, kb * BLOCK_K, m0, leader_full + 8u * s);
-                    tma_load_2d_pair(st + a_bytes, &map_w, kb * BLOCK_K, w_row, leader_full + 8u * s);
+                    if (it >= early) load_weights(it, kb, w_row);
+                    tma_load_2d_pair(smem + (size_t)s * stage_bytes, &map_x, kb * BLOCK_K, m0, leader_full + 8u * s);
                 }
             }
         }
@@ -1120,7 +1157,7 @@ __global__ void __launch_bounds__(PT_THREADS)
                 wait_drain += FERRIS_TL_CLOCK() - c0;
                 tcgen05_fence_after();
                 const uint32_t d0 = tmem + buf * n_mma;
-                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+                for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % PP_STAGES;
                     c0 = FERRIS_TL_CLOCK();
                     if (!mbar_wait(&full[s], (it / PP_STAGES) & 1, p.status, 32)) {
@@ -1135,11 +1172,11 @@ __global__ void __launch_bounds__(PT_THREADS)
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
                         const uint64_t adv = (uint64_t)((k * UMMA_K * 2) >> 4);
-                        tcgen05_mma_bf16_pair(d0, a_desc + adv, b_desc + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tcgen05_mma_bf16_pair(d0, a_desc + adv, b_desc + adv, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    tcgen05_commit_pair(&empty[s], 3);  // the stage is free in both CTAs
+                    tcgen05_commit_pair(&empty[s], both);  // the stage is free in both CTAs
                 }
-                if (ok) tcgen05_commit_pair(&tmem_full[buf], 3);
+                if (ok) tcgen05_commit_pair(&tmem_full[buf], both);
             }
             FERRIS_TL_VALUE(pair == 0, 0, (unsigned long long)wait_load);
             FERRIS_TL_VALUE(pair == 0, 1, (unsigned long long)wait_drain);
@@ -1158,11 +1195,66 @@ __global__ void __launch_bounds__(PT_THREADS)
             const int t = m0 + quarter * 32 + lane;
             if (!mbar_wait(&tmem_full[buf], (local >> 1) & 1, p.status, 33)) break;
             tcgen05_fence_after();
+            if (ACCS == 1 && splits > 1) break;  // one tile to a cluster: its pairs' sums meet below
             const uint32_t d0 = lane_addr + buf * n_mma;
-            pt_epilogue_tile<MODE, ACT>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
+            if constexpr (MODE == QKV_ROPE_BF16)
+                pt_epilogue_qkv_rope(p, d0, n0, half, t);
+            else
+                pt_epilogue_tile<MODE, ACT>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[buf]), 0));
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[buf]), leader));
+        }
+    }
+    if constexpr (ACCS == 1 && MODE != QKV_ROPE_BF16) {
+        if (splits > 1) {
+            __syncwarp();
+            cluster_sync();  // every pair's MMAs are done: the rings take partial sums now
+            const int e = warp - 2, quarter = warp & 3, half = e >> 2, row = quarter * 32 + lane;
+            const uint32_t d0 = tmem + ((uint32_t)(quarter * 32) << 16);
+            const int chunks = p.bn >> 5, per = (chunks + splits - 1) / splits;  // of a tile, of an owner
+            const uint32_t ring = smem_u32(smem);
+            if (warp >= 2) {
+                for (int c = half; c < chunks; c += 2) {
+                    const int owner = c / per;
+                    if (owner == split) continue;
+                    uint32_t ra[32];
+                    tmem_load_32x32(d0 + 32 * c, ra);
+                    tmem_load_wait();
+                    const int slot = (split < owner ? split : split - 1) * per + c - owner * per;
+                    const uint32_t at = map_to_cta(ring + slot * PP_CHUNK_BYTES + row * 16, 2 * owner + rank);
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) st_cluster_x4(at + v * (PT_BLOCK_M * 16), ra + 4 * v);
+                }
+            }
+            __syncwarp();
+            cluster_sync();
+            if (warp >= 2) {
+                const int m0 = (pair % p.m_tiles) * (2 * PT_BLOCK_M) + (int)rank * PT_BLOCK_M, n0 = (pair / p.m_tiles) * p.bn;
+                const float row_scale = pt_row_scale<MODE, ACT>(p, m0 + row);
+                for (int c = half; c < chunks; c += 2) {
+                    if (c / per != split) continue;
+                    uint32_t own[32], sum[32] = {};
+                    tmem_load_32x32(d0 + 32 * c, own);
+                    tmem_load_wait();
+                    for (int from = 0; from < splits; ++from) {
+                        const int slot = (from < split ? from : from - 1) * per + c - split * per;
+                        const uint8_t* part = smem + (size_t)slot * PP_CHUNK_BYTES + row * 16;
+#pragma unroll
+                        for (int v = 0; v < 8; ++v) {
+                            float4 x = make_float4(__uint_as_float(own[4 * v]), __uint_as_float(own[4 * v + 1]),
+                                                   __uint_as_float(own[4 * v + 2]), __uint_as_float(own[4 * v + 3]));
+                            if (from != split) x = *reinterpret_cast<const float4*>(part + v * (PT_BLOCK_M * 16));
+                            const float f[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                sum[4 * v + i] = __float_as_uint(from == 0 ? f[i] : __uint_as_float(sum[4 * v + i]) + f[i]);
+                        }
+                    }
+                    pt_epilogue_chunk<MODE, ACT>(p, map_out, sum, own, n0 + 32 * c, 32, m0 + quarter * 32, lane, m0 + row,
+                                                 row_scale, out_stage);
+                }
+            }
         }
     }
     if ((MODE == STORE_F32 || MODE == ACCUM_F32) && warp >= 2 && lane == 0) tma_store_wait_all();
@@ -1293,34 +1385,99 @@ static bool token_major_pays(int mode, int T, int N, int K) {
     return t_tm <= 1.15 * t_wm;
 }
 
-int g_pair = -1;  // 0: no product on pairs, 1: every long-step product, 2: the SwiGLU product only
-bool ferris_gemm_pair_enabled(int mode, int T) {
+// Weight rows per tile of the token-major kernel with one accumulator: the width among 128 .. 256 that costs least.  A CTA takes in (128 + bn) rows per K
+// slice, and the CTAs go through ceil(tiles / SMs) rounds; 192 or 224 rows often fit in one round what 128 rows
+// need two for (2,048 tokens x 1,536 outputs: 192 tiles of 128 in two rounds, 128 tiles of 192 in one).
+// head: the q/k/v mode takes whole heads (and pairs of 32-column chunks), steps of 64 or 128 rows; 0: any product.
+static int tokens_m_width(int T, int N, int head) {
+    const int step = head ? (head == 64 ? 64 : 128) : 32;
+    long long best = -1;
+    int width = 128;
+    for (int bn = 256; bn >= 128; bn -= step) {
+        const long long tiles = (long long)((T + PT_BLOCK_M - 1) / PT_BLOCK_M) * ((N + bn - 1) / bn);
+        const long long cost = ((tiles + g_sms - 1) / g_sms) * (PT_BLOCK_M + bn);
+        if (best < 0 || cost < best) {
+            best = cost;
+            width = bn;
+        }
+    }
+    return width;
+}
+
+int g_pair = -1;  // 0: no product on pairs, 1: every long-step product (no K splits), 2: the SwiGLU product, others where pair_plan's estimate says so
+int pair_clusters(int splits);
+
+struct PairPlan {
+    int bn = 0, splits = 1;  // bn 0: not on pairs
+};
+// Whether a long step runs on CTA pairs, with which tile width and K split.  head: the q/k/v mode's head size, 0 otherwise.
+// SwiGLU: a pair's tile has 256 tokens: with an odd number of 128-token tiles the last pair is half empty, which costs
+// more than pairs save while the tiles are few (384 tokens at the 0.5B sizes: 18.3 us on pairs, 14.1 us without).
+// One accumulator: from two estimates in microseconds.  Either kernel has about 192 KB on its way to an SM, which takes
+// PT_FEED bytes a microsecond in; a K slice on pairs costs 0.25 to 0.30 by the width; a launch costs about 7, on pairs 9, and 13
+// where the splits' sums meet.  Pairs are taken where they win by more than the estimates are off (8 %): products whose
+// tiles are few and whose K is long (split), and products that the other kernel needs two rounds for (us: 2,048 x 18,944 -> 3,584
+// 260 / 206 to 245 on pairs, 2,048 x 3,584 -> 4,608 57 / 47 to 55; the spread is that of several processes).  Without the 8 %, and with
+// splits wherever they fit: 1.5B output product of 512 tokens 12.4 / 12.1, of 1,024 13.2 / 13.3, 0.5B ones up to 30 % slower.
+PairPlan pair_plan(int mode, int T, int N, int K, int head) {
     if (g_pair < 0) {
         const char* v = getenv("FERRIS_GEMM_PAIR");
         g_pair = (v && v[0] >= '0' && v[0] <= '2') ? v[0] - '0' : 2;
     }
-    if (g_pair == 1) return true;
-    // A pair's tile has 256 tokens: with an odd number of 128-token tiles the last pair is half empty, which costs
-    // more than pairs save while the tiles are few (384 tokens at the 0.5B sizes: 18.3 us on pairs, 14.1 us without).
-    const int m128 = (T + PT_BLOCK_M - 1) / PT_BLOCK_M;
-    return g_pair == 2 && mode == SWIGLU_BF16 && (m128 % 2 == 0 || m128 >= 9);
+    sm_count();
+    PairPlan plan;
+    if (g_pair == 0) return plan;
+    const int m128 = (T + PT_BLOCK_M - 1) / PT_BLOCK_M, m256 = (m128 + 1) / 2, all = g_sms / 2;
+    if (mode == SWIGLU_BF16) {
+        if (g_pair == 1 || m128 % 2 == 0 || m128 >= 9) plan.bn = 128;
+        return plan;
+    }
+    if (g_pair == 1) {
+        plan.bn = m256 * ((N + 255) / 256) < all ? 128 : 256;
+        return plan;
+    }
+    const int kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+    const int width = tokens_m_width(T, N, head);
+    const double PT_FEED = 113e3;
+    const long long tiles_m = (long long)m128 * ((N + width - 1) / width), rounds_m = (tiles_m + g_sms - 1) / g_sms;
+    const double t_m = (double)rounds_m * kblocks * (PT_BLOCK_M + width) * (BLOCK_K * 2) / PT_FEED + 7.0;
+    double best = 0.92 * t_m;
+    for (int bn = 256; bn >= 128; bn -= head == 128 ? 128 : (head ? 64 : 32)) {
+        const long long tiles = (long long)m256 * ((N + bn - 1) / bn);
+        const double slice = bn > 224 ? 0.30 : (bn > 128 ? 0.28 : 0.25);
+        for (int splits = 1; splits <= (head ? 1 : PP_MAX_SPLITS); ++splits) {
+            const int per = (kblocks + splits - 1) / splits;
+            if (splits > 1 && (per < 4 || per * (splits - 1) >= kblocks)) continue;  // no split may be empty
+            if (splits == 1 && rounds_m < 2) continue;  // as fast at best (2,345 x 1,536 x 8,960: 62.9 us, on pairs 64.4)
+            const int room = splits == 1 ? all : pair_clusters(splits);
+            if (room <= 0) continue;
+            const long long rounds = (tiles + room - 1) / room;
+            const double t = splits == 1 ? rounds * per * slice + 9.0 : rounds * (per * slice + 13.0);
+            if (t < best) {
+                best = t;
+                plan.bn = bn;
+                plan.splits = splits;
+            }
+        }
+    }
+    return plan;
 }
 
 template <int MODE, bool ACT = false>
-int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const PTParams& p, int pairs,
+int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const PTParams& p, int clusters,
                 size_t smem, cudaStream_t s) {
     int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_pair_kernel<MODE, ACT>, smem);
     if (rc != FERRIS_OK) return rc;
     cudaError_t e = cudaSuccess;
     {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * pairs);
+        cfg.gridDim = dim3(2 * p.splits * clusters);
         cfg.blockDim = dim3(PT_THREADS);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.x = 2 * p.splits;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1383,6 +1540,37 @@ int active_clusters(int size) {
     }
     g_active_clusters[size] = clusters;
     return clusters;
+}
+
+// How many clusters of `splits` pairs the GPU holds at once (the CTAs of a cluster share a GPC); asked once for each size.
+int g_pair_clusters[PP_MAX_SPLITS + 1] = {};
+int pair_clusters(int splits) {
+    int& have = g_pair_clusters[splits];
+    if (have != 0) return have;
+    have = -1;
+    auto kernel = gemm_tokens_pair_kernel<ACCUM_F32, false>;
+    const int smem = PP_STAGES * 2 * PT_BLOCK_M * BLOCK_K * 2 + PT_EPI_WARPS * 4096 + 1024;
+    if (ferris_allow_dynamic_smem((const void*)kernel, smem) != FERRIS_OK) {
+        cudaGetLastError();
+        return have;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * splits);
+    cfg.blockDim = dim3(PT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0)
+        have = clusters;
+    else
+        cudaGetLastError();
+    return have;
 }
 
 template <int MODE, bool ACT = false>
@@ -1603,6 +1791,55 @@ FERRIS_API int ferris_merge_gemm_tcgen05(const float* scratch_parts, int heads, 
 // (a decode step of 1 / 8 / 64 rows at the 0.5B sizes: 0.751 / 0.757 / 1.673 ms with one, 0.725 / 0.752 / 1.64 ms without).
 static FerrisEpilogueAct g_launch_act = {0, 0.0f, 0.0f};
 
+// A long step on CTA pairs (see gemm_tokens_pair_kernel).
+static int run_pairs(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K, int ldx, int ldw,
+                     int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope, const PairPlan& plan, cudaStream_t s) {
+    const int accs = mode == SWIGLU_BF16 ? 2 : 1;
+    PTParams q;
+    q.out = out;
+    q.bias = bias;
+    q.act = g_launch_act;
+    q.T = T;
+    q.N = N;
+    q.K = K;
+    q.ldo = ldo;
+    q.m_tiles = (T + 2 * PT_BLOCK_M - 1) / (2 * PT_BLOCK_M);
+    q.bn = plan.bn;
+    q.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+    q.kb_per = (q.kblocks + plan.splits - 1) / plan.splits;
+    q.splits = plan.splits;
+    q.n_tiles = (N + q.bn - 1) / q.bn;
+    q.up_row_offset = up_row_offset;
+    q.status = ferris_status_ptr();
+    q.rope = rope ? *rope : RopeEpilogue{};
+    const int half_rows = accs * q.bn / 2;
+    CUtensorMap mx, mw;
+    int rc = ferris_make_tensor_map_2d(&mx, x, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, PT_BLOCK_M, BLOCK_K);
+    if (rc != FERRIS_OK) return rc;
+    rc = pt_weight_map(w, (uint64_t)rows_w, (uint64_t)K, (uint64_t)ldw, (uint32_t)half_rows, &mw);
+    if (rc != FERRIS_OK) return rc;
+    CUtensorMap mo = mx;  // unused by the bf16 modes
+    if (mode == STORE_F32 || mode == ACCUM_F32) {
+        rc = ferris_make_tensor_map_2d_f32(&mo, out, (uint64_t)T, (uint64_t)N, (uint64_t)ldo, 32);
+        if (rc != FERRIS_OK) return rc;
+    }
+    const int stage_bytes = PT_BLOCK_M * BLOCK_K * 2 + half_rows * BLOCK_K * 2;
+    const size_t smem = (size_t)PP_STAGES * stage_bytes + (size_t)PT_EPI_WARPS * 4096 + 1024;
+    int clusters = q.m_tiles * q.n_tiles;
+    if (q.splits == 1 && clusters > g_sms / 2) clusters = g_sms / 2;  // (with splits a cluster takes one tile)
+    switch (mode) {
+        case STORE_BF16:
+            if (q.act.kind) return launch_pair<STORE_BF16, true>(mx, mw, mo, q, clusters, smem, s);
+            return launch_pair<STORE_BF16>(mx, mw, mo, q, clusters, smem, s);
+        case STORE_F32: return launch_pair<STORE_F32>(mx, mw, mo, q, clusters, smem, s);
+        case ACCUM_F32: return launch_pair<ACCUM_F32>(mx, mw, mo, q, clusters, smem, s);
+        case QKV_ROPE_BF16: return launch_pair<QKV_ROPE_BF16>(mx, mw, mo, q, clusters, smem, s);
+        default:
+            if (q.act.kind || q.row_scale) return launch_pair<SWIGLU_BF16, true>(mx, mw, mo, q, clusters, smem, s);
+            return launch_pair<SWIGLU_BF16>(mx, mw, mo, q, clusters, smem, s);
+    }
+}
+
 // The persistent token-major kernel for a long step (T >= 128 tokens; output rows aligned for 16-byte stores).
 static int run_tokens_m(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
                         int ldx, int ldw, int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope,
@@ -1620,25 +1857,7 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
     q.K = K;
     q.ldo = ldo;
     q.m_tiles = (T + PT_BLOCK_M - 1) / PT_BLOCK_M;
-    // Weight rows per tile.  SwiGLU: 128 + 128.  Otherwise the width among 128 .. 256 that costs least: a CTA takes in (128 + bn) rows per K
-    // slice, and the CTAs go through ceil(tiles / SMs) rounds; 192 or 224 rows often fit in one round what 128 rows
-    // need two for (2,048 tokens x 1,536 outputs: 192 tiles of 128 in two rounds, 128 tiles of 192 in one).
-    if (accs == 2) {
-        q.bn = 128;
-    } else {
-        // the q/k/v mode takes whole heads (and pairs of 32-column chunks): steps of 64 or 128 rows
-        const int step = rope ? (rope->d == 64 ? 64 : 128) : 32;
-        long long best = -1;
-        q.bn = 128;
-        for (int bn = 256; bn >= 128; bn -= step) {
-            const long long tiles = (long long)q.m_tiles * ((N + bn - 1) / bn);
-            const long long cost = ((tiles + g_sms - 1) / g_sms) * (PT_BLOCK_M + bn);
-            if (best < 0 || cost < best) {
-                best = cost;
-                q.bn = bn;
-            }
-        }
-    }
+    q.bn = accs == 2 ? 128 : tokens_m_width(T, N, rope ? rope->d : 0);
     q.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
     q.n_tiles = (N + q.bn - 1) / q.bn;
     q.up_row_offset = up_row_offset;
@@ -1729,50 +1948,8 @@ static int gemm_tcgen05_impl(const void* x, const void* w, const float* bias, vo
     // long steps: the persistent token-major kernel (its 16-byte stores need aligned output rows)
     const int elt = (mode == STORE_BF16 || mode == SWIGLU_BF16) ? 2 : 4;
     const bool long_step = !built && token_major_pays(mode, T, N, K) && ((size_t)ldo * elt) % 16 == 0 && ((uintptr_t)out & 15) == 0;
-    if (long_step && T > PT_BLOCK_M && ferris_gemm_pair_enabled(mode, T)) {
-        // CTA pairs: tiles of 256 tokens x 256 weight rows (128 + 128 in SwiGLU mode), or x 128 where the
-        // wider tile would leave pairs of SMs without work
-        PTParams q;
-        q.out = out;
-        q.bias = bias;
-        q.act = g_launch_act;
-        q.T = T;
-        q.N = N;
-        q.K = K;
-        q.ldo = ldo;
-        q.m_tiles = (T + 2 * PT_BLOCK_M - 1) / (2 * PT_BLOCK_M);
-        const int pairs_all = g_sms / 2;
-        q.bn = (accs == 2 || q.m_tiles * ((N + 255) / 256) < pairs_all) ? 128 : 256;
-        q.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
-        q.n_tiles = (N + q.bn - 1) / q.bn;
-        q.up_row_offset = up_row_offset;
-        q.status = ferris_status_ptr();
-        const int half_rows = accs * q.bn / 2;
-        CUtensorMap mx, mw;
-        int rc = ferris_make_tensor_map_2d(&mx, x, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, PT_BLOCK_M, BLOCK_K);
-        if (rc != FERRIS_OK) return rc;
-        rc = pt_weight_map(w, (uint64_t)rows_w, (uint64_t)K, (uint64_t)ldw, (uint32_t)half_rows, &mw);
-        if (rc != FERRIS_OK) return rc;
-        CUtensorMap mo = mx;  // unused by the bf16 modes
-        if (elt == 4) {
-            rc = ferris_make_tensor_map_2d_f32(&mo, out, (uint64_t)T, (uint64_t)N, (uint64_t)ldo, 32);
-            if (rc != FERRIS_OK) return rc;
-        }
-        const int stage_bytes = PT_BLOCK_M * BLOCK_K * 2 + half_rows * BLOCK_K * 2;
-        const size_t smem = (size_t)PP_STAGES * stage_bytes + (size_t)PT_EPI_WARPS * 4096 + 1024;
-        int pairs = q.m_tiles * q.n_tiles;
-        if (pairs > pairs_all) pairs = pairs_all;
-        switch (mode) {
-            case STORE_BF16:
-                if (q.act.kind) return launch_pair<STORE_BF16, true>(mx, mw, mo, q, pairs, smem, s);
-                return launch_pair<STORE_BF16>(mx, mw, mo, q, pairs, smem, s);
-            case STORE_F32: return launch_pair<STORE_F32>(mx, mw, mo, q, pairs, smem, s);
-            case ACCUM_F32: return launch_pair<ACCUM_F32>(mx, mw, mo, q, pairs, smem, s);
-            default:
-                if (q.act.kind || q.row_scale) return launch_pair<SWIGLU_BF16, true>(mx, mw, mo, q, pairs, smem, s);
-                return launch_pair<SWIGLU_BF16>(mx, mw, mo, q, pairs, smem, s);
-        }
-    }
+    const PairPlan pairs = long_step && T > PT_BLOCK_M ? pair_plan(mode, T, N, K, 0) : PairPlan{};
+    if (pairs.bn) return run_pairs(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, nullptr, pairs, s);
     if (long_step)
         return run_tokens_m(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, nullptr, s);
 
@@ -1924,6 +2101,8 @@ FERRIS_API int ferris_qkv_rope_gemm_tcgen05(const void* x, const void* w, const 
     r.d = d;
     r.page_size = page_size;
     g_launch_act = FerrisEpilogueAct{0, 0.0f, 0.0f};
+    const PairPlan pairs = T > PT_BLOCK_M ? pair_plan(QKV_ROPE_BF16, T, N, K, d) : PairPlan{};
+    if (pairs.bn) return run_pairs(x, w, bias, out, QKV_ROPE_BF16, T, N, K, ldx, ldw, ldo, rows_w, 0, &r, pairs, (cudaStream_t)stream);
     return run_tokens_m(x, w, bias, out, QKV_ROPE_BF16, T, N, K, ldx, ldw, ldo, rows_w, 0, &r, (cudaStream_t)stream);
 }
 

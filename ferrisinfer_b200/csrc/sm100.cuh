@@ -121,6 +121,12 @@ __device__ __forceinline__ void st_peer_shared_f32(uint32_t addr, uint32_t rank,
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
+// 16 bytes to an address of the cluster's shared memory (map_to_cta).
+__device__ __forceinline__ void st_cluster_x4(uint32_t cluster_addr, const uint32_t* v) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------

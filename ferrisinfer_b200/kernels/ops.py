@@ -313,8 +313,9 @@ GEMM_PAIRS_NONE, GEMM_PAIRS_ALL, GEMM_PAIRS_SWIGLU = 0, 1, 2
 
 def set_gemm_pairs(which=GEMM_PAIRS_SWIGLU) -> None:
     """Which products of long steps (more than 128 tokens) run on pairs of CTAs that share one 256-row MMA
-    (cta_group::2): none, all, or the gate / up product only (the default, also of the library: see the
-    measurements beside ferris_gemm_pair_enabled in csrc/gemm_tcgen05.cu).  True / False mean all / none."""
+    (cta_group::2): none, all (without K splits: the numbers are then those of single CTAs bit for bit), or the gate / up
+    product and those that an estimate puts there, some with their K split over a cluster of pairs (the default, also
+    of the library: see pair_plan in csrc/gemm_tcgen05.cu).  True / False mean all / none."""
     _lib().ferris_set_gemm_pair(_c_int(int(which)))
 
 

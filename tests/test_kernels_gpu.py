@@ -281,6 +281,33 @@ def test_gemm_on_cta_pairs(T, N, K, mode, device):
     _close(paired, ref, K, dtype)
 
 
+@pytest.mark.parametrize("T, N, K", [(2048, 896, 4864), (1000, 896, 4864), (1001, 900, 4872), (769, 1540, 2504), (512, 1536, 8960),
+                                     (257, 3584, 5000), (130, 3590, 18944), (2048, 3592, 136)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_gemm_of_long_steps_as_they_are_launched(T, N, K, mode, device):
+    """Few tiles and a long K (pairs of CTAs with two, three or four K splits, the last one shorter), two rounds of tiles
+    (pairs without splits), token and weight rows and K slices that end inside a tile.  Against 64 bits: sums of K terms in
+    fp32, 2^-24 of the sum of their absolute values for the additions on the way (in order, then over four splits and the
+    base), and a bf16 result's own rounding; the same bits again."""
+    from ferrisinfer_b200.kernels import ops
+
+    N = N // 8 * 8 if mode == 0 else N // 4 * 4
+    x, w = rnd((T, K), BF16, device, 51), rnd((N, K), BF16, device, 52, scale=0.1)
+    bias = rnd((N,), F32, device, 53) if mode < 2 else None
+    base = rnd((T, N), F32, device, 54) if mode == 2 else None
+    outs = []
+    for _ in range(2):
+        out = base.clone() if mode == 2 else torch.full((T, N), float("nan"), dtype=F32 if mode else BF16, device=device)
+        ops.gemm_tcgen05(x, w, bias, out, mode)
+        outs.append(out)
+    assert ops.kernel_status() == 0 and torch.equal(outs[0], outs[1])
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    extra = base if mode == 2 else bias
+    want, size = want + extra.double(), size + extra.double().abs()
+    bound = (K / 16 + 8) * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if mode == 0 else 0.0)
+    assert ((outs[0].double() - want).abs() <= bound).all()
+
+
 @pytest.fixture
 def skinny_off():
     """The products of short steps on the tcgen05 kernel with its K split over a cluster, as before the skinny kernel."""
