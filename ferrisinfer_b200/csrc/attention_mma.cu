@@ -521,7 +521,6 @@ __global__ void __launch_bounds__(NW * 32)
     }
     mbar_fence_init();
     __syncthreads();
-    pdl_launch_dependents();
     if (splits > 1 && cluster_merge) cluster_arrive_relaxed();  // first phase of the cluster's barrier: "this CTA runs"
     // A kernel that rotates AND writes the cache reads nothing from the cache that this step wrote before it (the
     // token's own key and value come from its qkv row, which it patches into the tile), and the step's metadata was
@@ -536,8 +535,11 @@ __global__ void __launch_bounds__(NW * 32)
     const bool fused = rope.inv_freq != nullptr;
     const bool patches = fused && rope.slot_mapping != nullptr;
     const bool early = patches;
-    if (!early) {
+    if (early) {
+        pdl_launch_dependents();
+    } else {  // (the attention of portions may run beside this kernel without a wait of its own: it is let in after this one's)
         pdl_wait();
+        pdl_launch_dependents();
         FERRIS_TL_BEGIN();
     }
     // with a token list, only the listed rows of the step are attended (the others belong to another kernel)
@@ -1071,7 +1073,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
                                  const bf16* q, int ldq, bf16* __restrict__ out, int ldo,
                                  const int* __restrict__ block_tables, int max_blocks, const int* __restrict__ seq_q_start,
                                  const int* __restrict__ seq_start_pos, int nh, int nkv, int page_size, int window,
-                                 float scale, int skip_single, int* status) {
+                                 float scale, int num_seqs, int skip_single, int beside, int* status) {
     constexpr int ATOMS = D / 64;                      // 64-wide column groups of a head (one 128-byte swizzle row each)
     constexpr int TILE = TILE_KEYS * 64 * 2;           // one 16-key x 64-column box of K or of V: 2 KB
     constexpr int ATOM_BYTES = T5_KEYS * 64 * 2;       // 128 rows x 64 columns: 16 KB
@@ -1094,20 +1096,45 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     uint8_t* kv_smem = smem + BLOCK_BYTES + GROUPS * P_BYTES;  // stages x (K block, V block), each [column group][128 keys][64]
 
     const int G = nh / nkv;
-    const int seq = blockIdx.z, hk = blockIdx.y;
+    const int hk = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     FERRIS_TL_ENTRY();
-    pdl_wait();
+    if (!beside) pdl_wait();
     pdl_launch_dependents();
     FERRIS_TL_BEGIN();
-    const int q_start = seq_q_start[seq], q_len = seq_q_start[seq + 1] - q_start;
-    const int rows_total = q_len * G;
-    const int n_blocks = (rows_total + T5_ROWS - 1) / T5_ROWS;
-    if ((skip_single && q_len == 1) || (int)blockIdx.x >= n_blocks) {  // single tokens are the decode kernel's
+    // The grid holds no more CTAs a kv head than there are row blocks, whatever the requests' lengths (a CTA without rows still
+    // takes a whole SM's shared memory: a step of 31 single tokens and one portion of 481 tokens launched 1,472 CTAs for 46
+    // row blocks and took 31 us): each warp finds the CTA's request by itself.
+    int seq = -1, rank = 0;
+    for (int s0 = 0, before = 0; s0 < num_seqs && seq < 0; s0 += 32) {
+        int n = 0;
+        if (s0 + lane < num_seqs) {
+            const int len = seq_q_start[s0 + lane + 1] - seq_q_start[s0 + lane];
+            n = skip_single && len == 1 ? 0 : (len * G + T5_ROWS - 1) / T5_ROWS;  // single tokens are the decode kernel's
+        }
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+        }
+        const unsigned here = __ballot_sync(0xffffffffu, (int)blockIdx.x < before + upto);
+        if (here) {
+            const int at = __ffs(here) - 1;
+            seq = s0 + at;
+            rank = (int)blockIdx.x - before - __shfl_sync(0xffffffffu, upto - n, at);
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (seq < 0) {
+        if (beside) pdl_wait();
         FERRIS_TL_END(8);
         return;
     }
-    const int block = n_blocks - 1 - blockIdx.x;  // heavy row blocks (the last tokens see the most keys) first
+    const int q_start = seq_q_start[seq], q_len = seq_q_start[seq + 1] - q_start;
+    const int rows_total = q_len * G;
+    const int n_blocks = (rows_total + T5_ROWS - 1) / T5_ROWS;
+    const int block = n_blocks - 1 - rank;  // heavy row blocks (the last tokens see the most keys) first
     const int row0 = block * T5_ROWS;
     const int start_pos = seq_start_pos[seq];
     const int* table = block_tables + (size_t)seq * max_blocks;
@@ -1456,6 +1483,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
         tcgen05_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
+    if (beside) pdl_wait();  // the launch before has ended when this one ends, for those who wait for this one
     FERRIS_TL_END(8);
 }
 
@@ -1671,15 +1699,18 @@ FERRIS_API int ferris_decode_attention(const void* q, int ldq, void* out, int ld
 }
 
 // The same for the rows of a step that `token_list` (int32 [tokens]) names: the single tokens of a step
-// that also carries portions of prompts.  The scratch is indexed by place in the list.
+// that also carries portions of prompts.  The scratch is indexed by place in the list.  merge: 1 a merge kernel follows, 3 a
+// cluster merges the key ranges (see ferris_decode_attention_rope).
 FERRIS_API int ferris_decode_attention_listed(const void* q, int ldq, void* out, int ldo, const void* k_cache,
                                               const void* v_cache, long long cache_pages, const int* block_tables,
                                               int max_blocks, const int* token_seq, const int* positions,
                                               const int* token_list, int tokens, int nh, int nkv, int d, int page_size,
-                                              int window, float scale, int splits, float* scratch, void* stream) {
+                                              int window, float scale, int splits, float* scratch, int merge, void* stream) {
     if (!token_list) FERRIS_REFUSE("decode attention: no token list");
+    if (merge != 1 && merge != 3) FERRIS_REFUSE("decode attention of listed tokens: merge mode %d", merge);
     return decode_attention_impl(q, ldq, out, ldo, k_cache, v_cache, cache_pages, block_tables, max_blocks, token_seq,
-                                 positions, token_list, tokens, nh, nkv, d, page_size, window, scale, splits, scratch, stream);
+                                 positions, token_list, tokens, nh, nkv, d, page_size, window, scale, splits, scratch, stream,
+                                 nullptr, nullptr, merge);
 }
 
 // Single-token steps whose q and k have NOT been rotated and whose k and v are NOT in the cache yet: the kernel
@@ -1785,12 +1816,17 @@ FERRIS_API int ferris_set_prefill_tcgen05(int on) {
 }
 
 // Portions of prompts (and anything else: a request with one token is a portion of one, unless
-// skip_single leaves those to the decode kernel).
+// skip_single leaves those to the decode kernel).  tokens, requests: how many rows and requests it concerns (without the single
+// tokens that are left out), by which the grid is cut; 0: not known.  beside: the launch before this one in the stream is
+// ferris_decode_attention_listed for the same step; it reads nothing that this kernel writes and writes nothing that it
+// reads, so the two run side by side (a step of 31 single tokens and one portion of 481 at the 1.5B sizes 3.68 -> 3.12 ms, with
+// the grid cut to the row blocks and the key ranges to the SMs that are left).  The decode kernel lets this one in only when its
+// own wait is over, which says that all launches before it have ended, and this one ends only when the decode kernel has ended.
 FERRIS_API int ferris_prefill_attention(const void* q, int ldq, void* out, int ldo, const void* k_cache,
                                         const void* v_cache, long long cache_pages, const int* block_tables,
                                         int max_blocks, const int* seq_q_start, const int* seq_start_pos, int num_seqs,
                                         int max_q_len, int nh, int nkv, int d, int page_size, int window, float scale,
-                                        int skip_single, void* stream) {
+                                        int skip_single, int tokens, int requests, int beside, void* stream) {
     if (num_seqs <= 0 || max_q_len <= 0) return FERRIS_OK;
     int rc = check_common(nh, nkv, d, page_size, max_blocks);
     if (rc != FERRIS_OK) return rc;
@@ -1803,7 +1839,14 @@ FERRIS_API int ferris_prefill_attention(const void* q, int ldq, void* out, int l
     cudaStream_t s = (cudaStream_t)stream;
     int* status = ferris_status_ptr();
     if (prefill_on_tcgen05()) {
-        dim3 grid5(((size_t)max_q_len * G + T5_ROWS - 1) / T5_ROWS, nkv, num_seqs);
+        // row blocks: a request's last one may be part of one, so at most one a request beyond what all rows fill
+        long long blocks = ((long long)max_q_len * G + T5_ROWS - 1) / T5_ROWS * num_seqs;
+        if (tokens > 0 && requests > 0) {
+            const long long most = (long long)tokens * G / T5_ROWS + requests;
+            if (most < blocks) blocks = most;
+        }
+        if (blocks > 0x7fffffffLL) FERRIS_REFUSE("prefill attention: %lld blocks of rows exceed one launch", blocks);
+        dim3 grid5((unsigned)blocks, nkv);
         // Q, a P tile per softmax group, stages of (K block, V block).  Head size 64: two groups and four stages
         // (209 KB); head size 128: one group and two stages (193 KB), two groups would not fit.
         auto bytes = [&](int groups, int stages) {
@@ -1815,7 +1858,7 @@ FERRIS_API int ferris_prefill_attention(const void* q, int ldq, void* out, int l
         if ((rc = set_smem(prefill_attention_tc5_kernel<DD, GG, SS>, smem)) != FERRIS_OK) return rc;                       \
         ferris_launch(prefill_attention_tc5_kernel<DD, GG, SS>, grid5, dim3(t5_threads(GG)), smem, s, mk, mv, (const bf16*)q, \
                       ldq, (bf16*)out, ldo, block_tables, max_blocks, seq_q_start, seq_start_pos, nh, nkv, page_size,      \
-                      window, scale, skip_single, status);                                                                 \
+                      window, scale, num_seqs, skip_single, beside, status);                                               \
     } while (0)
         if (d == 64 && g_prefill_tc5 != 2)
             FERRIS_T5_LAUNCH(64, 2, 4);

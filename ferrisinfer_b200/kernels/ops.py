@@ -38,7 +38,8 @@ _SIGNATURES = {
     "ferris_rotary_angles": [_VP, _VP, _VP, _I, _I, _VP],
     "ferris_rmsnorm": [_VP, _VP, _VP, _VP, _I, _I, _I, _F, _VP],
     "ferris_rope_cache_write": [_VP, _I, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP],
-    "ferris_prefill_attention": [_VP, _I, _VP, _I, _VP, _VP, _LL, _VP, _I, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _F, _I, _VP],
+    "ferris_prefill_attention": [_VP, _I, _VP, _I, _VP, _VP, _LL, _VP, _I, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _I,
+                                 _VP],
     "ferris_decode_attention_rope": [_VP, _I, _VP, _I, _VP, _VP, _LL, _VP, _I, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I,
                                      _F, _I, _VP, _I, _VP],
     "ferris_gemm_argmax_tcgen05": [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP, _VP],
@@ -2042,33 +2043,37 @@ def decode_splits(tokens: int, num_kv_heads: int, max_kv_len: int) -> int:
 
 
 def decode_attention(qkv, out, k_cache, v_cache, block_tables, token_seq, positions, num_heads, num_kv_heads,
-                     head_dim, window, scale, splits, scratch, rows: Optional[torch.Tensor] = None):
+                     head_dim, window, scale, splits, scratch, rows: Optional[torch.Tensor] = None, cluster: bool = False):
     """Split-KV attention for single tokens (bf16, head size 64 or 128): every row of the step, or the rows
-    that ``rows`` (int32) names when the step also carries portions of prompts."""
+    that ``rows`` (int32) names when the step also carries portions of prompts; ``cluster`` (with ``rows``): the
+    key ranges of a token merge through a cluster's shared memory, without scratch."""
     T, _, ldq = _rows(qkv, "attention queries")
     _, _, ldo = _rows(out, "attention output")
     n = T if rows is None else rows.numel()
-    need = n * num_heads * splits * (head_dim + 2) if splits > 1 else 0
+    cluster = cluster and rows is not None
+    need = n * num_heads * splits * (head_dim + 2) if splits > 1 and not cluster else 0
     if need and (scratch is None or scratch.numel() < need or scratch.dtype != torch.float32):
         raise KernelError(f"decode attention with {splits} splits needs {need} floats of scratch")
     common = (_ptr(qkv), _c_int(ldq), _ptr(out), _c_int(ldo), _ptr(k_cache), _ptr(v_cache),
               ctypes.c_longlong(k_cache.shape[0]), _ptr(block_tables), _c_int(block_tables.shape[1]), _ptr(token_seq),
               _ptr(positions))
     tail = (_c_int(num_heads), _c_int(num_kv_heads), _c_int(head_dim), _c_int(k_cache.shape[2]), _c_int(window or 0),
-            _c_float(scale), _c_int(splits), _ptr(scratch if need else None), _stream())
-    kernels = 2 if splits > 1 else 1  # the attention kernel and the merge of its key ranges
+            _c_float(scale), _c_int(splits), _ptr(scratch if need else None))
+    kernels = 2 if splits > 1 and not cluster else 1  # the attention kernel and the merge of its key ranges
     if rows is None:
-        _check(_lib().ferris_decode_attention(*common, _c_int(T), *tail), "decode attention", kernels)
+        _check(_lib().ferris_decode_attention(*common, _c_int(T), *tail, _stream()), "decode attention", kernels)
     else:
         _need(rows, "rows of the single tokens", torch.int32)
-        _check(_lib().ferris_decode_attention_listed(*common, _ptr(rows), _c_int(rows.numel()), *tail), "decode attention",
-               kernels)
+        _check(_lib().ferris_decode_attention_listed(*common, _ptr(rows), _c_int(rows.numel()), *tail,
+                                                     _c_int(3 if cluster else 1), _stream()), "decode attention", kernels)
 
 
 def prefill_attention(qkv, out, k_cache, v_cache, block_tables, seq_q_start, seq_start_pos, num_seqs, max_q_len,
-                      num_heads, num_kv_heads, head_dim, window, scale, skip_single: bool = False):
+                      num_heads, num_kv_heads, head_dim, window, scale, skip_single: bool = False, singles: int = 0,
+                      beside_decode: bool = False):
     """Tensor-core attention for portions of prompts (bf16, head size 64 or 128).  ``skip_single``: requests
-    that bring one token are left out (the decode kernel takes them)."""
+    that bring one token are left out (the decode kernel takes them); ``singles``: how many those are.
+    ``beside_decode``: the launch before is ``decode_attention`` of those tokens, the two may run side by side."""
     _, _, ldq = _rows(qkv, "attention queries")
     _, _, ldo = _rows(out, "attention output")
     _check(
@@ -2077,7 +2082,8 @@ def prefill_attention(qkv, out, k_cache, v_cache, block_tables, seq_q_start, seq
                                         _c_int(block_tables.shape[1]), _ptr(seq_q_start), _ptr(seq_start_pos),
                                         _c_int(num_seqs), _c_int(max_q_len), _c_int(num_heads), _c_int(num_kv_heads),
                                         _c_int(head_dim), _c_int(k_cache.shape[2]), _c_int(window or 0), _c_float(scale),
-                                        _c_int(1 if skip_single else 0), _stream()),
+                                        _c_int(1 if skip_single else 0), _c_int(max(qkv.shape[0] - singles, 0)),
+                                        _c_int(max(num_seqs - singles, 0)), _c_int(1 if beside_decode else 0), _stream()),
         "prefill attention",
     )
 
@@ -2188,17 +2194,27 @@ def paged_attention(qkv, out, k_cache, v_cache, block_tables, ctx, num_heads, nu
         # single tokens: all rows of the step, or the listed ones beside portions of prompts
         n = T if ctx.max_q_len == 1 else singles.numel()
         kv_span = min(ctx.max_kv_len, window) if window else ctx.max_kv_len
-        splits = decode_splits(n, num_kv_heads, kv_span)
+        beside = ctx.max_q_len > 1 and gemm_skinny_enabled()  # (the switch of the merge through clusters)
+        if beside:
+            # the portions' row blocks run beside this kernel: key ranges for the SMs that they leave, at least for half of them
+            blocks = ((T - n) * (num_heads // num_kv_heads) // 128 + ctx.num_seqs - n) * num_kv_heads
+            left = sm_count() - min(blocks, sm_count() // 2)
+            splits = min(int(_lib().ferris_decode_cluster_splits(n, num_kv_heads, head_dim, kv_span)),
+                         max(1, left // (n * num_kv_heads)))
+            beside = splits >= 1
+        if not beside:
+            splits = decode_splits(n, num_kv_heads, kv_span)
         scratch = None
-        if splits > 1:
+        if splits > 1 and not beside:
             scratch = ctx.workspace.get("attn_split_scratch", (n * num_heads * splits * (head_dim + 2),), torch.float32)
         decode_attention(qkv, out, k_cache, v_cache, block_tables, ctx.token_seq, ctx.positions, num_heads,
                          num_kv_heads, head_dim, window, scale, splits, scratch,
-                         rows=None if ctx.max_q_len == 1 else singles)
+                         rows=None if ctx.max_q_len == 1 else singles, cluster=beside)
     if ctx.max_q_len > 1:
         prefill_attention(qkv, out, k_cache, v_cache, block_tables, ctx.seq_q_start, ctx.seq_start_pos, ctx.num_seqs,
                           ctx.max_q_len, num_heads, num_kv_heads, head_dim, window, scale,
-                          skip_single=singles is not None)
+                          skip_single=singles is not None, singles=0 if singles is None else singles.numel(),
+                          beside_decode=singles is not None)
 
 
 def sample(logits: torch.Tensor, out_token: torch.Tensor, out_prob: Optional[torch.Tensor] = None,

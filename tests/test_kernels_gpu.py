@@ -641,6 +641,22 @@ def test_attention_mixed_batch(nh, nkv, d, page, dtype, impl, device):
     assert torch.allclose(got, want, **ATT_TOL[dtype]), (got - want).abs().max()
 
 
+@pytest.mark.parametrize("nh, nkv, d", [(14, 2, 64), (6, 2, 128)])
+@pytest.mark.parametrize("singles", [0, 3, 60])
+def test_attention_of_many_requests_of_all_lengths(singles, nh, nkv, d, device):
+    """Portions whose row blocks fill up exactly, by one row less and one more, and of a row or two, in an order that puts
+    them on both sides of the 32nd and the 64th request, beside no, few (several key ranges each) and many single tokens."""
+    G = nh // nkv
+    lens = [2, 128 // G, 128 // G + 1, 256 // G, 3, 2, 200] + [2 + i % 5 for i in range(30)] + [90, 2]
+    seqs = [(n + 17 * i % 130, n) for i, n in enumerate(lens)]
+    for i in range(singles):
+        seqs.insert((5 * i) % len(seqs), (1 + 37 * i % 700, 1))
+    case = AttentionCase(device, BF16, nh, nkv, d, 16, seqs, seed=singles + d)
+    got, want = run_attention(case, "dispatch"), case.reference()
+    assert torch.isfinite(got).all()
+    assert torch.allclose(got, want, **ATT_TOL[BF16]), (got - want).abs().max()
+
+
 @pytest.mark.parametrize("impl", ["simt", "dispatch"])
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("q_len", [1, 5, 64])
