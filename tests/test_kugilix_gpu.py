@@ -351,6 +351,19 @@ def test_gated_rmsnorm(device, dtype):
     assert torch.allclose(out.double(), want, atol=tol, rtol=tol)
 
 
+@pytest.mark.parametrize("n", [504, 512, 520, 2048, 4096, 4104])  # eight columns a thread from 512 to 4,096
+def test_gated_rmsnorm_of_wide_rows(device, n):
+    """Against 64 bits: fp32 throughout (a few units of 2^-24, the sum over a row's squares among them), one rounding to bf16."""
+    ops = _ops()
+    torch.manual_seed(n)
+    o, g, w = torch.randn(5, n, device=device) * 4, torch.randn(5, n + 8, device=device).to(BF16), 1 + 0.3 * torch.randn(n, device=device)
+    out = torch.full((5, n + 16), 7.0, dtype=BF16, device=device)
+    ops.gated_rmsnorm(o, g[:, 8:], w, 1e-6, out[:, :n])
+    want = plain.rms_unit(o.double(), 1e-6) * w.double() * torch.sigmoid(g[:, 8:].double())
+    assert ((out[:, :n].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -18) * want.abs()).all()
+    assert bool((out[:, n:] == 7).all())
+
+
 @pytest.mark.parametrize("n", [1001, 4096])  # one value a thread; sixteen bytes a thread
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_xielu_activation(device, dtype, n):
