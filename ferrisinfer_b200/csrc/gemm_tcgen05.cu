@@ -690,10 +690,28 @@ struct PTParams {
     // Written by the launch before this one, so never read through a read-only path.
     const int* tile_expert = nullptr;
     int expert_rows = 0;
+    // with tile_expert: how many rows of each tile are a token's, its first ones; only the boxes of PT_ROW_BOX rows that hold them
+    // are loaded and stored.  (An expert of a decode step has a few rows: whole tiles of 128 are more bytes than half its weights.)
+    const int* tile_rows = nullptr;
     // SwiGLU mode, or the bf16 store with an activation: a factor per row (written by an earlier launch) on the accumulators
     // ahead of the activation: the product of a row that is multiplied by it.  Null: none.
     const float* row_scale = nullptr;
 };
+
+constexpr int PT_ROW_BOX = 32;  // an epilogue warp's rows
+
+// Token tiles up to the last one that meets an expert's weights (all of them without experts): the CTAs divide these among
+// themselves.  By a whole warp.
+__device__ __forceinline__ int pt_live_tiles(const PTParams& p) {
+    if (!p.tile_expert) return p.m_tiles;
+    int last = 0;
+    for (int i = threadIdx.x & 31; i < p.m_tiles; i += 32)
+        if (*(reinterpret_cast<const volatile int*>(p.tile_expert) + i) >= 0) last = i + 1;
+    return __reduce_max_sync(0xffffffffu, last);
+}
+__device__ __forceinline__ int pt_tile_rows(const PTParams& p, int mt) {
+    return p.tile_rows ? *(reinterpret_cast<const volatile int*>(p.tile_rows) + mt) : PT_BLOCK_M;
+}
 
 // The first weight row of the expert that token tile `mt` meets (0 without experts), or -1 to skip the tile.
 __device__ __forceinline__ int pt_tile_weight_row(const PTParams& p, int mt) {
@@ -896,7 +914,7 @@ __device__ __forceinline__ void pt_epilogue_tile(const PTParams& p, const CUtens
     }
 }
 
-template <int MODE, bool ACT>
+template <int MODE, bool ACT, bool GROUPED>
 __global__ void __launch_bounds__(PT_THREADS)
     gemm_tokens_m_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          const __grid_constant__ CUtensorMap map_out, const PTParams p) {
@@ -910,7 +928,6 @@ __global__ void __launch_bounds__(PT_THREADS)
     const int a_bytes = PT_BLOCK_M * BLOCK_K * 2, b_bytes = p.bn * BLOCK_K * 2;
     const int stage_bytes = a_bytes + ACCS * b_bytes;
     const int acc_cols = 256;  // columns of one accumulator buffer (ACCS * bn of them used)
-    const int tiles = p.m_tiles * p.n_tiles;
     // fp32 outputs leave through shared memory and TMA: 4 KB (32 tokens x 32 floats, swizzled) per epilogue warp
     uint8_t* out_stage = smem + (size_t)PT_STAGES * stage_bytes + (size_t)(warp >= 2 ? warp - 2 : 0) * 4096;
 
@@ -937,36 +954,40 @@ __global__ void __launch_bounds__(PT_THREADS)
     // expert says which they are), the tokens after it: a weight's first slices come from HBM while the launch before ends (us a
     // product in a row of them: 9,728 x 896 at 256 to 2,048 tokens 14.0 / 19.1 / 25.3 / 36.8 -> 13.5 / 18.1 / 24.3 / 35.7)
     int early = 0;
-    auto load_weights = [&](int it, int kb, int row) {
+    auto load_weights = [&](int it, int kb, int row, int token_bytes) {
         uint8_t* st = smem + (size_t)(it % PT_STAGES) * stage_bytes;
         uint64_t* bar = &full[it % PT_STAGES];
-        mbar_expect_tx(bar, stage_bytes);
+        mbar_expect_tx(bar, token_bytes + ACCS * b_bytes);
         tma_load_2d(st + a_bytes, &map_w, kb * BLOCK_K, row, bar);
         if (ACCS == 2) tma_load_2d(st + a_bytes + b_bytes, &map_w, kb * BLOCK_K, p.up_row_offset + row, bar);
     };
-    if (threadIdx.x == 0 && !p.tile_expert) {
+    if (threadIdx.x == 0 && !GROUPED) {
         early = min(PT_STAGES, p.kblocks);
-        for (int kb = 0; kb < early; ++kb) load_weights(kb, kb, ((int)blockIdx.x / p.m_tiles) * p.bn);
+        for (int kb = 0; kb < early; ++kb) load_weights(kb, kb, ((int)blockIdx.x / p.m_tiles) * p.bn, a_bytes);
     }
     pdl_wait();
     FERRIS_TL_BEGIN();
+    const int m_tiles = GROUPED ? pt_live_tiles(p) : p.m_tiles, tiles = m_tiles * p.n_tiles;
 
     if (warp == 0) {
         if (lane == 0) {
             int it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-                const int wrow = pt_tile_weight_row(p, tile % p.m_tiles);
+                const int wrow = GROUPED ? pt_tile_weight_row(p, tile % m_tiles) : 0;
                 if (wrow < 0) continue;
-                const int m0 = (tile % p.m_tiles) * PT_BLOCK_M, n0 = (tile / p.m_tiles) * p.bn;
+                const int m0 = (tile % m_tiles) * PT_BLOCK_M, n0 = (tile / m_tiles) * p.bn;
+                const int boxes = GROUPED && p.tile_rows ? (pt_tile_rows(p, tile % m_tiles) + PT_ROW_BOX - 1) / PT_ROW_BOX : 1;
+                const int box_bytes = GROUPED && p.tile_rows ? PT_ROW_BOX * BLOCK_K * 2 : a_bytes;
                 for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
                     const int s = it % PT_STAGES;
                     if (it >= PT_STAGES && !mbar_wait(&empty[s], ((it / PT_STAGES) - 1) & 1, p.status, 20)) {
                         ok = false;
                         break;
                     }
-                    if (it >= early) load_weights(it, kb, wrow + n0);
-                    tma_load_2d(smem + (size_t)s * stage_bytes, &map_x, kb * BLOCK_K, m0, &full[s]);
+                    if (it >= early) load_weights(it, kb, wrow + n0, boxes * box_bytes);
+                    for (int i = 0; i < boxes; ++i)
+                        tma_load_2d(smem + (size_t)s * stage_bytes + i * box_bytes, &map_x, kb * BLOCK_K, m0 + i * PT_ROW_BOX, &full[s]);
                 }
             }
         }
@@ -976,7 +997,7 @@ __global__ void __launch_bounds__(PT_THREADS)
             int it = 0, local = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-                if (pt_tile_weight_row(p, tile % p.m_tiles) < 0) continue;  // skipped by every role alike
+                if (GROUPED && pt_tile_weight_row(p, tile % m_tiles) < 0) continue;  // skipped by every role alike
                 const int buf = local & 1;
                 // the epilogue must have drained this accumulator buffer (two tiles ago)
                 if (local >= 2 && !mbar_wait(&tmem_empty[buf], ((local >> 1) - 1) & 1, p.status, 21)) break;
@@ -1013,9 +1034,9 @@ __global__ void __launch_bounds__(PT_THREADS)
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         int local = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            if (pt_tile_weight_row(p, tile % p.m_tiles) < 0) continue;
+            if (GROUPED && pt_tile_weight_row(p, tile % m_tiles) < 0) continue;
             const int buf = local & 1;
-            const int m0 = (tile % p.m_tiles) * PT_BLOCK_M, n0 = (tile / p.m_tiles) * p.bn;
+            const int m0 = (tile % m_tiles) * PT_BLOCK_M, n0 = (tile / m_tiles) * p.bn;
             const int t = m0 + quarter * 32 + lane;
             if (!mbar_wait(&tmem_full[buf], (local >> 1) & 1, p.status, 23)) break;
             ++local;
@@ -1023,7 +1044,7 @@ __global__ void __launch_bounds__(PT_THREADS)
             const uint32_t d0 = lane_addr + buf * acc_cols;
             if constexpr (MODE == QKV_ROPE_BF16)
                 pt_epilogue_qkv_rope(p, d0, n0, half, t);
-            else
+            else if (!GROUPED || quarter * PT_ROW_BOX < pt_tile_rows(p, tile % m_tiles))  // (rows that were not loaded are nobody's)
                 pt_epilogue_tile<MODE, ACT>(p, map_out, d0, m0, n0, quarter, half, lane, t, out_stage);
             // this warp has read its part of the buffer: the MMA warp may overwrite it
             tcgen05_fence_before();
@@ -1404,6 +1425,28 @@ static int tokens_m_width(int T, int N, int head) {
     return width;
 }
 
+// The same for a product per group of token tiles, of which only those with rows count: as many as there are experts while a step's
+// pairs are few, half an expert's tile beyond the full ones later on.  A tile with few rows costs its weights and a box of rows.
+// The experts' gate and up rows of 64 tokens x 2 of 8 (2 x 2,688 rows of 2,048 each): 8 x 21 tiles of 128 + 128 go through 148 CTAs in
+// two rounds, 8 x 34 of 80 + 80 do so too.  All of the experts' kernels, us, before / now (with boxes of rows): 17 to 64 tokens 75.6 / 68.4,
+// 256 78.4 / 71.2, 512 92.7 / 78.5, 1,024 119 / 112, 2,048 177 / 171; all tokens to two of the eight experts, 64 to 256 tokens
+// 47 to 51 / 49 to 53 (more boxes a slice).  Six stages of shared memory instead of four: the same.
+static int grouped_width(int m_tiles, int experts, int N, int accs) {
+    const int few = experts < m_tiles ? experts : m_tiles, many = m_tiles - experts / 2;
+    const int live = few > many ? few : many, rows = many <= few ? PT_ROW_BOX : PT_BLOCK_M;
+    long long best = -1;
+    int width = 128;
+    for (int bn = accs == 2 ? 128 : 256; bn >= (accs == 2 ? 64 : 128); bn -= accs == 2 ? 16 : 32) {
+        const long long tiles = (long long)live * ((N + bn - 1) / bn);
+        const long long cost = ((tiles + g_sms - 1) / g_sms) * (rows + accs * bn);
+        if (best < 0 || cost < best) {
+            best = cost;
+            width = bn;
+        }
+    }
+    return width;
+}
+
 int g_pair = -1;  // 0: no product on pairs, 1: every long-step product (no K splits), 2: the SwiGLU product, others where pair_plan's estimate says so
 int pair_clusters(int splits);
 
@@ -1573,12 +1616,12 @@ int pair_clusters(int splits) {
     return have;
 }
 
-template <int MODE, bool ACT = false>
+template <int MODE, bool ACT = false, bool GROUPED = false>
 int launch_pt(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const PTParams& p, int ctas,
               size_t smem, cudaStream_t s) {
-    int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_m_kernel<MODE, ACT>, smem);
+    int rc = ferris_allow_dynamic_smem((const void*)gemm_tokens_m_kernel<MODE, ACT, GROUPED>, smem);
     if (rc != FERRIS_OK) return rc;
-    cudaError_t e = ferris_launch(gemm_tokens_m_kernel<MODE, ACT>, dim3(ctas), dim3(PT_THREADS), smem, s, mx, mw, mo, p);
+    cudaError_t e = ferris_launch(gemm_tokens_m_kernel<MODE, ACT, GROUPED>, dim3(ctas), dim3(PT_THREADS), smem, s, mx, mw, mo, p);
     if (e != cudaSuccess) {
         ferris_set_error("gemm: %s", cudaGetErrorString(e));
         return (int)e;
@@ -1843,8 +1886,8 @@ static int run_pairs(const void* x, const void* w, const float* bias, void* out,
 // The persistent token-major kernel for a long step (T >= 128 tokens; output rows aligned for 16-byte stores).
 static int run_tokens_m(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
                         int ldx, int ldw, int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope,
-                        cudaStream_t s, const int* tile_expert = nullptr, int expert_rows = 0,
-                        const float* row_scale = nullptr) {
+                        cudaStream_t s, const int* tile_expert = nullptr, const int* tile_rows = nullptr, int experts = 0,
+                        int expert_rows = 0, const float* row_scale = nullptr) {
     const int accs = mode == SWIGLU_BF16 ? 2 : 1;
     const int elt = (mode == STORE_F32 || mode == ACCUM_F32) ? 4 : 2;
     sm_count();
@@ -1857,17 +1900,21 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
     q.K = K;
     q.ldo = ldo;
     q.m_tiles = (T + PT_BLOCK_M - 1) / PT_BLOCK_M;
-    q.bn = accs == 2 ? 128 : tokens_m_width(T, N, rope ? rope->d : 0);
+    if (tile_expert)
+        q.bn = grouped_width(q.m_tiles, experts, N, accs);
+    else
+        q.bn = accs == 2 ? 128 : tokens_m_width(T, N, rope ? rope->d : 0);
     q.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
     q.n_tiles = (N + q.bn - 1) / q.bn;
     q.up_row_offset = up_row_offset;
     q.status = ferris_status_ptr();
     q.rope = rope ? *rope : RopeEpilogue{};
     q.tile_expert = tile_expert;
+    q.tile_rows = tile_rows;
     q.expert_rows = expert_rows;
     q.row_scale = row_scale;
     CUtensorMap mx, mw;
-    int rc = ferris_make_tensor_map_2d(&mx, x, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, PT_BLOCK_M, BLOCK_K);
+    int rc = ferris_make_tensor_map_2d(&mx, x, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, tile_rows ? PT_ROW_BOX : PT_BLOCK_M, BLOCK_K);
     if (rc != FERRIS_OK) return rc;
     rc = pt_weight_map(w, (uint64_t)rows_w, (uint64_t)K, (uint64_t)ldw, (uint32_t)q.bn, &mw);
     if (rc != FERRIS_OK) return rc;
@@ -1880,6 +1927,12 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
     const size_t smem = (size_t)PT_STAGES * stage_bytes + (size_t)PT_EPI_WARPS * 4096 + 1024;
     int ctas = q.m_tiles * q.n_tiles;
     if (ctas > g_sms) ctas = g_sms;
+    if (tile_expert) {
+        if (mode == STORE_F32) return launch_pt<STORE_F32, false, true>(mx, mw, mo, q, ctas, smem, s);
+        if (mode == STORE_BF16) return launch_pt<STORE_BF16, true, true>(mx, mw, mo, q, ctas, smem, s);
+        if (q.act.kind || row_scale) return launch_pt<SWIGLU_BF16, true, true>(mx, mw, mo, q, ctas, smem, s);
+        return launch_pt<SWIGLU_BF16, false, true>(mx, mw, mo, q, ctas, smem, s);
+    }
     switch (mode) {
         case STORE_BF16:
             if (q.act.kind) return launch_pt<STORE_BF16, true>(mx, mw, mo, q, ctas, smem, s);
@@ -1887,7 +1940,7 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
         case STORE_F32: return launch_pt<STORE_F32>(mx, mw, mo, q, ctas, smem, s);
         case ACCUM_F32: return launch_pt<ACCUM_F32>(mx, mw, mo, q, ctas, smem, s);
         case SWIGLU_BF16:
-            if (q.act.kind || q.row_scale) return launch_pt<SWIGLU_BF16, true>(mx, mw, mo, q, ctas, smem, s);
+            if (q.act.kind) return launch_pt<SWIGLU_BF16, true>(mx, mw, mo, q, ctas, smem, s);
             return launch_pt<SWIGLU_BF16>(mx, mw, mo, q, ctas, smem, s);
         default: return launch_pt<QKV_ROPE_BF16>(mx, mw, mo, q, ctas, smem, s);
     }
@@ -1898,9 +1951,11 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
 // rows each, of which the first N (and, in SwiGLU mode, the N from up_row_offset on) meet the rows of their tiles.
 // Modes: 0 bf16 store (with the activation of ferris_gemm_set_activation), 1 fp32 store, 3 SwiGLU from two accumulators; with
 // row_scale (fp32 [rows]; mode 3, or mode 0 with an activation) the accumulators times the row's factor first.  A tile whose entry is negative is skipped.
+// tile_rows (int32 per tile, may be null): the rows of a tile that count, its first ones; rows from the next multiple of 32 on are
+// neither read nor written.
 FERRIS_API int ferris_gemm_grouped_tcgen05(const void* x, const void* w, void* out, int mode, int rows, int N, int K,
                                            int ldx, int ldw, int ldo, int experts, int expert_rows, int up_row_offset,
-                                           const int* tile_expert, const float* row_scale, void* stream) {
+                                           const int* tile_expert, const int* tile_rows, const float* row_scale, void* stream) {
     if (rows <= 0 || N <= 0) return FERRIS_OK;
     if (rows % PT_BLOCK_M) FERRIS_REFUSE("grouped gemm: %d rows are no multiple of %d", rows, PT_BLOCK_M);
     if (K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ldx < K || ldw < K)
@@ -1918,7 +1973,7 @@ FERRIS_API int ferris_gemm_grouped_tcgen05(const void* x, const void* w, void* o
     if (row_scale && mode != SWIGLU_BF16 && !(mode == STORE_BF16 && g_launch_act.kind))
         FERRIS_REFUSE("grouped gemm: a factor per row goes with an activation (mode %d)", mode);
     return run_tokens_m(x, w, nullptr, out, mode, rows, N, K, ldx, ldw, ldo, experts * expert_rows, up_row_offset, nullptr,
-                        (cudaStream_t)stream, tile_expert, expert_rows, row_scale);
+                        (cudaStream_t)stream, tile_expert, tile_rows, experts, expert_rows, row_scale);
 }
 
 static int gemm_tcgen05_impl(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,

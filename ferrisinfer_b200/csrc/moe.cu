@@ -701,11 +701,12 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) moe_down_few_kernel(const T* a
 
 // ------------------------------------------------------------------------------------------ expert-major: sort
 // One block.  pos[pair] = the row of pair (t, s) in the sorted order; row_token[row] = its token, or -1 for a row that
-// only fills a tile up; tile_expert[tile] = the expert of the tile's rows, or -1 beyond the last row.
+// only fills a tile up; tile_expert[tile] = the expert of the tile's rows, or -1 beyond the last row, tile_rows[tile] = how many of
+// its rows (the first ones) are pairs.
 constexpr int MOE_TILE = 128;
 // row_scale (may be null): the pair's weight at its row, 0 at the rows that only fill up.
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* ids, int* pos, int* row_token, int* tile_expert,
-                                                        int pairs, int top, int experts, int max_rows, int with_weights,
+                                                        int* tile_rows, int pairs, int top, int experts, int max_rows, int with_weights,
                                                         const float* weights, float* row_scale) {
     __shared__ int count[MOE_MAX_EXPERTS];
     __shared__ int first[MOE_MAX_EXPERTS + 1];
@@ -736,7 +737,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* ids, int* pos
     }
     for (int tile = threadIdx.x; tile < max_rows / MOE_TILE; tile += blockDim.x) {
         const int row = tile * MOE_TILE;
-        int e = -1;
+        int e = -1, held = 0;
         if (row < first[experts]) {
             int lo = 0, hi = experts - 1;  // the last expert whose first row is at or before this tile's
             while (lo < hi) {
@@ -744,8 +745,10 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* ids, int* pos
                 if (first[mid] <= row) lo = mid; else hi = mid - 1;
             }
             e = lo < with_weights ? lo : -1;  // the rows of identity experts meet no weights
+            held = min(MOE_TILE, first[lo] + count[lo] - row);
         }
         tile_expert[tile] = e;
+        tile_rows[tile] = held;
     }
 }
 
@@ -801,7 +804,7 @@ extern "C" void ferris_gemm_set_gated_activation(int kind, float limit);
 extern "C" void ferris_gemm_set_activation(int kind, float a, float b);
 extern "C" int ferris_gemm_grouped_tcgen05(const void* x, const void* w, void* out, int mode, int rows, int N, int K,
                                            int ldx, int ldw, int ldo, int experts, int expert_rows, int up_row_offset,
-                                           const int* tile_expert, const float* row_scale, void* stream);
+                                           const int* tile_expert, const int* tile_rows, const float* row_scale, void* stream);
 
 // Rows of the sorted order that `tokens` tokens choosing `top` of `experts` can need at most (whole tiles of 128).
 FERRIS_API int ferris_moe_sorted_rows(int tokens, int top, int experts) {
@@ -813,7 +816,7 @@ FERRIS_API int ferris_moe_sorted_rows(int tokens, int top, int experts) {
 // The experts of a long step in bf16.  x bf16 [tokens, width] rows ldx apart; gate_up bf16 [experts, 2 ff, width] (an
 // expert's gate rows, then its up rows); down bf16 [experts, width, ff]; ids, weights [tokens, top]; h fp32.
 // Scratch, all sized for rows = ferris_moe_sorted_rows(...): pos int32 [tokens x top], row_token int32 [rows],
-// tile_expert int32 [rows / 128], xs bf16 [rows, width], act bf16 [rows, ff], y fp32 [rows, width].
+// tile_expert int32 [2 x rows / 128] (the tiles' experts, then their counts of rows), xs bf16 [rows, width], act bf16 [rows, ff], y fp32 [rows, width].
 // identity_w (may be null): fp32 [tokens]; with it, ids may hold `experts` (an identity expert: the pair meets no weights)
 // and h also gets identity_w[t] x[t]; the scratch is then sized for experts + 1.  act_kind, act_limit: the gated
 // activation (ferris_gated_act).  row_scale: scratch, fp32 [rows], where the weights go onto the experts' inputs; else null.
@@ -833,7 +836,8 @@ FERRIS_API int ferris_moe_experts_grouped(const void* x, int ldx, const void* ga
     if (width % 8 || ff % 8 || ldx % 8 || ldh % 4 || (((uintptr_t)x | (uintptr_t)xs | (uintptr_t)y | (uintptr_t)h) & 15))
         FERRIS_REFUSE("experts: width %d, ff %d and the rows must be multiples of 8 elements and start on 16 bytes", width, ff);
     cudaStream_t s = (cudaStream_t)stream;
-    ferris_launch(moe_sort_kernel, dim3(1), dim3(1024), 0, s, ids, pos, row_token, tile_expert, tokens * top, top, sorted,
+    int* tile_rows = tile_expert + rows / MOE_TILE;
+    ferris_launch(moe_sort_kernel, dim3(1), dim3(1024), 0, s, ids, pos, row_token, tile_expert, tile_rows, tokens * top, top, sorted,
                   rows, experts, weights, row_scale);
     const size_t n16 = (size_t)rows * (width / 8);
     const size_t want = (n16 + 255) / 256;
@@ -842,16 +846,16 @@ FERRIS_API int ferris_moe_experts_grouped(const void* x, int ldx, const void* ga
     int rc;
     if (plain) {
         ferris_gemm_set_activation(act_kind, act_limit, 0.0f);  // taken by the product launched next
-        rc = ferris_gemm_grouped_tcgen05(xs, gate_up, act, 0, rows, ff, width, width, width, ff, experts, ff, 0, tile_expert, row_scale, stream);
+        rc = ferris_gemm_grouped_tcgen05(xs, gate_up, act, 0, rows, ff, width, width, width, ff, experts, ff, 0, tile_expert, tile_rows, row_scale, stream);
         ferris_gemm_set_activation(0, 0.0f, 0.0f);
     } else {
         ferris_gemm_set_gated_activation(act_kind, act_limit);
         rc = ferris_gemm_grouped_tcgen05(xs, gate_up, act, 3, rows, ff, width, width, width, ff, experts, 2 * ff, ff,
-                                         tile_expert, row_scale, stream);
+                                         tile_expert, tile_rows, row_scale, stream);
         ferris_gemm_set_gated_activation(0, 0.0f);
     }
     if (rc != FERRIS_OK) return rc;
-    rc = ferris_gemm_grouped_tcgen05(act, down, y, 1, rows, width, ff, ff, ff, width, experts, width, 0, tile_expert, nullptr, stream);
+    rc = ferris_gemm_grouped_tcgen05(act, down, y, 1, rows, width, ff, ff, ff, width, experts, width, 0, tile_expert, tile_rows, nullptr, stream);
     if (rc != FERRIS_OK || !h) return rc;  // without h the rows stay in y, for the caller to add
     const size_t n4 = (size_t)tokens * (width / 4);
     const size_t want4 = (n4 + 255) / 256;

@@ -1972,7 +1972,7 @@ def moe_experts(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, ids:
             raise KernelError(f"experts: {T} tokens x {top} choices are more than one launch takes")
         pos = get("moe_pos", (T * top,), torch.int32)
         row_token = get("moe_row_token", (rows,), torch.int32)
-        tile_expert = get("moe_tile_expert", (rows // 128,), torch.int32)
+        tile_expert = get("moe_tile_expert", (2 * (rows // 128),), torch.int32)  # experts, then counts of rows
         xs = get("moe_sorted_rows", (rows, W), x.dtype)
         act = get("moe_sorted_act", (rows, ff), x.dtype)
         y = get("moe_sorted_out", (rows, W), torch.float32)

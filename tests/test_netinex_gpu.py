@@ -439,6 +439,37 @@ def test_experts_give_a_token_the_same_bits_alone_and_among_others(device, W, ff
         assert torch.equal(alone[0], together[t]), t
 
 
+@pytest.mark.parametrize("ff", [72, 272, 2688])  # tile widths of the first product that end inside, at and behind its columns
+@pytest.mark.parametrize("counts", [(32, 33, 0, 128, 129, 1, 96, 97), (0, 0, 300, 0, 0, 0, 0, 31), (1, 0, 0, 0, 0, 0, 0, 0)])
+def test_sorted_experts_with_rows_at_the_edges_of_boxes(device, counts, ff):
+    """Rows of an expert that fill boxes of 32 and tiles of 128 exactly and by one more, experts without rows, also as the
+    last ones; scratch that holds NaN where no row is.  bf16: the products' rounding of the activations, 2^-8 of what enters
+    the second product, and of the weighted sum over ff of them."""
+    ops = _ops()
+    from ferrisinfer_b200.engine.workspace import Workspace
+
+    torch.manual_seed(ff)
+    E, W = len(counts), 136
+    gate_up = (torch.randn(E, 2 * ff, W) / math.sqrt(W)).to(device, BF16)
+    down = (torch.randn(E, W, ff) / math.sqrt(ff)).to(device, BF16)
+    of = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)])[torch.randperm(sum(counts))]
+    T = len(of)
+    x, weights, ids = torch.randn(T, W).to(device, BF16), torch.rand(T, 1, device=device) + 0.5, of.int().view(T, 1).to(device)
+    ws = Workspace(device)
+    for again in range(2):
+        h = torch.zeros(T, W, device=device)
+        ops.moe_experts(x, gate_up, down, ids, weights, h, ws, grouped=True)
+        both = torch.stack([gate_up[e].double() @ x[t].double() for t, e in enumerate(of.tolist())])
+        act = torch.nn.functional.silu(both[:, :ff]) * both[:, ff:]
+        each = torch.stack([down[e].double() @ act[t] for t, e in enumerate(of.tolist())])
+        size = torch.stack([down[e].double().abs() @ act[t].abs() for t, e in enumerate(of.tolist())])
+        assert ((h.double() - weights.double() * each).abs() <= 2.0 ** -8 * 1.1 * weights.double() * size + 1e-6).all()
+        for name, buf in ws._buffers.items():  # what no row writes is nobody's
+            if name[0] in ("moe_sorted_act", "moe_sorted_out"):
+                buf.fill_(float("nan"))
+    assert ops.kernel_status() == 0
+
+
 # ================================================================================================ whole models
 MODEL_CASES = sorted(cases.CASES)
 LENGTHS = {"long": (150, 11), "mid": (67, 12), "short": (23, 13), "one": (1, 14), "edge": (49, 15)}
