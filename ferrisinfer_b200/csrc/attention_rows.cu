@@ -723,7 +723,7 @@ FERRIS_API int ferris_attention_rows(const void* q, int ldq, void* out, int ldo,
     const ScoreTerms st = {slopes, log_r1, log_r2, sink, v_stride, softcap, gate, ldgate};
     const PooledKeys pk = keys_beside(pool_k, pool_v, pool_tables, pool_max_blocks, pool_every, keep, k_cache, v_cache, block_tables, max_blocks);
     if (int rc = check_pooled(pk, window, st)) return rc;
-    if ((log_r1 != nullptr) != (log_r2 != nullptr)) FERRIS_REFUSE("attention rows: half of a logarithmic penalty");
+    if ((log_r1 == nullptr) != (log_r2 == nullptr) || (slopes && log_r1)) FERRIS_REFUSE("attention rows: one kind of distance penalty, with all its numbers");
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)pool_k | (uintptr_t)pool_v) & 15) != 0 || ldq % 8 ||
         ((uintptr_t)out & 3) || (ldo & 1))
         FERRIS_REFUSE("attention rows: rows must start on 16 bytes");

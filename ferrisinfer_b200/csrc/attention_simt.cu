@@ -522,87 +522,93 @@ void launch_lanes(const void* q, int ldq, void* out, int ldo, const void* k_cach
 
 
 // ---------------------------------------------------------------------------------------------
-// Portions of prompts: a block takes up to TL_ROWS = 64 query rows that share their keys and values, namely the g query
-// heads of one kv head for floor(64 / g) consecutive tokens of the step (rows beyond those stay idle), and walks the keys those tokens see in tiles of 32, which
-// it brings into shared memory once for all 64 rows (fp32, a row's 16-byte pieces spread over the banks).  Eight
-// lanes share two rows: each forms 2 x 4 scores of a tile from shared memory, the eight exchange the rows' maxima
-// and sums by shuffles, write the weights to shared memory and add 2 x (dv / 8) columns of weighted values each.
-// Everything is fp32 FMAs: scores, weights and the sums over values.  Tokens of several requests in one tile are taken
-// request by request (the other rows masked), so any division of a step is served; a step of single tokens is the
+// Portions of prompts: a block takes up to ROWS = 32 query rows (64 where a kv head has more than 32 query heads) that share their
+// keys and values, namely the g query heads of one kv head for floor(ROWS / g) consecutive tokens of the step (rows beyond those stay
+// idle), and walks the keys those tokens see in tiles of 64, which it brings into shared memory once for all its rows (fp32, a row's
+// 16-byte pieces spread over the banks).  Sixteen lanes share four rows: each forms 4 x 4 scores of a tile from shared memory, the
+// sixteen exchange the rows' maxima and sums by shuffles, write the weights to shared memory and add 4 x (dv / 16) columns of
+// weighted values each.  Everything is fp32 FMAs: scores, weights and the sums over values.  Tokens of several requests in one tile
+// are taken request by request (the other rows masked), so any division of a step is served; a step of single tokens is the
 // kernel above's.
+// Bound by what shared memory returns to the lanes: 16 bytes a lane take four cycles of an SM a warp, and eight FMAs go with each.
+// Four blocks share an SM, so that the rows of one come in while others compute; blocks with the most keys begin first.
+// A prompt of 777 tokens, 14 heads of 64 over 2, fp32: 110 us, 137 with the head size known at run time only (the instructions),
+// 193 with blocks of 64 rows, tiles of 32 keys and two rows a lane.
 // ---------------------------------------------------------------------------------------------
-constexpr int TL_ROWS = 64, TL_KEYS = 32, TL_THREADS = 256;
+constexpr int TL_KEYS = 64;
 
-__device__ __forceinline__ void stage_row(const float* src, float* dst, int n, int part, int parts, float mul) {
-    for (int v = part; v * 4 < n; v += parts) {
-        float4 u = *reinterpret_cast<const float4*>(src + v * 4);
-        u.x *= mul, u.y *= mul, u.z *= mul, u.w *= mul;
-        *reinterpret_cast<float4*>(dst + v * 4) = u;
-    }
+// A row's n numbers (a multiple of 16 bytes), by the sixteen lanes that share it: asynchronously where nothing is converted.
+__device__ __forceinline__ void stage_row(const float* src, float* dst, int n, int sub) {
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int v = sub; v * 4 < n; v += 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + v * 16), "l"(src + v * 4) : "memory");
 }
-__device__ __forceinline__ void stage_row(const bf16* src, float* dst, int n, int part, int parts, float mul) {
-    for (int v = part; v * 8 < n; v += parts) {
+__device__ __forceinline__ void stage_row(const bf16* src, float* dst, int n, int sub) {
+    for (int v = sub; v * 8 < n; v += 16) {
         const uint4 u = *reinterpret_cast<const uint4*>(src + v * 8);
-        *reinterpret_cast<float4*>(dst + v * 8) = make_float4(bf16_lo(u.x) * mul, bf16_hi(u.x) * mul, bf16_lo(u.y) * mul, bf16_hi(u.y) * mul);
-        *reinterpret_cast<float4*>(dst + v * 8 + 4) = make_float4(bf16_lo(u.z) * mul, bf16_hi(u.z) * mul, bf16_lo(u.w) * mul, bf16_hi(u.w) * mul);
+        *reinterpret_cast<float4*>(dst + v * 8) = make_float4(bf16_lo(u.x), bf16_hi(u.x), bf16_lo(u.y), bf16_hi(u.y));
+        *reinterpret_cast<float4*>(dst + v * 8 + 4) = make_float4(bf16_lo(u.z), bf16_hi(u.z), bf16_lo(u.w), bf16_hi(u.w));
     }
 }
-__device__ __forceinline__ void zero_row(float* dst, int n, int part, int parts) {
-    for (int v = part; v * 4 < n; v += parts) *reinterpret_cast<float4*>(dst + v * 4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+__device__ __forceinline__ void zero_row(float* dst, int n, int sub) {
+    for (int v = sub; v * 4 < n; v += 16) *reinterpret_cast<float4*>(dst + v * 4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-template <typename T, int NC, bool POOL>  // NC: 4-column pieces of the value head that a lane adds up: dv <= 32 * NC
-__global__ void __launch_bounds__(TL_THREADS)
+// NC: 4-column pieces of the value head that a lane adds up: dv <= 64 * NC.  DF: the head size (keys' and values') where it is known
+// to the compiler, which halves the instructions; 0: any.
+template <typename T, int ROWS, int NC, bool POOL, int DF>
+__global__ void __launch_bounds__(ROWS * 4, ROWS == 32 && NC == 1 ? 4 : 1)
     paged_attention_tiled_kernel(const T* q, int ldq, T* __restrict__ out, int ldo, const T* k_cache, const T* v_cache,
                                  const int* __restrict__ block_tables, int max_blocks,
                                  const int* __restrict__ token_seq, const int* __restrict__ positions, int tokens, int nh,
-                                 int nkv, int d, int dv, int page_size, int window, float scale,
+                                 int nkv, int d_any, int dv_any, int page_size, int window, float scale,
                                  const ScoreTerms st, const PooledKeys pk) {
+    const int d = DF ? DF : d_any, dv = DF ? DF : dv_any;
+    constexpr int THREADS = ROWS * 4, P_PITCH = ROWS + 4;
     extern __shared__ __align__(16) float tl_smem[];
+    __shared__ int key_row[TL_KEYS];  // the tile's keys' rows in the cache, -1: none
     const int dp = d + 4, dvp = dv + 4;
-    float* Qs = tl_smem;                      // [64][d + 4], scaled
-    float* Ks = Qs + TL_ROWS * dp;            // [32][d + 4]
-    float* Vs = Ks + TL_KEYS * dp;            // [32][dv + 4]
-    float* Ps = Vs + TL_KEYS * dvp;           // [64][32 + 1]
+    float* Qs = tl_smem;                      // [ROWS][d + 4]
+    float* Ks = Qs + ROWS * dp;               // [64][d + 4]
+    float* Vs = Ks + TL_KEYS * dp;            // [64][dv + 4]
+    float* Ps = Vs + TL_KEYS * dvp;           // [64][ROWS + 4]: a key's weights for the rows
     pdl_wait();
     pdl_launch_dependents();
     const int tid = threadIdx.x;
-    const int g = nh / nkv, qt = TL_ROWS / g;
+    const int g = nh / nkv, qt = ROWS / g;
     const int hk = blockIdx.y;
-    const int t_first = blockIdx.x * qt;
+    const int t_first = (gridDim.x - 1 - blockIdx.x) * qt;  // the last tokens, which see most keys, first
     const int t_end = min(t_first + qt, tokens);
     const int pshift = (page_size & (page_size - 1)) == 0 ? __ffs(page_size) - 1 : -1;
+    const int ry = tid >> 4, kx = tid & 15;
+    const int r0 = 4 * ry;  // this lane's rows: r0 .. r0 + 3
 
-    // the queries, scaled once
-    {
-        const int row = tid >> 2, part = tid & 3;
-        const int t = t_first + row / g;
-        float* dst = Qs + row * dp;
+    for (int row = ry; row < ROWS; row += THREADS / 16) {
+        const int t = row < qt * g ? t_first + row / g : tokens;
         if (t < t_end)
-            stage_row(q + (size_t)t * ldq + (size_t)(hk * g + row % g) * d, dst, d, part, 4, scale);
+            stage_row(q + (size_t)t * ldq + (size_t)(hk * g + row % g) * d, Qs + row * dp, d, kx);
         else
-            zero_row(dst, d, part, 4);
+            zero_row(Qs + row * dp, d, kx);
     }
-    const int ry = tid >> 3, kx = tid & 7;
-    const int r0 = 2 * ry;  // this lane's rows: r0 and r0 + 1
-    int rt[2], rpos[2], rseq[2];
-    HeadTerms rterm[2];
+    int rt[4], rpos[4], rseq[4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
-        rt[a] = t_first + (r0 + a) / g;
+    for (int a = 0; a < 4; ++a) {
+        rt[a] = r0 + a < qt * g ? t_first + (r0 + a) / g : tokens;
         const bool ok = rt[a] < t_end;
         rpos[a] = ok ? positions[rt[a]] : -1;
         rseq[a] = ok ? token_seq[rt[a]] : -1;
-        rterm[a] = head_terms(st, hk * g + (r0 + a) % g);
     }
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
-    float acc[2][NC][4];
+    const bool terms = st.slopes || st.log_r1 || st.softcap > 0.0f;
+    float m[4], l[4];
+    float acc[4][NC][4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < 4; ++a) {
+        m[a] = -INFINITY, l[a] = 0.0f;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[a][c][e] = 0.0f;
+    }
 
     const int seq_first = token_seq[t_first], seq_last = token_seq[t_end - 1];
     int ta = t_first;  // first token of the current request within the tile
@@ -620,90 +626,105 @@ __global__ void __launch_bounds__(TL_THREADS)
         const T* keys = runs ? reinterpret_cast<const T*>(pk.k) : k_cache;
         const T* vals = runs ? reinterpret_cast<const T*>(pk.v) : v_cache;
         for (int j0 = kmin & ~(TL_KEYS - 1); j0 <= kmax; j0 += TL_KEYS) {
-            __syncthreads();  // the tile before has been used (and, the first time, the queries are in place)
-            {
-                const int key = tid >> 3, part = tid & 7;
-                const int j = j0 + key;
+            __syncthreads();  // the tile before has been used
+            if (tid < TL_KEYS) {
+                const int j = j0 + tid;
                 int page = -1;
                 if (j >= kmin && j <= kmax) page = table[pshift >= 0 ? (j >> pshift) : (j / page_size)];
-                if (page >= 0) {
-                    const int in_page = pshift >= 0 ? (j & (page_size - 1)) : (j % page_size);
-                    const size_t row = ((size_t)page * nkv + hk) * page_size + in_page;
-                    stage_row(keys + row * d, Ks + key * dp, d, part, 8, 1.0f);
-                    stage_row(vals + row * (st.v_stride ? (size_t)st.v_stride : (size_t)dv), Vs + key * dvp, dv, part, 8, 1.0f);
-                } else {
-                    zero_row(Ks + key * dp, d, part, 8);
-                    zero_row(Vs + key * dvp, dv, part, 8);
-                }
+                const int in_page = pshift >= 0 ? (j & (page_size - 1)) : (j % page_size);
+                key_row[tid] = page >= 0 ? (page * nkv + hk) * page_size + in_page : -1;
             }
             __syncthreads();
-            // 2 x 4 scores: rows r0, r0 + 1 against keys kx, kx + 8, kx + 16, kx + 24
-            float sc[2][4];
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) sc[a][c] = 0.0f;
-            const float* q0 = Qs + r0 * dp;
-            const float* kb = Ks + kx * dp;
-            for (int x = 0; x < d; x += 4) {
-                const float4 qa = *reinterpret_cast<const float4*>(q0 + x);
-                const float4 qb = *reinterpret_cast<const float4*>(q0 + dp + x);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float4 kv = *reinterpret_cast<const float4*>(kb + (size_t)(8 * c) * dp + x);
-                    sc[0][c] = fmaf(qa.x, kv.x, fmaf(qa.y, kv.y, fmaf(qa.z, kv.z, fmaf(qa.w, kv.w, sc[0][c]))));
-                    sc[1][c] = fmaf(qb.x, kv.x, fmaf(qb.y, kv.y, fmaf(qb.z, kv.z, fmaf(qb.w, kv.w, sc[1][c]))));
+#pragma unroll 4
+            for (int key = ry; key < TL_KEYS; key += THREADS / 16) {
+                const int row = key_row[key];
+                if (row >= 0) {
+                    stage_row(keys + (size_t)row * d, Ks + key * dp, d, kx);
+                    stage_row(vals + (size_t)row * (st.v_stride ? st.v_stride : dv), Vs + key * dvp, dv, kx);
+                } else {
+                    zero_row(Ks + key * dp, d, kx);
+                    zero_row(Vs + key * dvp, dv, kx);
                 }
             }
-            // the rows' maxima and sums over the tile, among the eight lanes that share the rows
-            float alpha[2];
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            // 4 x 4 scores: rows r0 .. r0 + 3 against keys kx, kx + 16, kx + 32, kx + 48
+            float sc[4][4];
 #pragma unroll
-            for (int a = 0; a < 2; ++a) {
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) sc[a][c] = 0.0f;
+            const float* qb = Qs + r0 * dp;
+            const float* kb = Ks + kx * dp;
+#pragma unroll(DF ? 4 : 2)
+            for (int x = 0; x < d; x += 4) {
+                float4 qv[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) qv[a] = *reinterpret_cast<const float4*>(qb + a * dp + x);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float4 kv = *reinterpret_cast<const float4*>(kb + (size_t)(16 * c) * dp + x);
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+                        sc[a][c] = fmaf(qv[a].x, kv.x, fmaf(qv[a].y, kv.y, fmaf(qv[a].z, kv.z, fmaf(qv[a].w, kv.w, sc[a][c]))));
+                }
+            }
+            // the rows' maxima and sums over the tile, among the sixteen lanes that share the rows
+            float alpha[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
                 int lo = first_key(rpos[a], window), hi = rpos[a];
                 if (runs) hi = ahead_rows(pk, lo) - 1, lo = 0;
+                if (rseq[a] != sq) hi = -1;
                 float best = -INFINITY;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const int j = j0 + kx + 8 * c;
-                    const bool seen = rseq[a] == sq && j >= lo && j <= hi;
-                    sc[a][c] = seen ? with_terms(sc[a][c], rterm[a], j, rpos[a]) : -INFINITY;
+                    const int j = j0 + kx + 16 * c;
+                    const bool seen = j >= lo && j <= hi;
+                    float s = sc[a][c] * scale;
+                    if (terms && seen) s = with_terms(s, head_terms(st, hk * g + (r0 + a) % g), j, rpos[a]);
+                    sc[a][c] = seen ? s : -INFINITY;
                     best = fmaxf(best, sc[a][c]);
                 }
 #pragma unroll
-                for (int o = 4; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+                for (int o = 8; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
                 const float m_new = fmaxf(m[a], best);
                 alpha[a] = (m_new == -INFINITY || m[a] == m_new) ? 1.0f : expf(m[a] - m_new);  // exp(-inf) = 0 at a row's first keys
                 float sum = 0.0f;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const float pw = sc[a][c] == -INFINITY ? 0.0f : expf(sc[a][c] - m_new);
-                    Ps[(r0 + a) * (TL_KEYS + 1) + kx + 8 * c] = pw;
-                    sum += pw;
+                    sc[a][c] = sc[a][c] == -INFINITY ? 0.0f : expf(sc[a][c] - m_new);
+                    sum += sc[a][c];
                 }
 #pragma unroll
-                for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
                 l[a] = l[a] * alpha[a] + sum;
                 m[a] = m_new;
             }
-            __syncwarp();  // a row's weights are written and read by the same eight lanes
 #pragma unroll
-            for (int a = 0; a < 2; ++a)
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<float4*>(Ps + (kx + 16 * c) * P_PITCH + r0) = make_float4(sc[0][c], sc[1][c], sc[2][c], sc[3][c]);
+            __syncwarp();  // a row's weights are written and read by the same sixteen lanes
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[a][c][e] *= alpha[a];
-            const float* p0 = Ps + r0 * (TL_KEYS + 1);
+#pragma unroll(DF ? 8 : 4)
             for (int kj = 0; kj < TL_KEYS; ++kj) {
-                const float pa0 = p0[kj], pa1 = p0[TL_KEYS + 1 + kj];
+                const float4 w = *reinterpret_cast<const float4*>(Ps + kj * P_PITCH + r0);
+                const float wa[4] = {w.x, w.y, w.z, w.w};
                 const float* vrow = Vs + kj * dvp + kx * 4;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    if (kx * 4 + 32 * c < dv) {
-                        const float4 vv = *reinterpret_cast<const float4*>(vrow + 32 * c);
-                        acc[0][c][0] = fmaf(pa0, vv.x, acc[0][c][0]), acc[0][c][1] = fmaf(pa0, vv.y, acc[0][c][1]);
-                        acc[0][c][2] = fmaf(pa0, vv.z, acc[0][c][2]), acc[0][c][3] = fmaf(pa0, vv.w, acc[0][c][3]);
-                        acc[1][c][0] = fmaf(pa1, vv.x, acc[1][c][0]), acc[1][c][1] = fmaf(pa1, vv.y, acc[1][c][1]);
-                        acc[1][c][2] = fmaf(pa1, vv.z, acc[1][c][2]), acc[1][c][3] = fmaf(pa1, vv.w, acc[1][c][3]);
+                    if (DF || kx * 4 + 64 * c < dv) {
+                        const float4 vv = *reinterpret_cast<const float4*>(vrow + 64 * c);
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) {
+                            acc[a][c][0] = fmaf(wa[a], vv.x, acc[a][c][0]), acc[a][c][1] = fmaf(wa[a], vv.y, acc[a][c][1]);
+                            acc[a][c][2] = fmaf(wa[a], vv.z, acc[a][c][2]), acc[a][c][3] = fmaf(wa[a], vv.w, acc[a][c][3]);
+                        }
                     }
                 }
             }
@@ -712,13 +733,14 @@ __global__ void __launch_bounds__(TL_THREADS)
         ta = tb + 1;
     }
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < 4; ++a) {
         if (rt[a] >= t_end) continue;
-        const float inv = head_gate<T>(st, rt[a], hk * g + (r0 + a) % g) / (l[a] + sink_share(st, hk * g + (r0 + a) % g, m[a]));
-        T* orow = out + (size_t)rt[a] * ldo + (size_t)(hk * g + (r0 + a) % g) * dv;
+        const int head = hk * g + (r0 + a) % g;
+        const float inv = head_gate<T>(st, rt[a], head) / (l[a] + sink_share(st, head, m[a]));
+        T* orow = out + (size_t)rt[a] * ldo + (size_t)head * dv;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const int col = kx * 4 + 32 * c;
+            const int col = kx * 4 + 64 * c;
             if (col < dv) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) orow[col + e] = from_float<T>(acc[a][c][e] * inv);
@@ -727,15 +749,52 @@ __global__ void __launch_bounds__(TL_THREADS)
     }
 }
 
-size_t tiled_smem_bytes(int d, int dv) {
-    return ((size_t)(TL_ROWS + TL_KEYS) * (d + 4) + (size_t)TL_KEYS * (dv + 4) + (size_t)TL_ROWS * (TL_KEYS + 1)) * sizeof(float);
+size_t tiled_smem_bytes(int rows, int d, int dv) {
+    return ((size_t)(rows + TL_KEYS) * (d + 4) + (size_t)TL_KEYS * (dv + 4) + (size_t)TL_KEYS * (rows + 4)) * sizeof(float);
 }
+int tiled_rows(int g) { return g <= 32 ? 32 : 64; }
 
 bool tiled_takes(int dtype, int nh, int nkv, int d, int dv) {
     const int g = nkv > 0 ? nh / nkv : 0;
     const int unit = dtype == FERRIS_F32 ? 4 : 8;  // elements of a 16-byte piece
-    return g >= 1 && g <= TL_ROWS && nh % nkv == 0 && d % unit == 0 && dv % unit == 0 && d <= 256 &&
-           dv <= 256 && tiled_smem_bytes(d, dv) <= 200 * 1024;
+    return g >= 1 && g <= 64 && nh % nkv == 0 && d % unit == 0 && dv % unit == 0 && d <= 256 &&
+           dv <= 256 && tiled_smem_bytes(tiled_rows(g), d, dv) <= 226 * 1024;
+}
+
+template <typename T, int ROWS, bool POOL>
+int launch_tiled_rows(const void* q, int ldq, void* out, int ldo, const void* k_cache, const void* v_cache,
+                      const int* block_tables, int max_blocks, const int* token_seq, const int* positions, int tokens, int nh,
+                      int nkv, int d, int dv, int page_size, int window, float scale, const ScoreTerms st, const PooledKeys pk,
+                      cudaStream_t s) {
+    const int qt = ROWS / (nh / nkv);
+    const dim3 grid((tokens + qt - 1) / qt, nkv), block(ROWS * 4);
+    const size_t smem = tiled_smem_bytes(ROWS, d, dv);
+#define FERRIS_TL_LAUNCH(NC, DF)                                                                                    \
+    do {                                                                                                            \
+        int e_ = ferris_allow_dynamic_smem((const void*)paged_attention_tiled_kernel<T, ROWS, NC, POOL, DF>, smem);       \
+        if (e_ != FERRIS_OK) return e_;                                                                             \
+        ferris_launch(paged_attention_tiled_kernel<T, ROWS, NC, POOL, DF>, grid, block, smem, s, (const T*)q, ldq, (T*)out, ldo, \
+                      (const T*)k_cache, (const T*)v_cache, block_tables, max_blocks, token_seq, positions, tokens, \
+                      nh, nkv, d, dv, page_size, window, scale, st, pk);                                       \
+    } while (0)
+    if constexpr (ROWS == 32 && !POOL && sizeof(T) == 4) {
+        if (d == 64 && dv == 64) {
+            FERRIS_TL_LAUNCH(1, 64);
+            FERRIS_LAUNCH_CHECK();
+        }
+        if (d == 128 && dv == 128) {
+            FERRIS_TL_LAUNCH(2, 128);
+            FERRIS_LAUNCH_CHECK();
+        }
+    }
+    if (dv <= 64)
+        FERRIS_TL_LAUNCH(1, 0);
+    else if (dv <= 128)
+        FERRIS_TL_LAUNCH(2, 0);
+    else
+        FERRIS_TL_LAUNCH(4, 0);
+#undef FERRIS_TL_LAUNCH
+    FERRIS_LAUNCH_CHECK();
 }
 
 template <typename T, bool POOL>
@@ -743,25 +802,9 @@ int launch_tiled(const void* q, int ldq, void* out, int ldo, const void* k_cache
                  const int* block_tables, int max_blocks, const int* token_seq, const int* positions, int tokens, int nh,
                  int nkv, int d, int dv, int page_size, int window, float scale, const ScoreTerms st, const PooledKeys pk,
                  cudaStream_t s) {
-    const int qt = TL_ROWS / (nh / nkv);
-    const dim3 grid((tokens + qt - 1) / qt, nkv), block(TL_THREADS);
-    const size_t smem = tiled_smem_bytes(d, dv);
-#define FERRIS_TL_LAUNCH(NC)                                                                                        \
-    do {                                                                                                            \
-        int e_ = ferris_allow_dynamic_smem((const void*)paged_attention_tiled_kernel<T, NC, POOL>, smem);                 \
-        if (e_ != FERRIS_OK) return e_;                                                                             \
-        ferris_launch(paged_attention_tiled_kernel<T, NC, POOL>, grid, block, smem, s, (const T*)q, ldq, (T*)out, ldo,   \
-                      (const T*)k_cache, (const T*)v_cache, block_tables, max_blocks, token_seq, positions, tokens, \
-                      nh, nkv, d, dv, page_size, window, scale, st, pk);                                       \
-    } while (0)
-    if (dv <= 64)
-        FERRIS_TL_LAUNCH(2);
-    else if (dv <= 128)
-        FERRIS_TL_LAUNCH(4);
-    else
-        FERRIS_TL_LAUNCH(8);
-#undef FERRIS_TL_LAUNCH
-    FERRIS_LAUNCH_CHECK();
+    auto* launch = tiled_rows(nh / nkv) == 32 ? launch_tiled_rows<T, 32, POOL> : launch_tiled_rows<T, 64, POOL>;
+    return launch(q, ldq, out, ldo, k_cache, v_cache, block_tables, max_blocks, token_seq, positions, tokens, nh, nkv, d, dv,
+                  page_size, window, scale, st, pk, s);
 }
 
 }  // namespace

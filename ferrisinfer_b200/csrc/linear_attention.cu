@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const float* o, int 
 
 // The same for bf16 rows of up to GN_THREADS x 8 x GN_CHUNKS columns that begin on 16 bytes: eight columns a thread at a time, with wide
 // loads all requested at once and kept in registers, so that a row is read once.  Bound by memory (8 bytes a column).  Rows of 512
-// columns and more: below, most of the threads would be idle.  2,048 rows of 2,048 columns 20 -> 10 us by the whole step's time
+// columns and more: below, most of the threads would be idle.  2,048 rows of 2,048 columns 20 -> 14 us by the whole step's time
 // (eight of them in 4.68 -> 4.63 ms).
 constexpr int GN_THREADS = 256, GN_CHUNKS = 2;
 __global__ void __launch_bounds__(GN_THREADS) gated_rmsnorm_vec_kernel(const float* o, int ldi, const bf16* g, int ldg,

@@ -460,9 +460,10 @@ def test_unit_norm_temperature_slopes_window_attention(device, nh, nkv, d, dv, w
 
 
 @pytest.mark.parametrize("kind", ["linear", "logarithmic"])
-@pytest.mark.parametrize("nh,nkv,d,dv", [(4, 1, 128, 128), (7, 1, 64, 64), (3, 3, 40, 24), (20, 2, 96, 200), (2, 1, 256, 256)])
-def test_distance_penalties_on_tensor_cores(device, nh, nkv, d, dv, kind):
-    """bf16 attention with a distance penalty: two requests' portions, and single tokens in one share and in several, with
+@pytest.mark.parametrize("nh,nkv,d,dv", [(4, 1, 128, 128), (7, 1, 64, 64), (3, 3, 40, 24), (20, 2, 96, 200), (2, 1, 256, 256), (40, 1, 64, 64)])
+@pytest.mark.parametrize("dtype", [BF16, F32])
+def test_distance_penalties_over_tiles_of_keys(device, nh, nkv, d, dv, kind, dtype):
+    """Attention with a distance penalty (bf16 on tensor cores, fp32 on CUDA cores): two requests' portions, and single tokens in one share and in several, with
     every key, a window, a chunk, a window with kept tokens; tiles of 64 keys end inside, at and after what a token sees.
     Against 64 bits: the output's own rounding (a bf16 has eight bits: up to 2^-8 of it), and scores of up to 2^7 that an fp32 sum leaves 2^-17 off."""
     ops = _ops()
@@ -474,9 +475,9 @@ def test_distance_penalties_on_tensor_cores(device, nh, nkv, d, dv, kind):
     order = torch.randperm(sum(blocks))
     table = torch.full((2, max(blocks)), -1, dtype=torch.int32)
     table[0, :blocks[0]], table[1, :blocks[1]] = order[:blocks[0]].int(), order[blocks[0]:].int()
-    k = torch.randn(sum(blocks), nkv, ps, d).to(BF16)
-    v = torch.randn(sum(blocks), nkv, ps, dv).to(BF16)
-    q = torch.randn(sum(lengths), nh * d).to(BF16)
+    k = torch.randn(sum(blocks), nkv, ps, d).to(dtype)
+    v = torch.randn(sum(blocks), nkv, ps, dv).to(dtype)
+    q = torch.randn(sum(lengths), nh * d).to(dtype)
     a, b = 0.02 + torch.rand(nh), 0.1 + torch.rand(nh)
     a[0] = 0.0
     terms = ops.ScoreTerms(slopes=a.to(device)) if kind == "linear" else ops.ScoreTerms(log_r1=a.to(device), log_r2=b.to(device))
@@ -500,10 +501,10 @@ def test_distance_penalties_on_tensor_cores(device, nh, nkv, d, dv, kind):
             s = torch.einsum("thd,shd->hts", q[at:at + n].double().view(n, nh, d), keys[:, of]) * scale - pen
             wgt = torch.softmax(s.masked_fill(~seen, -math.inf), -1)
             want[at:at + n] = torch.einsum("hts,shv->thv", wgt, values[:, of])
-        bound = 2.0 ** -8 * want.abs() + 2.0 ** -14 * vd.abs().max().item()
+        bound = (2.0 ** -8 * want.abs() if dtype == BF16 else 0.0) + 2.0 ** -14 * vd.abs().max().item()
         for form in ("portions", "single", "shares"):
             ctx = fake_ctx(device, lengths, starts, [0, 1])
-            out = torch.empty(sum(lengths), nh * dv, dtype=BF16, device=device)
+            out = torch.empty(sum(lengths), nh * dv, dtype=dtype, device=device)
             extra = dict(max_kv_len=max(p + n for p, n in zip(starts, lengths)), workspace=Workspace(device)) if form == "shares" else {}
             ops.paged_attention_simt(q.to(device), out, kd, vd, td, ctx.token_seq, ctx.positions, nh, nkv, d, window, scale,
                                      score_slopes=terms, v_head_dim=dv, max_q_len=max(lengths) if form == "portions" else 1,
