@@ -15,6 +15,9 @@
 // one 64 x 64 tile kernel for all sizes, 250 on the average product of a step of four): 1152 x 896 3.4 / 4.2 / 5.8, 896 x 896
 // 3.4 / 4.1 / 5.7, 9728 x 896 12.3 / 15.7 / 22.9, 896 x 4864 10.1 / 10.6 / 19.8, 151936 x 896 98 / 142 / 203 (5.5 TB/s at one).
 // Two or four weight rows a lane (a ring twice as large and one CTA an SM): 17 / 22 / 28 at 9728 x 896.
+// SwiGLU rides in it: a CTA takes the gate rows and the up rows of its outputs, eight by eight in turn (four requests
+// of 96 + 24 tokens at the 0.5B sizes 44.0 -> 40.4 ms; the RMSNorm formed in every CTA as well: 42.5, what its launch cost the wait for
+// the rows took twice).
 //
 // gemm_f32_tile_kernel: prompts.  Bound by the FMA pipes and, as closely, by what shared memory returns to the lanes (16
 // bytes a lane take four cycles of an SM a warp, whether lanes share them or not).  64 x 64 tiles, k-slices of 32 through a
@@ -48,6 +51,7 @@ struct RowsParams {
     int M, N, K, ldx, ldw, ldo, accumulate;
     int rows_per_cta, phases, stages;  // stages: a multiple of ROWS_WARPS, so that one warp takes a stage every time
     int* status;
+    int up_offset;  // > 0: SwiGLU, out[t, n] of gate row n and up row up_offset + n; N outputs of 2 N weight rows
 };
 
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -78,9 +82,13 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const RowsP
     const int xp = runs * X_PITCH;
     float* part = xs + TT * xp;  // [run][row of the CTA][token]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n0 = blockIdx.x * p.rows_per_cta, m0 = blockIdx.y * TT;
-    const int rows = min(p.rows_per_cta, p.N - n0), mt = min(TT, p.M - m0);
-    const int groups = (rows + RS - 1) / RS;
+    const bool pairs = p.up_offset > 0;  // groups of eight weight rows: gate, up, gate, up, ...
+    const int outs_per_cta = pairs ? p.rows_per_cta / 2 : p.rows_per_cta;
+    const int n0 = blockIdx.x * outs_per_cta, m0 = blockIdx.y * TT;
+    const int outs = min(outs_per_cta, p.N - n0), mt = min(TT, p.M - m0);
+    const int groups = (outs + RS - 1) / RS * (pairs ? 2 : 1);
+    auto group_outs = [&](int g) { return min(RS, outs - (pairs ? g >> 1 : g) * RS); };
+    auto group_row = [&](int g) { return n0 + (pairs ? (g & 1) * p.up_offset + (g >> 1) * RS : g * RS); };
     const int rowsp = p.rows_per_cta;
     if (tid == 0) {
         for (int i = 0; i < p.stages; ++i) {
@@ -97,12 +105,12 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const RowsP
             const int s = it % p.stages, round = it / p.stages;
             const int g = it / p.phases, k0 = (it % p.phases) * PHASE;
             if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, p.status, 0x60)) break;
-            const int nr = min(RS, rows - g * RS);
+            const int nr = group_outs(g);
             const uint32_t bytes = 4u * min(PHASE, p.K - k0);
             if (lane == 0) mbar_expect_tx(&full[s], bytes * nr);
             __syncwarp();
             if (lane < nr)
-                bulk_load(ring + s * stage_floats + lane * W_PITCH, p.w + (size_t)(n0 + g * RS + lane) * p.ldw + k0, bytes,
+                bulk_load(ring + s * stage_floats + lane * W_PITCH, p.w + (size_t)(group_row(g) + lane) * p.ldw + k0, bytes,
                           &full[s]);
         }
         return;
@@ -144,18 +152,14 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const RowsP
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
         const int row = g * RS + r;
-        if (len > 0 && row < rows) {
+        if (len > 0 && r < group_outs(g)) {
 #pragma unroll
             for (int t = 0; t < TT; ++t) part[((size_t)run * rowsp + row) * TT + t] = acc[t].x + acc[t].y;
         }
     }
     asm volatile("bar.sync 1, %0;" ::"n"(ROWS_WARPS * 32) : "memory");
     const int per = f32_runs_per_part(runs);
-    for (int i = tid; i < rows * mt; i += ROWS_WARPS * 32) {
-        const int row = i % rows, t = i / rows;
-        const int n = n0 + row;
-        float* o = p.out + (size_t)(m0 + t) * p.ldo + n;
-        const float old = p.accumulate ? *o : 0.0f;
+    auto total_of = [&](int row, int t) {
         float total = 0.0f;
         for (int c0 = 0; c0 < runs; c0 += per) {
             float sum = 0.0f;
@@ -163,6 +167,21 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const RowsP
             for (int c = c0; c < c1; ++c) sum += part[((size_t)c * rowsp + row) * TT + t];
             total += sum;
         }
+        return total;
+    };
+    for (int i = tid; i < outs * mt; i += ROWS_WARPS * 32) {
+        const int row = i % outs, t = i / outs;
+        const int n = n0 + row;
+        float* o = p.out + (size_t)(m0 + t) * p.ldo + n;
+        if (pairs) {
+            const int at = row / RS * 2 * RS + row % RS;
+            const float g = total_of(at, t), u = total_of(at + RS, t);
+            const float sg = g * (1.0f / (1.0f + expf(-g)));
+            *o = u * sg;
+            continue;
+        }
+        const float old = p.accumulate ? *o : 0.0f;
+        float total = total_of(row, t);
         if (p.bias) total += p.bias[n];
         *o = p.accumulate ? old + total : total;
     }
@@ -298,9 +317,21 @@ __global__ void __launch_bounds__(BM * BN / (TM * TN), 3) gemm_f32_tile_kernel(c
 template <int TT>
 int launch_rows(RowsParams& p, size_t smem, cudaStream_t s) {
     if (int rc = ferris_allow_dynamic_smem((const void*)gemm_f32_rows_kernel<TT>, smem)) return rc;
-    dim3 grid((p.N + p.rows_per_cta - 1) / p.rows_per_cta, (p.M + TT - 1) / TT);
+    const int outs = p.up_offset > 0 ? p.rows_per_cta / 2 : p.rows_per_cta;
+    dim3 grid((p.N + outs - 1) / outs, (p.M + TT - 1) / TT);
     ferris_launch(gemm_f32_rows_kernel<TT>, grid, dim3(ROWS_THREADS), smem, s, p);
     FERRIS_LAUNCH_CHECK();
+}
+
+struct RowsPlan {
+    int TT, rows_per_cta, phases, stages;
+    size_t smem;
+};
+int launch_rows_of(RowsParams& p, const RowsPlan& q, cudaStream_t s) {
+    if (q.TT == 8) return launch_rows<8>(p, q.smem, s);
+    if (q.TT == 4) return launch_rows<4>(p, q.smem, s);
+    if (q.TT == 2) return launch_rows<2>(p, q.smem, s);
+    return launch_rows<1>(p, q.smem, s);
 }
 
 int launch_tile(TileParams& p, dim3 grid, cudaStream_t s) {
@@ -316,18 +347,13 @@ int launch_tile(TileParams& p, dim3 grid, cudaStream_t s) {
 constexpr size_t MAX_SMEM = 227 * 1024;
 constexpr int TILE_SPLIT = 2 * 148;  // fewer tiles than two an SM: the parts of K side by side
 
-struct RowsPlan {
-    int TT, rows_per_cta, phases, stages;
-    size_t smem;
-};
-
-// How few tokens are cut; false: they do not fit.
-bool rows_plan(int M, int N, int K, RowsPlan& q) {
+// How few tokens are cut (N weight rows; unit: a CTA's are a multiple of so many); false: they do not fit.
+bool rows_plan(int M, int N, int K, int unit, RowsPlan& q) {
     const int runs = (K + F32_CHUNK - 1) / F32_CHUNK;
     q.phases = (K + PHASE - 1) / PHASE;
     for (int tt = M >= 5 ? 8 : M >= 3 ? 4 : M; tt >= 1; tt /= 2) {
         q.TT = tt;
-        const int rows = ((N + 147) / 148 + RS - 1) / RS * RS;
+        const int rows = ((N + 147) / 148 + unit - 1) / unit * unit;
         q.rows_per_cta = rows > ROWS_CAP ? ROWS_CAP : rows;
         const size_t round = (size_t)ROWS_WARPS * RS * W_PITCH * 4;  // a stage for every warp
         const size_t fixed = 2 * ROWS_MAX_STAGES * sizeof(uint64_t) + (size_t)tt * runs * X_PITCH * 4 +
@@ -357,12 +383,9 @@ int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* ou
     // Up to 16 tokens, and up to 32 where the weights are few: the rows kernel reads the weights once for every eight tokens,
     // the tiles do the work of 64 (us at 16 / 32 / 33 tokens: 9728 x 896 42 / 62 / 44, 896 x 4864 38 / 67 / 49, 151936 x 896
     // 379 / 730 / 422, but 1152 x 896 6 / 11 / 18).
-    if ((M <= 16 || (M <= 32 && (long long)N * K <= (1 << 21))) && rows_plan(M, N, K, q)) {
-        RowsParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr()};
-        if (q.TT == 8) return launch_rows<8>(p, q.smem, s);
-        if (q.TT == 4) return launch_rows<4>(p, q.smem, s);
-        if (q.TT == 2) return launch_rows<2>(p, q.smem, s);
-        return launch_rows<1>(p, q.smem, s);
+    if ((M <= 16 || (M <= 32 && (long long)N * K <= (1 << 21))) && rows_plan(M, N, K, RS, q)) {
+        RowsParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), 0};
+        return launch_rows_of(p, q, s);
     }
     const int runs = (K + F32_CHUNK - 1) / F32_CHUNK, per = f32_runs_per_part(runs);
     const int parts = (runs + per - 1) / per;
@@ -374,4 +397,24 @@ int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* ou
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if ((int)(grid.x * grid.y) < TILE_SPLIT) grid.z = parts;
     return launch_tile(p, grid, s);
+}
+
+constexpr int SWIGLU_MAX_TOKENS = 16;  // (beyond, the plain product may run the tiles)
+
+// Whether ferris_gemm_f32_swiglu takes a product of M tokens and N outputs: 16 tokens at most, rows that begin on 16 bytes.
+FERRIS_API int ferris_gemm_f32_swiglu_takes(const void* x, const void* w, int M, int N, int K, int ldx, int ldw) {
+    RowsPlan q;
+    return M > 0 && M <= SWIGLU_MAX_TOKENS && N > 0 && ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw) && rows_plan(M, 2 * N, K, 2 * RS, q);
+}
+// out[t, n] = silu(x[t] . w[n]) (x[t] . w[N + n]), fp32 throughout, with the sums of every other form of the product.
+FERRIS_API int ferris_gemm_f32_swiglu(const float* x, const float* w, float* out, int M, int N, int K, int ldx, int ldw, int ldo,
+                                      void* stream) {
+    if (M <= 0 || N <= 0) return FERRIS_OK;
+    if (K <= 0 || ldx < K || ldw < K || ldo < N) FERRIS_REFUSE("gemm: K=%d, row strides %d, %d, %d", K, ldx, ldw, ldo);
+    if (!ferris_gemm_f32_swiglu_takes(x, w, M, N, K, ldx, ldw))
+        FERRIS_REFUSE("gemm: %d tokens x %d outputs of %d do not take SwiGLU on the way", M, N, K);
+    RowsPlan q;
+    rows_plan(M, 2 * N, K, 2 * RS, q);
+    RowsParams p = {x, w, nullptr, out, M, N, K, ldx, ldw, ldo, 0, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), N};
+    return launch_rows_of(p, q, (cudaStream_t)stream);
 }

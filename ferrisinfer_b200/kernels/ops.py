@@ -566,7 +566,8 @@ def gemm_activation(x, w, out, kind: str, coefficients=(0.0, 0.0), params: Optio
 
 def gemm_swiglu(x, gate_up_weight, out, workspace=None):
     """out [T, I] = silu(x Wg^T) * (x Wu^T) with gate_up_weight = [Wg; Wu] ([2I, K]).  bf16: one tensor-core
-    kernel with two accumulators (the [T, 2I] intermediate never exists); otherwise a product and the SwiGLU kernel."""
+    kernel with two accumulators (the [T, 2I] intermediate never exists), so too 32-bit steps of at most 16 tokens; otherwise
+    a product and the SwiGLU kernel."""
     T, I = out.shape
     if gate_up_weight.shape[0] != 2 * I:
         raise KernelError(f"gemm_swiglu: weight {tuple(gate_up_weight.shape)} for {I} outputs")
@@ -581,6 +582,16 @@ def gemm_swiglu(x, gate_up_weight, out, workspace=None):
     if tensor_core_gemm_takes(x, gate_up_weight) and out.dtype == torch.bfloat16:
         gemm_tcgen05(x, gate_up_weight, None, out, 3, up_row_offset=I)
         return
+    if T <= 16 and x.dtype == gate_up_weight.dtype == out.dtype == torch.float32:
+        T2, K, ldx = _rows(x, "gemm input")
+        _, K2, ldw = _rows(gate_up_weight, "gemm weight")
+        _, _, ldo = _rows(out, "gemm output")
+        sizes = (_c_int(T), _c_int(I), _c_int(K), _c_int(ldx), _c_int(ldw))
+        if (T2 == T and K2 == K and x.untyped_storage().data_ptr() != out.untyped_storage().data_ptr()
+                and _lib().ferris_gemm_f32_swiglu_takes(_ptr(x), _ptr(gate_up_weight), *sizes)):
+            _check(_lib().ferris_gemm_f32_swiglu(_ptr(x), _ptr(gate_up_weight), _ptr(out), *sizes, _c_int(ldo), _stream()),
+                   "32-bit gemm")
+            return
     if workspace is not None:
         gate_up = workspace.get("ffn_gate_up", (T, 2 * I), x.dtype)
     else:

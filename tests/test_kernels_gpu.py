@@ -130,6 +130,25 @@ def test_gemm_fp32_sums_in_one_order_in_every_form(N, K, device):
     assert ops.kernel_status() == 0
 
 
+@pytest.mark.parametrize("N, K", [(8, 4), (150, 132), (67, 1028), (896, 896), (4864, 896), (40, 9220)])
+def test_gemm_fp32_with_swiglu_on_the_way(N, K, device):
+    """The 32-bit gate and up products of few tokens with SwiGLU in one launch: the bits of the product and the SwiGLU kernel
+    (which longer steps run)."""
+    from ferrisinfer_b200.kernels import ops
+
+    w = rnd((2 * N, K), F32, device, 30, scale=0.2)
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17):
+        x = rnd((M, K), F32, device, 33 + M)
+        gate_up, want = torch.empty(M, 2 * N, device=device), torch.empty(M, N, device=device)
+        ops.gemm_simt(x, w, None, gate_up)
+        ops.swiglu(gate_up, want)
+        out, before = torch.full((M, N), 7.0, device=device), ops.launch_count()
+        ops.gemm_swiglu(x, w, out)
+        assert torch.equal(out, want), M
+        assert ops.launch_count() - before == (1 if M <= 16 else 2), M
+    assert ops.kernel_status() == 0
+
+
 # ------------------------------------------------------------------------- tensor-core gemm
 TC_SHAPES = [(1, 1152, 896), (8, 1152, 896), (64, 896, 4864), (5, 130, 72), (16, 128, 64), (17, 300, 1000),
              (300, 256, 128), (2048, 384, 256), (33, 1000, 80), (257, 129, 200),
