@@ -1040,13 +1040,14 @@ struct MapCacheEntry {
 // One CTA per SM (shared memory and registers are each more than half an SM).  Measured with two per SM, by giving
 // K a single stage and capping registers at 96: batches of short prompts gain 10 %, but one long prompt loses 15 %,
 // because its time is that of the CTA of its last rows, which then shares its SM.
-// Head size 64 runs two groups of softmax warps and four stages, head size 128 one group and two stages (what
-// fits in shared memory).  Per block of keys the one-group chain costs about 2,600 cycles (wait for S 260, maximum
+// Head size 64 runs two groups of softmax warps and K and V of four blocks, head size 128 one group and K and V of two (what
+// fits in shared memory).  Per block of keys the one-group chain costs about 2,600 cycles at head size 64 (wait for S 260, maximum
 // and exchange 400, fold 400, exponentials and P 1,500, of which 1,024 is the special-function unit's time for
-// 16,384 exponentials); two groups take about 4,400 cycles for two blocks (the second group's wait for the tensor
+// 16,384 exponentials), 3,400 at head size 128 (350, 470, 900, 1,670); two groups take about 4,400 cycles for two blocks (the second group's wait for the tensor
 // core and the shared special-function unit keep it from halving): 2,048-token prompt 31.2 -> 29.8 us, a portion of
 // 512 at the end of 4,096 keys 53.4 -> 44.9 us, 8,192-token prompt 326 -> 281 us.
-// Measured and not kept: a ring of K blocks apart from a ring of V blocks, so that a K stage is free as soon as
+// Measured and not kept: one copy for the eight pages of a block where they lie one behind the other (3 to 10 % of the kernel, nothing of
+// a prompt's step); with the scores still in registers, a ring of K blocks apart from a ring of V blocks, so that a K stage is free as soon as
 // its scores are done (8,192-token prompt 281 -> 322 us at head size 64, 2,048 tokens at head size 128 43.7 -> 46.9 us).
 // =============================================================================================
 // 2^x by the special-function unit (ex2.approx: about two units in the last place; -inf gives 0).
@@ -1067,6 +1068,18 @@ constexpr int t5_threads(int groups) { return (T5_GROUP_WARPS * groups + 2) * 32
 // of its chain of key blocks (wait for S, maximum, exchange, fold, exponentials, one after the other: about
 // 1.4 us per block, of which the exponentials' share of the special-function unit is 0.54 us), and the kernel
 // lasts as long as the CTA of the prompt's last rows: two chains side by side shorten it.
+// Two score accumulators in either case: block i's scores stand in accumulator i % 2 (of two groups, each has one; one group
+// alternates, so that the tensor core forms the next block's scores while it works on this one's, without keeping them in registers).
+//
+// The ring.  Two groups: a stage holds K and V of a block, free when its product is done (a stage each: 8,192 tokens 281 -> 319
+// us).  One group (K and V of two blocks are all that fits): a stage holds one block of K or V, in the order of their use, K 0,
+// K 1, V 0, K 2, V 1, K 3, .., a K free as soon as its scores are done.  The stage, counted through, of a block's K and of its V
+// (n blocks in all):
+template <int GROUPS>
+__device__ __forceinline__ int t5_k_place(int i) { return GROUPS == 2 || i < 2 ? i : 2 * i - 1; }
+template <int GROUPS>
+__device__ __forceinline__ int t5_v_place(int i, int n) { return GROUPS == 2 ? i : i + 1 == n ? 2 * i + 1 : 2 * i + 2; }
+
 template <int D, int GROUPS, int STAGES>
 __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -1078,14 +1091,15 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     constexpr int TILE = TILE_KEYS * 64 * 2;           // one 16-key x 64-column box of K or of V: 2 KB
     constexpr int ATOM_BYTES = T5_KEYS * 64 * 2;       // 128 rows x 64 columns: 16 KB
     constexpr int BLOCK_BYTES = ATOMS * ATOM_BYTES;    // 128 keys of K or of V
+    constexpr int STAGE_BYTES = GROUPS * BLOCK_BYTES;  // two groups: K and V side by side; one: either
     constexpr int P_BYTES = 32768;                     // a group's P tile: [2 halves of 64 keys][128 rows][64] bf16
     constexpr int SW = T5_GROUP_WARPS * GROUPS;        // softmax warps; then the TMA warp and the MMA warp
-    constexpr int TMEM_COLS = GROUPS == 1 ? 256 : 512; // per group 128 columns of scores and D of the product
+    constexpr int TMEM_COLS = 512;                     // two times 128 columns of scores, per group D of the product
     static_assert(GROUPS == 1 || GROUPS == 2, "one or two softmax groups");
-    static_assert(128 * GROUPS + D * GROUPS <= TMEM_COLS, "tensor memory");
+    static_assert(256 + D * GROUPS <= TMEM_COLS, "tensor memory");
     static_assert(GROUPS == 1 || T5_ROWS * D * 4 <= P_BYTES, "the merge goes through a P tile");
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t kv_full[STAGES], kv_empty[STAGES], q_ready, s_ready[GROUPS], s_free[GROUPS], p_ready[GROUPS],
+    __shared__ uint64_t kv_full[STAGES], kv_empty[STAGES], q_ready, s_ready[2], s_free[2], p_ready[GROUPS],
         pv_done[GROUPS];
     __shared__ uint32_t tmem_base;
     __shared__ float row_share[GROUPS][2][2][T5_ROWS];  // [group][block parity][key half][row]: what the two threads of a row tell each other
@@ -1093,7 +1107,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     uint8_t* smem = align1024(smem_raw);
     uint8_t* q_smem = smem;                                  // [column group][128 rows][64] bf16, 128-byte swizzle
     uint8_t* p_smem = smem + BLOCK_BYTES;                    // per group: a P tile
-    uint8_t* kv_smem = smem + BLOCK_BYTES + GROUPS * P_BYTES;  // stages x (K block, V block), each [column group][128 keys][64]
+    uint8_t* kv_smem = smem + BLOCK_BYTES + GROUPS * P_BYTES;  // stages, each one or two blocks, [column group][128 keys][64]
 
     const int G = nh / nkv;
     const int hk = blockIdx.y;
@@ -1147,9 +1161,11 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
             mbar_init(&kv_empty[s], 1);
         }
         mbar_init(&q_ready, 4);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&s_ready[b], 1);
+            mbar_init(&s_free[b], T5_GROUP_WARPS);
+        }
         for (int g = 0; g < GROUPS; ++g) {
-            mbar_init(&s_ready[g], 1);
-            mbar_init(&s_free[g], T5_GROUP_WARPS);
             mbar_init(&p_ready[g], T5_GROUP_WARPS);
             mbar_init(&pv_done[g], 1);
         }
@@ -1159,7 +1175,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_s = tmem_base, tmem_pv = tmem_base + 128 * GROUPS;  // group g: scores at + 128 g, product at + D g
+    const uint32_t tmem_s = tmem_base, tmem_pv = tmem_base + 256;  // block i's scores at + 128 (i % 2); group g's product at + D g
 
     // keys of the block: from the first key its first token may see to its last token's position
     const int tok_first = row0 / G;
@@ -1184,23 +1200,50 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
                 }
             };
             look_up(0, rows);
-            for (int i = 0; i < n_kb; ++i) {
-                const int s = i % STAGES;
-                if (i + 1 < n_kb) look_up(i + 1, next_rows);
-                if (i >= STAGES && !mbar_wait(&kv_empty[s], ((i / STAGES) - 1) & 1, status, 40)) break;
-                uint8_t* ks = kv_smem + (size_t)s * 2 * BLOCK_BYTES;
-                uint8_t* vs = ks + BLOCK_BYTES;
-                mbar_expect_tx(&kv_full[s], 2 * BLOCK_BYTES);
+            if constexpr (GROUPS == 2) {
+                for (int i = 0; i < n_kb; ++i) {
+                    const int s = i % STAGES;
+                    if (i + 1 < n_kb) look_up(i + 1, next_rows);
+                    if (i >= STAGES && !mbar_wait(&kv_empty[s], ((i / STAGES) - 1) & 1, status, 40)) break;
+                    uint8_t* ks = kv_smem + (size_t)s * STAGE_BYTES;
+                    uint8_t* vs = ks + BLOCK_BYTES;
+                    mbar_expect_tx(&kv_full[s], 2 * BLOCK_BYTES);
 #pragma unroll
-                for (int t = 0; t < TILES; ++t) {
+                    for (int t = 0; t < TILES; ++t) {
 #pragma unroll
-                    for (int a = 0; a < ATOMS; ++a) {
-                        tma_load_2d(ks + a * ATOM_BYTES + t * TILE, &map_k, 64 * a, rows[t], &kv_full[s]);
-                        tma_load_2d(vs + a * ATOM_BYTES + t * TILE, &map_v, 64 * a, rows[t], &kv_full[s]);
+                        for (int a = 0; a < ATOMS; ++a) {
+                            tma_load_2d(ks + a * ATOM_BYTES + t * TILE, &map_k, 64 * a, rows[t], &kv_full[s]);
+                            tma_load_2d(vs + a * ATOM_BYTES + t * TILE, &map_v, 64 * a, rows[t], &kv_full[s]);
+                        }
                     }
-                }
 #pragma unroll
-                for (int t = 0; t < TILES; ++t) rows[t] = next_rows[t];
+                    for (int t = 0; t < TILES; ++t) rows[t] = next_rows[t];
+                }
+            } else {
+                auto load = [&](int n, const CUtensorMap* map, const int (&from)[TILES]) {
+                    const int s = n % STAGES;
+                    if (n >= STAGES && !mbar_wait(&kv_empty[s], ((n / STAGES) - 1) & 1, status, 40)) return false;
+                    uint8_t* dst = kv_smem + (size_t)s * STAGE_BYTES;
+                    mbar_expect_tx(&kv_full[s], BLOCK_BYTES);
+#pragma unroll
+                    for (int t = 0; t < TILES; ++t) {
+#pragma unroll
+                        for (int a = 0; a < ATOMS; ++a) tma_load_2d(dst + a * ATOM_BYTES + t * TILE, map, 64 * a, from[t], &kv_full[s]);
+                    }
+                    return true;
+                };
+                // (`rows` are those of block i, `next_rows` of block i + 1)
+                bool ok = load(0, &map_k, rows);
+                if (n_kb > 1) look_up(1, next_rows);
+                if (ok && n_kb > 1) ok = load(1, &map_k, next_rows);
+                for (int i = 0; i < n_kb && ok; ++i) {
+                    int after[TILES];
+                    if (i + 2 < n_kb) look_up(i + 2, after);
+                    ok = load(t5_v_place<1>(i, n_kb), &map_v, rows);
+                    if (ok && i + 2 < n_kb) ok = load(t5_k_place<1>(i + 2), &map_k, after);
+#pragma unroll
+                    for (int t = 0; t < TILES; ++t) rows[t] = next_rows[t], next_rows[t] = after[t];
+                }
             }
         }
     } else if (warp == SW + 1) {
@@ -1210,26 +1253,28 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
             bool ok = mbar_wait(&q_ready, 0, status, 41);
             // block i belongs to group i % GROUPS and is that group's block number i / GROUPS
             auto issue_qk = [&](int i) {
-                const int s = i % STAGES, g = i % GROUPS, j = i / GROUPS;
-                if (!mbar_wait(&kv_full[s], (i / STAGES) & 1, status, 42)) return false;
-                if (j > 0 && !mbar_wait(&s_free[g], (j - 1) & 1, status, 43)) return false;
+                const int n = t5_k_place<GROUPS>(i), s = n % STAGES, b = i % 2;
+                if (!mbar_wait(&kv_full[s], (n / STAGES) & 1, status, 42)) return false;
+                if (i > 1 && !mbar_wait(&s_free[b], (i / 2 - 1) & 1, status, 43)) return false;
                 tcgen05_fence_after();
-                const uint32_t k_addr = smem_u32(kv_smem + (size_t)s * 2 * BLOCK_BYTES);
+                const uint32_t k_addr = smem_u32(kv_smem + (size_t)s * STAGE_BYTES);
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k) {
                     // 16 columns of Q and of K: 32 bytes along the row within the column group of 64
                     const uint64_t qd = umma_desc_k_major_sw128(smem_u32(q_smem) + (k >> 2) * ATOM_BYTES) + (uint64_t)(2 * (k & 3));
                     const uint64_t kd = umma_desc_k_major_sw128(k_addr + (k >> 2) * ATOM_BYTES) + (uint64_t)(2 * (k & 3));
-                    tcgen05_mma_bf16(tmem_s + 128 * g, qd, kd, idesc_qk, k > 0 ? 1u : 0u);
+                    tcgen05_mma_bf16(tmem_s + 128 * b, qd, kd, idesc_qk, k > 0 ? 1u : 0u);
                 }
-                tcgen05_commit(&s_ready[g]);
+                tcgen05_commit(&s_ready[b]);
+                if (GROUPS == 1) tcgen05_commit(&kv_empty[s]);
                 return true;
             };
             auto issue_pv = [&](int i) {
-                const int s = i % STAGES, g = i % GROUPS;
+                const int n = t5_v_place<GROUPS>(i, n_kb), s = n % STAGES, g = i % GROUPS;
+                if (GROUPS == 1 && !mbar_wait(&kv_full[s], (n / STAGES) & 1, status, 48)) return false;
                 tcgen05_fence_after();
                 // V as an MN-major operand: column groups of 64 lie ATOM_BYTES apart (the leading byte offset)
-                const uint64_t v_desc = umma_desc_mn_major_sw128(smem_u32(kv_smem + (size_t)s * 2 * BLOCK_BYTES + BLOCK_BYTES), ATOM_BYTES);
+                const uint64_t v_desc = umma_desc_mn_major_sw128(smem_u32(kv_smem + (size_t)s * STAGE_BYTES + (STAGE_BYTES - BLOCK_BYTES)), ATOM_BYTES);
 #pragma unroll
                 for (int k = 0; k < T5_KEYS / 16; ++k) {
                     // A: 16 keys of P = 32 bytes along the row within the half of 64 keys; B: 16 rows of V = 2 KB further
@@ -1238,15 +1283,18 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
                 }
                 tcgen05_commit(&pv_done[g]);
                 tcgen05_commit(&kv_empty[s]);
+                return true;
             };
-            // In block order: the scores of block i + GROUPS as soon as its group has read those of block i, then the
-            // product of block i.  (Measured for two groups: serving whichever group is ready first, by polling the
-            // barriers, is 5 % slower; a group mostly waits for the tensor core, not for its turn.)
-            for (int i = 0; i < GROUPS && i < n_kb && ok; ++i) ok = issue_qk(i);
+            // In block order.  Two groups: the scores of block i + 2 as soon as its group has read those of block i, then the
+            // product of block i.  (Measured: serving whichever group is ready first, by polling the barriers, is 5 % slower;
+            // a group mostly waits for the tensor core, not for its turn.)  One group has the scores of block i + 1 already when
+            // it is done with block i, so the product, which it waits for next, goes first.
+            for (int i = 0; i < 2 && i < n_kb && ok; ++i) ok = issue_qk(i);
             for (int i = 0; i < n_kb && ok; ++i) {
-                if (i + GROUPS < n_kb) ok = issue_qk(i + GROUPS);
+                if (GROUPS == 2 && i + 2 < n_kb) ok = issue_qk(i + 2);
                 if (!ok || !mbar_wait(&p_ready[i % GROUPS], (i / GROUPS) & 1, status, 44)) break;
-                issue_pv(i);
+                ok = issue_pv(i);
+                if (GROUPS == 1 && ok && i + 2 < n_kb) ok = issue_qk(i + 2);
             }
         }
     } else {
@@ -1272,7 +1320,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
             if (lane == 0) mbar_arrive(&q_ready);
         }
         const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
-        const uint32_t my_s = tmem_s + 128 * g + lane_addr + 64 * kh;
+        const uint32_t s_base = tmem_s + (GROUPS == 2 ? 128 * g : 0) + lane_addr + 64 * kh;
         const uint32_t my_pv = tmem_pv + D * g + lane_addr + (D / 2) * kh;
         const float scale2 = scale * 1.4426950408889634f;  // scores in units of log 2
         float m = -INFINITY, l = 0.0f;
@@ -1285,51 +1333,33 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
         long long t_wait_s = 0, t_max = 0, t_fold = 0, t_exp = 0, c0 = FERRIS_TL_CLOCK(), c1;
         for (int j = 0; j < n_own; ++j) {
             const int i = j * GROUPS + g;
-            if (!mbar_wait(&s_ready[g], j & 1, status, 45)) break;
+            const int b = GROUPS == 2 ? g : j & 1;  // the accumulator of its scores
+            const uint32_t my_s = GROUPS == 2 ? s_base : s_base + 128 * b;
+            if (!mbar_wait(&s_ready[b], (GROUPS == 2 ? j : j >> 1) & 1, status, 45)) break;
             tcgen05_fence_after();
             c1 = FERRIS_TL_CLOCK();
             t_wait_s += c1 - c0;
             c0 = c1;
             const int key_base = (kb_begin + i) * T5_KEYS + 64 * kh;
             const bool interior = key_base >= lo && key_base + 63 <= hi;
-            // One group: this thread's 64 scores are read once and kept, so that the next block's scores may overwrite
-            // them while the exponentials are taken.  Two groups (18 warps leave a thread 96 registers): the scores
-            // stay in tensor memory, read in chunks for the maximum and again for the exponentials; the other group
-            // keeps the tensor core busy meanwhile.
-            constexpr int KEEP = GROUPS == 1 ? 64 : 1;
-            uint32_t sv[KEEP];
+            // The scores stay in tensor memory, read in chunks for the maximum and again for the exponentials.  (One group used to
+            // keep its 64 in registers beside 64 output columns at head size 128: 35 of them spilled, and bringing the row to
+            // the new maximum took 2,200 cycles of a block's 4,700; now 900 of 3,400.  Head size 128, us, before / now, one prompt
+            // of 2,048 tokens with 12 heads over 2 45.9 / 38.5, with 28 over 4 91.6 / 77.8, of 8,192 422 / 360, of 512 17.5 / 14.4.)
             float mx = -INFINITY;
-            if constexpr (GROUPS == 1) {
-                tmem_load_32x64(my_s, reinterpret_cast<uint32_t (&)[64]>(sv));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t sc[32];
+                tmem_load_32x32(my_s + 32 * h, sc);
                 tmem_load_wait();
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&s_free[g]);
                 if (interior) {
 #pragma unroll
-                    for (int c = 0; c < 64; ++c) mx = fmaxf(mx, __uint_as_float(sv[c % KEEP]));
+                    for (int c = 0; c < 32; ++c) mx = fmaxf(mx, __uint_as_float(sc[c]));
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 64; ++c) {
-                        const int key = key_base + c;
-                        mx = fmaxf(mx, (key <= hi && key >= lo) ? __uint_as_float(sv[c % KEEP]) : -INFINITY);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t sc[32];
-                    tmem_load_32x32(my_s + 32 * h, sc);
-                    tmem_load_wait();
-                    if (interior) {
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) mx = fmaxf(mx, __uint_as_float(sc[c]));
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) {
-                            const int key = key_base + 32 * h + c;
-                            mx = fmaxf(mx, (key <= hi && key >= lo) ? __uint_as_float(sc[c]) : -INFINITY);
-                        }
+                    for (int c = 0; c < 32; ++c) {
+                        const int key = key_base + 32 * h + c;
+                        mx = fmaxf(mx, (key <= hi && key >= lo) ? __uint_as_float(sc[c]) : -INFINITY);
                     }
                 }
             }
@@ -1370,13 +1400,8 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {  // 16 keys at a time
                     uint32_t sc[16], packed[8];
-                    if constexpr (GROUPS == 1) {
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) sc[c] = sv[(16 * h + c) % KEEP];
-                    } else {
-                        tmem_load_32x16(my_s + 16 * h, sc);
-                        tmem_load_wait();
-                    }
+                    tmem_load_32x16(my_s + 16 * h, sc);
+                    tmem_load_wait();
                     if (interior) {
 #pragma unroll
                         for (int c = 0; c < 16; c += 2) {
@@ -1402,12 +1427,10 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
                 }
                 l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
             }
-            if constexpr (GROUPS == 2) {
-                // the scores have been read for the last time: the group's next block may overwrite them
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&s_free[g]);
-            }
+            // the scores have been read for the last time: the block after next may overwrite them
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[b]);
             m = m_new;
             fence_proxy_async();  // the MMA reads P through the async proxy
             __syncwarp();
@@ -1847,10 +1870,10 @@ FERRIS_API int ferris_prefill_attention(const void* q, int ldq, void* out, int l
         }
         if (blocks > 0x7fffffffLL) FERRIS_REFUSE("prefill attention: %lld blocks of rows exceed one launch", blocks);
         dim3 grid5((unsigned)blocks, nkv);
-        // Q, a P tile per softmax group, stages of (K block, V block).  Head size 64: two groups and four stages
-        // (209 KB); head size 128: one group and two stages (193 KB), two groups would not fit.
+        // Q, a P tile per softmax group, the ring.  Head size 64: two groups and four stages of K and V (209 KB); head
+        // size 128: one group and four stages of K or V (193 KB), two groups would not fit.
         auto bytes = [&](int groups, int stages) {
-            return (size_t)T5_ROWS * d * 2 + (size_t)groups * 32768 + (size_t)stages * 2 * T5_KEYS * d * 2 + 1024;
+            return (size_t)T5_ROWS * d * 2 + (size_t)groups * 32768 + (size_t)groups * stages * T5_KEYS * d * 2 + 1024;
         };
 #define FERRIS_T5_LAUNCH(DD, GG, SS)                                                                                       \
     do {                                                                                                                   \
@@ -1863,9 +1886,9 @@ FERRIS_API int ferris_prefill_attention(const void* q, int ldq, void* out, int l
         if (d == 64 && g_prefill_tc5 != 2)
             FERRIS_T5_LAUNCH(64, 2, 4);
         else if (d == 64)
-            FERRIS_T5_LAUNCH(64, 1, 4);
+            FERRIS_T5_LAUNCH(64, 1, 8);
         else
-            FERRIS_T5_LAUNCH(128, 1, 2);
+            FERRIS_T5_LAUNCH(128, 1, 4);
 #undef FERRIS_T5_LAUNCH
         FERRIS_LAUNCH_CHECK();
     }
