@@ -1114,11 +1114,10 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     FERRIS_TL_ENTRY();
     if (!beside) pdl_wait();
-    pdl_launch_dependents();
     FERRIS_TL_BEGIN();
-    // The grid holds no more CTAs a kv head than there are row blocks, whatever the requests' lengths (a CTA without rows still
-    // takes a whole SM's shared memory: a step of 31 single tokens and one portion of 481 tokens launched 1,472 CTAs for 46
-    // row blocks and took 31 us): each warp finds the CTA's request by itself.
+    // The grid holds at most one CTA a request and kv head more than there are row blocks, whatever the requests' lengths (a CTA
+    // without rows still takes a whole SM's shared memory: a step of 31 single tokens and one portion of 481 tokens launched 1,472
+    // CTAs for 46 row blocks and took 31 us): each warp finds the CTA's request by itself.
     int seq = -1, rank = 0;
     for (int s0 = 0, before = 0; s0 < num_seqs && seq < 0; s0 += 32) {
         int n = 0;
@@ -1141,6 +1140,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
         before += __shfl_sync(0xffffffffu, upto, 31);
     }
     if (seq < 0) {
+        pdl_launch_dependents();
         if (beside) pdl_wait();
         FERRIS_TL_END(8);
         return;
@@ -1175,6 +1175,9 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    // Only now: this kernel takes all of an SM's tensor memory.  A dependent product whose shared memory fits beside it (one
+    // K slice of a few tokens, 20 KB) could otherwise take its columns first and then wait for this grid, which would wait for them.
+    pdl_launch_dependents();
     const uint32_t tmem_s = tmem_base, tmem_pv = tmem_base + 256;  // block i's scores at + 128 (i % 2); group g's product at + D g
 
     // keys of the block: from the first key its first token may see to its last token's position

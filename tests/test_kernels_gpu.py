@@ -796,6 +796,26 @@ def test_prefill_attention_on_tcgen05_and_on_mma_sync(nh, nkv, d, window, device
     assert (got[1] - got[2]).abs().max() <= 2 * ATT_TOL[BF16]["atol"]
 
 
+@pytest.mark.parametrize("q_len", [2, 16])
+def test_a_small_product_right_behind_the_attention_of_portions(q_len, device):
+    """The attention of portions takes all of an SM's tensor memory; the product behind it has one K slice, so that its
+    shared memory fits beside, and is let in while the attention runs: both end, and with the right numbers."""
+    from ferrisinfer_b200.kernels import ops
+
+    case = AttentionCase(device, BF16, 2, 1, 128, 16, [(q_len + 40 * i, q_len) for i in range(80)], seed=q_len)
+    qkv, k, v, tables, ctx, T = case.device_inputs()
+    x, w = rnd((16, 64), BF16, device, 1), rnd((1024, 64), BF16, device, 2)
+    out = torch.full((T, 256), float("nan"), dtype=BF16, device=device)
+    product = torch.empty(16, 1024, dtype=F32, device=device)
+    for _ in range(10):
+        ops.paged_attention(qkv, out, k, v, tables, ctx, 2, 1, 128, 0, 1.0 / math.sqrt(128))
+        ops.gemm_tcgen05(x, w, None, product, 1)
+    torch.cuda.synchronize()
+    assert ops.kernel_status() == 0
+    assert torch.allclose(out.cpu().double(), case.reference(), **ATT_TOL[BF16])
+    assert torch.allclose(product.cpu().double(), x.cpu().double() @ w.cpu().double().t(), atol=1e-4, rtol=1e-4)
+
+
 @pytest.mark.parametrize("impl", ["simt", "dispatch"])
 def test_attention_single_tokens_beside_portions_at_long_context(impl, device):
     """Single tokens whose keys are split into ranges, at rows of the step that come after portions of prompts
