@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(ROWS * 4, ROWS == 32 && NC == 1 ? 4 : 1)
     const int d = DF ? DF : d_any, dv = DF ? DF : dv_any;
     constexpr int THREADS = ROWS * 4, P_PITCH = ROWS + 4;
     extern __shared__ __align__(16) float tl_smem[];
-    __shared__ int key_row[TL_KEYS];  // the tile's keys' rows in the cache, -1: none
+    __shared__ long long key_row[TL_KEYS];  // the tile's keys' rows in the cache (small heads: more than 2^31), -1: none
     const int dp = d + 4, dvp = dv + 4;
     float* Qs = tl_smem;                      // [ROWS][d + 4]
     float* Ks = Qs + ROWS * dp;               // [64][d + 4]
@@ -632,15 +632,15 @@ __global__ void __launch_bounds__(ROWS * 4, ROWS == 32 && NC == 1 ? 4 : 1)
                 int page = -1;
                 if (j >= kmin && j <= kmax) page = table[pshift >= 0 ? (j >> pshift) : (j / page_size)];
                 const int in_page = pshift >= 0 ? (j & (page_size - 1)) : (j % page_size);
-                key_row[tid] = page >= 0 ? (page * nkv + hk) * page_size + in_page : -1;
+                key_row[tid] = page >= 0 ? ((long long)page * nkv + hk) * page_size + in_page : -1;
             }
             __syncthreads();
 #pragma unroll 4
             for (int key = ry; key < TL_KEYS; key += THREADS / 16) {
-                const int row = key_row[key];
+                const long long row = key_row[key];
                 if (row >= 0) {
-                    stage_row(keys + (size_t)row * d, Ks + key * dp, d, kx);
-                    stage_row(vals + (size_t)row * (st.v_stride ? st.v_stride : dv), Vs + key * dvp, dv, kx);
+                    stage_row(keys + row * d, Ks + key * dp, d, kx);
+                    stage_row(vals + row * (st.v_stride ? st.v_stride : dv), Vs + key * dvp, dv, kx);
                 } else {
                     zero_row(Ks + key * dp, d, kx);
                     zero_row(Vs + key * dvp, dv, kx);

@@ -816,6 +816,35 @@ def test_a_small_product_right_behind_the_attention_of_portions(q_len, device):
     assert torch.allclose(product.cpu().double(), x.cpu().double() @ w.cpu().double().t(), atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("q_len", [1, 40])
+def test_attention_of_a_cache_with_more_rows_than_32_bits_count(q_len, device):
+    """Heads of four elements in 32-bit: 2^31 rows of keys are 34 GB, which the card holds.  A request on the last pages
+    gets what it gets on the first ones, from the kernel for portions and from the one for single tokens."""
+    from ferrisinfer_b200.kernels import ops
+
+    page, d, pages = 16, 4, (1 << 31) // 16 + 8
+    if torch.cuda.mem_get_info(device)[0] < 2 * pages * page * d * 4:
+        pytest.skip("the cache does not fit into the free memory")
+    kv = 70
+    rows = rnd((1, kv + 10, d), F32, device, 1).view(5, 1, page, d)
+    cache = torch.empty(pages, 1, page, d, dtype=F32, device=device)  # keys and values in one: only the pages in use are ever touched
+    qkv = rnd((q_len, 3 * d), F32, device, 2)
+    token_seq = torch.zeros(q_len, dtype=torch.int32, device=device)
+    positions = torch.arange(kv - q_len, kv, dtype=torch.int32, device=device)
+    outs = []
+    for first in (0, pages - 5):
+        cache[first:first + 5] = rows
+        tables = torch.arange(first, first + 5, dtype=torch.int32, device=device)[None]
+        out = torch.empty(q_len, d, dtype=F32, device=device)
+        ops.paged_attention_simt(qkv, out, cache, cache, tables, token_seq, positions, 1, 1, d, 0, 0.5, max_q_len=q_len,
+                                 max_kv_len=kv)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    k = rows.view(-1, d)[:kv].double()
+    want = [torch.softmax((qkv[i, :d].double() @ k[:p + 1].t()) * 0.5, -1) @ k[:p + 1] for i, p in enumerate(positions.tolist())]
+    assert torch.allclose(outs[1].double(), torch.stack(want), **ATT_TOL[F32])
+
+
 @pytest.mark.parametrize("impl", ["simt", "dispatch"])
 def test_attention_single_tokens_beside_portions_at_long_context(impl, device):
     """Single tokens whose keys are split into ranges, at rows of the step that come after portions of prompts
