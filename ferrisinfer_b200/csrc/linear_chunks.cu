@@ -182,6 +182,43 @@ __device__ __forceinline__ Chunk chunk_of(const ChunkArgs& p, int head) {
     return c;
 }
 
+// A chunk whose products are not finite, token by token as the walk does it: an infinity cut into parts leaves inf - inf, a
+// weight of zero meets a later token's, a power of the decay that falls to zero an earlier one's.  `cols` columns of one head,
+// four threads each: their values begin at v and the keys and queries at k and q, rows of `width`; the state goes from `start`
+// (null: zeros) to `end` (null: not wanted), the outputs to rows of `ldo` at `out` (null: not wanted).  Not inlined: the kernels
+// keep their registers.
+template <int D>
+__device__ __noinline__ void walk_chunk(const float* q, const float* k, const float* v, int width, int n, int dim, int cols, float lam,
+                                        const float* start, float* end, float* out, int ldo) {
+    const int col = threadIdx.x >> 2, part = threadIdx.x & 3;
+    const bool mine = col < cols;
+    const size_t at = (size_t)col * dim;
+    float S[D / 4];
+#pragma unroll
+    for (int i = 0; i < D / 4; ++i) S[i] = start && mine && part + 4 * i < dim ? start[at + part + 4 * i] : 0.0f;
+    for (int t = 0; t < n; ++t, q += width, k += width, v += width) {
+        const float value = mine ? v[col] : 0.0f;
+        float o = 0.0f;
+#pragma unroll
+        for (int i = 0; i < D / 4; ++i) {
+            const int d = part + 4 * i;
+            if (d < dim) {
+                S[i] = fmaf(k[d], value, lam * S[i]);
+                o = fmaf(S[i], q[d], o);
+            }
+        }
+        o += __shfl_xor_sync(0xffffffffu, o, 1);
+        o += __shfl_xor_sync(0xffffffffu, o, 2);
+        if (out && mine && part == 0) out[(size_t)t * ldo + col] = o;
+    }
+    if (end && mine) {
+#pragma unroll
+        for (int i = 0; i < D / 4; ++i)
+            if (part + 4 * i < dim) end[at + part + 4 * i] = S[i];
+    }
+}
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
 template <int D>
 __global__ void __launch_bounds__(LC_THREADS, 2) linear_chunk_sums_kernel(const ChunkArgs p) {
     extern __shared__ __align__(16) float lc_smem[];
@@ -210,16 +247,23 @@ __global__ void __launch_bounds__(LC_THREADS, 2) linear_chunk_sums_kernel(const 
     CutSums<D / 16> acc;
     for (int t = 0; t < c.n; t += 8)
         cut_products<D / 16, true>(acc, vs + t * V_PITCH + m0, 1, V_PITCH, ks + t * K_PITCH + d0, K_PITCH, 1, 8, D / 16, pw + t);
+    bool odd = false;
 #pragma unroll
     for (int j = 0; j < D / 16; ++j) {
         const int d = d0 + 8 * j + 2 * t4;
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
             const int v = m0 + g + 8 * a;
-            if (v < cols && d < p.dim)
-                *reinterpret_cast<float2*>(c.state + (size_t)(col0 + v) * p.dim + d) = make_float2(acc.get(j, 2 * a), acc.get(j, 2 * a + 1));
+            const float2 sum = make_float2(acc.get(j, 2 * a), acc.get(j, 2 * a + 1));
+            if (v < cols && d < p.dim) {
+                odd |= !is_finite(sum.x) || !is_finite(sum.y);
+                *reinterpret_cast<float2*>(c.state + (size_t)(col0 + v) * p.dim + d) = sum;
+            }
         }
     }
+    if (__syncthreads_or(odd))
+        walk_chunk<D>(row + head * p.dim, row + qk + head * p.dim, row + 2 * qk + head * p.vdim + col0, (int)width, c.n, p.dim, cols,
+                      p.decay[head], nullptr, c.state + (size_t)col0 * p.dim, nullptr, 0);
 }
 
 // scratch holds each chunk's own sum; afterwards it holds the state at each chunk's start, and the request's slot its new state.
@@ -234,6 +278,8 @@ __global__ void __launch_bounds__(256) linear_chunk_starts_kernel(const ChunkArg
     if (e >= per_state || row1 - row0 <= p.above) return;
     const float lam = p.decay[e / ((size_t)p.vdim * p.dim)];
     const float step = power(lam, LC_TOKENS);
+    // for a power of zero: an infinity stays one however often it decays, also where the power is too small for 32 bits
+    auto decayed = [lam](float f, float x) { return lam != 0.0f && isinf(x) ? copysignf(1.0f, f) * x : f * x; };
     float4* slot = reinterpret_cast<float4*>(p.state + (size_t)p.seq_state_slot[seq] * per_state + e);
     float4 S = *slot;
     const int chunks = (row1 - row0 + LC_TOKENS - 1) / LC_TOKENS;
@@ -250,7 +296,12 @@ __global__ void __launch_bounds__(256) linear_chunk_starts_kernel(const ChunkArg
             if (c0 + i < chunks) *place(c0 + i) = S;
             if (c0 + i < sums) {
                 const float f = c0 + i + 1 < chunks ? step : power(lam, row1 - row0 - (chunks - 1) * LC_TOKENS);
-                S.x = fmaf(f, S.x, own[i].x), S.y = fmaf(f, S.y, own[i].y), S.z = fmaf(f, S.z, own[i].z), S.w = fmaf(f, S.w, own[i].w);
+                if (f != 0.0f) {
+                    S.x = fmaf(f, S.x, own[i].x), S.y = fmaf(f, S.y, own[i].y), S.z = fmaf(f, S.z, own[i].z), S.w = fmaf(f, S.w, own[i].w);
+                } else {
+                    S.x = decayed(f, S.x) + own[i].x, S.y = decayed(f, S.y) + own[i].y;
+                    S.z = decayed(f, S.z) + own[i].z, S.w = decayed(f, S.w) + own[i].w;
+                }
             }
         }
     }
@@ -300,33 +351,18 @@ __global__ void __launch_bounds__(LC_THREADS, 2) linear_chunk_outputs_kernel(con
                 as[t * A_PITCH + i] = i <= t ? acc.get(j, e) * pw[t - i] : 0.0f;
             }
     }
-    wait_rows<0>();  // this thread's pieces of v: does one hold an infinity or a NaN?
-    bool odd_piece = false;
-    for (int x = tid; x < LC_TOKENS * (LC_COLS / 4); x += LC_THREADS) {
-        const float4 f = *reinterpret_cast<const float4*>(vs + (x / (LC_COLS / 4)) * V_PITCH + (x % (LC_COLS / 4)) * 4);
-        odd_piece |= !(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))) <= 3.4028234e38f) || f.x != f.x || f.y != f.y ||
-                     f.z != f.z || f.w != f.w;
-    }
-    const bool odd_values = __syncthreads_or(odd_piece);  // (and the keys have been read)
+    wait_rows<0>();
+    __syncthreads();  // v is there, and the keys have been read
     request_rows(ks, K_PITCH, c.state + (size_t)col0 * p.dim, p.dim, cols, p.dim, D);  // the state's columns as rows
     commit_rows();
     const int v0 = 8 * odd;  // tiles 2 j + odd of the columns
     CutSums<4> within, before;
-    if (odd_values) {  // a weight of zero must not meet a later token's infinity
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int t = m0 + g + 8 * (e >> 1);
-                for (int i = 0; i <= t; ++i)
-                    within.big[j][e] = fmaf(as[t * A_PITCH + i], vs[i * V_PITCH + 16 * j + v0 + 2 * t4 + (e & 1)], within.big[j][e]);
-            }
-    }
-    for (int i = 0; i < (odd_values ? 0 : m0 + 16); i += 8)
+    for (int i = 0; i < m0 + 16; i += 8)
         cut_products<4>(within, as + m0 * A_PITCH + i, A_PITCH, 1, vs + i * V_PITCH + v0, V_PITCH, 1, 16, 4);
     wait_rows<0>();
     __syncthreads();
     for (int d = 0; d < D; d += 8) cut_products<4>(before, qs + m0 * K_PITCH + d, K_PITCH, 1, ks + v0 * K_PITCH + d, 1, K_PITCH, 16, 4);
+    bool odd_sum = false;
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
         const int t = m0 + g + 8 * a;
@@ -336,11 +372,17 @@ __global__ void __launch_bounds__(LC_THREADS, 2) linear_chunk_outputs_kernel(con
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int v = 16 * j + v0 + 2 * t4;
-            if (v < cols)
-                *reinterpret_cast<float2*>(orow + v) = make_float2(fmaf(f, before.get(j, 2 * a), within.get(j, 2 * a)),
-                                                                   fmaf(f, before.get(j, 2 * a + 1), within.get(j, 2 * a + 1)));
+            const float2 o = make_float2(fmaf(f, before.get(j, 2 * a), within.get(j, 2 * a)), fmaf(f, before.get(j, 2 * a + 1), within.get(j, 2 * a + 1)));
+            if (v < cols) {
+                odd_sum |= !is_finite(o.x) || !is_finite(o.y);
+                *reinterpret_cast<float2*>(orow + v) = o;
+            }
         }
     }
+    if (__syncthreads_or(odd_sum))
+        walk_chunk<D>(row + head * p.dim, row + qk + head * p.dim, row + 2 * qk + head * p.vdim + col0, (int)width, c.n, p.dim, cols,
+                      p.decay[head], c.state + (size_t)col0 * p.dim, nullptr,
+                      p.out + (size_t)c.row0 * p.ldo + (size_t)head * p.vdim + col0, p.ldo);
 }
 
 template <int D>

@@ -311,6 +311,49 @@ def test_linear_attention_chunks_keep_an_infinity_from_earlier_tokens(device):
     assert torch.allclose(outs[0][:75], outs[1][:75], atol=1e-4) and not bool(torch.isfinite(outs[1][75:, 5]).any())
 
 
+@pytest.mark.parametrize("decay", [0.1, 0.9, 1.0, 0.0])  # 0.1: a chunk's power of it is zero in 32 bits
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 72)])
+@pytest.mark.parametrize("where", ["v", "k", "q", "state", "both signs", "nan", "largest"])
+def test_linear_attention_chunks_pass_infinities_on_as_the_walk_does(device, where, dim, vdim, decay):
+    """An infinity or a NaN among the values, keys, queries or in the state that a request begins with, chunks before its end:
+    outputs and state are infinite, with the same sign, NaN and finite where those of the walk token by token are."""
+    ops = _ops()
+    torch.manual_seed(dim)
+    lens, slots = [200, 130], [1, 0]
+    T = sum(lens)
+    # (keys and queries above zero, so that an infinity stays one instead of meeting its opposite)
+    proj = torch.cat([torch.rand(T, 2 * dim) + 0.1, torch.randn(T, vdim)], 1).to(BF16)
+    start = torch.randn(2, 1, vdim, dim)
+    if where == "v":
+        proj[30, 2 * dim + 5], proj[T - 3, 2 * dim + 63] = math.inf, -math.inf
+    elif where == "k":
+        proj[70, dim + 3] = math.inf
+    elif where == "q":
+        proj[70, 9], proj[140, 1] = math.inf, -math.inf
+    elif where == "state":
+        start[1, 0, 7, 11], start[0, 0, 0, 1] = math.inf, -math.inf
+    elif where == "both signs":
+        start[1, 0, 7, 11] = math.inf
+        proj[100, 2 * dim + 7] = -math.inf
+    elif where == "nan":
+        proj[64, 2 * dim + 5] = math.nan
+    else:
+        proj[10, 2 * dim + 2] = 3.38e38  # of bf16: finite, and so is its product with a key below one
+        proj[10, dim:2 * dim] = proj[10, dim:2 * dim].clamp(max=0.5)
+    got = {}
+    for form in ("chunks", "walk"):
+        state, out = start.clone().to(device), torch.empty(T, vdim, device=device)
+        ops.linear_attention(proj.to(device), (0, dim, 2 * dim), out, state, torch.tensor([decay], device=device),
+                             fake_ctx(device, lens, [0, 0], slots), 1, dim, vdim, segment=None if form == "chunks" else 1024)
+        got[form] = (out.cpu(), state.cpu())
+    for a, b in zip(got["chunks"], got["walk"]):
+        assert torch.equal(torch.isnan(a), torch.isnan(b))
+        odd = ~torch.isfinite(b)
+        assert torch.equal(a[odd & ~torch.isnan(b)], b[odd & ~torch.isnan(b)])
+        assert torch.equal(torch.isfinite(a), ~odd)
+        assert torch.allclose(a[~odd], b[~odd], rtol=1e-5, atol=1e-4)
+
+
 def test_linear_attention_keeps_a_key_from_hundreds_of_tokens_ago(device):
     """With a decay of one, a key that matches the last query, 600 tokens back among keys that do not, comes through
     with its value: one wrong state row or a lost update shows at full size."""
