@@ -488,7 +488,7 @@ __device__ __forceinline__ void rotate_q(WarpStateT<D>& st, const float2* cos_si
 // copy costs the TMA unit ~30 ns whatever it brings, and a CTA of a long context issues hundreds).  A tile then lies
 // in shared memory as (K box, V box) per 64 columns instead of all K boxes followed by all V boxes.
 // TR: the group has at most 8 query heads and the warps work on the transposed products (attend_block_t).
-template <int D, int STAGES, bool PAIR, int NW, bool TR>
+template <int D, int STAGES, bool PAIR, int NW, bool TR, bool LISTED>
 __global__ void __launch_bounds__(NW * 32)
     decode_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                             const bf16* q, int ldq, bf16* __restrict__ out, int ldo,
@@ -521,6 +521,9 @@ __global__ void __launch_bounds__(NW * 32)
     }
     mbar_fence_init();
     __syncthreads();
+    // With a token list the launch behind is the attention of portions, which may run beside this kernel without a wait of its
+    // own: it is let in after this one's.
+    if (!LISTED) pdl_launch_dependents();
     if (splits > 1 && cluster_merge) cluster_arrive_relaxed();  // first phase of the cluster's barrier: "this CTA runs"
     // A kernel that rotates AND writes the cache reads nothing from the cache that this step wrote before it (the
     // token's own key and value come from its qkv row, which it patches into the tile), and the step's metadata was
@@ -535,15 +538,13 @@ __global__ void __launch_bounds__(NW * 32)
     const bool fused = rope.inv_freq != nullptr;
     const bool patches = fused && rope.slot_mapping != nullptr;
     const bool early = patches;
-    if (early) {
-        pdl_launch_dependents();
-    } else {  // (the attention of portions may run beside this kernel without a wait of its own: it is let in after this one's)
+    if (!early) {
         pdl_wait();
-        pdl_launch_dependents();
+        if (LISTED) pdl_launch_dependents();
         FERRIS_TL_BEGIN();
     }
     // with a token list, only the listed rows of the step are attended (the others belong to another kernel)
-    const int tok = token_list ? token_list[blockIdx.z] : (int)blockIdx.z;
+    const int tok = LISTED ? token_list[blockIdx.z] : (int)blockIdx.z;
     const int seq = token_seq[tok];
     const int P = positions[tok];
     const int lo = (window > 0 && P - window + 1 > 0) ? P - window + 1 : 0;
@@ -1650,7 +1651,8 @@ static int decode_attention_impl(const void* q, int ldq, void* out, int ldo, con
     const int G = nh / nkv;
     const size_t recv_bytes = cluster ? (size_t)splits * (2 * G + (G * d + splits - 1) / splits) * 4 : 0;
     const size_t smem = (size_t)nw * st * 16384 + 1024 + recv_bytes;
-    auto launch = [&](auto kernel) -> cudaError_t {
+    auto launch = [&](auto kernel) -> int {
+        if (int refused = set_smem(kernel, smem)) return refused;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
         cfg.blockDim = dim3(nw * 32);
@@ -1665,8 +1667,8 @@ static int decode_attention_impl(const void* q, int ldq, void* out, int ldo, con
             attr[n].val.clusterDim.z = 1;
             ++n;
             if (splits > 8) {
-                const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                if (allowed != cudaSuccess) return allowed;
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                if (e != cudaSuccess) return FERRIS_OK;  // said below
             }
         }
         if (ferris_pdl_enabled()) {
@@ -1676,19 +1678,20 @@ static int decode_attention_impl(const void* q, int ldq, void* out, int ldo, con
         }
         cfg.attrs = attr;
         cfg.numAttrs = n;
-        return cudaLaunchKernelEx(&cfg, kernel, mk, mv, (const bf16*)q, ldq, (bf16*)out, ldo, part_o, part_ml, block_tables,
-                                  max_blocks, token_seq, positions, token_list, nh, nkv, page_size, window, scale, splits,
-                                  rope, cluster, status);
+        e = cudaLaunchKernelEx(&cfg, kernel, mk, mv, (const bf16*)q, ldq, (bf16*)out, ldo, part_o, part_ml, block_tables,
+                               max_blocks, token_seq, positions, token_list, nh, nkv, page_size, window, scale, splits,
+                               rope, cluster, status);
+        return FERRIS_OK;
     };
 #define FERRIS_DECODE_LAUNCH_AS(DD, PP, NWW, STT)                                                                \
     do {                                                                                                         \
-        if (G <= 8) {                                                                                            \
-            if ((rc = set_smem(decode_attention_kernel<DD, STT, PP, NWW, true>, smem)) != FERRIS_OK) return rc;  \
-            e = launch(decode_attention_kernel<DD, STT, PP, NWW, true>);                                         \
-        } else {                                                                                                 \
-            if ((rc = set_smem(decode_attention_kernel<DD, STT, PP, NWW, false>, smem)) != FERRIS_OK) return rc; \
-            e = launch(decode_attention_kernel<DD, STT, PP, NWW, false>);                                        \
-        }                                                                                                        \
+        if (G <= 8)                                                                                              \
+            rc = token_list ? launch(decode_attention_kernel<DD, STT, PP, NWW, true, true>)                      \
+                            : launch(decode_attention_kernel<DD, STT, PP, NWW, true, false>);                    \
+        else                                                                                                     \
+            rc = token_list ? launch(decode_attention_kernel<DD, STT, PP, NWW, false, true>)                     \
+                            : launch(decode_attention_kernel<DD, STT, PP, NWW, false, false>);                   \
+        if (rc != FERRIS_OK) return rc;                                                                          \
     } while (0)
 #define FERRIS_DECODE_LAUNCH(DD, PP)                              \
     do {                                                          \
@@ -1799,15 +1802,15 @@ FERRIS_API int ferris_decode_cluster_splits(int tokens, int nkv, int d, int max_
             cudaError_t e = cudaSuccess;
             cfg.dynamicSmemBytes = (size_t)12 * 16384 + 1024 + (size_t)(MAX_CLUSTER * 2 * 16 + 16 * d + MAX_CLUSTER) * 4;
             if (sp > 8) {
-                if (d == 64) cudaFuncSetAttribute(decode_attention_kernel<64, 1, true, 12, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                else cudaFuncSetAttribute(decode_attention_kernel<128, 1, true, 12, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                if (d == 64) cudaFuncSetAttribute(decode_attention_kernel<64, 1, true, 12, true, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                else cudaFuncSetAttribute(decode_attention_kernel<128, 1, true, 12, true, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             }
             if (d == 64) {
-                set_smem(decode_attention_kernel<64, 1, true, 12, true>, cfg.dynamicSmemBytes);
-                e = cudaOccupancyMaxActiveClusters(&clusters, decode_attention_kernel<64, 1, true, 12, true>, &cfg);
+                set_smem(decode_attention_kernel<64, 1, true, 12, true, false>, cfg.dynamicSmemBytes);
+                e = cudaOccupancyMaxActiveClusters(&clusters, decode_attention_kernel<64, 1, true, 12, true, false>, &cfg);
             } else {
-                set_smem(decode_attention_kernel<128, 1, true, 12, true>, cfg.dynamicSmemBytes);
-                e = cudaOccupancyMaxActiveClusters(&clusters, decode_attention_kernel<128, 1, true, 12, true>, &cfg);
+                set_smem(decode_attention_kernel<128, 1, true, 12, true, false>, cfg.dynamicSmemBytes);
+                e = cudaOccupancyMaxActiveClusters(&clusters, decode_attention_kernel<128, 1, true, 12, true, false>, &cfg);
             }
             if (e == cudaSuccess && clusters > 0) have = clusters;
             else cudaGetLastError();

@@ -59,3 +59,12 @@ def test_tensor_memory_is_allocated_before_dependents_are_let_in(file, kernel, b
     for at in triggers:
         if at < allocated:
             assert "return;" in block_after(body, at), f"{file}: {kernel} lets dependents in before it has its tensor memory"
+
+
+def test_only_the_attention_of_listed_tokens_lets_the_next_launch_in_after_its_wait():
+    """The attention of portions may run beside it without a wait of its own, which is safe only when the launches before have
+    ended; every other launch behind this kernel waits by itself and is let in at once."""
+    (_, _, body), = [k for k in kernels_with("LISTED") if k[1] == "decode_attention_kernel"]
+    wait = body.index("pdl_wait();")
+    assert "if (!LISTED) pdl_launch_dependents();" in body[:wait]
+    assert body[wait:].split("pdl_wait();")[1].strip().startswith("if (LISTED) pdl_launch_dependents();")
