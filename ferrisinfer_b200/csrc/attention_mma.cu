@@ -1046,7 +1046,7 @@ struct MapCacheEntry {
 // and exchange 400, fold 400, exponentials and P 1,500, of which 1,024 is the special-function unit's time for
 // 16,384 exponentials), 3,400 at head size 128 (350, 470, 900, 1,670); two groups take about 4,400 cycles for two blocks (the second group's wait for the tensor
 // core and the shared special-function unit keep it from halving): 2,048-token prompt 31.2 -> 29.8 us, a portion of
-// 512 at the end of 4,096 keys 53.4 -> 44.9 us, 8,192-token prompt 326 -> 281 us.
+// 512 at the end of 4,096 keys 53.4 -> 44.9 us, 8,192-token prompt 326 -> 281 us (as it was measured then; now 27.4, 44.3 and 274).
 // Measured and not kept: one copy for the eight pages of a block where they lie one behind the other (3 to 10 % of the kernel, nothing of
 // a prompt's step); with the scores still in registers, a ring of K blocks apart from a ring of V blocks, so that a K stage is free as soon as
 // its scores are done (8,192-token prompt 281 -> 322 us at head size 64, 2,048 tokens at head size 128 43.7 -> 46.9 us).
@@ -1114,46 +1114,6 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     const int hk = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     FERRIS_TL_ENTRY();
-    if (!beside) pdl_wait();
-    FERRIS_TL_BEGIN();
-    // The grid holds at most one CTA a request and kv head more than there are row blocks, whatever the requests' lengths (a CTA
-    // without rows still takes a whole SM's shared memory: a step of 31 single tokens and one portion of 481 tokens launched 1,472
-    // CTAs for 46 row blocks and took 31 us): each warp finds the CTA's request by itself.
-    int seq = -1, rank = 0;
-    for (int s0 = 0, before = 0; s0 < num_seqs && seq < 0; s0 += 32) {
-        int n = 0;
-        if (s0 + lane < num_seqs) {
-            const int len = seq_q_start[s0 + lane + 1] - seq_q_start[s0 + lane];
-            n = skip_single && len == 1 ? 0 : (len * G + T5_ROWS - 1) / T5_ROWS;  // single tokens are the decode kernel's
-        }
-        int upto = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int x = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += x;
-        }
-        const unsigned here = __ballot_sync(0xffffffffu, (int)blockIdx.x < before + upto);
-        if (here) {
-            const int at = __ffs(here) - 1;
-            seq = s0 + at;
-            rank = (int)blockIdx.x - before - __shfl_sync(0xffffffffu, upto - n, at);
-        }
-        before += __shfl_sync(0xffffffffu, upto, 31);
-    }
-    if (seq < 0) {
-        pdl_launch_dependents();
-        if (beside) pdl_wait();
-        FERRIS_TL_END(8);
-        return;
-    }
-    const int q_start = seq_q_start[seq], q_len = seq_q_start[seq + 1] - q_start;
-    const int rows_total = q_len * G;
-    const int n_blocks = (rows_total + T5_ROWS - 1) / T5_ROWS;
-    const int block = n_blocks - 1 - rank;  // heavy row blocks (the last tokens see the most keys) first
-    const int row0 = block * T5_ROWS;
-    const int start_pos = seq_start_pos[seq];
-    const int* table = block_tables + (size_t)seq * max_blocks;
-
     if (threadIdx.x == 0) {
         tma_prefetch_descriptor(&map_k);
         tma_prefetch_descriptor(&map_v);
@@ -1178,7 +1138,53 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
     tcgen05_fence_after();
     // Only now: this kernel takes all of an SM's tensor memory.  A dependent product whose shared memory fits beside it (one
     // K slice of a few tokens, 20 KB) could otherwise take its columns first and then wait for this grid, which would wait for them.
+    // (Ahead of the wait as well, the output product's weights came in against those of the q/k/v product: a step of 40 tokens at
+    // the 1.5B sizes 1,842 -> 1,878 us.)
+    if (!beside) pdl_wait();
     pdl_launch_dependents();
+    FERRIS_TL_BEGIN();
+    // The grid holds at most one CTA a request and kv head more than there are row blocks, whatever the requests' lengths (a CTA
+    // without rows still takes a whole SM's shared memory: a step of 31 single tokens and one portion of 481 tokens launched 1,472
+    // CTAs for 46 row blocks and took 31 us): each warp finds the CTA's request by itself, a lane a request, with one trip to
+    // memory.
+    int seq = -1, rank = 0, q_start = 0, q_len = 0, start_pos = 0;
+    for (int s0 = 0, before = 0; s0 < num_seqs && seq < 0; s0 += 32) {
+        int n = 0, first = 0, len = 0, pos = 0;
+        if (s0 + lane < num_seqs) {
+            first = seq_q_start[s0 + lane];
+            len = seq_q_start[s0 + lane + 1] - first;
+            pos = seq_start_pos[s0 + lane];
+            n = skip_single && len == 1 ? 0 : (len * G + T5_ROWS - 1) / T5_ROWS;  // single tokens are the decode kernel's
+        }
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+        }
+        const unsigned here = __ballot_sync(0xffffffffu, (int)blockIdx.x < before + upto);
+        if (here) {
+            const int at = __ffs(here) - 1;
+            seq = s0 + at;
+            rank = (int)blockIdx.x - before - __shfl_sync(0xffffffffu, upto - n, at);
+            q_start = __shfl_sync(0xffffffffu, first, at);
+            q_len = __shfl_sync(0xffffffffu, len, at);
+            start_pos = __shfl_sync(0xffffffffu, pos, at);
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (seq < 0) {
+        if (warp == SW + 1) tmem_dealloc(tmem_base, TMEM_COLS);
+        if (beside) pdl_wait();
+        FERRIS_TL_END(8);
+        return;
+    }
+    const int rows_total = q_len * G;
+    const int n_blocks = (rows_total + T5_ROWS - 1) / T5_ROWS;
+    const int block = n_blocks - 1 - rank;  // heavy row blocks (the last tokens see the most keys) first
+    const int row0 = block * T5_ROWS;
+    const int* table = block_tables + (size_t)seq * max_blocks;
+
     const uint32_t tmem_s = tmem_base, tmem_pv = tmem_base + 256;  // block i's scores at + 128 (i % 2); group g's product at + D g
 
     // keys of the block: from the first key its first token may see to its last token's position
@@ -1348,10 +1354,16 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
             const bool interior = key_base >= lo && key_base + 63 <= hi;
             // The scores stay in tensor memory, read in chunks for the maximum and again for the exponentials.  (One group used to
             // keep its 64 in registers beside 64 output columns at head size 128: 35 of them spilled, and bringing the row to
-            // the new maximum took 2,200 cycles of a block's 4,700; now 900 of 3,400.  Head size 128, us, before / now, one prompt
-            // of 2,048 tokens with 12 heads over 2 45.9 / 38.5, with 28 over 4 91.6 / 77.8, of 8,192 422 / 360, of 512 17.5 / 14.4.)
+            // the new maximum took 2,200 cycles of a block's 4,700; now 900 of 3,400.)
+            // Both loops over the chunks stay loops.  Where a layer's weights (1.5B sizes and more) push the kernel's code out of
+            // L2 between two layers, a short prompt pays for every instruction that it fetches once: unrolled, the only
+            // block's exponentials took 7,000 cycles, and not 4,300 with the scores in registers.  us, scores in registers /
+            // in tensor memory and unrolled / now: a step of 16 tokens at the 1.5B sizes 1,853 / 1,885 / 1,810, of 40 tokens 1,903 / 1,971 /
+            // 1,842, at the 7B sizes 4,119 / 4,157 / 4,069; the kernel alone, code at hand, head size 128, one prompt of 2,048
+            // tokens with 12 heads over 2 46.6 / 39.3 / 37.2, with 28 over 4 91.7 / 80.0 / 73.6, of 8,192 429 / 365 / 354, of 512 17.3 /
+            // 14.0 / 14.0; head size 64 (in tensor memory before too), 14 heads over 2, 2,048 tokens 29.6 / 27.4, 8,192 280 / 274.
             float mx = -INFINITY;
-#pragma unroll
+#pragma unroll 1  // (see above)
             for (int h = 0; h < 2; ++h) {
                 uint32_t sc[32];
                 tmem_load_32x32(my_s + 32 * h, sc);
@@ -1401,7 +1413,7 @@ __global__ void __launch_bounds__(t5_threads(GROUPS), 1)
             {
                 float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // four partial sums: the additions do not wait for one another
                 uint8_t* half = p_smem + g * P_BYTES + kh * 16384;
-#pragma unroll
+#pragma unroll 1  // (see above)
                 for (int h = 0; h < 4; ++h) {  // 16 keys at a time
                     uint32_t sc[16], packed[8];
                     tmem_load_32x16(my_s + 16 * h, sc);
