@@ -345,7 +345,8 @@ int launch_tile(TileParams& p, dim3 grid, cudaStream_t s) {
 }
 
 constexpr size_t MAX_SMEM = 227 * 1024;
-constexpr int TILE_SPLIT = 2 * 148;  // fewer tiles than two an SM: the parts of K side by side
+constexpr int SMS = 148;
+constexpr int TILE_SPLIT = 2 * SMS;  // fewer tiles than two an SM: the parts of K side by side
 
 // How few tokens are cut (N weight rows; unit: a CTA's are a multiple of so many); false: they do not fit.
 bool rows_plan(int M, int N, int K, int unit, RowsPlan& q) {
@@ -353,7 +354,7 @@ bool rows_plan(int M, int N, int K, int unit, RowsPlan& q) {
     q.phases = (K + PHASE - 1) / PHASE;
     for (int tt = M >= 5 ? 8 : M >= 3 ? 4 : M; tt >= 1; tt /= 2) {
         q.TT = tt;
-        const int rows = ((N + 147) / 148 + unit - 1) / unit * unit;
+        const int rows = ((N + SMS - 1) / SMS + unit - 1) / unit * unit;
         q.rows_per_cta = rows > ROWS_CAP ? ROWS_CAP : rows;
         const size_t round = (size_t)ROWS_WARPS * RS * W_PITCH * 4;  // a stage for every warp
         const size_t fixed = 2 * ROWS_MAX_STAGES * sizeof(uint64_t) + (size_t)tt * runs * X_PITCH * 4 +
@@ -370,7 +371,45 @@ bool rows_plan(int M, int N, int K, int unit, RowsPlan& q) {
     return false;
 }
 
+// Whether few tokens are better off with the rows kernel, cut so, than with the tiles.  The rows kernel goes over the weights
+// once for every q.TT tokens, and the longer K is the fewer tokens' rows fit (eight up to K = 3,584 or so, four at 4,864 to 8,960 and for
+// 37,888 rows of 3,584, one at 18,944); the tiles do the work of 64 tokens whatever their number.  Both from estimates: a round of the
+// rows kernel's CTAs takes in weights at the rates below (KB a microsecond a CTA; two share an SM where their memory allows), a
+// tile's CTA 0.09 us a k, three to an SM.  They are within a fifth or so, and the rows kernel is left only where it loses by more
+// (us, rows / tiles, tokens: 3,584 x 18,944 three 263 / 280, four 351 / 280, eight 614 / 281, sixteen 1,139 / 280; 37,888 x 3,584 eight 282 / 409, twelve
+// 423 / 409, sixteen 563 / 409; sixteen tokens: 9,728 x 896 38 / 44, 896 x 4,864 35 / 51, 17,920 x 1,536 85 / 98, 1,536 x 8,960 82 / 92, 4,608 x 3,584
+// 55 / 79, 3,584 x 3,584 53 / 50).
+bool rows_pay(int M, int N, int K, const RowsPlan& q) {
+    const int each = q.smem <= ROWS_SMEM ? 2 : 1;
+    const long long ctas = (long long)((N + q.rows_per_cta - 1) / q.rows_per_cta) * ((M + q.TT - 1) / q.TT);
+    const double rate = each == 2 ? 12.5e3 : q.TT == 8 ? 17.5e3 : q.TT == 4 ? 23e3 : 27e3;
+    const double t_rows = (double)((ctas + SMS * each - 1) / (SMS * each)) * q.rows_per_cta * K * 4.0 / rate;
+    const int runs = (K + F32_CHUNK - 1) / F32_CHUNK, per = f32_runs_per_part(runs);
+    long long tiles = (long long)((N + BN - 1) / BN) * ((M + BM - 1) / BM);
+    double k = K;
+    if (tiles < TILE_SPLIT) {
+        tiles *= (runs + per - 1) / per;
+        k = runs > per ? per * F32_CHUNK : K;
+    }
+    const double t_tiles = 0.09 * k * (tiles > 3 * SMS ? (double)tiles / (3 * SMS) : 1.0);
+    return t_rows <= 1.25 * t_tiles;
+}
+
+// The rows kernel up to 16 tokens, and up to 32 where the weights are few (us at 32 / 33 tokens: 9728 x 896 62 / 44, 896 x 4864 67 / 49,
+// 151936 x 896 730 / 422, but 1152 x 896 11 / 18), where it pays.
+bool rows_take(int M, int N, int K, int unit, RowsPlan& q) {
+    return (M <= 16 || (M <= 32 && (long long)N * K <= (1 << 21))) && rows_plan(M, N, K, unit, q) && rows_pay(M, N, K, q);
+}
+
 }  // namespace
+
+// How a 32-bit product of aligned rows is cut: tokens of a CTA of the rows kernel, 0 where the tiles take it (swiglu: N outputs of
+// 2 N weight rows; 0 also where SwiGLU does not ride along).
+FERRIS_API int ferris_gemm_f32_plan(int M, int N, int K, int swiglu) {
+    RowsPlan q;
+    if (M <= 0 || N <= 0 || K <= 0 || K & 3) return 0;
+    return rows_take(M, swiglu ? 2 * N : N, K, swiglu ? 2 * RS : RS, q) ? q.TT : 0;
+}
 
 bool ferris_gemm_f32_takes(const void* x, const void* w, const void* out, int K, int ldx, int ldw) {
     return !(K & 3) && !(ldx & 3) && !(ldw & 3) && !(((uintptr_t)x | (uintptr_t)w) & 15) && K <= 65536;
@@ -380,10 +419,7 @@ int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* ou
                     int ldo, int accumulate, cudaStream_t s, bool* taken) {
     *taken = true;
     RowsPlan q;
-    // Up to 16 tokens, and up to 32 where the weights are few: the rows kernel reads the weights once for every eight tokens,
-    // the tiles do the work of 64 (us at 16 / 32 / 33 tokens: 9728 x 896 42 / 62 / 44, 896 x 4864 38 / 67 / 49, 151936 x 896
-    // 379 / 730 / 422, but 1152 x 896 6 / 11 / 18).
-    if ((M <= 16 || (M <= 32 && (long long)N * K <= (1 << 21))) && rows_plan(M, N, K, RS, q)) {
+    if (rows_take(M, N, K, RS, q)) {
         RowsParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), 0};
         return launch_rows_of(p, q, s);
     }
@@ -401,10 +437,11 @@ int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* ou
 
 constexpr int SWIGLU_MAX_TOKENS = 16;  // (beyond, the plain product may run the tiles)
 
-// Whether ferris_gemm_f32_swiglu takes a product of M tokens and N outputs: 16 tokens at most, rows that begin on 16 bytes.
+// Whether ferris_gemm_f32_swiglu takes a product of M tokens and N outputs: 16 tokens at most, rows that begin on 16 bytes, and
+// weights that the rows kernel reads in fewer microseconds than the tiles.
 FERRIS_API int ferris_gemm_f32_swiglu_takes(const void* x, const void* w, int M, int N, int K, int ldx, int ldw) {
     RowsPlan q;
-    return M > 0 && M <= SWIGLU_MAX_TOKENS && N > 0 && ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw) && rows_plan(M, 2 * N, K, 2 * RS, q);
+    return M > 0 && M <= SWIGLU_MAX_TOKENS && N > 0 && ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw) && rows_take(M, 2 * N, K, 2 * RS, q);
 }
 // out[t, n] = silu(x[t] . w[n]) (x[t] . w[N + n]), fp32 throughout, with the sums of every other form of the product.
 FERRIS_API int ferris_gemm_f32_swiglu(const float* x, const float* w, float* out, int M, int N, int K, int ldx, int ldw, int ldo,

@@ -252,6 +252,11 @@ def gemm_tcgen05(x, w, bias, out, mode: int, n_out: Optional[int] = None, up_row
     )
 
 
+def gemm_f32_plan(tokens: int, outputs: int, k: int, swiglu: bool = False) -> int:
+    """Tokens that a block of the 32-bit kernel for few tokens takes (aligned rows); 0: the product runs the tiles."""
+    return int(_lib().ferris_gemm_f32_plan(_c_int(tokens), _c_int(outputs), _c_int(k), _c_int(1 if swiglu else 0)))
+
+
 def gemm_plan(tokens: int, outputs: int, k: int, accumulators: int = 1) -> tuple[int, int]:
     """How the short-step tcgen05 kernel would cut a product: (token tile, K splits)."""
     bt, splits, floats, counters = _c_int(), _c_int(), ctypes.c_longlong(), _c_int()
@@ -566,7 +571,7 @@ def gemm_activation(x, w, out, kind: str, coefficients=(0.0, 0.0), params: Optio
 
 def gemm_swiglu(x, gate_up_weight, out, workspace=None):
     """out [T, I] = silu(x Wg^T) * (x Wu^T) with gate_up_weight = [Wg; Wu] ([2I, K]).  bf16: one tensor-core
-    kernel with two accumulators (the [T, 2I] intermediate never exists), so too 32-bit steps of at most 16 tokens; otherwise
+    kernel with two accumulators (the [T, 2I] intermediate never exists), so too 32-bit steps of few tokens; otherwise
     a product and the SwiGLU kernel."""
     T, I = out.shape
     if gate_up_weight.shape[0] != 2 * I:

@@ -149,6 +149,31 @@ def test_gemm_fp32_with_swiglu_on_the_way(N, K, device):
     assert ops.kernel_status() == 0
 
 
+@pytest.mark.parametrize("N, K", [(3584, 18944), (18944, 3584)])
+def test_gemm_fp32_gives_a_row_the_same_bits_on_either_side_of_the_rule(N, K, device):
+    """Long rows (the 7B down projection) and many of them: from some number of tokens on the tiles take the product."""
+    from ferrisinfer_b200.kernels import ops
+
+    w, x = rnd((N, K), F32, device, 50, scale=0.05), rnd((16, K), F32, device, 51)
+    plans = [ops.gemm_f32_plan(M, N, K) for M in (1, 3, 8, 16)] + [ops.gemm_f32_plan(M, N // 2, K, True) for M in (8, 16)]
+    assert 0 in plans and any(plans)
+    full = torch.empty(16, N, device=device)
+    ops.gemm_simt(x, w, None, full)
+    bound = (128 + K / 1024 + 8 + 3) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert ((full.double() - x.double() @ w.double().t()).abs() <= bound).all()
+    for M in (1, 2, 3, 4, 8, 12):
+        out = torch.empty(M, N, device=device)
+        ops.gemm_simt(x[:M], w, None, out)
+        assert torch.equal(out, full[:M]), M
+    want = torch.empty(16, N // 2, device=device)
+    ops.swiglu(full, want)
+    for M in (2, 8, 12, 16):
+        out = torch.empty(M, N // 2, device=device)
+        ops.gemm_swiglu(x[:M], w, out)
+        assert torch.equal(out, want[:M]), M
+    assert ops.kernel_status() == 0
+
+
 # ------------------------------------------------------------------------- tensor-core gemm
 TC_SHAPES = [(1, 1152, 896), (8, 1152, 896), (64, 896, 4864), (5, 130, 72), (16, 128, 64), (17, 300, 1000),
              (300, 256, 128), (2048, 384, 256), (33, 1000, 80), (257, 129, 200),
