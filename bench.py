@@ -406,19 +406,19 @@ def kernel_numbers(engine, cfg, peaks) -> dict:
     x = torch.randn(T, H, device=dev).to(torch.bfloat16)
     act = torch.empty(T, I, dtype=torch.bfloat16, device=dev)
     h = torch.zeros(T, H, dtype=torch.float32, device=dev)
-    sec = timed(lambda: [ops.gemm_swiglu(x, b.feed_forward.gate_up, act) for b in blocks])
+    sec = timed(lambda: [ops.gemm_swiglu(x, b.feed_forward.gate_up, act, fixed_weight=True) for b in blocks])
     out["decode_gate_up_gbs"] = round(2 * I * H * 2 / sec / 1e9, 1)
-    sec = timed(lambda: [ops.gemm(act, b.feed_forward.down, None, h, accumulate=True) for b in blocks])
+    sec = timed(lambda: [ops.gemm(act, b.feed_forward.down, None, h, accumulate=True, fixed_weight=True) for b in blocks])
     out["decode_down_gbs"] = round(I * H * 2 / sec / 1e9, 1)
     # the output head, 8 rows
     logits = torch.empty(T, n["V"], dtype=torch.float32, device=dev)
     w_head = engine.model.output.weight
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    ops.gemm(x, w_head, None, logits)
+    ops.gemm(x, w_head, None, logits, fixed_weight=True)
     torch.cuda.synchronize()
     e0.record()
     for _ in range(4):
-        ops.gemm(x, w_head, None, logits)
+        ops.gemm(x, w_head, None, logits, fixed_weight=True)
     e1.record()
     torch.cuda.synchronize()
     out["lm_head_gbs"] = round(n["V"] * H * 2 / (e0.elapsed_time(e1) * 1e-3 / 4) / 1e9, 1)
@@ -449,7 +449,7 @@ def kernel_numbers(engine, cfg, peaks) -> dict:
     Tp = PREFILL_TOKENS
     xp = torch.randn(Tp, H, device=dev).to(torch.bfloat16)
     actp = torch.empty(Tp, I, dtype=torch.bfloat16, device=dev)
-    sec = timed(lambda: [ops.gemm_swiglu(xp, b.feed_forward.gate_up, actp) for b in blocks])
+    sec = timed(lambda: [ops.gemm_swiglu(xp, b.feed_forward.gate_up, actp, fixed_weight=True) for b in blocks])
     out["prefill_gate_up_tflops"] = round(2.0 * Tp * 2 * I * H / sec / 1e12, 1)
     if have >= Tp // 16:
         tables = torch.arange(Tp // 16, dtype=torch.int32, device=dev).view(1, -1)

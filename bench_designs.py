@@ -556,8 +556,8 @@ def netinex_kernel_numbers(s: dict, peaks: dict) -> dict:
         act = torch.empty(T, ff, dtype=bf, device=dev)
 
         def dense():
-            ops.gemm_activation(x, w_up, act, "silu")
-            ops.gemm(act, w_down, None, hrow, accumulate=True)
+            ops.gemm_activation(x, w_up, act, "silu", fixed_weight=True)
+            ops.gemm(act, w_down, None, hrow, accumulate=True, fixed_weight=True)
 
         t = _timed(dense, flush)
         record(f"dense_feed_forward_{tag}", t, bytes_=2 * W * ff * 2 + T * W * (2 + 8), tensor_flops=2.0 * T * 2 * W * ff)
@@ -690,7 +690,7 @@ def sumevik_kernel_numbers(s: dict, peaks: dict) -> dict:
         x = torch.randn(T, W, device=dev).to(bf)
         act = torch.empty(T, inter, dtype=bf, device=dev)
         for kind in ("gelu_tanh", "silu"):
-            t = _timed(lambda: ops.gemm_gated(x, gate_up_w, act, kind, 0.0, ws), flush)
+            t = _timed(lambda: ops.gemm_gated(x, gate_up_w, act, kind, 0.0, ws, fixed_weight=True), flush)
             record(f"gated_product_{kind}_{tag}", t, bytes_=2 * inter * W * 2 + T * (W + inter) * 2,
                    tensor_flops=2.0 * T * 2 * inter * W)
     # ---- the scored router and the experts with a clamped gate and identity experts
@@ -822,7 +822,7 @@ def retezen_kernel_numbers(s: dict, peaks: dict) -> dict:
         x = torch.randn(T, W, device=dev).to(bf)
         act = torch.empty(T, inter, dtype=bf, device=dev)
         for kind in ("clamped_swish", "silu"):
-            t = _timed(lambda: ops.gemm_gated(x, gate_up_w, act, kind, 7.0, ws), flush)
+            t = _timed(lambda: ops.gemm_gated(x, gate_up_w, act, kind, 7.0, ws, fixed_weight=True), flush)
             record(f"gated_product_{kind}_{tag}", t, bytes_=2 * inter * W * 2 + T * (W + inter) * 2,
                    tensor_flops=2.0 * T * 2 * inter * W)
     # ---- the sigmoid router and the experts with weights on their inputs
@@ -965,7 +965,7 @@ def lukelorn_kernel_numbers(s: dict, peaks: dict) -> dict:
         t = _timed(lambda: ops.short_conv(wide[:, :C], conv, cw, cs, ctx, residual=False, silu=True), flush, reps=reps)
         record(f"conv_silu_{name}", t, bytes_=T * C * 4 + (S * 3 * C * 8 if q_len == 1 else 0))
         a1, a2, dt = randn(T, d).to(bf), (randn(H * d, d) / math.sqrt(d)).to(bf), torch.zeros(H * d, device=dev)
-        t = _timed(lambda: ops.gemm(a1, a2, dt, z), flush, reps=reps)
+        t = _timed(lambda: ops.gemm(a1, a2, dt, z, fixed_weight=True), flush, reps=reps)
         record(f"decay_product_{name}", t, bytes_=T * (d * 2 + H * d * 4) + H * d * d * 2, tensor_flops=2.0 * T * H * d * d)
         y, gate = torch.empty(T, H * d, dtype=bf, device=dev), randn(T, H * d).to(bf)
         nw = torch.ones(d, device=dev)

@@ -45,7 +45,9 @@ typedef __nv_bfloat16 bf16;
 // Programmatic dependent launch: a kernel launched through ferris_launch may begin while the kernel
 // before it in the stream is still draining.  Its set-up (barriers, tensor memory, descriptor
 // prefetch) overlaps that tail; pdl_wait() then blocks until the earlier kernel has completed and its
-// writes are visible, and must come before the first access to global memory.
+// writes are visible, and must come before the first access to global memory that an earlier launch may have written.
+// A model's weights and a step's metadata are written by none; where a product's second operand may be something else, its
+// kernel is told (early_weights: ferris_gemm_simt, ferris_gemm_tcgen05, ferris_qkv_rope_gemm_tcgen05, ferris_gemm_f32_swiglu).
 // pdl_launch_dependents() lets the NEXT kernel start its own set-up early; it takes effect once every
 // CTA of this grid has called it (or exited), so CTAs that are not resident yet are never starved.
 // Launched without the attribute (FERRIS_PDL=0), both are no-ops.
@@ -58,7 +60,7 @@ typedef __nv_bfloat16 bf16;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-bool ferris_pdl_enabled();
+bool ferris_pdl_enabled();  // (not while the calling thread asks for stream order: ferris_in_stream_order)
 
 template <typename Kernel, typename... Args>
 inline cudaError_t ferris_launch(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

@@ -6,8 +6,8 @@
 // and CTAs work on one output; they also halve the rounding error of one long chain.
 //
 // gemm_f32_rows_kernel: few tokens (decode steps).  Bound by reading the weights once.  The weight ROWS are divided among
-// the CTAs; a producer warp streams them through a ring of stages (bulk copies, a row a copy, requested before the launch
-// wait), the step's rows lie in shared memory, and a lane sums one run of one weight row for all tokens: eight
+// the CTAs; a producer warp streams them through a ring of stages (bulk copies, a row a copy; a model's weights before the
+// launch wait), the step's rows lie in shared memory, and a lane sums one run of one weight row for all tokens: eight
 // lanes take eight rows, four such groups four runs, so that every shared-memory read of weights is free of conflicts and
 // every read of a token's values is shared by eight lanes.  The runs' sums meet in shared memory and are added in order.
 // What binds it beside HBM is what shared memory returns to the lanes: 16 bytes a lane take four cycles, shared or not, so a
@@ -51,6 +51,7 @@ struct RowsParams {
     int M, N, K, ldx, ldw, ldo, accumulate;
     int rows_per_cta, phases, stages;  // stages: a multiple of ROWS_WARPS, so that one warp takes a stage every time
     int* status;
+    int early_weights;  // no launch that may still run writes w: its rows are requested ahead of the launch wait
     int up_offset;  // > 0: SwiGLU, out[t, n] of gate row n and up row up_offset + n; N outputs of 2 N weight rows
 };
 
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const RowsP
     __syncthreads();
     pdl_launch_dependents();
     if (warp == ROWS_WARPS) {
+        if (!p.early_weights) pdl_wait();
         const int total = groups * p.phases;
         for (int it = 0; it < total; ++it) {
             const int s = it % p.stages, round = it / p.stages;
@@ -416,11 +418,12 @@ bool ferris_gemm_f32_takes(const void* x, const void* w, const void* out, int K,
 }
 
 int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx, int ldw,
-                    int ldo, int accumulate, cudaStream_t s, bool* taken) {
+                    int ldo, int accumulate, int early_weights, cudaStream_t s, bool* taken) {
     *taken = true;
     RowsPlan q;
     if (rows_take(M, N, K, RS, q)) {
-        RowsParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), 0};
+        RowsParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(),
+                        early_weights, 0};
         return launch_rows_of(p, q, s);
     }
     const int runs = (K + F32_CHUNK - 1) / F32_CHUNK, per = f32_runs_per_part(runs);
@@ -444,14 +447,15 @@ FERRIS_API int ferris_gemm_f32_swiglu_takes(const void* x, const void* w, int M,
     return M > 0 && M <= SWIGLU_MAX_TOKENS && N > 0 && ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw) && rows_take(M, 2 * N, K, 2 * RS, q);
 }
 // out[t, n] = silu(x[t] . w[n]) (x[t] . w[N + n]), fp32 throughout, with the sums of every other form of the product.
+// early_weights: no launch that may still run writes w.
 FERRIS_API int ferris_gemm_f32_swiglu(const float* x, const float* w, float* out, int M, int N, int K, int ldx, int ldw, int ldo,
-                                      void* stream) {
+                                      int early_weights, void* stream) {
     if (M <= 0 || N <= 0) return FERRIS_OK;
     if (K <= 0 || ldx < K || ldw < K || ldo < N) FERRIS_REFUSE("gemm: K=%d, row strides %d, %d, %d", K, ldx, ldw, ldo);
     if (!ferris_gemm_f32_swiglu_takes(x, w, M, N, K, ldx, ldw))
         FERRIS_REFUSE("gemm: %d tokens x %d outputs of %d do not take SwiGLU on the way", M, N, K);
     RowsPlan q;
     rows_plan(M, 2 * N, K, 2 * RS, q);
-    RowsParams p = {x, w, nullptr, out, M, N, K, ldx, ldw, ldo, 0, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), N};
+    RowsParams p = {x, w, nullptr, out, M, N, K, ldx, ldw, ldo, 0, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), early_weights, N};
     return launch_rows_of(p, q, (cudaStream_t)stream);
 }

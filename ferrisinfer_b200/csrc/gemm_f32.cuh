@@ -12,5 +12,6 @@ __host__ __device__ inline int f32_runs_per_part(int runs) {
 
 bool ferris_gemm_f32_takes(const void* x, const void* w, const void* out, int K, int ldx, int ldw);
 // `taken` false: nothing was launched (sizes that no form takes).
+// early_weights: no launch that may still run writes w.
 int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx, int ldw,
-                    int ldo, int accumulate, cudaStream_t s, bool* taken);
+                    int ldo, int accumulate, int early_weights, cudaStream_t s, bool* taken);

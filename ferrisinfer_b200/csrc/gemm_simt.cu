@@ -109,8 +109,9 @@ int launch(const void* x, const void* w, const float* bias, void* out, int M, in
 
 // x: [M, K] rows ldx apart; w: [N, K] rows ldw apart; out: [M, N] rows ldo apart.
 // in_dtype is the type of x and w; out_dtype that of out; accumulate != 0 needs an fp32 out.
+// early_weights: no launch that may still run writes w (the 32-bit kernel for few tokens then requests it ahead of its launch wait).
 FERRIS_API int ferris_gemm_simt(const void* x, const void* w, const float* bias, void* out, int in_dtype,
-                                int out_dtype, int M, int N, int K, int ldx, int ldw, int ldo, int accumulate,
+                                int out_dtype, int M, int N, int K, int ldx, int ldw, int ldo, int accumulate, int early_weights,
                                 void* stream) {
     if (M <= 0 || N <= 0) return FERRIS_OK;
     if (K <= 0) FERRIS_REFUSE("gemm: K=%d", K);
@@ -120,7 +121,8 @@ FERRIS_API int ferris_gemm_simt(const void* x, const void* w, const float* bias,
     cudaStream_t s = (cudaStream_t)stream;
     if (in_dtype == FERRIS_F32 && out_dtype == FERRIS_F32 && ferris_gemm_f32_takes(x, w, out, K, ldx, ldw)) {
         bool taken;
-        const int rc = ferris_gemm_f32((const float*)x, (const float*)w, bias, (float*)out, M, N, K, ldx, ldw, ldo, accumulate, s, &taken);
+        const int rc = ferris_gemm_f32((const float*)x, (const float*)w, bias, (float*)out, M, N, K, ldx, ldw, ldo, accumulate, early_weights, s,
+                                       &taken);
         if (taken) return rc;
     }
     if (in_dtype == FERRIS_F32 && out_dtype == FERRIS_F32)

@@ -681,6 +681,7 @@ struct PTParams {
     int m_tiles, n_tiles;
     int up_row_offset;
     int* status;
+    int early_weights = 0;  // no launch that may still run writes the weights: the first slices are requested ahead of the wait
     int splits, kb_per;  // CTA pairs only: pairs that share a tile's K slices, and the slices of each but the last
     RopeEpilogue rope;  // mode QKV_ROPE_BF16 only
     FerrisEpilogueAct act;  // applied by the bf16 store (mode STORE_BF16)
@@ -950,7 +951,7 @@ __global__ void __launch_bounds__(PT_THREADS)
     tcgen05_fence_after();
     const uint32_t tmem = tmem_base;
     pdl_launch_dependents();
-    // The weights of the first tile's first slices are requested ahead of the wait (no launch writes them, unless the tile's
+    // The weights of the first tile's first slices are requested ahead of the wait (where no launch writes them, and no tile's
     // expert says which they are), the tokens after it: a weight's first slices come from HBM while the launch before ends (us a
     // product in a row of them: 9,728 x 896 at 256 to 2,048 tokens 14.0 / 19.1 / 25.3 / 36.8 -> 13.5 / 18.1 / 24.3 / 35.7)
     int early = 0;
@@ -961,7 +962,7 @@ __global__ void __launch_bounds__(PT_THREADS)
         tma_load_2d(st + a_bytes, &map_w, kb * BLOCK_K, row, bar);
         if (ACCS == 2) tma_load_2d(st + a_bytes + b_bytes, &map_w, kb * BLOCK_K, p.up_row_offset + row, bar);
     };
-    if (threadIdx.x == 0 && !GROUPED) {
+    if (threadIdx.x == 0 && !GROUPED && p.early_weights) {
         early = min(PT_STAGES, p.kblocks);
         for (int kb = 0; kb < early; ++kb) load_weights(kb, kb, ((int)blockIdx.x / p.m_tiles) * p.bn, a_bytes);
     }
@@ -1139,7 +1140,7 @@ __global__ void __launch_bounds__(PT_THREADS)
         tma_load_2d_pair(smem + (size_t)s * stage_bytes + a_bytes, &map_w, kb * BLOCK_K, row, leader_full + 8u * s);
     };
     int early = 0;  // slices whose weights are requested ahead of the wait, as above
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && p.early_weights) {
         early = min(PP_STAGES, kb1 - kb0);
         for (int i = 0; i < early; ++i) load_weights(i, kb0 + i, weight_row(pair));
     }
@@ -1780,13 +1781,15 @@ FERRIS_API int ferris_gemm_tcgen05_fuses_gated_activation(int T, int N, int K, i
 
 static int gemm_tcgen05_impl(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
                              int ldx, int ldw, int ldo, int rows_w, int up_row_offset, float* scratch, int* counters,
-                             void* stream, const TokenSource& src);
+                             int early_weights, void* stream, const TokenSource& src);
 
+// early_weights: no launch that may still run writes w (long steps then request it ahead of the launch wait; the kernel of short
+// steps always does).
 FERRIS_API int ferris_gemm_tcgen05(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N,
                                    int K, int ldx, int ldw, int ldo, int rows_w, int up_row_offset, float* scratch,
-                                   int* counters, void* stream) {
+                                   int* counters, int early_weights, void* stream) {
     return gemm_tcgen05_impl(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, scratch, counters,
-                             stream, TokenSource());
+                             early_weights, stream, TokenSource());
 }
 
 // The same product with RMSNorm fused in front: x = bf16((h * rstd(h)) * norm_w) is formed inside the kernel from the
@@ -1802,7 +1805,7 @@ FERRIS_API int ferris_norm_gemm_tcgen05(const float* h, const float* norm_w, flo
     src.norm_h = h;
     src.norm_w = norm_w;
     src.norm_eps = norm_eps;
-    return gemm_tcgen05_impl(w, w, bias, out, mode, T, N, K, K, ldw, ldo, rows_w, up_row_offset, nullptr, nullptr, stream,
+    return gemm_tcgen05_impl(w, w, bias, out, mode, T, N, K, K, ldw, ldo, rows_w, up_row_offset, nullptr, nullptr, 1, stream,
                              src);
 }
 
@@ -1825,7 +1828,7 @@ FERRIS_API int ferris_merge_gemm_tcgen05(const float* scratch_parts, int heads, 
     src.merge_heads = heads;
     src.merge_d = d;
     const int K = heads * d;
-    return gemm_tcgen05_impl(w, w, bias, out, mode, T, N, K, K, ldw, ldo, rows_w, 0, nullptr, nullptr, stream, src);
+    return gemm_tcgen05_impl(w, w, bias, out, mode, T, N, K, K, ldw, ldo, rows_w, 0, nullptr, nullptr, 1, stream, src);
 }
 
 // The activation that the product being launched applies in its bf16 store (taken from ferris_gemm_set_activation at
@@ -1836,7 +1839,8 @@ static FerrisEpilogueAct g_launch_act = {0, 0.0f, 0.0f};
 
 // A long step on CTA pairs (see gemm_tokens_pair_kernel).
 static int run_pairs(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K, int ldx, int ldw,
-                     int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope, const PairPlan& plan, cudaStream_t s) {
+                     int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope, const PairPlan& plan, int early_weights,
+                     cudaStream_t s) {
     const int accs = mode == SWIGLU_BF16 ? 2 : 1;
     PTParams q;
     q.out = out;
@@ -1849,6 +1853,7 @@ static int run_pairs(const void* x, const void* w, const float* bias, void* out,
     q.m_tiles = (T + 2 * PT_BLOCK_M - 1) / (2 * PT_BLOCK_M);
     q.bn = plan.bn;
     q.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+    q.early_weights = early_weights;
     q.kb_per = (q.kblocks + plan.splits - 1) / plan.splits;
     q.splits = plan.splits;
     q.n_tiles = (N + q.bn - 1) / q.bn;
@@ -1886,7 +1891,7 @@ static int run_pairs(const void* x, const void* w, const float* bias, void* out,
 // The persistent token-major kernel for a long step (T >= 128 tokens; output rows aligned for 16-byte stores).
 static int run_tokens_m(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
                         int ldx, int ldw, int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope,
-                        cudaStream_t s, const int* tile_expert = nullptr, const int* tile_rows = nullptr, int experts = 0,
+                        int early_weights, cudaStream_t s, const int* tile_expert = nullptr, const int* tile_rows = nullptr, int experts = 0,
                         int expert_rows = 0, const float* row_scale = nullptr) {
     const int accs = mode == SWIGLU_BF16 ? 2 : 1;
     const int elt = (mode == STORE_F32 || mode == ACCUM_F32) ? 4 : 2;
@@ -1909,6 +1914,7 @@ static int run_tokens_m(const void* x, const void* w, const float* bias, void* o
     q.up_row_offset = up_row_offset;
     q.status = ferris_status_ptr();
     q.rope = rope ? *rope : RopeEpilogue{};
+    q.early_weights = early_weights;
     q.tile_expert = tile_expert;
     q.tile_rows = tile_rows;
     q.expert_rows = expert_rows;
@@ -1973,12 +1979,12 @@ FERRIS_API int ferris_gemm_grouped_tcgen05(const void* x, const void* w, void* o
     if (row_scale && mode != SWIGLU_BF16 && !(mode == STORE_BF16 && g_launch_act.kind))
         FERRIS_REFUSE("grouped gemm: a factor per row goes with an activation (mode %d)", mode);
     return run_tokens_m(x, w, nullptr, out, mode, rows, N, K, ldx, ldw, ldo, experts * expert_rows, up_row_offset, nullptr,
-                        (cudaStream_t)stream, tile_expert, tile_rows, experts, expert_rows, row_scale);
+                        0, (cudaStream_t)stream, tile_expert, tile_rows, experts, expert_rows, row_scale);
 }
 
 static int gemm_tcgen05_impl(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
                              int ldx, int ldw, int ldo, int rows_w, int up_row_offset, float* scratch, int* counters,
-                             void* stream, const TokenSource& src) {
+                             int early_weights, void* stream, const TokenSource& src) {
     const bool built = src.norm_h || src.merge_o;
     if (T <= 0 || N <= 0) return FERRIS_OK;
     if (K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ldx < K || ldw < K)
@@ -2004,9 +2010,9 @@ static int gemm_tcgen05_impl(const void* x, const void* w, const float* bias, vo
     const int elt = (mode == STORE_BF16 || mode == SWIGLU_BF16) ? 2 : 4;
     const bool long_step = !built && token_major_pays(mode, T, N, K) && ((size_t)ldo * elt) % 16 == 0 && ((uintptr_t)out & 15) == 0;
     const PairPlan pairs = long_step && T > PT_BLOCK_M ? pair_plan(mode, T, N, K, 0) : PairPlan{};
-    if (pairs.bn) return run_pairs(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, nullptr, pairs, s);
+    if (pairs.bn) return run_pairs(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, nullptr, pairs, early_weights, s);
     if (long_step)
-        return run_tokens_m(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, nullptr, s);
+        return run_tokens_m(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset, nullptr, early_weights, s);
 
     CUtensorMap mw, mx;
     int rc = weight_map(w, (uint64_t)rows_w, (uint64_t)K, (uint64_t)ldw, &mw);
@@ -2133,7 +2139,7 @@ FERRIS_API int ferris_gemm_argmax_tcgen05(const void* x, const void* w, int* out
 FERRIS_API int ferris_qkv_rope_gemm_tcgen05(const void* x, const void* w, const float* bias, void* out, int T, int K, int ldx,
                                             int ldw, int ldo, int rows_w, const float* angles, const int* slots,
                                             void* k_cache, void* v_cache, int nh, int nkv, int d, int page_size,
-                                            void* stream) {
+                                            int early_weights, void* stream) {
     if (T <= 0) return FERRIS_OK;
     if (nh <= 0 || nkv <= 0 || page_size <= 0 || (d != 64 && d != 128))
         FERRIS_REFUSE("q/k/v product with rotation: %d + 2 x %d heads of %d, pages of %d", nh, nkv, d, page_size);
@@ -2157,8 +2163,9 @@ FERRIS_API int ferris_qkv_rope_gemm_tcgen05(const void* x, const void* w, const 
     r.page_size = page_size;
     g_launch_act = FerrisEpilogueAct{0, 0.0f, 0.0f};
     const PairPlan pairs = T > PT_BLOCK_M ? pair_plan(QKV_ROPE_BF16, T, N, K, d) : PairPlan{};
-    if (pairs.bn) return run_pairs(x, w, bias, out, QKV_ROPE_BF16, T, N, K, ldx, ldw, ldo, rows_w, 0, &r, pairs, (cudaStream_t)stream);
-    return run_tokens_m(x, w, bias, out, QKV_ROPE_BF16, T, N, K, ldx, ldw, ldo, rows_w, 0, &r, (cudaStream_t)stream);
+    if (pairs.bn) return run_pairs(x, w, bias, out, QKV_ROPE_BF16, T, N, K, ldx, ldw, ldo, rows_w, 0, &r, pairs, early_weights,
+                                    (cudaStream_t)stream);
+    return run_tokens_m(x, w, bias, out, QKV_ROPE_BF16, T, N, K, ldx, ldw, ldo, rows_w, 0, &r, early_weights, (cudaStream_t)stream);
 }
 
 FERRIS_TIMELINE_TU(gemm_tcgen05)

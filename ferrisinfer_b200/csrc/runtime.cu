@@ -19,13 +19,17 @@ FERRIS_API const char* ferris_last_error() { return g_error; }
 
 // Programmatic dependent launch is on unless the environment says FERRIS_PDL=0.
 static int g_pdl = -1;
+static thread_local int t_stream_order = 0;
 bool ferris_pdl_enabled() {
+    if (t_stream_order) return false;
     if (g_pdl < 0) {
         const char* v = getenv("FERRIS_PDL");
         g_pdl = (v && v[0] == '0') ? 0 : 1;
     }
     return g_pdl != 0;
 }
+// While on, the calling thread's launches begin when the launch before has ended: whatever they read ahead of a wait is there.
+FERRIS_API void ferris_in_stream_order(int on) { t_stream_order = on; }
 FERRIS_API void ferris_set_pdl(int on) { g_pdl = on ? 1 : 0; }
 
 // The activation that the next bf16-storing product applies in its epilogue (see common.cuh).

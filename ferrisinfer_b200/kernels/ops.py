@@ -31,10 +31,10 @@ _VP, _I, _F, _LL = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longl
 # Argument types of the launchers on the model's path: with these declared, plain Python ints and floats go straight
 # to C (a pointer would otherwise be cut to 32 bits, and wrapping every argument in a ctypes object costs microseconds).
 _SIGNATURES = {
-    "ferris_gemm_tcgen05": [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _I, _I, _VP, _VP, _VP],
+    "ferris_gemm_tcgen05": [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _I, _I, _VP, _VP, _I, _VP],
     "ferris_norm_gemm_tcgen05": [_VP, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _I, _VP],
     "ferris_merge_gemm_tcgen05": [_VP, _I, _I, _I, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP],
-    "ferris_qkv_rope_gemm_tcgen05": [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP],
+    "ferris_qkv_rope_gemm_tcgen05": [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _VP],
     "ferris_rotary_angles": [_VP, _VP, _VP, _I, _I, _VP],
     "ferris_rmsnorm": [_VP, _VP, _VP, _VP, _I, _I, _I, _F, _VP],
     "ferris_rope_cache_write": [_VP, _I, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP],
@@ -162,9 +162,20 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
     )
 
 
+class _StreamOrder:
+    """Launches of this thread begin when the launch before has ended (no programmatic launch)."""
+
+    def __enter__(self):
+        _lib().ferris_in_stream_order(_c_int(1))
+
+    def __exit__(self, *exc):
+        _lib().ferris_in_stream_order(_c_int(0))
+
+
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-              accumulate: bool = False):
-    """out[t, n] (+)= sum_k x[t, k] w[n, k] + bias[n] with fp32 FMAs on the CUDA cores."""
+              accumulate: bool = False, fixed_weight: Optional[bool] = None):
+    """out[t, n] (+)= sum_k x[t, k] w[n, k] + bias[n] with fp32 FMAs on the CUDA cores.  ``fixed_weight`` as in ``gemm``
+    (None and False: w may come from the launch before)."""
     M, K, ldx = _rows(x, "gemm input")
     N, K2, ldw = _rows(w, "gemm weight")
     M2, N2, ldo = _rows(out, "gemm output")
@@ -177,7 +188,7 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     _check(
         _lib().ferris_gemm_simt(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _dt(x, "gemm input"), _dt(out, "gemm output"),
                                 _c_int(M), _c_int(N), _c_int(K), _c_int(ldx), _c_int(ldw), _c_int(ldo),
-                                _c_int(1 if accumulate else 0), _stream()),
+                                _c_int(1 if accumulate else 0), _c_int(1 if fixed_weight else 0), _stream()),
         "gemm",
     )
 
@@ -216,9 +227,13 @@ def tensor_core_gemm_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
 _uses_clusters = None
 
 
-def gemm_tcgen05(x, w, bias, out, mode: int, n_out: Optional[int] = None, up_row_offset: int = 0):
+def gemm_tcgen05(x, w, bias, out, mode: int, n_out: Optional[int] = None, up_row_offset: int = 0,
+                 fixed_weight: Optional[bool] = None):
     """out = x w^T on the tcgen05 tensor cores.  mode 0: bf16 store (+bias); 1: fp32 store (+bias);
-    2: fp32 out += ; 3: bf16 silu(x w[:N]^T) * (x w[up_row_offset:up_row_offset+N]^T)."""
+    2: fp32 out += ; 3: bf16 silu(x w[:N]^T) * (x w[up_row_offset:up_row_offset+N]^T).  ``fixed_weight`` as in ``gemm``."""
+    if fixed_weight is False:
+        with _StreamOrder():
+            return gemm_tcgen05(x, w, bias, out, mode, n_out, up_row_offset, True)
     global _uses_clusters
     T, K, ldx = _rows(x, "gemm input")
     rows_w, K2, ldw = _rows(w, "gemm weight")
@@ -247,7 +262,7 @@ def gemm_tcgen05(x, w, bias, out, mode: int, n_out: Optional[int] = None, up_row
         lib.ferris_gemm_tcgen05(x.data_ptr(), w.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(),
                                 mode, T, N, K, ldx, ldw, ldo, rows_w, up_row_offset,
                                 None if scratch is None else scratch.data_ptr(), None if cnt is None else cnt.data_ptr(),
-                                _stream()),
+                                1 if fixed_weight else 0, _stream()),
         "tensor-core gemm",
     )
 
@@ -310,7 +325,7 @@ def greedy_head(y, w, out_token, out_prob, workspace):
         gemm_argmax(y, w, out_token, out_prob, scratch)
         return
     logits = workspace.get("logits", (n, V), torch.float32)
-    gemm(y, w, None, logits)
+    gemm(y, w, None, logits, fixed_weight=True)
     sample(logits, out_token, out_prob)
 
 
@@ -504,10 +519,17 @@ def _mode_of(out, accumulate: bool) -> int:
     return 2 if accumulate else (0 if out.dtype == torch.bfloat16 else 1)
 
 
-def gemm(x, w, bias, out, accumulate: bool = False):
+def gemm(x, w, bias, out, accumulate: bool = False, fixed_weight: Optional[bool] = None):
     """The matrix product of the model, out (+)= x w^T + bias: for bf16 operands the skinny kernel (at most 16
     tokens) or the tcgen05 kernels, the CUDA-core kernel for everything else (all of the 32-bit path).  ``x`` may
-    be a LazyRMSNorm or a LazySplitMerge."""
+    be a LazyRMSNorm or a LazySplitMerge.
+    ``fixed_weight``: True: no launch that may still run writes ``w`` (a model's weight), so every kernel requests it
+    before the launch before it has ended.  False: ``w`` may be what the launch before writes; the product begins when
+    that has ended.  None: bf16 steps of at most a few hundred tokens, whose kernels have always been meant for weights, as with True;
+    the 32-bit path and long steps read ``w`` after their wait for the launch before."""
+    if fixed_weight is False:
+        with _StreamOrder():
+            return gemm(x, w, bias, out, accumulate, True)
     if isinstance(x, LazySplitMerge):
         if w.shape[0] == out.shape[1] and _merge_gemm_takes(x, w):
             merge_gemm_tcgen05(x, w, bias, out, 2 if accumulate else (0 if out.dtype == torch.bfloat16 else 1))
@@ -523,24 +545,28 @@ def gemm(x, w, bias, out, accumulate: bool = False):
         x = x.materialize()
     if tensor_core_gemm_takes(x, w) and w.shape[0] == out.shape[1]:
         if accumulate:
-            gemm_tcgen05(x, w, bias, out, 2)
+            gemm_tcgen05(x, w, bias, out, 2, fixed_weight=fixed_weight)
         else:
-            gemm_tcgen05(x, w, bias, out, 0 if out.dtype == torch.bfloat16 else 1)
+            gemm_tcgen05(x, w, bias, out, 0 if out.dtype == torch.bfloat16 else 1, fixed_weight=fixed_weight)
         return
-    gemm_simt(x, w, bias, out, accumulate)
+    gemm_simt(x, w, bias, out, accumulate, fixed_weight)
 
 
 _EPILOGUE_ACTIVATIONS = {"xielu": 1, "silu": 2, "relu2": 3}
 _set_activation = None
 
 
-def gemm_activation(x, w, out, kind: str, coefficients=(0.0, 0.0), params: Optional[torch.Tensor] = None):
+def gemm_activation(x, w, out, kind: str, coefficients=(0.0, 0.0), params: Optional[torch.Tensor] = None,
+                    fixed_weight: Optional[bool] = None):
     """out = a(x w^T): the plain feed-forward's up product with its activation.  bf16 on the weight-stationary kernel
     (at most 16 tokens) or the tcgen05 kernels of long steps: the activation is applied to the fp32 accumulator in
     the product's epilogue, before the one rounding to bf16
     (``coefficients``: for xIELU, (softplus(p), 1/2 + softplus(q)) as Python floats).  Anything else: the product,
-    then the activation kernel with ``params`` (the two raw numbers on the device)."""
+    then the activation kernel with ``params`` (the two raw numbers on the device).  ``fixed_weight`` as in ``gemm``."""
     global _set_activation
+    if fixed_weight is False:
+        with _StreamOrder():
+            return gemm_activation(x, w, out, kind, coefficients, params, True)
     if kind not in _EPILOGUE_ACTIVATIONS:
         raise KernelError(f"activation '{kind}' is not known")
     if out.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[0] == out.shape[1]:
@@ -561,18 +587,21 @@ def gemm_activation(x, w, out, kind: str, coefficients=(0.0, 0.0), params: Optio
             if tensor_core_gemm_takes(x, w) and _lib().ferris_gemm_tcgen05_fuses_activation(
                     _c_int(x.shape[0]), _c_int(out.shape[1]), _c_int(x.shape[1]), _c_int(out.stride(0)), _ptr(out)):
                 _set_activation(code, a, b)
-                gemm_tcgen05(x, w, None, out, 0)
+                gemm_tcgen05(x, w, None, out, 0, fixed_weight=fixed_weight)
                 return
         finally:
             _set_activation(0, 0.0, 0.0)
-    gemm(x, w, None, out)
+    gemm(x, w, None, out, fixed_weight=fixed_weight)
     activation(out, out, kind, params)
 
 
-def gemm_swiglu(x, gate_up_weight, out, workspace=None):
+def gemm_swiglu(x, gate_up_weight, out, workspace=None, fixed_weight: Optional[bool] = None):
     """out [T, I] = silu(x Wg^T) * (x Wu^T) with gate_up_weight = [Wg; Wu] ([2I, K]).  bf16: one tensor-core
     kernel with two accumulators (the [T, 2I] intermediate never exists), so too 32-bit steps of few tokens; otherwise
-    a product and the SwiGLU kernel."""
+    a product and the SwiGLU kernel.  ``fixed_weight`` as in ``gemm``."""
+    if fixed_weight is False:
+        with _StreamOrder():
+            return gemm_swiglu(x, gate_up_weight, out, workspace, True)
     T, I = out.shape
     if gate_up_weight.shape[0] != 2 * I:
         raise KernelError(f"gemm_swiglu: weight {tuple(gate_up_weight.shape)} for {I} outputs")
@@ -585,7 +614,7 @@ def gemm_swiglu(x, gate_up_weight, out, workspace=None):
             return
         x = x.materialize()
     if tensor_core_gemm_takes(x, gate_up_weight) and out.dtype == torch.bfloat16:
-        gemm_tcgen05(x, gate_up_weight, None, out, 3, up_row_offset=I)
+        gemm_tcgen05(x, gate_up_weight, None, out, 3, up_row_offset=I, fixed_weight=fixed_weight)
         return
     if T <= 16 and x.dtype == gate_up_weight.dtype == out.dtype == torch.float32:
         T2, K, ldx = _rows(x, "gemm input")
@@ -594,14 +623,15 @@ def gemm_swiglu(x, gate_up_weight, out, workspace=None):
         sizes = (_c_int(T), _c_int(I), _c_int(K), _c_int(ldx), _c_int(ldw))
         if (T2 == T and K2 == K and x.untyped_storage().data_ptr() != out.untyped_storage().data_ptr()
                 and _lib().ferris_gemm_f32_swiglu_takes(_ptr(x), _ptr(gate_up_weight), *sizes)):
-            _check(_lib().ferris_gemm_f32_swiglu(_ptr(x), _ptr(gate_up_weight), _ptr(out), *sizes, _c_int(ldo), _stream()),
+            _check(_lib().ferris_gemm_f32_swiglu(_ptr(x), _ptr(gate_up_weight), _ptr(out), *sizes, _c_int(ldo),
+                                                 _c_int(1 if fixed_weight else 0), _stream()),
                    "32-bit gemm")
             return
     if workspace is not None:
         gate_up = workspace.get("ffn_gate_up", (T, 2 * I), x.dtype)
     else:
         gate_up = torch.empty(T, 2 * I, dtype=x.dtype, device=x.device)
-    gemm_simt(x, gate_up_weight, None, gate_up)
+    gemm_simt(x, gate_up_weight, None, gate_up, fixed_weight=fixed_weight)
     swiglu(gate_up, out)
 
 
@@ -622,14 +652,18 @@ def gated_activation(gate_up: torch.Tensor, out: torch.Tensor, kind: str = "silu
            "gated activation")
 
 
-def gemm_gated(x, gate_up_weight, out, kind: str = "silu", limit: float = 0.0, workspace=None):
+def gemm_gated(x, gate_up_weight, out, kind: str = "silu", limit: float = 0.0, workspace=None,
+               fixed_weight: Optional[bool] = None):
     """out [T, I] = f(x Wg^T, x Wu^T) with gate_up_weight = [Wg; Wu] ([2I, K]) and f a gated activation (see
     ``gated_activation``).  "silu" is ``gemm_swiglu``.  The others in bf16: the weight-stationary kernel (at most 16
     tokens) and the tcgen05 kernels of long steps apply f to the two fp32 accumulators in their epilogue; anything else
-    is the product followed by the activation kernel."""
+    is the product followed by the activation kernel.  ``fixed_weight`` as in ``gemm``."""
     global _set_gated
+    if fixed_weight is False:
+        with _StreamOrder():
+            return gemm_gated(x, gate_up_weight, out, kind, limit, workspace, True)
     if kind == "silu":
-        return gemm_swiglu(x, gate_up_weight, out, workspace)
+        return gemm_swiglu(x, gate_up_weight, out, workspace, fixed_weight)
     if kind not in GATED_ACTIVATIONS:
         raise KernelError(f"gated activation '{kind}' is not known ({', '.join(GATED_ACTIVATIONS)})")
     T, I = out.shape
@@ -651,7 +685,7 @@ def gemm_gated(x, gate_up_weight, out, kind: str = "silu", limit: float = 0.0, w
             if tensor_core_gemm_takes(x, gate_up_weight) and _lib().ferris_gemm_tcgen05_fuses_gated_activation(
                     _c_int(T), _c_int(I), _c_int(x.shape[1]), _c_int(out.stride(0)), _ptr(out)):
                 _set_gated(code, float(limit))
-                gemm_tcgen05(x, gate_up_weight, None, out, 3, up_row_offset=I)
+                gemm_tcgen05(x, gate_up_weight, None, out, 3, up_row_offset=I, fixed_weight=fixed_weight)
                 return
         finally:
             _set_gated(0, 0.0)
@@ -659,7 +693,7 @@ def gemm_gated(x, gate_up_weight, out, kind: str = "silu", limit: float = 0.0, w
         gate_up = workspace.get("ffn_gate_up", (T, 2 * I), out.dtype)
     else:
         gate_up = torch.empty(T, 2 * I, dtype=out.dtype, device=out.device)
-    gemm(x, gate_up_weight, None, gate_up)
+    gemm(x, gate_up_weight, None, gate_up, fixed_weight=fixed_weight)
     gated_activation(gate_up, out, kind, limit)
 
 
@@ -713,11 +747,13 @@ def qkv_rope_gemm_takes(x, w, qkv, num_heads, num_kv_heads, head_dim, rotary_dim
             and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and tensor_core_gemm_takes(x, w))
 
 
-def qkv_rope_gemm(x, w, bias, qkv, angles, slot_mapping, k_cache, v_cache, num_heads, num_kv_heads, head_dim):
+def qkv_rope_gemm(x, w, bias, qkv, angles, slot_mapping, k_cache, v_cache, num_heads, num_kv_heads, head_dim,
+                  fixed_weight: Optional[bool] = None):
     """The q/k/v product of a long step with rotation and cache write in its epilogue: ``qkv[:, :nh d]`` gets the
     rotated queries (its key and value columns are left as they were), the paged cache the rotated keys and
     the values at ``slot_mapping`` (None: nothing is stored, for a layer that reads another layer's cache).
-    ``angles``: from ``rotary_angles`` for the step's positions."""
+    ``angles``: from ``rotary_angles`` for the step's positions.  ``fixed_weight`` as in ``gemm`` (None and False: w may come
+    from the launch before)."""
     T, K, ldx = _rows(x, "q/k/v input")
     rows_w, K2, ldw = _rows(w, "q/k/v weight")
     T2, N, ldo = _rows(qkv, "q/k/v output")
@@ -743,7 +779,7 @@ def qkv_rope_gemm(x, w, bias, qkv, angles, slot_mapping, k_cache, v_cache, num_h
                                             qkv.data_ptr(), T, K, ldx, ldw, ldo, rows_w, angles.data_ptr(),
                                             None if slot_mapping is None else slot_mapping.data_ptr(),
                                             k_cache.data_ptr(), v_cache.data_ptr(), num_heads, num_kv_heads, head_dim,
-                                            page_size, _stream()),
+                                            page_size, 1 if fixed_weight else 0, _stream()),
         "q/k/v product with rotation",
     )
 

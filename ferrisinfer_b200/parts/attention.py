@@ -265,7 +265,7 @@ class GroupedQueryAttention(Mixer):
         qkv = ctx.workspace.get("attn_qkv", (T, self.qkv_weight.shape[0]), x.dtype)
         if not self.plain:
             dv = self.v_head_dim
-            ops.gemm(x, self.qkv_weight, self.qkv_bias, qkv)
+            ops.gemm(x, self.qkv_weight, self.qkv_bias, qkv, fixed_weight=True)
             gate = None
             if self.output_gate is not None:
                 qkv, gate = qkv[:, :n_qkv], qkv[:, n_qkv:n_qkv + self.gate_size]
@@ -297,7 +297,7 @@ class GroupedQueryAttention(Mixer):
                                 fp32_weights=self.fp32_weights, pooled=pooled, keep_first=self.keep_first)
             if gate is not None and not self.gate_per_head:
                 ops.gate_mul(out, gate, out, self.output_gate[1], self.output_scale)
-            ops.gemm(out, self.o_weight, None, h, accumulate=accumulate)
+            ops.gemm(out, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
             return
         table = self.position.rotary_table(qkv.device)
         inv_freq, rotary = table if table is not None else (None, 0)
@@ -310,16 +310,16 @@ class GroupedQueryAttention(Mixer):
             fused = ops.qkv_rope_gemm_takes(x, self.qkv_weight, qkv, nh, nkv, d, rotary, cache.k)
         if fused:
             ops.qkv_rope_gemm(x, self.qkv_weight, self.qkv_bias, qkv, self.position.angles(ctx),
-                              meta.slot_mapping if owns_cache else None, cache.k, cache.v, nh, nkv, d)
+                              meta.slot_mapping if owns_cache else None, cache.k, cache.v, nh, nkv, d, fixed_weight=True)
         else:
-            ops.gemm(x, self.qkv_weight, self.qkv_bias, qkv)
+            ops.gemm(x, self.qkv_weight, self.qkv_bias, qkv, fixed_weight=True)
             if table is None:
                 self.position.apply(qkv, ctx.positions, nh, nkv, d)
         out = ctx.workspace.get("attn_out", (T, self.q_size), x.dtype)
         attended = ops.attention_step(qkv, out, cache.k, cache.v, meta, ctx, nh, nkv, d, inv_freq, rotary,
                                       self.window or 0, self.scale, write_kv=owns_cache, lazy_merge=True,
                                       rotated=fused, score_slopes=slopes)
-        ops.gemm(attended, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(attended, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 register_part("mixer", "gqa_attention", GroupedQueryAttention)

@@ -128,7 +128,7 @@ class OutputHead(Part):
 
     def forward(self, y, logits):
         """logits fp32 [n, V] = y [n, H] W^T."""
-        ops.gemm(y, self.weight, None, logits)
+        ops.gemm(y, self.weight, None, logits, fixed_weight=True)
         if self.logit_scale != 1.0:
             ops.scale_(logits, self.logit_scale)
         if self.softcap is not None:

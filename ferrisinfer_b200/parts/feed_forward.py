@@ -47,8 +47,8 @@ class SwiGLU(FeedForward):
     def forward(self, x, h, ctx):
         T, I = x.shape[0], self.intermediate_size
         act = ctx.workspace.get("ffn_act", (T, I), x.dtype)
-        ops.gemm_swiglu(x, self.gate_up, act, ctx.workspace)
-        ops.gemm(act, self.down, None, h, accumulate=True)
+        ops.gemm_swiglu(x, self.gate_up, act, ctx.workspace, fixed_weight=True)
+        ops.gemm(act, self.down, None, h, accumulate=True, fixed_weight=True)
 
 
 class GatedFeedForward(FeedForward):
@@ -82,8 +82,8 @@ class GatedFeedForward(FeedForward):
     def forward(self, x, h, ctx, accumulate: bool = True):
         T, I = x.shape[0], self.intermediate_size
         act = ctx.workspace.get("ffn_act", (T, I), ctx.act_dtype)
-        ops.gemm_gated(x, self.gate_up, act, self.activation, self.limit, ctx.workspace)
-        ops.gemm(act, self.down, None, h, accumulate=accumulate)
+        ops.gemm_gated(x, self.gate_up, act, self.activation, self.limit, ctx.workspace, fixed_weight=True)
+        ops.gemm(act, self.down, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 class DenseActivation(FeedForward):
@@ -127,8 +127,8 @@ class DenseActivation(FeedForward):
     def forward(self, x, h, ctx, accumulate: bool = True):
         T, I = x.shape[0], self.intermediate_size
         z = ctx.workspace.get("ffn_act", (T, I), ctx.act_dtype)
-        ops.gemm_activation(x, self.up, z, self.activation, self.coefficients, self.act)
-        ops.gemm(z, self.down, None, h, accumulate=accumulate)
+        ops.gemm_activation(x, self.up, z, self.activation, self.coefficients, self.act, fixed_weight=True)
+        ops.gemm(z, self.down, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 class MixtureOfExperts(FeedForward):

@@ -102,7 +102,7 @@ class LatentAttention(Mixer):
         ws = ctx.workspace
         meta = ctx.paged[cache.group]
         proj = ws.get("latent_in", (T, self.in_weight.shape[0]), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, None, proj)
+        ops.gemm(x, self.in_weight, None, proj, fixed_weight=True)
         q_att = ws.get("latent_queries", (T, nh * row), ctx.act_dtype)
         table = self.rotary.table(proj.device)
         keys = None
@@ -116,7 +116,7 @@ class LatentAttention(Mixer):
             ops.latent_prepare(ctx.positions, table, self.norm_eps, nh, d, r, rank, keys=keys,
                                q_latent=(latent, self.q_norm, latent))
             q = ws.get("latent_q", (T, self.q_size), ctx.act_dtype)
-            ops.gemm(proj[:, :self.q_cols], self.uq, None, q)
+            ops.gemm(proj[:, :self.q_cols], self.uq, None, q, fixed_weight=True)
             ops.latent_prepare(ctx.positions, table, self.norm_eps, nh, d, r, rank, queries=(q, q_att))
         ops.head_gemm(q, d + r, self.uk, q_att, row)  # the plain queries through the key up-projection
         mixed = ws.get("latent_mixed", (T, nh * rank), ctx.act_dtype)
@@ -125,7 +125,7 @@ class LatentAttention(Mixer):
         out = ws.get("latent_out", (T, nh * dv), ctx.act_dtype)
         gate = proj[:, self.gate_off:self.gate_off + nh] if self.output_gate else None
         ops.head_gemm(mixed, rank, self.uv, out, dv, gate=gate)
-        ops.gemm(out, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(out, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 register_part("mixer", "latent_attention", LatentAttention)

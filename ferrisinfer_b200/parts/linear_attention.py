@@ -89,7 +89,7 @@ class DecayedLinearAttention(Mixer):
         T = x.shape[0]
         nh, d, dv = self.num_heads, self.head_dim, self.v_head_dim
         proj = ctx.workspace.get("linear_attn_in", (T, 2 * self.qk_size + 2 * self.v_size), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, None, proj)
+        ops.gemm(x, self.in_weight, None, proj, fixed_weight=True)
         o = ctx.workspace.get("linear_attn_out", (T, self.v_size), torch.float32)
         ops.linear_attention(proj, (0, self.qk_size, 2 * self.qk_size), o, cache.state, self._decays(o.device), ctx,
                              nh, d, dv, silu=self.activation == "silu", write_state=owns_cache,
@@ -101,7 +101,7 @@ class DecayedLinearAttention(Mixer):
                                  gate_kind=self.gate)
         else:
             ops.gated_rmsnorm(o, g, self.norm_weight, self.norm_eps, y)
-        ops.gemm(y, self.o_weight, None, h, accumulate=True)
+        ops.gemm(y, self.o_weight, None, h, accumulate=True, fixed_weight=True)
 
 
 register_part("mixer", "decayed_linear_attention", DecayedLinearAttention)

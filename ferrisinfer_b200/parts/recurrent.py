@@ -132,7 +132,7 @@ class GatedDeltaRule(Mixer):
         history, state = cache.parts
         ws = ctx.workspace
         proj = ws.get("recurrent_in", (T, self.in_weight.shape[0]), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, None, proj)
+        ops.gemm(x, self.in_weight, None, proj, fixed_weight=True)
         conv = ws.get("recurrent_conv", (T, C), ctx.act_dtype)
         ops.short_conv(proj[:, :C], conv, self.conv_weight, None if history is None else history.state, ctx,
                        advance=owns_cache, residual=False, silu=True)
@@ -145,7 +145,7 @@ class GatedDeltaRule(Mixer):
                              delta_rule=True, qscale=qscale, kscale=kscale, write_state=owns_cache)
         y = ws.get("recurrent_gated", (T, V), ctx.act_dtype)
         ops.gated_group_norm(o, proj[:, C:C + V], self.norm_weight, self.norm_eps, y, group=dv, gate_kind="silu")
-        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 class ChannelDeltaRule(GatedDeltaRule):
@@ -191,14 +191,14 @@ class ChannelDeltaRule(GatedDeltaRule):
         history, state = cache.parts
         ws = ctx.workspace
         proj = ws.get("recurrent_in", (T, self.in_weight.shape[0]), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, None, proj)
+        ops.gemm(x, self.in_weight, None, proj, fixed_weight=True)
         conv = ws.get("recurrent_conv", (T, C), ctx.act_dtype)
         ops.short_conv(proj[:, :C], conv, self.conv_weight, None if history is None else history.state, ctx,
                        advance=owns_cache, residual=False, silu=True)
         z = ws.get("recurrent_row_decay", (T, nh * d), torch.float32)
-        ops.gemm(proj[:, self.a_off:self.a_off + self.a2.shape[1]], self.a2, self.dt_bias, z)
+        ops.gemm(proj[:, self.a_off:self.a_off + self.a2.shape[1]], self.a2, self.dt_bias, z, fixed_weight=True)
         gate = ws.get("recurrent_gate", (T, V), ctx.act_dtype)
-        ops.gemm(proj[:, self.g_off:self.g_off + self.g2.shape[1]], self.g2, None, gate)
+        ops.gemm(proj[:, self.g_off:self.g_off + self.g2.shape[1]], self.g2, None, gate, fixed_weight=True)
         beta = ws.get("recurrent_beta", (T, nh), torch.float32)
         qscale, kscale = ws.get("recurrent_qscale", (T, g), torch.float32), ws.get("recurrent_kscale", (T, g), torch.float32)
         ops.recurrence_gates(proj, None, self.b_off, None, None, None, beta, nh,
@@ -208,7 +208,7 @@ class ChannelDeltaRule(GatedDeltaRule):
                              delta_rule=True, qscale=qscale, kscale=kscale, write_state=owns_cache, row_decay=(z, self.rates))
         y = ws.get("recurrent_gated", (T, V), ctx.act_dtype)
         ops.gated_group_norm(o, gate, self.norm_weight, self.norm_eps, y, group=dv, gate_kind="sigmoid")
-        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 class StateSpaceDuality(Mixer):
@@ -261,7 +261,7 @@ class StateSpaceDuality(Mixer):
         history, state = cache.parts
         ws = ctx.workspace
         proj = ws.get("recurrent_in", (T, self.in_weight.shape[0]), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, None, proj)
+        ops.gemm(x, self.in_weight, None, proj, fixed_weight=True)
         conv = ws.get("recurrent_conv", (T, C), ctx.act_dtype)
         ops.short_conv(proj[:, inner:inner + C], conv, self.conv_weight, None if history is None else history.state, ctx,
                        advance=owns_cache, bias=self.conv_bias, residual=False, silu=True)
@@ -274,7 +274,7 @@ class StateSpaceDuality(Mixer):
         y = ws.get("recurrent_gated", (T, inner), ctx.act_dtype)
         ops.gated_group_norm(o, proj[:, :inner], self.norm_weight, self.norm_eps, y, group=inner // self.norm_groups,
                              gate_kind="silu", gate_first=True)
-        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 class GatedLinearUnit(Mixer):
@@ -337,7 +337,7 @@ class GatedLinearUnit(Mixer):
         history, state = cache.parts
         ws = ctx.workspace
         proj = ws.get("recurrent_in", (T, self.in_weight.shape[0]), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, self.in_bias, proj)
+        ops.gemm(x, self.in_weight, self.in_bias, proj, fixed_weight=True)
         u = ws.get("recurrent_conv", (T, C), ctx.act_dtype)
         ops.short_conv(proj[:, C:2 * C], u, self.conv_weight, None if history is None else history.state, ctx,
                        advance=owns_cache, bias=self.conv_bias, residual=False, silu=False)
@@ -351,7 +351,7 @@ class GatedLinearUnit(Mixer):
             ops.rglru_gates(u, self.ra_t, self.ri_t, self.ra_bias, self.ri_bias, self.rate, a, b, self.decay_factor,
                             stored=(self.ra, self.ri))
             ops.rglru_scan(a, b, proj[:, :C], y, state.state, ctx, gelu=gelu, write_state=owns_cache)
-        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 class GatedLinearAttention(Mixer):
@@ -418,16 +418,16 @@ class GatedLinearAttention(Mixer):
         nh, d, dv, QK, V = self.num_heads, self.head_dim, self.v_head_dim, self.qk_size, self.v_size
         ws = ctx.workspace
         proj = ws.get("linear_attn_in", (T, self.in_weight.shape[0]), ctx.act_dtype)
-        ops.gemm(x, self.in_weight, None, proj)
+        ops.gemm(x, self.in_weight, None, proj, fixed_weight=True)
         z = ws.get("linear_attn_decay", (T, QK), torch.float32)
-        ops.gemm(proj[:, self.a_off:self.a_off + self.rank_cols], self.a2_weight, self.a2_bias, z)
+        ops.gemm(proj[:, self.a_off:self.a_off + self.rank_cols], self.a2_weight, self.a2_bias, z, fixed_weight=True)
         o = ws.get("linear_attn_out", (T, V), torch.float32)
         ops.row_decay_recurrence(proj[:, :QK], proj[:, QK:2 * QK], proj[:, 2 * QK:2 * QK + V], z, 1.0 / self.tau, o,
                                  cache.state, ctx, nh, d, dv, q_scale=d ** -0.5, write_state=owns_cache)
         y = ws.get("linear_attn_gated", (T, V), ctx.act_dtype)
         ops.gated_group_norm(o, proj[:, 2 * QK + V:2 * QK + 2 * V], self.norm_weight, self.norm_eps, y, group=dv,
                              gate_kind="silu")
-        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate)
+        ops.gemm(y, self.o_weight, None, h, accumulate=accumulate, fixed_weight=True)
 
 
 register_part("mixer", "gated_linear_unit", GatedLinearUnit)

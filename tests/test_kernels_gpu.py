@@ -149,7 +149,7 @@ def test_gemm_fp32_with_swiglu_on_the_way(N, K, device):
     assert ops.kernel_status() == 0
 
 
-@pytest.mark.parametrize("N, K", [(3584, 18944), (18944, 3584)])
+@pytest.mark.parametrize("N, K", [(3584, 18944), (37888, 3584)])
 def test_gemm_fp32_gives_a_row_the_same_bits_on_either_side_of_the_rule(N, K, device):
     """Long rows (the 7B down projection) and many of them: from some number of tokens on the tiles take the product."""
     from ferrisinfer_b200.kernels import ops
@@ -171,6 +171,40 @@ def test_gemm_fp32_gives_a_row_the_same_bits_on_either_side_of_the_rule(N, K, de
         out = torch.empty(M, N // 2, device=device)
         ops.gemm_swiglu(x[:M], w, out)
         assert torch.equal(out, want[:M]), M
+    assert ops.kernel_status() == 0
+
+
+# A second operand that the launch before writes, in the forms that request a model's weights ahead of their wait.
+@pytest.mark.parametrize("dtype, T, N, K, swiglu, told", [
+    (F32, 4, 4864, 896, False, None), (F32, 4, 2432, 896, True, None), (BF16, 256, 4864, 896, False, None),
+    (BF16, 512, 1536, 8960, False, None), (BF16, 512, 4480, 1536, True, None),  # single CTAs, pairs with K splits, pairs
+    (F32, 4, 4864, 896, False, False), (BF16, 8, 4864, 896, False, False), (BF16, 64, 4864, 896, False, False),
+    (BF16, 8, 2432, 896, True, False), (BF16, 512, 1536, 8960, False, False)])
+def test_products_of_a_second_operand_that_the_launch_before_writes(dtype, T, N, K, swiglu, told, device):
+    """By default (the 32-bit path and long steps), or told that it is no fixed weight (every form), a product reads w
+    after the launch before it has ended; with a weight that stays as it is, the same bits."""
+    from ferrisinfer_b200.kernels import ops
+
+    rows = 2 * N if swiglu else N
+    x = rnd((T, K), dtype, device, 60, scale=0.2)
+    halves = [rnd((rows, 2 * K), dtype, device, 61 + i, scale=0.5) for i in range(2)]  # w = silu(left) * right of either
+    product = ops.gemm_swiglu if swiglu else (lambda x, w, out, **kw: ops.gemm(x, w, None, out, **kw))
+    out = torch.empty(T, N, dtype=dtype, device=device)
+    want = []
+    for h in halves:
+        w = torch.empty(rows, K, dtype=dtype, device=device)
+        ops.swiglu(h, w)
+        torch.cuda.synchronize()
+        product(x, w, out, fixed_weight=True)
+        want.append(out.clone())
+    w = torch.zeros(rows, K, dtype=dtype, device=device)
+    outs = [torch.empty(T, N, dtype=dtype, device=device) for _ in range(12)]
+    for i, o in enumerate(outs):
+        ops.swiglu(halves[i % 2], w)
+        product(x, w, o, fixed_weight=told)
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        assert torch.equal(o, want[i % 2]), i
     assert ops.kernel_status() == 0
 
 
