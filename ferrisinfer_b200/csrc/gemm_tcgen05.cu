@@ -1888,6 +1888,35 @@ static int run_pairs(const void* x, const void* w, const float* bias, void* out,
     }
 }
 
+// The plan by which a long step of T tokens runs on CTA pairs (bn 0: it does not).  head: 64 or 128 for the q/k/v product, else 0.
+FERRIS_API int ferris_gemm_pair_plan(int mode, int T, int N, int K, int head, int* bn, int* splits) {
+    *bn = 0, *splits = 1;
+    if (T <= PT_BLOCK_M || N <= 0 || K <= 0) return FERRIS_OK;
+    const PairPlan plan = pair_plan(head ? QKV_ROPE_BF16 : mode, T, N, K, head);
+    *bn = plan.bn, *splits = plan.splits;
+    return FERRIS_OK;
+}
+
+// ferris_gemm_tcgen05 for one accumulator (modes 0 to 2) on CTA pairs by a plan of the caller's: tiles of bn weight rows (128 to 256, a
+// multiple of 32), `splits` pairs to a tile.
+FERRIS_API int ferris_gemm_on_pairs(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
+                                    int ldx, int ldw, int ldo, int rows_w, int bn, int splits, void* stream) {
+    if (T <= 0 || N <= 0) return FERRIS_OK;
+    const int elt = mode == STORE_BF16 ? 2 : 4, kblocks = (K + BLOCK_K - 1) / BLOCK_K, per = splits > 0 ? (kblocks + splits - 1) / splits : 0;
+    if (mode != STORE_BF16 && mode != STORE_F32 && mode != ACCUM_F32) FERRIS_REFUSE("gemm on pairs: mode %d", mode);
+    if (K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ldx < K || ldw < K || ldo < N || N > rows_w || ((size_t)ldo * elt) % 16 ||
+        (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15))
+        FERRIS_REFUSE("gemm on pairs: K=%d and row strides %d, %d, %d of %d rows must start on 16 bytes", K, ldx, ldw, ldo, rows_w);
+    if (bn < 128 || bn > 256 || bn % 32 || splits < 1 || splits > PP_MAX_SPLITS || per * (splits - 1) >= kblocks ||
+        (splits > 1 && pair_clusters(splits) <= 0))
+        FERRIS_REFUSE("gemm on pairs: tiles of %d weight rows, %d splits of %d K slices", bn, splits, kblocks);
+    sm_count();
+    g_launch_act = FerrisEpilogueAct{0, 0.0f, 0.0f};
+    PairPlan plan;
+    plan.bn = bn, plan.splits = splits;
+    return run_pairs(x, w, bias, out, mode, T, N, K, ldx, ldw, ldo, rows_w, 0, nullptr, plan, 0, (cudaStream_t)stream);
+}
+
 // The persistent token-major kernel for a long step (T >= 128 tokens; output rows aligned for 16-byte stores).
 static int run_tokens_m(const void* x, const void* w, const float* bias, void* out, int mode, int T, int N, int K,
                         int ldx, int ldw, int ldo, int rows_w, int up_row_offset, const RopeEpilogue* rope,

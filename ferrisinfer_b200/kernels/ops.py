@@ -340,6 +340,31 @@ def set_gemm_pairs(which=GEMM_PAIRS_SWIGLU) -> None:
     _lib().ferris_set_gemm_pair(_c_int(int(which)))
 
 
+def gemm_pair_plan(tokens: int, outputs: int, k: int, mode: int = 1, head_dim: int = 0) -> tuple[int, int]:
+    """How a long step's product (modes as ``gemm_tcgen05``; ``head_dim``: the q/k/v product with its rotation) runs on pairs of CTAs:
+    (weight rows of a tile, K splits), (0, 1) where it does not."""
+    bn, splits = _c_int(), _c_int()
+    _lib().ferris_gemm_pair_plan(_c_int(mode), _c_int(tokens), _c_int(outputs), _c_int(k), _c_int(head_dim), ctypes.byref(bn),
+                                 ctypes.byref(splits))
+    return bn.value, splits.value
+
+
+def gemm_on_pairs(x, w, bias, out, mode: int, tile_rows: int, splits: int):
+    """``gemm_tcgen05`` of one accumulator (modes 0 to 2) on pairs of CTAs, cut as told."""
+    T, K, ldx = _rows(x, "gemm input")
+    N, K2, ldw = _rows(w, "gemm weight")
+    T2, N2, ldo = _rows(out, "gemm output")
+    if K != K2 or T != T2 or N != N2 or not x.dtype == w.dtype == torch.bfloat16 or out.dtype != (torch.float32 if mode else torch.bfloat16):
+        raise KernelError(f"gemm on pairs: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} {out.dtype}, mode {mode}")
+    if bias is not None:
+        _need(bias, "gemm bias", torch.float32)
+        if bias.numel() != N:
+            raise KernelError("gemm: bias length differs from the output width")
+    _check(_lib().ferris_gemm_on_pairs(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(ldx),
+                                       _c_int(ldw), _c_int(ldo), _c_int(N), _c_int(tile_rows), _c_int(splits), _stream()),
+           "gemm on pairs")
+
+
 def set_gemm_long_min(tokens: int = 0) -> None:
     """From how many tokens on a product runs the token-major kernel (never below 128); 0: the library's default."""
     _lib().ferris_set_gemm_long_min(_c_int(int(tokens)))

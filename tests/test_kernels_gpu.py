@@ -363,8 +363,8 @@ def test_gemm_on_cta_pairs(T, N, K, mode, device):
                                      (257, 3584, 5000), (130, 3590, 18944), (2048, 3592, 136)])
 @pytest.mark.parametrize("mode", [0, 1, 2])
 def test_gemm_of_long_steps_as_they_are_launched(T, N, K, mode, device):
-    """Few tiles and a long K (pairs of CTAs with two, three or four K splits, the last one shorter), two rounds of tiles
-    (pairs without splits), token and weight rows and K slices that end inside a tile.  Against 64 bits: sums of K terms in
+    """Few tiles and a long K, two rounds of tiles, token and weight rows and K slices that end inside a tile, on whichever kernel
+    and plan they get (the two tests below say which).  Against 64 bits: sums of K terms in
     fp32, 2^-24 of the sum of their absolute values for the additions on the way (in order, then over four splits and the
     base), and a bf16 result's own rounding; the same bits again."""
     from ferrisinfer_b200.kernels import ops
@@ -384,6 +384,65 @@ def test_gemm_of_long_steps_as_they_are_launched(T, N, K, mode, device):
     want, size = want + extra.double(), size + extra.double().abs()
     bound = (K / 16 + 8) * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if mode == 0 else 0.0)
     assert ((outs[0].double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("splits", [1, 2, 3, 4])
+@pytest.mark.parametrize("bn", [128, 160, 192, 224, 256])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_gemm_on_cta_pairs_of_every_width_and_split(bn, splits, mode, device):
+    """All widths of a tile and K splits of a cluster that a plan can hold: an odd number of token tiles, ragged last rows, columns
+    and slices, owners of several, one and no columns.  The bound as above; without splits the bits of single CTAs."""
+    from ferrisinfer_b200.kernels import ops
+
+    T, N, K = 385, 616, 64 * 13 + 8
+    x, w = rnd((T, K), BF16, device, 55), rnd((N, K), BF16, device, 56, scale=0.1)
+    bias = rnd((N,), F32, device, 57) if mode < 2 else None
+    base = rnd((T, N), F32, device, 58) if mode == 2 else None
+    fresh = lambda: base.clone() if mode == 2 else torch.full((T, N), float("nan"), dtype=F32 if mode else BF16, device=device)
+    outs = [fresh(), fresh()]
+    for out in outs:
+        ops.gemm_on_pairs(x, w, bias, out, mode, bn, splits)
+    assert torch.equal(outs[0], outs[1])
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    extra = base if mode == 2 else bias
+    want, size = want + extra.double(), size + extra.double().abs()
+    bound = (K / 16 + 8) * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if mode == 0 else 0.0)
+    assert ((outs[0].double() - want).abs() <= bound).all()
+    if splits == 1:
+        single = fresh()
+        ops.set_gemm_pairs(ops.GEMM_PAIRS_NONE)
+        try:
+            ops.gemm_tcgen05(x, w, bias, single, mode)
+        finally:
+            ops.set_gemm_pairs()
+        assert torch.equal(outs[0], single)
+    assert ops.kernel_status() == 0
+
+
+@pytest.mark.parametrize("T, N, K, split", [(512, 1536, 8960, True), (1000, 896, 4864, True), (2048, 896, 4864, True),
+                                            (256, 3584, 18944, True), (2048, 4608, 3584, False)])
+def test_products_that_the_plan_puts_on_cta_pairs(T, N, K, split, device):
+    """With and without K splits, as launched by default: on pairs by the plan, against the kernel on single CTAs: the same bits
+    without splits, with them the sums regrouped."""
+    from ferrisinfer_b200.kernels import ops
+
+    bn, splits = ops.gemm_pair_plan(T, N, K)
+    assert bn > 0 and (splits > 1) == split
+    x, w = rnd((T, K), BF16, device, 55), rnd((N, K), BF16, device, 56, scale=0.1)
+    planned, single, told = (torch.empty(T, N, device=device) for _ in range(3))
+    ops.gemm_tcgen05(x, w, None, planned, 1)
+    ops.gemm_on_pairs(x, w, None, told, 1, bn, splits)
+    ops.set_gemm_pairs(ops.GEMM_PAIRS_NONE)
+    try:
+        ops.gemm_tcgen05(x, w, None, single, 1)
+    finally:
+        ops.set_gemm_pairs()
+    assert torch.equal(planned, told)
+    if not split:
+        assert torch.equal(planned, single)
+    size = x.double().abs() @ w.double().abs().t()
+    assert ((planned.double() - single.double()).abs() <= 2 * (K / 16 + 8) * 2.0 ** -24 * size).all()
+    assert ops.kernel_status() == 0
 
 
 @pytest.fixture
@@ -601,6 +660,42 @@ def test_qkv_product_with_rotation_and_cache_write_in_its_epilogue(T, nh, nkv, d
     ops.rope_cache_write(ref, positions, inv_freq, slots, k2, v2, nh, nkv, d, d, page)
     assert torch.allclose(ref.view(T, -1, d)[:, :nh].float(), qkv.view(T, -1, d)[:, :nh].float(), atol=3e-2, rtol=2e-2)
     assert torch.allclose(k2.float(), k_cache.float(), atol=3e-2, rtol=2e-2)
+
+@pytest.mark.parametrize("T, nh, nkv, d, K, page, planned", [
+    (300, 14, 2, 64, 896, 64, False), (129, 3, 1, 64, 72, 16, False), (257, 3, 1, 128, 136, 32, False), (640, 12, 2, 128, 200, 16, False),
+    (2048, 28, 4, 128, 3584, 16, True), (2048, 28, 8, 64, 3584, 64, None)])
+def test_qkv_product_on_cta_pairs_writes_what_single_ctas_write(T, nh, nkv, d, K, page, planned, device):
+    """Odd numbers of token tiles, a last pair with an empty half, ragged last rows, both head sizes, slots of -1: queries, keys
+    and values bit for bit; the prompts of the 7B sizes run there by themselves."""
+    from ferrisinfer_b200.kernels import ops
+
+    N = (nh + 2 * nkv) * d
+    x, w, bias = rnd((T, K), BF16, device, 71), rnd((N, K), BF16, device, 72, scale=K ** -0.5), rnd((N,), F32, device, 73)
+    g = torch.Generator().manual_seed(6)
+    positions = torch.randint(0, 5000, (T,), generator=g, dtype=torch.int32).to(device)
+    pages = (T + page - 1) // page + 2
+    slots = torch.randperm(pages * page, generator=g)[:T].to(torch.int32)
+    slots[5] = slots[T - 1] = -1
+    slots = slots.to(device)
+    angles = torch.empty(T, d // 2, 2, dtype=F32, device=device)
+    ops.rotary_angles(positions, torch.tensor(plain.rotary_inverse_frequencies(d, d, 1e6).numpy(), device=device), angles)
+    got = {}
+    try:
+        for which in (ops.GEMM_PAIRS_NONE, ops.GEMM_PAIRS_ALL, 2):
+            ops.set_gemm_pairs(which)
+            on_pairs = ops.gemm_pair_plan(T, N, K, head_dim=d)[0] > 0
+            assert on_pairs == {0: False, 1: True}.get(which, on_pairs if planned is None else planned)
+            out = [torch.full((T, N), 7.0, dtype=BF16, device=device)] + \
+                [torch.full((pages, nkv, page, d), 7.0, dtype=BF16, device=device) for _ in range(2)]
+            ops.qkv_rope_gemm(x, w, bias, out[0], angles, slots, out[1], out[2], nh, nkv, d)
+            got[which] = out
+    finally:
+        ops.set_gemm_pairs()
+    assert ops.kernel_status() == 0
+    for a, b, c in zip(*got.values()):
+        assert torch.equal(a, b) and torch.equal(a, c)
+    assert bool((got[0][1] != 7.0).any())
+
 
 
 
