@@ -1363,8 +1363,8 @@ bool ferris_gemm_cluster_enabled() {
     return g_cluster != 0;
 }
 
-// Which long-step products run on CTA pairs: FERRIS_GEMM_PAIR / ferris_set_gemm_pair = 0 none, 1 all, 2 (the
-// default) the gate / up product only.  Measured inside the prefill step of 2,048 tokens, per launch: gate / up
+// Which long-step products run on CTA pairs: FERRIS_GEMM_PAIR / ferris_set_gemm_pair = 0 none, 1 all (without K splits), 2 (the
+// default) by pair_plan.  Measured inside the prefill step of 2,048 tokens before K splits, per launch: gate / up
 // 38.4 us on pairs against 41.6 us, the products with one accumulator 20.5 us against 19.3 us (same number of
 // CTAs either way, and the pair's barriers cost more than the halved weight traffic saves).  Prefill with the
 // default against no pairs: 0.5B sizes 3.49-3.58 against 3.51-3.59 ms, 1.5B sizes 8.13-8.20 against 8.47-8.51 ms.
@@ -1677,8 +1677,8 @@ FERRIS_API int ferris_set_gemm_long_min(int tokens) {
     return FERRIS_OK;
 }
 
-// Long steps on CTA pairs (cta_group::2) instead of single CTAs: 0 none, 1 every product, 2 the gate / up product
-// only (the default); any other value selects the default.
+// Long steps on CTA pairs (cta_group::2) instead of single CTAs: 0 none, 1 every product (without K splits), 2 by pair_plan (the
+// default); any other value selects the default.
 FERRIS_API int ferris_set_gemm_pair(int on) {
     g_pair = (on >= 0 && on <= 2) ? on : 2;
     return FERRIS_OK;

@@ -329,10 +329,11 @@ def greedy_head(y, w, out_token, out_prob, workspace):
     sample(logits, out_token, out_prob)
 
 
-GEMM_PAIRS_NONE, GEMM_PAIRS_ALL, GEMM_PAIRS_SWIGLU = 0, 1, 2
+GEMM_PAIRS_NONE, GEMM_PAIRS_ALL, GEMM_PAIRS_PLANNED = 0, 1, 2
+GEMM_PAIRS_SWIGLU = GEMM_PAIRS_PLANNED  # its older name
 
 
-def set_gemm_pairs(which=GEMM_PAIRS_SWIGLU) -> None:
+def set_gemm_pairs(which=GEMM_PAIRS_PLANNED) -> None:
     """Which products of long steps (more than 128 tokens) run on pairs of CTAs that share one 256-row MMA
     (cta_group::2): none, all (without K splits: the numbers are then those of single CTAs bit for bit), or the gate / up
     product and those that an estimate puts there, some with their K split over a cluster of pairs (the default, also
@@ -905,7 +906,7 @@ def paged_attention_simt(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Te
     denominator).  ``v_head_dim``: size of a value head where it differs from the keys'.  ``values_in_keys``: a key's
     first ``v_head_dim`` elements are its value (``v_cache`` is then not read and may be None).
     ``max_q_len``: the most tokens a request brings; above one (portions of prompts) the kernel that shares tiles of
-    keys among 64 query rows runs where it takes the geometry.  ``max_kv_len`` and ``workspace`` (a step of single
+    keys among 32 or 64 query rows runs where it takes the geometry.  ``max_kv_len`` and ``workspace`` (a step of single
     tokens): the most keys a request holds, and where scratch comes from; the keys of a token are then cut into
     shares that run side by side, and query heads of one kv head share its keys.  ``pooled`` (with a window): beside the
     window's tokens the query sees one row of ``pooled`` for every run of positions that lies wholly before the window.
