@@ -1,0 +1,517 @@
+// The 32-bit path's products of many tokens on the tensor cores: out[t, n] (+)= sum_k x[t, k] * w[n, k] (+ bias[n]) with operands and
+// sums of 32 bits.
+//
+// Every operand is written as the sum of three bf16 numbers, v = v1 + v2 + v3 (each the rest rounded to nearest; the third is
+// exact, so 24 bits of significand are kept whole), and a product is the six of their nine products that reach into 32 bits:
+// x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1; what is left out is below 2^-26 of |x w|, under half of an fp32 rounding.  The products
+// themselves are exact.  The tensor core's own additions cut off instead of rounding, so a sum stays there for 32 k's only, the
+// small products first (the cuts then fall on sums a 256th as large) and the two steps of large ones last; after that it is
+// added to sums in registers, rounded to nearest, and these every 1,024 k's to a sum of their own.  Error against 64 bits
+// (2-norm, relative, normal numbers; this kernel / the FMA kernels of gemm_f32.cu): K = 64 0.7 / 1.1, 896 0.9 to 1.15 / 1.55, 4,864
+// 1.2 to 1.3 / 1.6, 9,220 1.3 / 1.65, each 1e-7.
+//
+// A cluster of two CTAs (cta_group::2) takes 256 weight rows x NT tokens.  Nothing reads the fp32 operands twice from
+// shared memory: every thread loads runs of 8 k's straight into registers one slice ahead (a warp: 4 rows x 64 k's, whole 128-byte
+// lines), splits them and stores three 16-byte chunks into bf16 tiles in the 128-byte swizzle that the MMA reads; the SAME warps
+// drain the accumulators, because with two slices of 64 k's in shared memory and two accumulators both jobs fit beside the MMAs.
+//
+// K SPLITS: where tiles are few a cluster of up to four pairs takes one tile, each a run of slices; the sums meet through
+// shared memory and are added in the runs' order.  SwiGLU: a CTA's rows 0..63 are gate rows, 64..127 their up rows.
+//
+// Infinities and overflow: a part of an infinity times a part that is zero is not a number, so a result that is not finite is
+// formed again with FMAs in the order of gemm_f32.cuh.
+#include "common.cuh"
+#include "gemm_f32.cuh"
+#include "sm100.cuh"
+
+namespace {
+
+constexpr int SP_WARPS = 16;
+constexpr int SP_THREADS = SP_WARPS * 32;  // 128 registers a thread; lane 0 of the leader's warp 0 issues the MMAs beside its work
+constexpr int SP_M = 128;                  // weight rows of a CTA, 256 of a pair
+constexpr int SP_K = 64;                   // k's of a slice: two runs of 32
+constexpr int SP_LEVEL = 16;               // slices whose runs are added up before they join the outer sum
+constexpr int SP_MAX_SPLITS = 4;
+constexpr int SP_A_PART = SP_M * 128;      // bytes of one part of a slice of the weights
+
+struct SplitParams {
+    const float* x;
+    const float* w;
+    const float* bias;
+    float* out;
+    int M, N, K, ldx, ldw, ldo, accumulate;
+    int up_offset;  // > 0: SwiGLU of weight rows n and up_offset + n; N outputs
+    int m_tiles, n_tiles, slices, slices_per, splits;
+    int early_weights;
+    int* status;
+};
+
+// a + b and a - b of two pairs, an instruction each.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return reinterpret_cast<float2&>(r);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    const float2 minus = make_float2(-1.0f, -1.0f);  // (a - b in one rounding: -b is exact)
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(r)
+        : "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<const unsigned long long&>(minus)),
+          "l"(reinterpret_cast<unsigned long long&>(a)));
+    return reinterpret_cast<float2&>(r);
+}
+
+// Eight fp32 values as three runs of eight bf16: the value rounded, the rest rounded, what then is left.
+__device__ __forceinline__ float2 unpack2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+__device__ __forceinline__ void split8(const float4 a, const float4 b, uint4& p1, uint4& p2, uint4& p3) {
+    const float2 v[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
+    uint32_t o1[4], o2[4], o3[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o1[i] = pack_bf16(v[i].x, v[i].y);
+        float2 rest = sub2(v[i], unpack2(o1[i]));
+        o2[i] = pack_bf16(rest.x, rest.y);
+        rest = sub2(rest, unpack2(o2[i]));
+        o3[i] = pack_bf16(rest.x, rest.y);
+    }
+    p1 = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+    p2 = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+    p3 = make_uint4(o3[0], o3[1], o3[2], o3[3]);
+}
+
+// One output in the order of the FMA kernels.
+__device__ __noinline__ float dot_in_order(const float* x, const float* w, int K) {
+    const int runs = (K + F32_CHUNK - 1) / F32_CHUNK, per = f32_runs_per_part(runs);
+    float total = 0.0f, part = 0.0f;
+    for (int c = 0; c < runs; ++c) {
+        float even = 0.0f, odd = 0.0f;
+        const int k1 = min(K, (c + 1) * F32_CHUNK);
+        for (int k = c * F32_CHUNK; k < k1; k += 2) {
+            even = fmaf(x[k], w[k], even);
+            if (k + 1 < k1) odd = fmaf(x[k + 1], w[k + 1], odd);
+        }
+        part += even + odd;
+        if ((c + 1) % per == 0 || c + 1 == runs) {
+            total += part;
+            part = 0.0f;
+        }
+    }
+    return total;
+}
+
+__device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+
+__device__ __forceinline__ void tmem_load_32x8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_store_32x8(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+template <int CW>  // tokens of a warp's columns; a tile has four times as many
+struct SplitShape {
+    static constexpr int NT = 4 * CW;
+    static constexpr int XR = NT / 2;  // token rows that a CTA holds
+    static constexpr int B_PART = XR * 128;
+    static constexpr int SLOT = 3 * (SP_A_PART + B_PART);
+    static constexpr int EXCHANGE = 64 * NT * 4;  // SwiGLU: the up rows' sums
+};
+
+template <int CW, bool SWIGLU>
+__global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const SplitParams p) {
+    using S = SplitShape<CW>;
+    constexpr int XG = S::XR > 64 ? 2 : 1;  // runs of token rows that a thread may load
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t full[2], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_base;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t cta = cluster_ctarank(), rank = cta & 1, leader = cta & ~1u;
+    const int splits = SWIGLU ? 1 : p.splits, split = SWIGLU ? 0 : (int)(cta >> 1);
+    const int first = (int)blockIdx.x / (2 * splits), stride = (int)gridDim.x / (2 * splits);  // clusters
+    const int s0 = split * p.slices_per, per_tile = min(p.slices, s0 + p.slices_per) - s0;
+    const int tiles = p.m_tiles * p.n_tiles;
+    const int total = first < tiles ? (tiles - first + stride - 1) / stride * per_tile : 0;  // slices of this CTA
+    const uint16_t both = (uint16_t)(3u << leader);
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&full[i], 2 * SP_WARPS);       // the warps of both CTAs (used in the leader only)
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], 2 * SP_WARPS);  // (the leader's only)
+        }
+        mbar_fence_init();
+    }
+    if (warp == 0) tmem_alloc_pair(&tmem_base, 512);
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tcgen05_fence_after();
+    const uint32_t tmem = tmem_base;
+    pdl_launch_dependents();
+
+    const int quarter = warp & 3, wc = warp >> 2;
+    const int lr = tid >> 3, ch = tid & 7;  // this thread's rows (and those 64 further) and its 8 k's of a slice
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + wc * CW;
+    const uint32_t full_at = map_to_cta(smem_u32(&full[0]), leader), empty_at = map_to_cta(smem_u32(&acc_empty[0]), leader);
+    float4 wa[2][2], xb[XG][2];
+    // the slice that is loaded next; of its tile this thread's rows (null: beyond the operand), and the rows 64 further if `more`
+    int l_tile = first, l_slice = 0, l_it = 0;
+    const float* w_row = nullptr;
+    const float* x_row = nullptr;
+    bool w_more = false, x_more = false;
+    auto rows_of_tile = [&]() {
+        const int nt = l_tile / p.m_tiles, n = nt * (SWIGLU ? SP_M : 2 * SP_M) + (int)rank * (SWIGLU ? 64 : SP_M) + lr;
+        const int t = (l_tile - nt * p.m_tiles) * S::NT + (int)rank * S::XR + lr;
+        w_row = n < p.N ? p.w + (size_t)n * p.ldw + 8 * ch : nullptr;
+        w_more = SWIGLU ? n < p.N : n + 64 < p.N;
+        x_row = lr < S::XR && t < p.M ? p.x + (size_t)t * p.ldx + 8 * ch : nullptr;
+        x_more = lr + 64 < S::XR && t + 64 < p.M;
+    };
+    const size_t w_further = (size_t)(SWIGLU ? p.up_offset : 64) * p.ldw, x_further = (size_t)64 * p.ldx;
+    auto load8 = [&](float4 (&v)[2], const float* at, bool lo, bool hi) {
+        const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[0] = lo ? *reinterpret_cast<const float4*>(at) : none;
+        v[1] = hi ? *reinterpret_cast<const float4*>(at + 4) : none;
+    };
+    auto load_w = [&]() {
+        if (l_it >= total) return;
+        if (l_slice == 0) rows_of_tile();
+        const int k = (s0 + l_slice) * SP_K;
+        const bool lo = k + 8 * ch < p.K, hi = k + 8 * ch + 4 < p.K;
+        load8(wa[0], w_row + k, w_row && lo, w_row && hi);
+        load8(wa[1], w_row + k + w_further, w_more && lo, w_more && hi);
+        if (w_row && (ch & 3) == 0) {  // two slices on: from HBM into L2
+            const int far = k + 2 * SP_K;
+            if (far + 8 * ch < p.K) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(w_row + far));
+                if (w_more) asm volatile("prefetch.global.L2 [%0];" ::"l"(w_row + far + w_further));
+            }
+        }
+    };
+    auto load_x = [&]() {
+        if (l_it >= total) return;
+        const int k = (s0 + l_slice) * SP_K;
+        const bool lo = k + 8 * ch < p.K, hi = k + 8 * ch + 4 < p.K;
+        load8(xb[0], x_row + k, x_row && lo, x_row && hi);
+        if (XG > 1) load8(xb[XG - 1], x_row + k + x_further, x_more && lo, x_more && hi);
+        ++l_it;
+        if (++l_slice == per_tile) {
+            l_slice = 0;
+            l_tile += stride;
+        }
+    };
+    auto store = [&](int it) {  // the loaded slice goes to its slot, in parts
+        if (it >= total) return;
+        uint8_t* slot = smem + (it & 1) * S::SLOT;
+        uint4 p1, p2, p3;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            split8(wa[j][0], wa[j][1], p1, p2, p3);
+            uint8_t* at = slot + swizzle128(lr + 64 * j, ch);
+            *reinterpret_cast<uint4*>(at) = p1;
+            *reinterpret_cast<uint4*>(at + SP_A_PART) = p2;
+            *reinterpret_cast<uint4*>(at + 2 * SP_A_PART) = p3;
+        }
+#pragma unroll
+        for (int j = 0; j < XG; ++j) {
+            const int r = lr + 64 * j;
+            if (r >= S::XR) continue;
+            split8(xb[j][0], xb[j][1], p1, p2, p3);
+            uint8_t* at = slot + 3 * SP_A_PART + swizzle128(r, ch);
+            *reinterpret_cast<uint4*>(at) = p1;
+            *reinterpret_cast<uint4*>(at + S::B_PART) = p2;
+            *reinterpret_cast<uint4*>(at + 2 * S::B_PART) = p3;
+        }
+        asm volatile("fence.proxy.async;" ::: "memory");  // the tensor core reads what every lane wrote
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(full_at + 8u * (it & 1));
+    };
+    int ok = 1;  // 0: a wait ran out; no MMA is issued and nothing waited for any more, every barrier is still met
+    // Half h of slice `it`: 32 k's into accumulator h, the smallest products first.
+    auto issue = [&](int it, int h) {
+        if (warp != 0) return;
+        if (lane == 0 && rank == 0 && it < total && ok) {
+            const int s = it & 1;
+            ok = mbar_wait(&full[s], (it >> 1) & 1, p.status, 0x70) &&
+                 (it == 0 || mbar_wait(&acc_empty[h], (it - 1) & 1, p.status, 0x71));
+            if (ok) {
+                tcgen05_fence_after();
+                constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
+                const uint32_t at = smem_u32(smem + s * S::SLOT), idesc = umma_idesc_bf16(2 * SP_M, S::NT);
+                const uint64_t a = umma_desc_k_major_sw128(at), b = umma_desc_k_major_sw128(at + 3 * SP_A_PART);
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const uint64_t step = (uint64_t)(2 * (2 * h + k));
+                        tcgen05_mma_bf16_pair(tmem + h * S::NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
+                                              b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
+                    }
+                tcgen05_commit_pair(&acc_full[h], both);
+            }
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+    };
+    if (p.early_weights) load_w();
+    pdl_wait();
+    if (!p.early_weights) load_w();
+    load_x();
+    store(0);
+    load_w();
+    load_x();
+    issue(0, 0);
+    issue(0, 1);
+    store(1);
+    load_w();
+    load_x();
+
+    float acc[CW];
+#pragma unroll
+    for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
+    int tile = first, slice = 0;
+    for (int it = 0; it < total; ++it) {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[h], it & 1, p.status, 0x72));
+            tcgen05_fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < CW; c0 += 24) {  // up to 24 columns under way
+                constexpr int AT_ONCE = 24;
+                uint32_t r[AT_ONCE];
+#pragma unroll
+                for (int c = 0; c < AT_ONCE && c0 + c < CW; c += 8) tmem_load_32x8(lane_addr + h * S::NT + c0 + c, r + c);
+                tmem_load_wait();
+#pragma unroll
+                for (int c = 0; c < AT_ONCE && c0 + c < CW; c += 2) {
+                    const float2 sum = add2(make_float2(acc[c0 + c], acc[c0 + c + 1]),
+                                            make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+                    acc[c0 + c] = sum.x;
+                    acc[c0 + c + 1] = sum.y;
+                }
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(empty_at + 8u * h);
+            issue(it + 1, h);
+        }
+        // both accumulators of slice `it` are complete: its slot is free
+        store(it + 2);
+        load_w();
+        load_x();
+        const bool last = slice + 1 == per_tile;
+        if ((slice + 1) % SP_LEVEL == 0 || (last && slice >= SP_LEVEL)) {  // the runs so far join the outer sum
+#pragma unroll
+            for (int c = 0; c < CW; c += 8) {
+                uint32_t r[8];
+                if (slice >= SP_LEVEL) {
+                    tmem_load_32x8(lane_addr + 2 * S::NT + c, r);
+                    tmem_load_wait();
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float sum = slice >= SP_LEVEL ? __uint_as_float(r[i]) + acc[c + i] : acc[c + i];
+                    r[i] = __float_as_uint(sum);
+                    acc[c + i] = last ? sum : 0.0f;
+                }
+                if (!last) tmem_store_32x8(lane_addr + 2 * S::NT + c, r);
+            }
+            if (!last) tmem_store_wait();
+        }
+        ++slice;
+        if (!last) continue;
+        slice = 0;
+        if (!SWIGLU && splits > 1) break;  // one tile to a cluster: its sums meet below
+        const int t0 = (tile % p.m_tiles) * S::NT + wc * CW, nt = tile / p.m_tiles;
+        if (SWIGLU) {
+            float* up = reinterpret_cast<float*>(smem + 2 * S::SLOT) + (wc * CW) * 64 + (quarter & 1) * 32 + lane;
+            const int bar = 1 + wc * 2 + (quarter & 1);  // the warp of the gate rows and that of their up rows
+            if (quarter >= 2) {
+#pragma unroll
+                for (int c = 0; c < CW; ++c) up[c * 64] = acc[c];
+            }
+            asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+            if (quarter < 2) {
+                const int n = nt * SP_M + (int)rank * 64 + quarter * 32 + lane;
+#pragma unroll
+                for (int c = 0; c < CW; ++c) {
+                    if (n < p.N && t0 + c < p.M) {
+                        float g = acc[c], u = up[c * 64];
+                        const float* row = p.x + (size_t)(t0 + c) * p.ldx;
+                        if (!is_finite(g)) g = dot_in_order(row, p.w + (size_t)n * p.ldw, p.K);
+                        if (!is_finite(u)) u = dot_in_order(row, p.w + (size_t)(n + p.up_offset) * p.ldw, p.K);
+                        p.out[(size_t)(t0 + c) * p.ldo + n] = u * (g * (1.0f / (1.0f + expf(-g))));
+                    }
+                }
+            }
+            asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+        } else {
+            const int n = nt * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
+            if (n < p.N) {
+                const float bias = p.bias ? p.bias[n] : 0.0f;
+#pragma unroll
+                for (int c = 0; c < CW; ++c) {
+                    if (t0 + c < p.M) {
+                        float v = acc[c];
+                        if (!is_finite(v)) v = dot_in_order(p.x + (size_t)(t0 + c) * p.ldx, p.w + (size_t)n * p.ldw, p.K);
+                        if (p.bias) v += bias;
+                        float* o = p.out + (size_t)(t0 + c) * p.ldo + n;
+                        *o = p.accumulate ? *o + v : v;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
+        tile += stride;
+    }
+    if (!SWIGLU && splits > 1) {
+        // groups of four tokens of a warp belong to the pairs in turn; a pair sends the others theirs
+        __syncwarp();
+        cluster_sync();  // every MMA of the cluster is done: the slots take partial sums now
+        constexpr int GROUPS = CW / 4;
+        const int each = (GROUPS + splits - 1) / splits;  // groups of an owner
+        const uint32_t ring = smem_u32(smem);
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            const int owner = g % splits;
+            if (owner == split) continue;
+            const int place = (split < owner ? split : split - 1) * each + g / splits;
+            uint32_t v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = __float_as_uint(acc[4 * g + i]);
+            st_cluster_x4(map_to_cta(ring + (place * SP_THREADS + tid) * 16, 2 * owner + rank), v);
+        }
+        cluster_sync();
+        const int t0 = (first % p.m_tiles) * S::NT + wc * CW;
+        const int n = first / p.m_tiles * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
+        if (n < p.N) {
+            const float bias = p.bias ? p.bias[n] : 0.0f;
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) {
+                if (g % splits != split) continue;
+                float sum[4];
+                for (int from = 0; from < splits; ++from) {
+                    float4 v = make_float4(acc[4 * g], acc[4 * g + 1], acc[4 * g + 2], acc[4 * g + 3]);
+                    if (from != split) {
+                        const int place = (from < split ? from : from - 1) * each + g / splits;
+                        v = *reinterpret_cast<const float4*>(smem + (size_t)(place * SP_THREADS + tid) * 16);
+                    }
+                    const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[i] = from ? sum[i] + f[i] : f[i];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int t = t0 + 4 * g + i;
+                    if (t >= p.M) continue;
+                    float v = sum[i];
+                    if (!is_finite(v)) v = dot_in_order(p.x + (size_t)t * p.ldx, p.w + (size_t)n * p.ldw, p.K);
+                    if (p.bias) v += bias;
+                    float* o = p.out + (size_t)t * p.ldo + n;
+                    *o = p.accumulate ? *o + v : v;
+                }
+            }
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_sync();  // neither CTA frees tensor memory or leaves while the pair's MMAs or arrivals may still come
+    if (warp == 0) {
+        tcgen05_fence_after();
+        tmem_dealloc_pair(tmem, 512);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------- launching
+template <int CW, bool SWIGLU>
+int launch_split(const SplitParams& p, int clusters, cudaStream_t s) {
+    const size_t smem = 2 * SplitShape<CW>::SLOT + (SWIGLU ? SplitShape<CW>::EXCHANGE : 0) + 1024;
+    if (int rc = ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<CW, SWIGLU>, smem)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * p.splits * clusters);
+    cfg.blockDim = dim3(SP_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * p.splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ferris_pdl_enabled() ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_split_kernel<CW, SWIGLU>, p);
+    if (e != cudaSuccess) {
+        ferris_set_error("32-bit gemm: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    FERRIS_LAUNCH_CHECK();
+}
+template <bool SWIGLU>
+int launch_split_of(int cw, const SplitParams& p, int clusters, cudaStream_t s) {
+    if (cw == 8) return launch_split<8, SWIGLU>(p, clusters, s);
+    if (cw == 16) return launch_split<16, SWIGLU>(p, clusters, s);
+    if (cw == 24) return launch_split<24, SWIGLU>(p, clusters, s);
+    if (cw == 32) return launch_split<32, SWIGLU>(p, clusters, s);
+    return launch_split<40, SWIGLU>(p, clusters, s);
+}
+
+// Clusters of 1 to 4 pairs that the GPU's 148 SMs hold at once, a CTA an SM (a cluster keeps to a GPC).
+constexpr int CLUSTERS[SP_MAX_SPLITS + 1] = {0, 74, 35, 22, 16};
+
+struct SplitPlan {
+    int cw, splits, clusters, m_tiles, n_tiles, slices_per;
+    double cycles;
+};
+SplitPlan split_plan(int M, int rows, int K, bool swiglu, int cw_only = 0, int splits_only = 0) {
+    SplitPlan best = {};
+    const int slices = (K + SP_K - 1) / SP_K, n_tiles = (rows + 2 * SP_M - 1) / (2 * SP_M);
+    for (int cw = 8; cw <= 40; cw += 8) {
+        if (cw_only && cw != cw_only) continue;
+        const int nt = 4 * cw;
+        const long long m_tiles = (M + nt - 1) / nt;
+        const double slice = 250.0 + (12 * nt > 700 + 3 * nt ? 12 * nt : 700 + 3 * nt);  // cycles: MMAs, or splitting and draining
+        for (int sp = 1; sp <= (swiglu ? 1 : SP_MAX_SPLITS); ++sp) {
+            if (splits_only && sp != splits_only) continue;
+            const int per = (slices + sp - 1) / sp;
+            if (sp > 1 && (per < 4 || (sp - 1) * per >= slices)) continue;
+            const long long tiles = m_tiles * n_tiles, rounds = (tiles + CLUSTERS[sp] - 1) / CLUSTERS[sp];
+            const double cycles = rounds * (per * slice + (sp > 1 ? 9000.0 : 1500.0)) + 5000.0;
+            if (best.cw && cycles >= best.cycles) continue;
+            best = {cw, sp, (int)(sp > 1 || tiles < CLUSTERS[1] ? tiles : CLUSTERS[1]), (int)m_tiles, n_tiles, per, cycles};
+        }
+    }
+    return best;
+}
+
+int run_split(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx, int ldw, int ldo,
+              int accumulate, int up_offset, int early_weights, const SplitPlan& q, cudaStream_t s) {
+    const SplitParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, up_offset, q.m_tiles, q.n_tiles, (K + SP_K - 1) / SP_K,
+                           q.slices_per, q.splits, early_weights, ferris_status_ptr()};
+    return up_offset > 0 ? launch_split_of<true>(q.cw, p, q.clusters, s) : launch_split_of<false>(q.cw, p, q.clusters, s);
+}
+
+}  // namespace
+
+// The product on the tensor cores, cut as told (token_tile 32 to 160 in steps of 32, splits 1 to 4; 0: by the plan).  Rows aligned as
+// ferris_gemm_f32_takes has it; swiglu: N outputs of 2 N weight rows, gate rows first.
+FERRIS_API int ferris_gemm_f32_split_run(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx,
+                                         int ldw, int ldo, int accumulate, int swiglu, int token_tile, int splits, void* stream) {
+    if (M <= 0 || N <= 0) return FERRIS_OK;
+    if (K <= 0 || ldx < K || ldw < K || ldo < N) FERRIS_REFUSE("gemm: K=%d, row strides %d, %d, %d", K, ldx, ldw, ldo);
+    if (!ferris_gemm_f32_takes(x, w, out, K, ldx, ldw)) FERRIS_REFUSE("gemm: rows that do not begin on 16 bytes");
+    if ((long long)((M + 31) / 32) * ((2LL * N + 255) / 256) >= (1 << 28)) FERRIS_REFUSE("gemm: %d x %d outputs", M, N);
+    if (token_tile % 32 || token_tile < 0 || token_tile > 160 || splits < 0 || splits > SP_MAX_SPLITS || (swiglu && (splits > 1 || bias || accumulate)))
+        FERRIS_REFUSE("gemm: token tile %d, %d splits", token_tile, splits);
+    const SplitPlan q = split_plan(M, swiglu ? 2 * N : N, K, swiglu != 0, token_tile / 4, splits);
+    if (!q.cw) FERRIS_REFUSE("gemm: %d k's in %d splits", K, splits);
+    return run_split(x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, swiglu ? N : 0, 0, q, (cudaStream_t)stream);
+}

@@ -272,6 +272,26 @@ def gemm_f32_plan(tokens: int, outputs: int, k: int, swiglu: bool = False) -> in
     return int(_lib().ferris_gemm_f32_plan(_c_int(tokens), _c_int(outputs), _c_int(k), _c_int(1 if swiglu else 0)))
 
 
+def gemm_f32_split(x, w, bias, out, accumulate: bool = False, swiglu: bool = False, token_tile: int = 0, splits: int = 0):
+    """The 32-bit product of many tokens on the tensor cores, whatever its size, cut as told: tokens of a tile (32 to 160 in steps of
+    32) and K splits (1 to 4), 0: by the plan.  ``swiglu``: out = silu(x Wg^T) * (x Wu^T) of w = [Wg; Wu]."""
+    M, K, ldx = _rows(x, "gemm input")
+    N, K2, ldw = _rows(w, "gemm weight")
+    M2, N2, ldo = _rows(out, "gemm output")
+    if K != K2 or M != M2 or N != (2 * N2 if swiglu else N2) or not x.dtype == w.dtype == out.dtype == torch.float32:
+        raise KernelError(f"gemm: x {tuple(x.shape)} {x.dtype}, w {tuple(w.shape)} {w.dtype}, out {tuple(out.shape)}")
+    if bias is not None:
+        _need(bias, "gemm bias", torch.float32)
+        if bias.numel() != N2:
+            raise KernelError("gemm: bias length differs from the output width")
+    _check(
+        _lib().ferris_gemm_f32_split_run(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _c_int(M), _c_int(N2), _c_int(K), _c_int(ldx),
+                                         _c_int(ldw), _c_int(ldo), _c_int(1 if accumulate else 0), _c_int(1 if swiglu else 0),
+                                         _c_int(token_tile), _c_int(splits), _stream()),
+        "32-bit gemm",
+    )
+
+
 def gemm_plan(tokens: int, outputs: int, k: int, accumulators: int = 1) -> tuple[int, int]:
     """How the short-step tcgen05 kernel would cut a product: (token tile, K splits)."""
     bt, splits, floats, counters = _c_int(), _c_int(), ctypes.c_longlong(), _c_int()

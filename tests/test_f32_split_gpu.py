@@ -1,0 +1,102 @@
+"""The 32-bit path's products of many tokens on tensor cores (operands in three bf16 parts), against 64 bits and against the FMA
+kernels where numbers are not finite."""
+
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import rnd
+
+pytestmark = pytest.mark.gpu
+
+F32 = torch.float32
+
+
+def bound(x, w, K):
+    """|error| of a product: in a run of 32 k's two additions of large products cut off (2^-23 each) and the 32 large products, laid
+    out at the largest one's exponent before they are added, may lose 2^-23 each; the rest is added in rounded fp32: at most 32
+    runs to a sum, the sums of 1,024 k's, at most four splits, the bias.  The small products and what is left out: 2^-24."""
+    steps = 2 * (2 + 32) + min(32, K / 32 + 1) + K / 1024 + 1 + 4 + 1 + 1
+    return steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+
+
+# token tiles of 32 to 160: one token more than a tile, one less, exactly; weight rows around 128 and 256; k's around slices of 64 and
+# around the 1,024 of the outer sum
+@pytest.mark.parametrize("M, N, K", [(1, 1, 4), (33, 40, 60), (160, 256, 128), (161, 129, 68), (95, 257, 1024), (31, 300, 1092),
+                                     (130, 896, 896), (50, 33, 9220)])
+def test_split_products_against_64_bits(M, N, K, device):
+    from ferrisinfer_b200.kernels import ops
+
+    x, w, bias, acc0 = rnd((M, K), F32, device, 1), rnd((N, K), F32, device, 2, 0.1), rnd((N,), F32, device, 3), rnd((M, N), F32, device, 4)
+    want, limit = x.double() @ w.double().t(), bound(x, w, K)
+    slices = (K + 63) // 64
+    for splits in (0, 1, 2, 3, 4):
+        per = -(-slices // max(1, splits))
+        if splits > 1 and (per < 4 or (splits - 1) * per >= slices):
+            with pytest.raises(Exception, match="splits"):
+                ops.gemm_f32_split(x, w, None, torch.empty(M, N, device=device), splits=splits)
+            continue
+        first = None
+        for tile in (0, 32, 64, 96, 128, 160):
+            out = torch.full((M, N + 3), 7.0, device=device)
+            ops.gemm_f32_split(x, w, None, out[:, :N], token_tile=tile, splits=splits)
+            assert ((out[:, :N].double() - want).abs() <= limit).all(), (tile, splits)
+            assert (out[:, N:] == 7.0).all()
+            if splits:  # a row's sums do not depend on the tile that it lies in
+                first = out if first is None else first
+                assert torch.equal(out, first), (tile, splits)
+        out = acc0.clone()
+        ops.gemm_f32_split(x, w, bias, out, accumulate=True, splits=splits)
+        total = want + bias.double() + acc0.double()
+        assert ((out.double() - total).abs() <= limit + 3 * 2.0 ** -24 * (total.abs() + acc0.double().abs() + bias.double().abs() + want.abs())).all()
+    # rows of wider buffers
+    wx, ww = rnd((M, K + 8), F32, device, 5), rnd((N, K + 4), F32, device, 6, 0.1)
+    out = torch.empty(M, N, device=device)
+    ops.gemm_f32_split(wx[:, 4:4 + K], ww[:, :K], None, out)
+    assert ((out.double() - wx[:, 4:4 + K].double() @ ww[:, :K].double().t()).abs() <= bound(wx[:, 4:4 + K], ww[:, :K], K)).all()
+    assert ops.kernel_status() == 0
+
+
+@pytest.mark.parametrize("M, I, K", [(33, 64, 64), (161, 65, 132), (96, 200, 1100), (300, 4864, 896)])
+def test_split_products_with_swiglu_on_the_way(M, I, K, device):
+    """The bits of the product without K splits and the SwiGLU kernel."""
+    from ferrisinfer_b200.kernels import ops
+
+    x, w = rnd((M, K), F32, device, 11), rnd((2 * I, K), F32, device, 12, 0.1)
+    gate_up, want = torch.empty(M, 2 * I, device=device), torch.empty(M, I, device=device)
+    ops.gemm_f32_split(x, w, None, gate_up, splits=1)
+    ops.swiglu(gate_up, want)
+    for tile in (0, 32, 64, 96, 128, 160):
+        out = torch.full((M, I), 7.0, device=device)
+        ops.gemm_f32_split(x, w, None, out, swiglu=True, token_tile=tile)
+        assert torch.equal(out, want), tile
+    assert ops.kernel_status() == 0
+
+
+def test_split_products_of_infinities_and_of_the_largest_numbers(device):
+    """Where parts would make infinity times zero or round beyond the largest bf16, the FMA kernel's result."""
+    from ferrisinfer_b200.kernels import ops
+
+    M, N, K = 64, 300, 200
+    x, w = rnd((M, K), F32, device, 21), rnd((N, K), F32, device, 22, 0.1).bfloat16().float()  # (their second and third parts are zero)
+    x[3, 7], x[5, 9], x[7, 11] = math.inf, -math.inf, math.nan
+    x[9] = 0.0
+    x[9, 13] = 3.4e38
+    w[17, 3], w[19, 5] = math.inf, 0.0
+    x[11, 3] = 0.0
+    for splits in (1, 0):
+        out, want = torch.empty(M, N, device=device), torch.empty(1, N, device=device)
+        ops.gemm_f32_split(x, w, None, out, splits=splits)
+        for t in (3, 5, 7, 9, 11, 0):
+            ops.gemm_simt(x[t:t + 1], w, None, want)
+            odd = ~torch.isfinite(want[0]) | (t == 9)
+            assert torch.allclose(out[t], want[0], rtol=1e-5, atol=1e-5 if t != 9 else 0.0, equal_nan=True), t
+            assert torch.equal(out[t][odd].nan_to_num(nan=3.0), want[0][odd].nan_to_num(nan=3.0)), t
+    # an infinity in a gate row: silu(-inf) = -inf * 0
+    out, gate_up, want = torch.empty(M, N // 2, device=device), torch.empty(1, N, device=device), torch.empty(1, N // 2, device=device)
+    ops.gemm_f32_split(x, w, None, out, swiglu=True)
+    for t in (3, 7, 11):
+        ops.gemm_simt(x[t:t + 1], w, None, gate_up)
+        ops.swiglu(gate_up, want)
+        assert torch.allclose(out[t], want[0], rtol=1e-4, atol=1e-4, equal_nan=True), t
