@@ -42,6 +42,7 @@ constexpr int SK_MAX_MT = 4;                      // 16-row tiles of a slab (per
 constexpr int SK_MAX_ROWS = 16 * SK_MAX_MT;
 constexpr int SK_MAX_STAGES = 96;
 constexpr int SK_MAX_TOKENS = 16;
+constexpr int SK_PASS_SMEM = 224 * 1024;          // of a CTA that works in passes (beside 1 KB of alignment and its barriers)
 
 enum SkMode { SK_STORE_BF16 = 0, SK_STORE_F32 = 1, SK_ACCUM_F32 = 2, SK_SWIGLU_BF16 = 3 };
 
@@ -89,6 +90,49 @@ __device__ __forceinline__ void sk_write(const SkParams& p, int t, int n, float 
         reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = old + (a + bias_v);
     } else {
         reinterpret_cast<bf16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16_rn(sk_silu_mul(a, b));
+    }
+}
+
+// Columns 4 idx .. 4 idx + 3 of row t as (x r) w, rounded to bf16, where TMA would have put them (zeros where the row is not `live` or beyond K).
+__device__ __forceinline__ void sk_put_row(const SkParams& p, uint8_t* x_smem, int x_box_bytes, int t, bool live, int idx, float4 h,
+                                           float4 w, float r) {
+    uint2 v = make_uint2(0u, 0u);
+    if (live && idx < p.K / 4) {
+        v.x = pack_bf16((h.x * r) * w.x, (h.y * r) * w.y);
+        v.y = pack_bf16((h.z * r) * w.z, (h.w * r) * w.w);
+    }
+    const int kb = idx >> 4;  // K block of these columns; group kb / nb, line t * nb + kb % nb of its box
+    const int grp = p.nb == 1 ? kb : (int)__umulhi((unsigned)kb, p.nb_magic);  // kb / nb, exact for small kb
+    *reinterpret_cast<uint2*>(x_smem + (size_t)grp * x_box_bytes + swizzle128(t * p.nb + (kb - grp * p.nb), (idx >> 1) & 7) + (idx & 1) * 8) = v;
+}
+// Row t of the step (a row of any length) as an RMSNorm, by one warp.
+__device__ __forceinline__ void sk_norm_row(const SkParams& p, uint8_t* x_smem, int x_box_bytes, int t, int lane) {
+    const int n4 = p.K / 4, tile4 = p.kblocks * 16;
+    const float4* w4 = reinterpret_cast<const float4*>(p.norm_w);
+    const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4* row = reinterpret_cast<const float4*>(p.norm_h + (size_t)(t < p.T ? t : 0) * p.K);
+    const bool live = t < p.T;
+    float ss = 0.0f;
+    for (int base = 0; base < n4 && live; base += 256) {
+        float4 hv[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) hv[j] = base + j * 32 + lane < n4 ? row[base + j * 32 + lane] : zero4;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += (hv[j].x * hv[j].x + hv[j].y * hv[j].y) + (hv[j].z * hv[j].z + hv[j].w * hv[j].w);
+    }
+    ss = warp_sum(ss);
+    const float r = 1.0f / sqrtf(ss / (float)p.K + p.norm_eps);
+    for (int base = 0; base < tile4; base += 256) {
+        float4 hv[8], wl[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int idx = base + j * 32 + lane;
+            hv[j] = (live && idx < n4) ? row[idx] : zero4;
+            wl[j] = idx < n4 ? w4[idx] : zero4;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (base + j * 32 + lane < tile4) sk_put_row(p, x_smem, x_box_bytes, t, live, base + j * 32 + lane, hv[j], wl[j], r);
     }
 }
 
@@ -229,19 +273,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
         for (int t = warp; t < p.x_rows; t += SK_WARPS) {
             const float4* row = reinterpret_cast<const float4*>(p.norm_h + (size_t)(t < p.T ? t : 0) * p.K);
             const bool live = t < p.T;
-            auto put = [&](int idx, float4 h, float4 w, float r) {  // columns 4 idx .. 4 idx + 3 of row t
-                uint2 v = make_uint2(0u, 0u);
-                if (live && idx < n4) {
-                    v.x = pack_bf16((h.x * r) * w.x, (h.y * r) * w.y);
-                    v.y = pack_bf16((h.z * r) * w.z, (h.w * r) * w.w);
-                }
-                const int kb = idx >> 4;  // K block of these columns; group kb / nb, line t * nb + kb % nb of its box
-                const int grp = p.nb == 1 ? kb : (int)__umulhi((unsigned)kb, p.nb_magic);  // kb / nb, exact for small kb
-                *reinterpret_cast<uint2*>(x_smem + (size_t)grp * x_box_bytes +
-                                          swizzle128(t * p.nb + (kb - grp * p.nb), (idx >> 1) & 7) + (idx & 1) * 8) = v;
-            };
-            float ss = 0.0f;
             if (tile4 <= 256) {
+                float ss = 0.0f;
                 float4 hv[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) hv[j] = (live && j * 32 + lane < n4) ? row[j * 32 + lane] : zero4;
@@ -251,29 +284,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
                 const float r = 1.0f / sqrtf(ss / (float)p.K + p.norm_eps);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    if (j * 32 + lane < tile4) put(j * 32 + lane, hv[j], wv[j], r);
+                    if (j * 32 + lane < tile4) sk_put_row(p, x_smem, x_box_bytes, t, live, j * 32 + lane, hv[j], wv[j], r);
             } else {
-                for (int base = 0; base < n4 && live; base += 256) {
-                    float4 hv[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) hv[j] = base + j * 32 + lane < n4 ? row[base + j * 32 + lane] : zero4;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) ss += (hv[j].x * hv[j].x + hv[j].y * hv[j].y) + (hv[j].z * hv[j].z + hv[j].w * hv[j].w);
-                }
-                ss = warp_sum(ss);
-                const float r = 1.0f / sqrtf(ss / (float)p.K + p.norm_eps);
-                for (int base = 0; base < tile4; base += 256) {
-                    float4 hv[8], wl[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int idx = base + j * 32 + lane;
-                        hv[j] = (live && idx < n4) ? row[idx] : zero4;
-                        wl[j] = idx < n4 ? w4[idx] : zero4;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (base + j * 32 + lane < tile4) put(base + j * 32 + lane, hv[j], wl[j], r);
-                }
+                sk_norm_row(p, x_smem, x_box_bytes, t, lane);
             }
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -394,6 +407,143 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     FERRIS_TL_END(40 + p.mode + (p.norm_h ? 4 : 0));
 }
 
+// SwiGLU products whose slab does not fit (the gate and up rows of the larger sizes): a CTA's outputs eight at a time, in PASSES, their gate
+// rows on rows 0-7 of the MMA's tile and their up rows on rows 8-15, so that a thread holds both sums of an output.  A slab of
+// 2 x 64 rows at once leaves a copy one K block (128 bytes) of each row, which comes out of HBM at 4.2 TB/s, and CTAs of 64 outputs two
+// rounds with a gap between; sixteen rows at once let a copy bring nine K blocks of them, and the ring runs on from pass to pass,
+// so that the copies never stop.  The step's rows are formed or brought in once for all passes.  Bound by HBM (figures: sk_passes).
+template <int NT, bool ACT = false>
+__global__ void __launch_bounds__(SK_THREADS, 1)
+    gemm_skinny_passes_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SkParams p) {
+    FERRIS_TL_ENTRY();
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t full[SK_WARPS], empty[SK_WARPS], full_x;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int box_bytes = 8 * p.nb * 128, stage_bytes = 2 * box_bytes;  // eight gate rows, eight up rows; a stage for every warp
+    const int x_box_bytes = p.x_rows * p.nb * 128;
+    uint8_t* x_smem = smem + (size_t)SK_WARPS * stage_bytes;
+    float* red = reinterpret_cast<float*>(x_smem + (size_t)p.groups * x_box_bytes);  // [pass & 1][warp][NT * 4][lane]
+    const int all = (p.N + 7) / 8;  // passes of the product, dealt to the CTAs in turn
+    const int passes = ((int)blockIdx.x < all) ? (all - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int total = passes * p.groups;
+    auto first_row = [&](int pass) { return 8 * ((int)blockIdx.x + pass * (int)gridDim.x); };
+    if (threadIdx.x == 0) {
+        tma_prefetch_descriptor(&map_w);
+        if (!p.norm_h) tma_prefetch_descriptor(&map_x);
+        for (int s = 0; s < SK_WARPS; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&full_x, 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    pdl_launch_dependents();
+
+    if (warp == SK_WARPS) {
+        int pass = 0, g = 0;  // of the group that is requested next
+        auto request = [&](int it) {
+            const int s = it % SK_WARPS, n0 = first_row(pass);
+            uint8_t* st = smem + (size_t)s * stage_bytes;
+            mbar_expect_tx(&full[s], stage_bytes);
+            tma_load_3d(st, &map_w, 0, g * p.nb, n0, &full[s]);
+            tma_load_3d(st + box_bytes, &map_w, 0, g * p.nb, p.up_row_offset + n0, &full[s]);
+            if (++g == p.groups) g = 0, ++pass;
+        };
+        const int first = min(total, SK_WARPS);
+        if (lane == 0)
+            for (int it = 0; it < first; ++it) request(it);  // a model's weights: ahead of the wait
+        if (!p.norm_h) {
+            pdl_wait();
+            if (lane == 0) mbar_expect_tx(&full_x, p.groups * x_box_bytes);
+            __syncwarp();
+            for (int i = lane; i < p.groups; i += 32) tma_load_3d(x_smem + (size_t)i * x_box_bytes, &map_x, 0, i * p.nb, 0, &full_x);
+        }
+        if (lane == 0)
+            for (int it = first; it < total; ++it) {
+                if (!mbar_wait(&empty[it % SK_WARPS], ((it / SK_WARPS) - 1) & 1, p.status, 43)) break;
+                request(it);
+            }
+        return;
+    }
+
+    if (p.norm_h)
+        for (int i = threadIdx.x; i * 32 < p.K; i += SK_WARPS * 32)  // one 128-byte line of the norm's weight per thread
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.norm_w + i * 32));
+    pdl_wait();
+    FERRIS_TL_BEGIN();
+    if (p.norm_h) {
+        for (int t = warp; t < p.x_rows; t += SK_WARPS) sk_norm_row(p, x_smem, x_box_bytes, t, lane);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+    } else {
+        mbar_wait(&full_x, 0, p.status, 42);
+    }
+    const int mi = lane >> 3, r8 = lane & 7;
+    const uint32_t x_base = smem_u32(x_smem), st = smem_u32(smem + (size_t)warp * stage_bytes);
+    // A operands: matrices (gate rows | up rows) x (columns 0-7 | 8-15 of the K step)
+    const uint32_t wg = st + (mi & 1) * box_bytes;
+    int it = warp, phase = 0;  // this warp's next group and its stage's phase
+    bool ok = true;
+    for (int pass = 0; pass < passes; ++pass) {
+        float acc[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[nt][j] = 0.0f;
+        const int g0 = pass * p.groups;
+        for (; it < g0 + p.groups; it += SK_WARPS, phase ^= 1) {
+            if (ok) ok = mbar_wait(&full[warp], phase, p.status, 44);
+            const int g = it - g0;
+            const uint32_t xg = x_base + g * x_box_bytes;
+            const int blocks = min(p.nb, p.kblocks - g * p.nb);
+            for (int kbi = 0; kbi < blocks; ++kbi) {
+                uint32_t b[4][NT][2], af[4][4];
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                    if (NT == 2) {
+                        uint32_t r[4];
+                        ldmatrix_x4(r, xg + swizzle128(((mi >> 1) * 8 + r8) * p.nb + kbi, ks * 2 + (mi & 1)));
+                        b[ks][0][0] = r[0], b[ks][0][1] = r[1], b[ks][NT - 1][0] = r[2], b[ks][NT - 1][1] = r[3];
+                    } else {
+                        uint32_t r[2];
+                        ldmatrix_x2(r, xg + swizzle128(r8 * p.nb + kbi, ks * 2 + (mi & 1)));
+                        b[ks][0][0] = r[0], b[ks][0][1] = r[1];
+                    }
+                    ldmatrix_x4(af[ks], wg + swizzle128(r8 * p.nb + kbi, ks * 2 + (mi >> 1)));
+                }
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[nt], af[ks], b[ks][nt][0], b[ks][nt][1]);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[warp]);
+        }
+        // the warps' sums, added in their order
+        float* mine = red + (size_t)(pass & 1) * (SK_WARPS * NT * 4 * 32);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mine[((warp * NT + nt) * 4 + j) * 32 + lane] = acc[nt][j];
+        asm volatile("bar.sync 1, 256;" ::: "memory");  // (the pass after the next writes here again, behind the next one's barrier)
+        if (threadIdx.x < NT * 64) {
+            const int ln = threadIdx.x & 31, e = threadIdx.x >> 5, j = e & 1, nt = e >> 1;
+            const int n = first_row(pass) + (ln >> 2), t = nt * 8 + (ln & 3) * 2 + j;
+            if (n < p.N && t < p.T) {
+                float gate = 0.0f, up = 0.0f;
+#pragma unroll
+                for (int w = 0; w < SK_WARPS; ++w) {
+                    gate += mine[((w * NT + nt) * 4 + j) * 32 + ln];
+                    up += mine[((w * NT + nt) * 4 + 2 + j) * 32 + ln];
+                }
+                sk_write<ACT>(p, t, n, gate, up, 0.0f, 0.0f);
+            }
+        }
+    }
+    FERRIS_TL_END(40 + p.mode + (p.norm_h ? 4 : 0));
+}
+
 int g_sk_sms = 0;
 int g_sk_enabled = -1;
 
@@ -497,6 +647,45 @@ bool sk_plan(int T, int N, int K, int accs, bool rows_by_tma, SkPlan* out) {
     return true;
 }
 
+// SwiGLU in passes of eight outputs: where the slab does not stand whole in shared memory, and copies of nine K blocks (or seven, where the
+// step's rows leave no more) fit beside the rows.  Fewer blocks a copy lose what the passes gain; more stages than one a warp bring
+// nothing (the others' copies are under way while a warp works on its own).  Measured (us a launch, weights from HBM, 1 / 8 / 16 tokens,
+// before and in passes of copies of nine): 2 x 18,944 x 3,584 56.7 / 57.1 / 59.4 -> 41.2 / 41.2 (6.6 TB/s) / as before, eight tokens at
+// seven blocks 44.6; 2 x 8,960 x 1,536 13.2 / 13.4 / 14.5 -> 11.8 / 11.5 / 12.4, at three 16.4; 2 x 11,008 x 4,096 61 / 62 / 64 -> 30.5 / 30.5 / as before, at
+// three blocks 64.
+bool sk_passes(int T, int N, int K, const SkPlan& whole, SkPlan* out) {
+    if ((K & 63) || whole.groups <= whole.stages) return false;
+    const int x_rows = T > 8 ? 16 : 8, nt = T > 8 ? 2 : 1, kblocks = K / SK_BLOCK_K;
+    const size_t red = (size_t)2 * SK_WARPS * nt * 4 * 32 * 4;
+    for (int nb = 9; nb >= 7; nb -= 2) {
+        const int groups = (kblocks + nb - 1) / nb;
+        const size_t smem = (size_t)groups * x_rows * nb * 128 + (size_t)SK_WARPS * 16 * nb * 128 + red;
+        if (nb > kblocks || smem > SK_PASS_SMEM) continue;
+        SkPlan q = whole;
+        q.nb = nb, q.groups = groups, q.stages = SK_WARPS, q.x_rows = x_rows, q.x_in_stages = 0;
+        q.smem = smem + 1024;
+        q.rows = q.box_rows = 8;
+        q.mt = 1;
+        const int sms = sk_sm_count(), all = (N + 7) / 8;
+        q.ctas = all < sms ? all : sms;
+        *out = q;
+        return true;
+    }
+    return false;
+}
+
+template <int NT, bool ACT = false>
+int sk_launch_passes(const CUtensorMap& mw, const CUtensorMap& mx, const SkParams& p, int ctas, size_t smem, cudaStream_t s) {
+    int rc = ferris_allow_dynamic_smem((const void*)gemm_skinny_passes_kernel<NT, ACT>, smem);
+    if (rc != FERRIS_OK) return rc;
+    cudaError_t e = ferris_launch(gemm_skinny_passes_kernel<NT, ACT>, dim3(ctas), dim3(SK_THREADS), smem, s, mw, mx, p);
+    if (e != cudaSuccess) {
+        ferris_set_error("skinny gemm: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    FERRIS_LAUNCH_CHECK();
+}
+
 template <int ACCS, int NT, bool ACT = false>
 int sk_launch(const CUtensorMap& mw, const CUtensorMap& mx, const SkParams& p, int ctas, size_t smem, cudaStream_t s) {
     int rc = ferris_allow_dynamic_smem((const void*)gemm_skinny_kernel<ACCS, NT, ACT>, smem);
@@ -550,6 +739,7 @@ FERRIS_API int ferris_gemm_skinny(const void* x, int ldx, const float* norm_h, c
         FERRIS_REFUSE("skinny gemm: %d tokens x %d outputs x K=%d is not a shape it takes (at most %d tokens, K a "
                       "multiple of 8, at most %d rows)", T, N, K, SK_MAX_TOKENS, 2 * SK_MAX_ROWS * sk_sm_count());
     if ((ldw & 7) || ldw < K || ((uintptr_t)w & 15)) FERRIS_REFUSE("skinny gemm: weight rows must be 16-byte aligned");
+    const bool passes = accs == 2 && sk_passes(T, N, K, plan, &plan);
     if (norm_h) {
         if (!norm_w || ((uintptr_t)norm_h & 15) || ((uintptr_t)norm_w & 15))
             FERRIS_REFUSE("skinny gemm: the rows to normalise and the norm's weight must be 16-byte aligned");
@@ -600,6 +790,10 @@ FERRIS_API int ferris_gemm_skinny(const void* x, int ldx, const float* norm_h, c
     p.status = ferris_status_ptr();
     p.act = act;
     cudaStream_t s = (cudaStream_t)stream;
+    if (passes && act.kind)
+        return T > 8 ? sk_launch_passes<2, true>(mw, mx, p, plan.ctas, plan.smem, s) : sk_launch_passes<1, true>(mw, mx, p, plan.ctas, plan.smem, s);
+    if (passes)
+        return T > 8 ? sk_launch_passes<2>(mw, mx, p, plan.ctas, plan.smem, s) : sk_launch_passes<1>(mw, mx, p, plan.ctas, plan.smem, s);
     if (accs == 2 && act.kind)
         return T > 8 ? sk_launch<2, 2, true>(mw, mx, p, plan.ctas, plan.smem, s) : sk_launch<2, 1, true>(mw, mx, p, plan.ctas, plan.smem, s);
     if (accs == 2)
