@@ -26,8 +26,10 @@
 
 namespace {
 
-constexpr int SP_WARPS = 16;
-constexpr int SP_THREADS = SP_WARPS * 32;  // 128 registers a thread; lane 0 of the leader's warp 0 issues the MMAs beside its work
+constexpr int SP_DRAINERS = 8;   // warps that add the accumulators up and write; lane 0 of the leader's first issues the MMAs
+constexpr int SP_SPLITTERS = 8;  // warps that load and split the operands
+constexpr int SP_THREADS = (SP_DRAINERS + SP_SPLITTERS) * 32;  // (128 registers a thread)
+constexpr int SP_ROWS = SP_SPLITTERS * 4;  // rows that the splitting warps take at a time, eight threads a row
 constexpr int SP_M = 128;                  // weight rows of a CTA, 256 of a pair
 constexpr int SP_K = 64;                   // k's of a slice: two runs of 32
 constexpr int SP_LEVEL = 16;               // slices whose runs are added up before they join the outer sum
@@ -115,21 +117,21 @@ __device__ __forceinline__ void tmem_store_32x8(uint32_t taddr, const uint32_t* 
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-template <int CW>  // tokens of a warp's columns; a tile has four times as many
+template <int NT>  // tokens of a tile
 struct SplitShape {
-    static constexpr int NT = 4 * CW;
+    static constexpr int CW = NT / 2;  // columns of a draining warp
     static constexpr int XR = NT / 2;  // token rows that a CTA holds
     static constexpr int B_PART = XR * 128;
     static constexpr int SLOT = 3 * (SP_A_PART + B_PART);
     static constexpr int EXCHANGE = 64 * NT * 4;  // SwiGLU: the up rows' sums
 };
 
-template <int CW, bool SWIGLU>
+template <int NT, bool SWIGLU>
 __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const SplitParams p) {
-    using S = SplitShape<CW>;
-    constexpr int XG = S::XR > 64 ? 2 : 1;  // runs of token rows that a thread may load
+    using S = SplitShape<NT>;
+    constexpr int CW = S::CW;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[2], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full[2], slot_free[2], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -142,9 +144,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
     const uint16_t both = (uint16_t)(3u << leader);
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&full[i], 2 * SP_WARPS);       // the warps of both CTAs (used in the leader only)
+            mbar_init(&full[i], 2 * SP_SPLITTERS);   // the splitting warps of both CTAs (used in the leader only)
+            mbar_init(&slot_free[i], 1);
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], 2 * SP_WARPS);  // (the leader's only)
+            mbar_init(&acc_empty[i], 2 * SP_DRAINERS);  // (the leader's only)
         }
         mbar_fence_init();
     }
@@ -156,242 +159,246 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
     const uint32_t tmem = tmem_base;
     pdl_launch_dependents();
 
-    const int quarter = warp & 3, wc = warp >> 2;
-    const int lr = tid >> 3, ch = tid & 7;  // this thread's rows (and those 64 further) and its 8 k's of a slice
-    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + wc * CW;
-    const uint32_t full_at = map_to_cta(smem_u32(&full[0]), leader), empty_at = map_to_cta(smem_u32(&acc_empty[0]), leader);
-    float4 wa[2][2], xb[XG][2];
-    // the slice that is loaded next; of its tile this thread's rows (null: beyond the operand), and the rows 64 further if `more`
-    int l_tile = first, l_slice = 0, l_it = 0;
-    const float* w_row = nullptr;
-    const float* x_row = nullptr;
-    bool w_more = false, x_more = false;
-    auto rows_of_tile = [&]() {
-        const int nt = l_tile / p.m_tiles, n = nt * (SWIGLU ? SP_M : 2 * SP_M) + (int)rank * (SWIGLU ? 64 : SP_M) + lr;
-        const int t = (l_tile - nt * p.m_tiles) * S::NT + (int)rank * S::XR + lr;
-        w_row = n < p.N ? p.w + (size_t)n * p.ldw + 8 * ch : nullptr;
-        w_more = SWIGLU ? n < p.N : n + 64 < p.N;
-        x_row = lr < S::XR && t < p.M ? p.x + (size_t)t * p.ldx + 8 * ch : nullptr;
-        x_more = lr + 64 < S::XR && t + 64 < p.M;
-    };
-    const size_t w_further = (size_t)(SWIGLU ? p.up_offset : 64) * p.ldw, x_further = (size_t)64 * p.ldx;
-    auto load8 = [&](float4 (&v)[2], const float* at, bool lo, bool hi) {
-        const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        v[0] = lo ? *reinterpret_cast<const float4*>(at) : none;
-        v[1] = hi ? *reinterpret_cast<const float4*>(at + 4) : none;
-    };
-    auto load_w = [&]() {
-        if (l_it >= total) return;
-        if (l_slice == 0) rows_of_tile();
-        const int k = (s0 + l_slice) * SP_K;
-        const bool lo = k + 8 * ch < p.K, hi = k + 8 * ch + 4 < p.K;
-        load8(wa[0], w_row + k, w_row && lo, w_row && hi);
-        load8(wa[1], w_row + k + w_further, w_more && lo, w_more && hi);
-        if (w_row && (ch & 3) == 0) {  // two slices on: from HBM into L2
-            const int far = k + 2 * SP_K;
-            if (far + 8 * ch < p.K) {
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(w_row + far));
-                if (w_more) asm volatile("prefetch.global.L2 [%0];" ::"l"(w_row + far + w_further));
-            }
-        }
-    };
-    auto load_x = [&]() {
-        if (l_it >= total) return;
-        const int k = (s0 + l_slice) * SP_K;
-        const bool lo = k + 8 * ch < p.K, hi = k + 8 * ch + 4 < p.K;
-        load8(xb[0], x_row + k, x_row && lo, x_row && hi);
-        if (XG > 1) load8(xb[XG - 1], x_row + k + x_further, x_more && lo, x_more && hi);
-        ++l_it;
-        if (++l_slice == per_tile) {
-            l_slice = 0;
-            l_tile += stride;
-        }
-    };
-    auto store = [&](int it) {  // the loaded slice goes to its slot, in parts
-        if (it >= total) return;
-        uint8_t* slot = smem + (it & 1) * S::SLOT;
-        uint4 p1, p2, p3;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            split8(wa[j][0], wa[j][1], p1, p2, p3);
-            uint8_t* at = slot + swizzle128(lr + 64 * j, ch);
-            *reinterpret_cast<uint4*>(at) = p1;
-            *reinterpret_cast<uint4*>(at + SP_A_PART) = p2;
-            *reinterpret_cast<uint4*>(at + 2 * SP_A_PART) = p3;
-        }
-#pragma unroll
-        for (int j = 0; j < XG; ++j) {
-            const int r = lr + 64 * j;
-            if (r >= S::XR) continue;
-            split8(xb[j][0], xb[j][1], p1, p2, p3);
-            uint8_t* at = slot + 3 * SP_A_PART + swizzle128(r, ch);
-            *reinterpret_cast<uint4*>(at) = p1;
-            *reinterpret_cast<uint4*>(at + S::B_PART) = p2;
-            *reinterpret_cast<uint4*>(at + 2 * S::B_PART) = p3;
-        }
-        asm volatile("fence.proxy.async;" ::: "memory");  // the tensor core reads what every lane wrote
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(full_at + 8u * (it & 1));
-    };
-    int ok = 1;  // 0: a wait ran out; no MMA is issued and nothing waited for any more, every barrier is still met
-    // Half h of slice `it`: 32 k's into accumulator h, the smallest products first.
-    auto issue = [&](int it, int h) {
-        if (warp != 0) return;
-        if (lane == 0 && rank == 0 && it < total && ok) {
-            const int s = it & 1;
-            ok = mbar_wait(&full[s], (it >> 1) & 1, p.status, 0x70) &&
-                 (it == 0 || mbar_wait(&acc_empty[h], (it - 1) & 1, p.status, 0x71));
-            if (ok) {
-                tcgen05_fence_after();
-                constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
-                const uint32_t at = smem_u32(smem + s * S::SLOT), idesc = umma_idesc_bf16(2 * SP_M, S::NT);
-                const uint64_t a = umma_desc_k_major_sw128(at), b = umma_desc_k_major_sw128(at + 3 * SP_A_PART);
-#pragma unroll
-                for (int i = 0; i < 6; ++i)
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const uint64_t step = (uint64_t)(2 * (2 * h + k));
-                        tcgen05_mma_bf16_pair(tmem + h * S::NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
-                                              b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
-                    }
-                tcgen05_commit_pair(&acc_full[h], both);
-            }
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-    };
-    if (p.early_weights) load_w();
-    pdl_wait();
-    if (!p.early_weights) load_w();
-    load_x();
-    store(0);
-    load_w();
-    load_x();
-    issue(0, 0);
-    issue(0, 1);
-    store(1);
-    load_w();
-    load_x();
-
     float acc[CW];
-#pragma unroll
-    for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
-    int tile = first, slice = 0;
-    for (int it = 0; it < total; ++it) {
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[h], it & 1, p.status, 0x72));
-            tcgen05_fence_after();
-#pragma unroll
-            for (int c0 = 0; c0 < CW; c0 += 24) {  // up to 24 columns under way
-                constexpr int AT_ONCE = 24;
-                uint32_t r[AT_ONCE];
-#pragma unroll
-                for (int c = 0; c < AT_ONCE && c0 + c < CW; c += 8) tmem_load_32x8(lane_addr + h * S::NT + c0 + c, r + c);
-                tmem_load_wait();
-#pragma unroll
-                for (int c = 0; c < AT_ONCE && c0 + c < CW; c += 2) {
-                    const float2 sum = add2(make_float2(acc[c0 + c], acc[c0 + c + 1]),
-                                            make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
-                    acc[c0 + c] = sum.x;
-                    acc[c0 + c + 1] = sum.y;
-                }
+    int ok = 1;  // 0: a wait ran out; no MMA is issued and nothing waited for any more, every barrier is still met
+    if (warp >= SP_DRAINERS) {
+        // -------------------------------------------------------------------------------- operands: fp32 -> three bf16 tiles
+        constexpr int WG = SP_M / SP_ROWS, XG = (S::XR + SP_ROWS - 1) / SP_ROWS;  // rows of a thread, SP_ROWS apart
+        const int ct = tid - SP_DRAINERS * 32, lr = ct >> 3, ch = ct & 7;         // its first row, its 8 k's of a slice
+        const uint32_t full_at = map_to_cta(smem_u32(&full[0]), leader);
+        float4 wa[WG][2], xb[XG][2];
+        int l_tile = first, l_slice = 0, l_it = 0;  // the slice that is loaded next
+        const float* w_row = nullptr;               // its tile's first row of this thread (the product's first where there is none)
+        const float* x_row = nullptr;
+        int w_left = 0, x_left = 0;                 // the operand's rows from there on
+        const int w_step = SP_ROWS * p.ldw, x_step = SP_ROWS * p.ldx;
+        const size_t w_up = SWIGLU ? (size_t)p.up_offset * p.ldw - (size_t)64 * p.ldw : 0;  // from a row 64 further to the up row
+        auto rows_of_tile = [&]() {
+            const int nt = l_tile / p.m_tiles, n = nt * (SWIGLU ? SP_M : 2 * SP_M) + (int)rank * (SWIGLU ? 64 : SP_M) + lr;
+            const int t = (l_tile - nt * p.m_tiles) * NT + (int)rank * S::XR + lr;
+            w_left = p.N - n, x_left = p.M - t;
+            w_row = p.w + (w_left > 0 ? (size_t)n * p.ldw : 0) + 8 * ch;
+            x_row = p.x + (x_left > 0 ? (size_t)t * p.ldx : 0) + 8 * ch;
+        };
+        auto load8 = [&](float4 (&v)[2], const float* at, bool lo, bool hi) {
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            v[0] = lo ? *reinterpret_cast<const float4*>(at) : none;
+            v[1] = hi ? *reinterpret_cast<const float4*>(at + 4) : none;
+        };
+        bool w_lo = false, w_hi = false, w_far = false;  // which of this thread's k's the slice has, and whether the one two further on
+        int w_k = 0;
+        // Turns to the slice that is loaded next; then its rows may be loaded, in any order (none beyond the last slice).
+        auto turn = [&]() {
+            if (l_it > 0 && ++l_slice == per_tile) {
+                l_slice = 0;
+                l_tile += stride;
             }
-            tcgen05_fence_before();
+            const bool any = l_it++ < total;
+            if (any && l_slice == 0) rows_of_tile();
+            w_k = (s0 + l_slice) * SP_K;
+            const int left = p.K - w_k - 8 * ch;  // k's from this thread's first on
+            w_lo = any && left > 0, w_hi = any && left > 4, w_far = any && left > 2 * SP_K && (ch & 3) == 0;
+        };
+        auto load_w = [&](int j) {
+            const bool there = (SWIGLU ? SP_ROWS * j % 64 : SP_ROWS * j) < w_left;
+            const float* at = w_row + w_k + j * w_step + (SWIGLU && SP_ROWS * j >= 64 ? w_up : 0);
+            load8(wa[j], at, there && w_lo, there && w_hi);
+            if (there && w_far) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 2 * SP_K));  // from HBM into L2
+        };
+        auto load_x = [&](int j) {
+            const bool there = SP_ROWS * j < x_left && SP_ROWS * j + lr < S::XR;
+            load8(xb[j], x_row + w_k + j * x_step, there && w_lo, there && w_hi);
+        };
+        const uint32_t at0 = swizzle128(lr, ch);  // (rows a multiple of eight further: the same swizzle)
+        turn();
+        if (!p.early_weights) pdl_wait();
+#pragma unroll
+        for (int j = 0; j < WG; ++j) load_w(j);
+        if (p.early_weights) pdl_wait();
+#pragma unroll
+        for (int j = 0; j < XG; ++j) load_x(j);
+        for (int it = 0; it < total; ++it) {
+            uint8_t* slot = smem + (it & 1) * S::SLOT + at0;
+            if (it >= 2 && ok) ok = __all_sync(0xffffffffu, mbar_wait(&slot_free[it & 1], ((it >> 1) - 1) & 1, p.status, 0x73));
+            turn();
+            uint4 p1, p2, p3;
+            // a run of rows is split and stored, and its registers take the next slice's at once
+#pragma unroll
+            for (int j = 0; j < WG; ++j) {
+                split8(wa[j][0], wa[j][1], p1, p2, p3);
+                load_w(j);
+                uint8_t* at = slot + j * SP_ROWS * 128;
+                *reinterpret_cast<uint4*>(at) = p1;
+                *reinterpret_cast<uint4*>(at + SP_A_PART) = p2;
+                *reinterpret_cast<uint4*>(at + 2 * SP_A_PART) = p3;
+            }
+#pragma unroll
+            for (int j = 0; j < XG; ++j) {
+                split8(xb[j][0], xb[j][1], p1, p2, p3);
+                load_x(j);
+                if (SP_ROWS * j + lr >= S::XR) continue;
+                uint8_t* at = slot + 3 * SP_A_PART + j * SP_ROWS * 128;
+                *reinterpret_cast<uint4*>(at) = p1;
+                *reinterpret_cast<uint4*>(at + S::B_PART) = p2;
+                *reinterpret_cast<uint4*>(at + 2 * S::B_PART) = p3;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what every lane wrote
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(empty_at + 8u * h);
-            issue(it + 1, h);
+            if (lane == 0) mbar_arrive_cluster(full_at + 8u * (it & 1));
         }
-        // both accumulators of slice `it` are complete: its slot is free
-        store(it + 2);
-        load_w();
-        load_x();
-        const bool last = slice + 1 == per_tile;
-        if ((slice + 1) % SP_LEVEL == 0 || (last && slice >= SP_LEVEL)) {  // the runs so far join the outer sum
+    } else {
+        // ---------------------------------------------------------------------------------------- MMAs, sums, outputs
+        const int quarter = warp & 3, wc = warp >> 2;
+        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + wc * CW;
+        const uint32_t empty_at = map_to_cta(smem_u32(&acc_empty[0]), leader);
+        // Half h of slice `it`: 32 k's into accumulator h, the smallest products first.
+        auto issue = [&](int it, int h) {
+            if (warp != 0) return;
+            if (lane == 0 && rank == 0 && it < total && ok) {
+                const int s = it & 1;
+                ok = (h == 1 || mbar_wait(&full[s], (it >> 1) & 1, p.status, 0x70)) &&
+                     (it == 0 || mbar_wait(&acc_empty[h], (it - 1) & 1, p.status, 0x71));
+                if (ok) {
+                    tcgen05_fence_after();
+                    constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
+                    const uint32_t at = smem_u32(smem + s * S::SLOT), idesc = umma_idesc_bf16(2 * SP_M, NT);
+                    const uint64_t a = umma_desc_k_major_sw128(at), b = umma_desc_k_major_sw128(at + 3 * SP_A_PART);
 #pragma unroll
-            for (int c = 0; c < CW; c += 8) {
-                uint32_t r[8];
-                if (slice >= SP_LEVEL) {
-                    tmem_load_32x8(lane_addr + 2 * S::NT + c, r);
-                    tmem_load_wait();
-                }
+                    for (int i = 0; i < 6; ++i)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float sum = slice >= SP_LEVEL ? __uint_as_float(r[i]) + acc[c + i] : acc[c + i];
-                    r[i] = __float_as_uint(sum);
-                    acc[c + i] = last ? sum : 0.0f;
-                }
-                if (!last) tmem_store_32x8(lane_addr + 2 * S::NT + c, r);
-            }
-            if (!last) tmem_store_wait();
-        }
-        ++slice;
-        if (!last) continue;
-        slice = 0;
-        if (!SWIGLU && splits > 1) break;  // one tile to a cluster: its sums meet below
-        const int t0 = (tile % p.m_tiles) * S::NT + wc * CW, nt = tile / p.m_tiles;
-        if (SWIGLU) {
-            float* up = reinterpret_cast<float*>(smem + 2 * S::SLOT) + (wc * CW) * 64 + (quarter & 1) * 32 + lane;
-            const int bar = 1 + wc * 2 + (quarter & 1);  // the warp of the gate rows and that of their up rows
-            if (quarter >= 2) {
-#pragma unroll
-                for (int c = 0; c < CW; ++c) up[c * 64] = acc[c];
-            }
-            asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
-            if (quarter < 2) {
-                const int n = nt * SP_M + (int)rank * 64 + quarter * 32 + lane;
-#pragma unroll
-                for (int c = 0; c < CW; ++c) {
-                    if (n < p.N && t0 + c < p.M) {
-                        float g = acc[c], u = up[c * 64];
-                        const float* row = p.x + (size_t)(t0 + c) * p.ldx;
-                        if (!is_finite(g)) g = dot_in_order(row, p.w + (size_t)n * p.ldw, p.K);
-                        if (!is_finite(u)) u = dot_in_order(row, p.w + (size_t)(n + p.up_offset) * p.ldw, p.K);
-                        p.out[(size_t)(t0 + c) * p.ldo + n] = u * (g * (1.0f / (1.0f + expf(-g))));
-                    }
+                        for (int k = 0; k < 2; ++k) {
+                            const uint64_t step = (uint64_t)(2 * (2 * h + k));
+                            tcgen05_mma_bf16_pair(tmem + h * NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
+                                                  b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
+                        }
+                    tcgen05_commit_pair(&acc_full[h], both);
+                    if (h == 1) tcgen05_commit_pair(&slot_free[s], both);
                 }
             }
-            asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
-        } else {
-            const int n = nt * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
-            if (n < p.N) {
-                const float bias = p.bias ? p.bias[n] : 0.0f;
-#pragma unroll
-                for (int c = 0; c < CW; ++c) {
-                    if (t0 + c < p.M) {
-                        float v = acc[c];
-                        if (!is_finite(v)) v = dot_in_order(p.x + (size_t)(t0 + c) * p.ldx, p.w + (size_t)n * p.ldw, p.K);
-                        if (p.bias) v += bias;
-                        float* o = p.out + (size_t)(t0 + c) * p.ldo + n;
-                        *o = p.accumulate ? *o + v : v;
-                    }
-                }
-            }
-        }
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+        };
+        pdl_wait();  // (an accumulating product reads what the launch before wrote)
+        issue(0, 0);
+        issue(0, 1);
 #pragma unroll
         for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
-        tile += stride;
+        int tile = first, slice = 0;
+        for (int it = 0; it < total; ++it) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[h], it & 1, p.status, 0x72));
+                tcgen05_fence_after();
+                constexpr int AT_ONCE = 16;
+#pragma unroll
+                for (int c0 = 0; c0 < CW; c0 += AT_ONCE) {
+                    uint32_t r[AT_ONCE];
+                    tmem_load_32x16(lane_addr + h * NT + c0, r);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int c = 0; c < AT_ONCE; c += 2) {
+                        const float2 sum = add2(make_float2(acc[c0 + c], acc[c0 + c + 1]),
+                                                make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+                        acc[c0 + c] = sum.x;
+                        acc[c0 + c + 1] = sum.y;
+                    }
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(empty_at + 8u * h);
+                issue(it + 1, h);
+            }
+            const bool last = slice + 1 == per_tile;
+            if ((slice + 1) % SP_LEVEL == 0 || (last && slice >= SP_LEVEL)) {  // the runs so far join the outer sum
+#pragma unroll
+                for (int c = 0; c < CW; c += 8) {
+                    uint32_t r[8];
+                    if (slice >= SP_LEVEL) {
+                        tmem_load_32x8(lane_addr + 2 * NT + c, r);
+                        tmem_load_wait();
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float sum = slice >= SP_LEVEL ? __uint_as_float(r[i]) + acc[c + i] : acc[c + i];
+                        r[i] = __float_as_uint(sum);
+                        acc[c + i] = last ? sum : 0.0f;
+                    }
+                    if (!last) tmem_store_32x8(lane_addr + 2 * NT + c, r);
+                }
+                if (!last) tmem_store_wait();
+            }
+            ++slice;
+            if (!last) continue;
+            slice = 0;
+            if (!SWIGLU && splits > 1) break;  // one tile to a cluster: its sums meet below
+            const int t0 = (tile % p.m_tiles) * NT + wc * CW, nt = tile / p.m_tiles;
+            if (SWIGLU) {
+                float* up = reinterpret_cast<float*>(smem + 2 * S::SLOT) + (wc * CW) * 64 + (quarter & 1) * 32 + lane;
+                const int bar = 1 + wc * 2 + (quarter & 1);  // the warp of the gate rows and that of their up rows
+                if (quarter >= 2) {
+#pragma unroll
+                    for (int c = 0; c < CW; ++c) up[c * 64] = acc[c];
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+                if (quarter < 2) {
+                    const int n = nt * SP_M + (int)rank * 64 + quarter * 32 + lane;
+#pragma unroll
+                    for (int c = 0; c < CW; ++c) {
+                        if (n < p.N && t0 + c < p.M) {
+                            float g = acc[c], u = up[c * 64];
+                            const float* row = p.x + (size_t)(t0 + c) * p.ldx;
+                            if (!is_finite(g)) g = dot_in_order(row, p.w + (size_t)n * p.ldw, p.K);
+                            if (!is_finite(u)) u = dot_in_order(row, p.w + (size_t)(n + p.up_offset) * p.ldw, p.K);
+                            p.out[(size_t)(t0 + c) * p.ldo + n] = u * (g * (1.0f / (1.0f + expf(-g))));
+                        }
+                    }
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+            } else {
+                const int n = nt * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
+                if (n < p.N) {
+                    const float bias = p.bias ? p.bias[n] : 0.0f;
+#pragma unroll
+                    for (int c = 0; c < CW; ++c) {
+                        if (t0 + c < p.M) {
+                            float v = acc[c];
+                            if (!is_finite(v)) v = dot_in_order(p.x + (size_t)(t0 + c) * p.ldx, p.w + (size_t)n * p.ldw, p.K);
+                            if (p.bias) v += bias;
+                            float* o = p.out + (size_t)(t0 + c) * p.ldo + n;
+                            *o = p.accumulate ? *o + v : v;
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
+            tile += stride;
+        }
     }
     if (!SWIGLU && splits > 1) {
         // groups of four tokens of a warp belong to the pairs in turn; a pair sends the others theirs
-        __syncwarp();
-        cluster_sync();  // every MMA of the cluster is done: the slots take partial sums now
-        constexpr int GROUPS = CW / 4;
+        constexpr int GROUPS = CW / 4, THREADS = SP_DRAINERS * 32;
         const int each = (GROUPS + splits - 1) / splits;  // groups of an owner
         const uint32_t ring = smem_u32(smem);
+        __syncwarp();
+        cluster_sync();  // every MMA of the cluster is done: the slots take partial sums now
+        if (warp < SP_DRAINERS) {
 #pragma unroll
-        for (int g = 0; g < GROUPS; ++g) {
-            const int owner = g % splits;
-            if (owner == split) continue;
-            const int place = (split < owner ? split : split - 1) * each + g / splits;
-            uint32_t v[4];
+            for (int g = 0; g < GROUPS; ++g) {
+                const int owner = g % splits;
+                if (owner == split) continue;
+                const int place = (split < owner ? split : split - 1) * each + g / splits;
+                uint32_t v[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = __float_as_uint(acc[4 * g + i]);
-            st_cluster_x4(map_to_cta(ring + (place * SP_THREADS + tid) * 16, 2 * owner + rank), v);
+                for (int i = 0; i < 4; ++i) v[i] = __float_as_uint(acc[4 * g + i]);
+                st_cluster_x4(map_to_cta(ring + (place * THREADS + tid) * 16, 2 * owner + rank), v);
+            }
         }
+        __syncwarp();
         cluster_sync();
-        const int t0 = (first % p.m_tiles) * S::NT + wc * CW;
+        const int quarter = warp & 3, wc = warp >> 2;
+        const int t0 = (first % p.m_tiles) * NT + wc * CW;
         const int n = first / p.m_tiles * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
-        if (n < p.N) {
+        if (warp < SP_DRAINERS && n < p.N) {
             const float bias = p.bias ? p.bias[n] : 0.0f;
 #pragma unroll
             for (int g = 0; g < GROUPS; ++g) {
@@ -401,7 +408,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
                     float4 v = make_float4(acc[4 * g], acc[4 * g + 1], acc[4 * g + 2], acc[4 * g + 3]);
                     if (from != split) {
                         const int place = (from < split ? from : from - 1) * each + g / splits;
-                        v = *reinterpret_cast<const float4*>(smem + (size_t)(place * SP_THREADS + tid) * 16);
+                        v = *reinterpret_cast<const float4*>(smem + (size_t)(place * THREADS + tid) * 16);
                     }
                     const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -420,6 +427,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             }
         }
     }
+    __syncwarp();
     tcgen05_fence_before();
     __syncthreads();
     cluster_sync();  // neither CTA frees tensor memory or leaves while the pair's MMAs or arrivals may still come
@@ -430,10 +438,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
 }
 
 // ------------------------------------------------------------------------------------------------- launching
-template <int CW, bool SWIGLU>
+template <int NT, bool SWIGLU>
 int launch_split(const SplitParams& p, int clusters, cudaStream_t s) {
-    const size_t smem = 2 * SplitShape<CW>::SLOT + (SWIGLU ? SplitShape<CW>::EXCHANGE : 0) + 1024;
-    if (int rc = ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<CW, SWIGLU>, smem)) return rc;
+    const size_t smem = 2 * SplitShape<NT>::SLOT + (SWIGLU ? SplitShape<NT>::EXCHANGE : 0) + 1024;
+    if (int rc = ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<NT, SWIGLU>, smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * p.splits * clusters);
     cfg.blockDim = dim3(SP_THREADS);
@@ -448,7 +456,7 @@ int launch_split(const SplitParams& p, int clusters, cudaStream_t s) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ferris_pdl_enabled() ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_split_kernel<CW, SWIGLU>, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_split_kernel<NT, SWIGLU>, p);
     if (e != cudaSuccess) {
         ferris_set_error("32-bit gemm: %s", cudaGetErrorString(e));
         return (int)e;
@@ -456,37 +464,63 @@ int launch_split(const SplitParams& p, int clusters, cudaStream_t s) {
     FERRIS_LAUNCH_CHECK();
 }
 template <bool SWIGLU>
-int launch_split_of(int cw, const SplitParams& p, int clusters, cudaStream_t s) {
-    if (cw == 8) return launch_split<8, SWIGLU>(p, clusters, s);
-    if (cw == 16) return launch_split<16, SWIGLU>(p, clusters, s);
-    if (cw == 24) return launch_split<24, SWIGLU>(p, clusters, s);
-    if (cw == 32) return launch_split<32, SWIGLU>(p, clusters, s);
-    return launch_split<40, SWIGLU>(p, clusters, s);
+int launch_split_of(int nt, const SplitParams& p, int clusters, cudaStream_t s) {
+    if (nt == 32) return launch_split<32, SWIGLU>(p, clusters, s);
+    if (nt == 64) return launch_split<64, SWIGLU>(p, clusters, s);
+    if (nt == 96) return launch_split<96, SWIGLU>(p, clusters, s);
+    if (nt == 128) return launch_split<128, SWIGLU>(p, clusters, s);
+    return launch_split<160, SWIGLU>(p, clusters, s);
 }
 
-// Clusters of 1 to 4 pairs that the GPU's 148 SMs hold at once, a CTA an SM (a cluster keeps to a GPC).
-constexpr int CLUSTERS[SP_MAX_SPLITS + 1] = {0, 74, 35, 22, 16};
+// Clusters of so many pairs that the GPU holds at once, a CTA an SM (a cluster keeps to a GPC).
+int active_clusters(int pairs) {
+    static int known[SP_MAX_SPLITS + 1] = {};
+    if (known[pairs] > 0) return known[pairs];
+    constexpr int UNKNOWN[SP_MAX_SPLITS + 1] = {0, 74, 32, 20, 12};
+    const size_t smem = 2 * SplitShape<128>::SLOT + 1024;
+    int n = 0;
+    if (ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<128, false>, smem) == FERRIS_OK) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * pairs);
+        cfg.blockDim = dim3(SP_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2 * pairs;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_split_kernel<128, false>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+    }
+    return known[pairs] = n > 0 ? n : UNKNOWN[pairs];
+}
 
 struct SplitPlan {
-    int cw, splits, clusters, m_tiles, n_tiles, slices_per;
-    double cycles;
+    int nt, splits, clusters, m_tiles, n_tiles, slices_per;
+    double us;
 };
-SplitPlan split_plan(int M, int rows, int K, bool swiglu, int cw_only = 0, int splits_only = 0) {
+// The cut of the least time, from what a slice was measured to take (us, token tiles of 32 to 160), a tile's end, the launch and a cluster's
+// exchange.
+SplitPlan split_plan(int M, int rows, int K, bool swiglu, int nt_only = 0, int splits_only = 0) {
+    constexpr double SLICE[5] = {2.0, 2.3, 2.5, 3.15, 4.5};
     SplitPlan best = {};
     const int slices = (K + SP_K - 1) / SP_K, n_tiles = (rows + 2 * SP_M - 1) / (2 * SP_M);
-    for (int cw = 8; cw <= 40; cw += 8) {
-        if (cw_only && cw != cw_only) continue;
-        const int nt = 4 * cw;
+    for (int nt = 32; nt <= 160; nt += 32) {
+        if (nt_only && nt != nt_only) continue;
         const long long m_tiles = (M + nt - 1) / nt;
-        const double slice = 250.0 + (12 * nt > 700 + 3 * nt ? 12 * nt : 700 + 3 * nt);  // cycles: MMAs, or splitting and draining
         for (int sp = 1; sp <= (swiglu ? 1 : SP_MAX_SPLITS); ++sp) {
             if (splits_only && sp != splits_only) continue;
             const int per = (slices + sp - 1) / sp;
             if (sp > 1 && (per < 4 || (sp - 1) * per >= slices)) continue;
-            const long long tiles = m_tiles * n_tiles, rounds = (tiles + CLUSTERS[sp] - 1) / CLUSTERS[sp];
-            const double cycles = rounds * (per * slice + (sp > 1 ? 9000.0 : 1500.0)) + 5000.0;
-            if (best.cw && cycles >= best.cycles) continue;
-            best = {cw, sp, (int)(sp > 1 || tiles < CLUSTERS[1] ? tiles : CLUSTERS[1]), (int)m_tiles, n_tiles, per, cycles};
+            const int at_once = active_clusters(sp);
+            const long long tiles = m_tiles * n_tiles, rounds = (tiles + at_once - 1) / at_once;
+            const double us = rounds * (per * SLICE[nt / 32 - 1] + (sp > 1 ? 7.0 : 1.0)) + 3.0;
+            if (best.nt && us >= best.us) continue;
+            best = {nt, sp, (int)(sp > 1 || tiles < at_once ? tiles : at_once), (int)m_tiles, n_tiles, per, us};
         }
     }
     return best;
@@ -496,7 +530,7 @@ int run_split(const float* x, const float* w, const float* bias, float* out, int
               int accumulate, int up_offset, int early_weights, const SplitPlan& q, cudaStream_t s) {
     const SplitParams p = {x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, up_offset, q.m_tiles, q.n_tiles, (K + SP_K - 1) / SP_K,
                            q.slices_per, q.splits, early_weights, ferris_status_ptr()};
-    return up_offset > 0 ? launch_split_of<true>(q.cw, p, q.clusters, s) : launch_split_of<false>(q.cw, p, q.clusters, s);
+    return up_offset > 0 ? launch_split_of<true>(q.nt, p, q.clusters, s) : launch_split_of<false>(q.nt, p, q.clusters, s);
 }
 
 }  // namespace
@@ -511,7 +545,7 @@ FERRIS_API int ferris_gemm_f32_split_run(const float* x, const float* w, const f
     if ((long long)((M + 31) / 32) * ((2LL * N + 255) / 256) >= (1 << 28)) FERRIS_REFUSE("gemm: %d x %d outputs", M, N);
     if (token_tile % 32 || token_tile < 0 || token_tile > 160 || splits < 0 || splits > SP_MAX_SPLITS || (swiglu && (splits > 1 || bias || accumulate)))
         FERRIS_REFUSE("gemm: token tile %d, %d splits", token_tile, splits);
-    const SplitPlan q = split_plan(M, swiglu ? 2 * N : N, K, swiglu != 0, token_tile / 4, splits);
-    if (!q.cw) FERRIS_REFUSE("gemm: %d k's in %d splits", K, splits);
+    const SplitPlan q = split_plan(M, swiglu ? 2 * N : N, K, swiglu != 0, token_tile, splits);
+    if (!q.nt) FERRIS_REFUSE("gemm: %d k's in %d splits", K, splits);
     return run_split(x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, swiglu ? N : 0, 0, q, (cudaStream_t)stream);
 }
