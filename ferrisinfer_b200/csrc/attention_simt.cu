@@ -18,6 +18,7 @@
 // cache when this runs, so prompts, portions of prompts and single decoded tokens are one case.
 #include <math.h>
 
+#include "attention_f32_split.cuh"
 #include "attention_general.cuh"
 #include "common.cuh"
 
@@ -921,7 +922,7 @@ FERRIS_API int ferris_paged_attention_tiled_takes(int dtype, int nh, int nkv, in
     return tiled_takes(dtype, nh, nkv, d, dv) ? 1 : 0;
 }
 
-// The same attention as ferris_paged_attention_simt (same arguments), for steps that bring portions of prompts.
+// The same attention as ferris_paged_attention_simt (same arguments), for steps that bring portions of prompts; seqs: the step's requests.
 FERRIS_API int ferris_paged_attention_tiled(const void* q, int ldq, void* out, int ldo, const void* k_cache,
                                             const void* v_cache, int dtype, const int* block_tables, int max_blocks,
                                             const int* token_seq, const int* positions, int tokens, int nh, int nkv,
@@ -929,8 +930,9 @@ FERRIS_API int ferris_paged_attention_tiled(const void* q, int ldq, void* out, i
                                             const float* log_r1, const float* log_r2, const float* sink, int v_stride,
                                             const void* pool_k, const void* pool_v, const int* pool_tables,
                                             int pool_max_blocks, int pool_every, int keep, float softcap,
-                                            const void* gate, int ldgate, void* stream) {
+                                            const void* gate, int ldgate, int seqs, void* stream) {
     if (tokens <= 0) return FERRIS_OK;
+    if (seqs <= 0) FERRIS_REFUSE("tiled attention: %d requests", seqs);
     if ((log_r1 == nullptr) != (log_r2 == nullptr) || (slopes && log_r1)) FERRIS_REFUSE("tiled attention: one kind of distance penalty, with all its numbers");
     if (v_stride < 0 || (v_stride > 0 && v_stride < dv)) FERRIS_REFUSE("tiled attention: value rows %d apart hold no %d values", v_stride, dv);
     const ScoreTerms st = {slopes, log_r1, log_r2, sink, v_stride, softcap, gate, ldgate};
@@ -944,6 +946,10 @@ FERRIS_API int ferris_paged_attention_tiled(const void* q, int ldq, void* out, i
         FERRIS_REFUSE("tiled attention: rows must start on 16 bytes");
     if (nkv > 65535) FERRIS_REFUSE("attention: %d kv heads are more than one launch takes", nkv);
     cudaStream_t s = (cudaStream_t)stream;
+    const bool plain = !slopes && !log_r1 && !sink && !gate && softcap == 0.0f && pk.every == 0 && pk.keep == 0 && (v_stride == 0 || v_stride == dv);
+    if (dtype == FERRIS_F32 && plain && ferris_attention_f32_split_takes(nh, nkv, d, dv))
+        return ferris_attention_f32_split((const float*)q, ldq, (float*)out, ldo, (const float*)k_cache, (const float*)v_cache, block_tables,
+                                          max_blocks, token_seq, positions, tokens, nh, nkv, page_size, window, scale, seqs, s);
 #define FERRIS_TILED(T, POOL)                                                                                             \
     return launch_tiled<T, POOL>(q, ldq, out, ldo, k_cache, v_cache, block_tables, max_blocks, token_seq, positions, tokens, \
                                  nh, nkv, d, dv, page_size, window, scale, st, pk, s)

@@ -1,6 +1,7 @@
-// The 32-bit path's matrix products: out[t, n] (+)= sum_k x[t, k] * w[n, k] (+ bias[n]), every product and sum an fp32 FMA
+// The 32-bit path's matrix products of up to 150 million multiply-adds or 32 rows (gemm_f32_split.cu takes the larger ones): out[t, n] (+)=
+// sum_k x[t, k] * w[n, k] (+ bias[n]), every product and sum an fp32 FMA
 // or an fp32 add on the CUDA cores (no tensor cores, no reduced precision), in ONE order of summation for every number of
-// rows, so that a row's result does not depend on what else is in the batch: within runs of F32_CHUNK the even and the odd k's
+// rows that comes here, so that a row's result does not depend on what else is in the batch: within runs of F32_CHUNK the even and the odd k's
 // ascending, each a chain of FMAs, and the two added; the runs added in ascending order within at most F32_PARTS parts of K, the parts in ascending order (gemm_simt.cu, which takes
 // what is not aligned, sums in the same order).  Runs that add up by themselves are what lets several lanes, warps
 // and CTAs work on one output; they also halve the rounding error of one long chain.
@@ -426,6 +427,8 @@ int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* ou
                         early_weights, 0};
         return launch_rows_of(p, q, s);
     }
+    if (ferris_gemm_f32_split_takes(M, N, K, ldx, ldw))
+        return ferris_gemm_f32_split(x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, 0, early_weights, s);
     const int runs = (K + F32_CHUNK - 1) / F32_CHUNK, per = f32_runs_per_part(runs);
     const int parts = (runs + per - 1) / per;
     if ((M + BM - 1) / BM > 65535) {
@@ -440,11 +443,12 @@ int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* ou
 
 constexpr int SWIGLU_MAX_TOKENS = 16;  // (beyond, the plain product may run the tiles)
 
-// Whether ferris_gemm_f32_swiglu takes a product of M tokens and N outputs: 16 tokens at most, rows that begin on 16 bytes, and
-// weights that the rows kernel reads in fewer microseconds than the tiles.
+// Whether ferris_gemm_f32_swiglu takes a product of M tokens and N outputs, of rows that begin on 16 bytes: few tokens whose weights the
+// rows kernel reads in fewer microseconds than the tiles, and what goes to the tensor cores.
 FERRIS_API int ferris_gemm_f32_swiglu_takes(const void* x, const void* w, int M, int N, int K, int ldx, int ldw) {
     RowsPlan q;
-    return M > 0 && M <= SWIGLU_MAX_TOKENS && N > 0 && ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw) && rows_take(M, 2 * N, K, 2 * RS, q);
+    if (M <= 0 || N <= 0 || N > (1 << 30) || !ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw)) return 0;
+    return M <= SWIGLU_MAX_TOKENS ? rows_take(M, 2 * N, K, 2 * RS, q) : ferris_gemm_f32_split_takes(M, 2 * N, K, ldx, ldw);
 }
 // out[t, n] = silu(x[t] . w[n]) (x[t] . w[N + n]), fp32 throughout, with the sums of every other form of the product.
 // early_weights: no launch that may still run writes w.
@@ -454,6 +458,8 @@ FERRIS_API int ferris_gemm_f32_swiglu(const float* x, const float* w, float* out
     if (K <= 0 || ldx < K || ldw < K || ldo < N) FERRIS_REFUSE("gemm: K=%d, row strides %d, %d, %d", K, ldx, ldw, ldo);
     if (!ferris_gemm_f32_swiglu_takes(x, w, M, N, K, ldx, ldw))
         FERRIS_REFUSE("gemm: %d tokens x %d outputs of %d do not take SwiGLU on the way", M, N, K);
+    if (M > SWIGLU_MAX_TOKENS)
+        return ferris_gemm_f32_split(x, w, nullptr, out, M, N, K, ldx, ldw, ldo, 0, N, early_weights, (cudaStream_t)stream);
     RowsPlan q;
     rows_plan(M, 2 * N, K, 2 * RS, q);
     RowsParams p = {x, w, nullptr, out, M, N, K, ldx, ldw, ldo, 0, q.rows_per_cta, q.phases, q.stages, ferris_status_ptr(), early_weights, N};

@@ -15,3 +15,10 @@ bool ferris_gemm_f32_takes(const void* x, const void* w, const void* out, int K,
 // early_weights: no launch that may still run writes w.
 int ferris_gemm_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx, int ldw,
                     int ldo, int accumulate, int early_weights, cudaStream_t s, bool* taken);
+
+// Products of many tokens on the tensor cores, operands and sums of 32 bits (gemm_f32_split.cu): which it takes (rows as
+// ferris_gemm_f32_takes has them; `rows`: weight rows), and the product (up_offset > 0: SwiGLU of N gate rows and the N rows up_offset
+// further).
+bool ferris_gemm_f32_split_takes(int M, int rows, int K, int ldx, int ldw);
+int ferris_gemm_f32_split(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx, int ldw,
+                          int ldo, int accumulate, int up_offset, int early_weights, cudaStream_t s);

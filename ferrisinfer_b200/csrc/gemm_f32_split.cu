@@ -34,6 +34,7 @@ constexpr int SP_M = 128;                  // weight rows of a CTA, 256 of a pai
 constexpr int SP_K = 64;                   // k's of a slice: two runs of 32
 constexpr int SP_LEVEL = 16;               // slices whose runs are added up before they join the outer sum
 constexpr int SP_MAX_SPLITS = 4;
+constexpr int SP_MAX_LD = 1 << 24;         // elements between rows (offsets of a thread's rows are 32-bit numbers)
 constexpr int SP_A_PART = SP_M * 128;      // bytes of one part of a slice of the weights
 
 struct SplitParams {
@@ -535,14 +536,27 @@ int run_split(const float* x, const float* w, const float* bias, float* out, int
 
 }  // namespace
 
-// The product on the tensor cores, cut as told (token_tile 32 to 160 in steps of 32, splits 1 to 4; 0: by the plan).  Rows aligned as
+// More than 32 tokens and 150 million multiply-adds.  Up to there every form of the product adds in one order, so that a row's bits do not depend
+// on how many others the step brings; from 33 tokens on this kernel would win there too, by 4 to 6 us of 18 to 27.
+bool ferris_gemm_f32_split_takes(int M, int rows, int K, int ldx, int ldw) {
+    return M > 32 && (long long)M * rows * K >= 150000000LL && (long long)((M + 31) / 32) * ((rows + 255) / 256) < (1 << 28) &&
+           ldx <= SP_MAX_LD && ldw <= SP_MAX_LD;
+}
+
+int ferris_gemm_f32_split(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx, int ldw,
+                          int ldo, int accumulate, int up_offset, int early_weights, cudaStream_t s) {
+    return run_split(x, w, bias, out, M, N, K, ldx, ldw, ldo, accumulate, up_offset, early_weights,
+                     split_plan(M, up_offset > 0 ? 2 * N : N, K, up_offset > 0), s);
+}
+
+// The product on the tensor cores whatever its size, cut as told (token_tile 32 to 160 in steps of 32, splits 1 to 4; 0: by the plan).  Rows aligned as
 // ferris_gemm_f32_takes has it; swiglu: N outputs of 2 N weight rows, gate rows first.
 FERRIS_API int ferris_gemm_f32_split_run(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx,
                                          int ldw, int ldo, int accumulate, int swiglu, int token_tile, int splits, void* stream) {
     if (M <= 0 || N <= 0) return FERRIS_OK;
     if (K <= 0 || ldx < K || ldw < K || ldo < N) FERRIS_REFUSE("gemm: K=%d, row strides %d, %d, %d", K, ldx, ldw, ldo);
     if (!ferris_gemm_f32_takes(x, w, out, K, ldx, ldw)) FERRIS_REFUSE("gemm: rows that do not begin on 16 bytes");
-    if ((long long)((M + 31) / 32) * ((2LL * N + 255) / 256) >= (1 << 28)) FERRIS_REFUSE("gemm: %d x %d outputs", M, N);
+    if ((long long)((M + 31) / 32) * ((2LL * N + 255) / 256) >= (1 << 28) || ldx > SP_MAX_LD || ldw > SP_MAX_LD) FERRIS_REFUSE("gemm: %d x %d outputs", M, N);
     if (token_tile % 32 || token_tile < 0 || token_tile > 160 || splits < 0 || splits > SP_MAX_SPLITS || (swiglu && (splits > 1 || bias || accumulate)))
         FERRIS_REFUSE("gemm: token tile %d, %d splits", token_tile, splits);
     const SplitPlan q = split_plan(M, swiglu ? 2 * N : N, K, swiglu != 0, token_tile, splits);

@@ -643,7 +643,7 @@ def gemm_activation(x, w, out, kind: str, coefficients=(0.0, 0.0), params: Optio
 
 def gemm_swiglu(x, gate_up_weight, out, workspace=None, fixed_weight: Optional[bool] = None):
     """out [T, I] = silu(x Wg^T) * (x Wu^T) with gate_up_weight = [Wg; Wu] ([2I, K]).  bf16: one tensor-core
-    kernel with two accumulators (the [T, 2I] intermediate never exists), so too 32-bit steps of few tokens; otherwise
+    kernel with two accumulators (the [T, 2I] intermediate never exists), so too 32-bit steps of few tokens and of many; otherwise
     a product and the SwiGLU kernel.  ``fixed_weight`` as in ``gemm``."""
     if fixed_weight is False:
         with _StreamOrder():
@@ -662,7 +662,7 @@ def gemm_swiglu(x, gate_up_weight, out, workspace=None, fixed_weight: Optional[b
     if tensor_core_gemm_takes(x, gate_up_weight) and out.dtype == torch.bfloat16:
         gemm_tcgen05(x, gate_up_weight, None, out, 3, up_row_offset=I, fixed_weight=fixed_weight)
         return
-    if T <= 16 and x.dtype == gate_up_weight.dtype == out.dtype == torch.float32:
+    if x.dtype == gate_up_weight.dtype == out.dtype == torch.float32:
         T2, K, ldx = _rows(x, "gemm input")
         _, K2, ldw = _rows(gate_up_weight, "gemm weight")
         _, _, ldo = _rows(out, "gemm output")
@@ -1013,7 +1013,7 @@ def paged_attention_simt(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Te
             and _lib().ferris_paged_attention_tiled_takes(_c_int(_dt(qkv, "attention")), _c_int(num_heads),
                                                           _c_int(num_kv_heads), _c_int(head_dim), _c_int(dv)):
         fn = _lib().ferris_paged_attention_tiled
-        extra = ()
+        extra = (_c_int(block_tables.shape[0]),)
     _check(
         fn(_ptr(qkv), _c_int(ldq), _ptr(out), _c_int(ldo), _ptr(k_cache), _ptr(v_cache),
                                            _dt(qkv, "attention"), _ptr(block_tables), _c_int(block_tables.shape[1]),
@@ -1023,7 +1023,7 @@ def paged_attention_simt(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Te
                                            _ptr(terms.log_r1),
                                            _ptr(terms.log_r2), _ptr(terms.sink), _c_int(v_stride), *pool_args, *extra,
                                            _stream()),
-        "paged attention", 2 if extra and extra[0].value > 0 else 1,
+        "paged attention", 2 if len(extra) == 3 and extra[0].value > 0 else 1,
     )
 
 

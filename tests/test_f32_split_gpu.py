@@ -1,4 +1,4 @@
-"""The 32-bit path's products of many tokens on tensor cores (operands in three bf16 parts), against 64 bits and against the FMA
+"""The 32-bit path's products of many tokens and its attention of prompts on tensor cores (operands in three bf16 parts), against 64 bits and against the FMA
 kernels where numbers are not finite."""
 
 import math
@@ -6,7 +6,7 @@ import math
 import pytest
 import torch
 
-from test_kernels_gpu import rnd
+from test_kernels_gpu import AttentionCase, rnd
 
 pytestmark = pytest.mark.gpu
 
@@ -100,3 +100,73 @@ def test_split_products_of_infinities_and_of_the_largest_numbers(device):
         ops.gemm_simt(x[t:t + 1], w, None, gate_up)
         ops.swiglu(gate_up, want)
         assert torch.allclose(out[t], want[0], rtol=1e-4, atol=1e-4, equal_nan=True), t
+
+
+def test_long_products_go_to_the_tensor_cores_by_their_size(device):
+    """``gemm`` of a long step: the split product's bits; the weight may be what the launch before writes; SwiGLU in one launch."""
+    from ferrisinfer_b200.kernels import ops
+
+    x, w = rnd((300, 896), F32, device, 31), rnd((1152, 896), F32, device, 32, 0.1)
+    out, want, late = torch.empty(300, 1152, device=device), torch.empty(300, 1152, device=device), torch.empty_like(w)
+    ops.gemm_f32_split(x, w, None, want)
+    ops.gemm(x, w, None, out, fixed_weight=True)
+    assert torch.equal(out, want)
+    late.copy_(w)
+    ops.gemm(x, late, None, out, fixed_weight=False)
+    assert torch.equal(out, want)
+    act, one = torch.empty(300, 576, device=device), torch.empty(300, 576, device=device)
+    ops.gemm_f32_split(x, w, None, one, swiglu=True)
+    before = ops.launch_count()
+    ops.gemm_swiglu(x, w, act, fixed_weight=True)
+    assert ops.launch_count() - before == 1 and torch.equal(act, one)
+    assert ops.kernel_status() == 0
+
+
+# ------------------------------------------------------------------------------------------------------------------ attention
+@pytest.mark.parametrize("window", [0, 50])
+@pytest.mark.parametrize("nh, nkv, page", [(14, 2, 16), (5, 5, 8), (3, 1, 5), (64, 1, 32), (22, 2, 16)])
+def test_split_attention_of_all_lengths(nh, nkv, page, window, device):
+    """Groups that fill a block's 64 rows and that leave some idle; requests that end inside a tile of keys, at its edge and one
+    beyond, several in a block, single tokens among them."""
+    seqs = [(1, 1), (64, 64), (65, 2), (63, 63), (129, 70), (200, 1), (7, 3), (128, 64), (300, 11)]
+    case = AttentionCase(device, F32, nh, nkv, 64, page, seqs, seed=nh + window, window=window)
+    from ferrisinfer_b200.kernels import ops
+
+    qkv, k, v, tables, ctx, T = case.device_inputs()
+    out = torch.full((T, nh * 64 + 3), 7.0, device=device)
+    ops.paged_attention_simt(qkv, out[:, :nh * 64], k, v, tables, ctx.token_seq, ctx.positions, nh, nkv, 64, window, 0.125, max_q_len=70)
+    got, want = out[:, :nh * 64].cpu().double(), case.reference()
+    # scores to 40 2^-24 of their size (at most 64 products of a few units each), as much again for weights and sums over 300 keys
+    assert (got - want).abs().max() <= 2e-5 and (got - want).norm() <= 1e-6 * want.norm()
+    assert (out[:, nh * 64:] == 7.0).all()
+
+
+def test_split_attention_of_single_tokens_beside_a_prompt(device):
+    """More requests than a block's tokens."""
+    from ferrisinfer_b200.kernels import ops
+
+    seqs = [(1 + 67 * i % 400, 1) for i in range(40)] + [(90, 90), (3, 2)]
+    case = AttentionCase(device, F32, 14, 2, 64, 16, seqs, seed=8)
+    qkv, k, v, tables, ctx, T = case.device_inputs()
+    out = torch.full((T, 14 * 64), float("nan"), device=device)
+    ops.paged_attention_simt(qkv, out, k, v, tables, ctx.token_seq, ctx.positions, 14, 2, 64, 0, 0.125, max_q_len=90)
+    want = case.reference()
+    assert (out.cpu().double() - want).norm() <= 1e-6 * want.norm()
+
+
+def test_split_attention_of_infinities(device):
+    """Rows that meet an infinity: the numbers of the kernel for single tokens; the others are left alone."""
+    from ferrisinfer_b200.kernels import ops
+
+    case = AttentionCase(device, F32, 14, 2, 64, 16, [(100, 100), (30, 20)], seed=5)
+    qkv, k, v, tables, ctx, T = case.device_inputs()
+    page = int(tables[0, 2])  # positions 32 .. 47 of the first request
+    k[page, 0, 3, 5] = -math.inf
+    v[page, 1, 4, 6] = math.inf
+    qkv[70, 64 + 9] = math.inf
+    out, want = torch.empty(T, 14 * 64, device=device), torch.empty(T, 14 * 64, device=device)
+    args = (k, v, tables, ctx.token_seq, ctx.positions, 14, 2, 64, 0, 0.125)
+    ops.paged_attention_simt(qkv, out, *args, max_q_len=100)
+    ops.paged_attention_simt(qkv, want, *args, max_q_len=1)
+    assert torch.allclose(out, want, rtol=1e-4, atol=2e-5, equal_nan=True)
+    assert not torch.isfinite(out).all() and torch.isfinite(out[:32]).all()
