@@ -27,14 +27,20 @@
 namespace {
 
 constexpr int SP_DRAINERS = 8;   // warps that add the accumulators up and write; lane 0 of the leader's first issues the MMAs
-constexpr int SP_SPLITTERS = 8;  // warps that load and split the operands
-constexpr int SP_THREADS = (SP_DRAINERS + SP_SPLITTERS) * 32;  // (128 registers a thread)
+constexpr int SP_SPLITTERS = 16; // warps that load and split the operands
+constexpr int SP_THREADS = (SP_DRAINERS + SP_SPLITTERS) * 32;
+// Registers a thread: 80 at the launch, then so many for either kind of warp, which together are no more.
+constexpr int SP_LAUNCH_REGS = 80, SP_DRAIN_REGS = 128, SP_SPLIT_REGS = 56;
+static_assert(SP_DRAINERS * SP_DRAIN_REGS + SP_SPLITTERS * SP_SPLIT_REGS <= (SP_DRAINERS + SP_SPLITTERS) * SP_LAUNCH_REGS &&
+                  SP_THREADS * SP_LAUNCH_REGS <= 65536 && SP_DRAINERS % 4 == 0 && SP_SPLITTERS % 4 == 0,
+              "the shares come out of the launch's registers, by groups of four warps");
 constexpr int SP_ROWS = SP_SPLITTERS * 4;  // rows that the splitting warps take at a time, eight threads a row
 constexpr int SP_M = 128;                  // weight rows of a CTA, 256 of a pair
 constexpr int SP_K = 64;                   // k's of a slice: two runs of 32
-constexpr int SP_LEVEL = 16;               // slices whose runs are added up before they join the outer sum
+constexpr int SP_LEVEL = 20;               // slices whose runs are added up before they join the outer sum
 constexpr int SP_MAX_SPLITS = 4;
 constexpr int SP_MAX_LD = 1 << 24;         // elements between rows (offsets of a thread's rows are 32-bit numbers)
+constexpr int SP_EXCHANGE = 4 * 16 * 32 * 4;  // SwiGLU: sums of up rows on their way, of sixteen tokens for each pair of warps
 constexpr int SP_A_PART = SP_M * 128;      // bytes of one part of a slice of the weights
 
 struct SplitParams {
@@ -84,7 +90,7 @@ __device__ __forceinline__ void split8(const float4 a, const float4 b, uint4& p1
 }
 
 // One output in the order of the FMA kernels.
-__device__ __noinline__ float dot_in_order(const float* x, const float* w, int K) {
+__device__ __forceinline__ float dot_in_order(const float* x, const float* w, int K) {
     const int runs = (K + F32_CHUNK - 1) / F32_CHUNK, per = f32_runs_per_part(runs);
     float total = 0.0f, part = 0.0f;
     for (int c = 0; c < runs; ++c) {
@@ -101,6 +107,21 @@ __device__ __noinline__ float dot_in_order(const float* x, const float* w, int K
         }
     }
     return total;
+}
+
+// An output whose sum is not finite.
+template <bool SWIGLU>
+__device__ __forceinline__ void write_in_order(const SplitParams& p, int t, int n) {
+    const float* x = p.x + (size_t)t * p.ldx;
+    float* o = p.out + (size_t)t * p.ldo + n;
+    float v = dot_in_order(x, p.w + (size_t)n * p.ldw, p.K);
+    if (SWIGLU) {
+        const float u = dot_in_order(x, p.w + (size_t)(n + p.up_offset) * p.ldw, p.K);
+        *o = u * (v * (1.0f / (1.0f + expf(-v))));
+    } else {
+        if (p.bias) v += p.bias[n];
+        *o = p.accumulate ? *o + v : v;
+    }
 }
 
 __device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
@@ -124,7 +145,6 @@ struct SplitShape {
     static constexpr int XR = NT / 2;  // token rows that a CTA holds
     static constexpr int B_PART = XR * 128;
     static constexpr int SLOT = 3 * (SP_A_PART + B_PART);
-    static constexpr int EXCHANGE = 64 * NT * 4;  // SwiGLU: the up rows' sums
 };
 
 template <int NT, bool SWIGLU>
@@ -160,9 +180,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
     const uint32_t tmem = tmem_base;
     pdl_launch_dependents();
 
-    float acc[CW];
     int ok = 1;  // 0: a wait ran out; no MMA is issued and nothing waited for any more, every barrier is still met
     if (warp >= SP_DRAINERS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SP_SPLIT_REGS));
         // -------------------------------------------------------------------------------- operands: fp32 -> three bf16 tiles
         constexpr int WG = SP_M / SP_ROWS, XG = (S::XR + SP_ROWS - 1) / SP_ROWS;  // rows of a thread, SP_ROWS apart
         const int ct = tid - SP_DRAINERS * 32, lr = ct >> 3, ch = ct & 7;         // its first row, its 8 k's of a slice
@@ -247,74 +267,83 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(full_at + 8u * (it & 1));
         }
+        if (!SWIGLU && splits > 1) {  // (the draining warps' exchange)
+            __syncwarp();
+            cluster_sync();
+            cluster_sync();
+        }
     } else {
         // ---------------------------------------------------------------------------------------- MMAs, sums, outputs
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SP_DRAIN_REGS));
         const int quarter = warp & 3, wc = warp >> 2;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + wc * CW;
         const uint32_t empty_at = map_to_cta(smem_u32(&acc_empty[0]), leader);
-        // Half h of slice `it`: 32 k's into accumulator h, the smallest products first.
-        auto issue = [&](int it, int h) {
+        // Slice `it`: the two runs of 32 k's into the two accumulators of its set, the smallest products first.  A product waits for the one
+        // before it in the same accumulator (some 190 cycles whatever the width), so the runs take turns.
+        auto issue = [&](int it) {
             if (warp != 0) return;
             if (lane == 0 && rank == 0 && it < total && ok) {
                 const int s = it & 1;
-                ok = (h == 1 || mbar_wait(&full[s], (it >> 1) & 1, p.status, 0x70)) &&
-                     (it == 0 || mbar_wait(&acc_empty[h], (it - 1) & 1, p.status, 0x71));
+                ok = mbar_wait(&full[s], (it >> 1) & 1, p.status, 0x70) &&
+                     (it < 2 || mbar_wait(&acc_empty[s], ((it >> 1) - 1) & 1, p.status, 0x71));
                 if (ok) {
                     tcgen05_fence_after();
                     constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
-                    const uint32_t at = smem_u32(smem + s * S::SLOT), idesc = umma_idesc_bf16(2 * SP_M, NT);
+                    const uint32_t at = smem_u32(smem + s * S::SLOT), idesc = umma_idesc_bf16(2 * SP_M, NT), d = tmem + s * 2 * NT;
                     const uint64_t a = umma_desc_k_major_sw128(at), b = umma_desc_k_major_sw128(at + 3 * SP_A_PART);
 #pragma unroll
                     for (int i = 0; i < 6; ++i)
 #pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            const uint64_t step = (uint64_t)(2 * (2 * h + k));
-                            tcgen05_mma_bf16_pair(tmem + h * NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
-                                                  b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
-                        }
-                    tcgen05_commit_pair(&acc_full[h], both);
-                    if (h == 1) tcgen05_commit_pair(&slot_free[s], both);
+                        for (int k = 0; k < 2; ++k)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const uint64_t step = (uint64_t)(2 * (2 * h + k));
+                                tcgen05_mma_bf16_pair(d + h * NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
+                                                      b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
+                            }
+                    tcgen05_commit_pair(&acc_full[s], both);
+                    tcgen05_commit_pair(&slot_free[s], both);
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
         };
         pdl_wait();  // (an accumulating product reads what the launch before wrote)
-        issue(0, 0);
-        issue(0, 1);
+        issue(0);
+        issue(1);
+        float acc[CW];
 #pragma unroll
         for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
         int tile = first, slice = 0;
         for (int it = 0; it < total; ++it) {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[h], it & 1, p.status, 0x72));
-                tcgen05_fence_after();
-                constexpr int AT_ONCE = 16;
+            const int set = it & 1;
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[set], (it >> 1) & 1, p.status, 0x72));
+            tcgen05_fence_after();
+            const uint32_t from = lane_addr + set * 2 * NT;
 #pragma unroll
-                for (int c0 = 0; c0 < CW; c0 += AT_ONCE) {
-                    uint32_t r[AT_ONCE];
-                    tmem_load_32x16(lane_addr + h * NT + c0, r);
-                    tmem_load_wait();
+            for (int c0 = 0; c0 < CW; c0 += 16) {
+                uint32_t r[16], q[16];
+                tmem_load_32x16(from + c0, r);
+                tmem_load_32x16(from + NT + c0, q);
+                tmem_load_wait();
 #pragma unroll
-                    for (int c = 0; c < AT_ONCE; c += 2) {
-                        const float2 sum = add2(make_float2(acc[c0 + c], acc[c0 + c + 1]),
-                                                make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
-                        acc[c0 + c] = sum.x;
-                        acc[c0 + c + 1] = sum.y;
-                    }
+                for (int c = 0; c < 16; c += 2) {
+                    float2 sum = add2(make_float2(acc[c0 + c], acc[c0 + c + 1]), make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+                    sum = add2(sum, make_float2(__uint_as_float(q[c]), __uint_as_float(q[c + 1])));
+                    acc[c0 + c] = sum.x;
+                    acc[c0 + c + 1] = sum.y;
                 }
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(empty_at + 8u * h);
-                issue(it + 1, h);
             }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(empty_at + 8u * set);
+            issue(it + 2);
             const bool last = slice + 1 == per_tile;
             if ((slice + 1) % SP_LEVEL == 0 || (last && slice >= SP_LEVEL)) {  // the runs so far join the outer sum
 #pragma unroll
                 for (int c = 0; c < CW; c += 8) {
                     uint32_t r[8];
                     if (slice >= SP_LEVEL) {
-                        tmem_load_32x8(lane_addr + 2 * NT + c, r);
+                        tmem_load_32x8(lane_addr + 4 * NT + c, r);
                         tmem_load_wait();
                     }
 #pragma unroll
@@ -323,7 +352,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
                         r[i] = __float_as_uint(sum);
                         acc[c + i] = last ? sum : 0.0f;
                     }
-                    if (!last) tmem_store_32x8(lane_addr + 2 * NT + c, r);
+                    if (!last) tmem_store_32x8(lane_addr + 4 * NT + c, r);
                 }
                 if (!last) tmem_store_wait();
             }
@@ -332,57 +361,60 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             slice = 0;
             if (!SWIGLU && splits > 1) break;  // one tile to a cluster: its sums meet below
             const int t0 = (tile % p.m_tiles) * NT + wc * CW, nt = tile / p.m_tiles;
-            if (SWIGLU) {
-                float* up = reinterpret_cast<float*>(smem + 2 * S::SLOT) + (wc * CW) * 64 + (quarter & 1) * 32 + lane;
-                const int bar = 1 + wc * 2 + (quarter & 1);  // the warp of the gate rows and that of their up rows
-                if (quarter >= 2) {
+            const int n = SWIGLU ? nt * SP_M + (int)rank * 64 + (quarter & 1) * 32 + lane : nt * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
+            // sixteen tokens at a time; those whose sums are not finite are left for the loop behind
+            float* up = reinterpret_cast<float*>(smem + 2 * S::SLOT) + (wc * 2 + (quarter & 1)) * (16 * 32) + lane;
+            const int bar = 1 + wc * 2 + (quarter & 1);  // the warp of the gate rows and that of their up rows
+            const float bias = !SWIGLU && p.bias && n < p.N ? p.bias[n] : 0.0f;
 #pragma unroll
-                    for (int c = 0; c < CW; ++c) up[c * 64] = acc[c];
+            for (int c0 = 0; c0 < CW; c0 += 16) {
+                uint32_t odd = 0;
+                if (SWIGLU) {
+                    if (quarter >= 2) {
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) up[c * 32] = acc[c0 + c];
+                    }
+                    asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
                 }
-                asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
-                if (quarter < 2) {
-                    const int n = nt * SP_M + (int)rank * 64 + quarter * 32 + lane;
+                if (n < p.N && (!SWIGLU || quarter < 2)) {
+                    float* o = p.out + (size_t)(t0 + c0) * p.ldo + n;
 #pragma unroll
-                    for (int c = 0; c < CW; ++c) {
-                        if (n < p.N && t0 + c < p.M) {
-                            float g = acc[c], u = up[c * 64];
-                            const float* row = p.x + (size_t)(t0 + c) * p.ldx;
-                            if (!is_finite(g)) g = dot_in_order(row, p.w + (size_t)n * p.ldw, p.K);
-                            if (!is_finite(u)) u = dot_in_order(row, p.w + (size_t)(n + p.up_offset) * p.ldw, p.K);
-                            p.out[(size_t)(t0 + c) * p.ldo + n] = u * (g * (1.0f / (1.0f + expf(-g))));
+                    for (int c = 0; c < 16; ++c) {
+                        if (t0 + c0 + c >= p.M) continue;
+                        const float v = acc[c0 + c];
+                        float* at = o + (size_t)c * p.ldo;
+                        if (SWIGLU) {
+                            const float u = up[c * 32];
+                            if (is_finite(v) && is_finite(u))
+                                *at = u * (v * (1.0f / (1.0f + expf(-v))));
+                            else
+                                odd |= 1u << c;
+                        } else if (is_finite(v)) {
+                            const float sum = p.bias ? v + bias : v;
+                            *at = p.accumulate ? *at + sum : sum;
+                        } else {
+                            odd |= 1u << c;
                         }
                     }
                 }
-                asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
-            } else {
-                const int n = nt * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
-                if (n < p.N) {
-                    const float bias = p.bias ? p.bias[n] : 0.0f;
-#pragma unroll
-                    for (int c = 0; c < CW; ++c) {
-                        if (t0 + c < p.M) {
-                            float v = acc[c];
-                            if (!is_finite(v)) v = dot_in_order(p.x + (size_t)(t0 + c) * p.ldx, p.w + (size_t)n * p.ldw, p.K);
-                            if (p.bias) v += bias;
-                            float* o = p.out + (size_t)(t0 + c) * p.ldo + n;
-                            *o = p.accumulate ? *o + v : v;
-                        }
-                    }
+                if (SWIGLU) asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+                while (odd) {
+                    const int c = __ffs(odd) - 1;
+                    odd &= odd - 1;
+                    write_in_order<SWIGLU>(p, t0 + c0 + c, n);
                 }
             }
 #pragma unroll
             for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
             tile += stride;
         }
-    }
-    if (!SWIGLU && splits > 1) {
-        // groups of four tokens of a warp belong to the pairs in turn; a pair sends the others theirs
-        constexpr int GROUPS = CW / 4, THREADS = SP_DRAINERS * 32;
-        const int each = (GROUPS + splits - 1) / splits;  // groups of an owner
-        const uint32_t ring = smem_u32(smem);
-        __syncwarp();
-        cluster_sync();  // every MMA of the cluster is done: the slots take partial sums now
-        if (warp < SP_DRAINERS) {
+        if (!SWIGLU && splits > 1) {
+            // groups of four tokens of a warp belong to the pairs in turn; a pair sends the others theirs
+            constexpr int GROUPS = CW / 4, THREADS = SP_DRAINERS * 32;
+            const int each = (GROUPS + splits - 1) / splits;  // groups of an owner
+            const uint32_t ring = smem_u32(smem);
+            __syncwarp();
+            cluster_sync();  // every MMA of the cluster is done: the slots take partial sums now
 #pragma unroll
             for (int g = 0; g < GROUPS; ++g) {
                 const int owner = g % splits;
@@ -393,37 +425,43 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
                 for (int i = 0; i < 4; ++i) v[i] = __float_as_uint(acc[4 * g + i]);
                 st_cluster_x4(map_to_cta(ring + (place * THREADS + tid) * 16, 2 * owner + rank), v);
             }
-        }
-        __syncwarp();
-        cluster_sync();
-        const int quarter = warp & 3, wc = warp >> 2;
-        const int t0 = (first % p.m_tiles) * NT + wc * CW;
-        const int n = first / p.m_tiles * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
-        if (warp < SP_DRAINERS && n < p.N) {
-            const float bias = p.bias ? p.bias[n] : 0.0f;
+            __syncwarp();
+            cluster_sync();
+            const int t0 = (first % p.m_tiles) * NT + wc * CW;
+            const int n = first / p.m_tiles * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
+            if (n < p.N) {
+                const float bias = p.bias ? p.bias[n] : 0.0f;
 #pragma unroll
-            for (int g = 0; g < GROUPS; ++g) {
-                if (g % splits != split) continue;
-                float sum[4];
-                for (int from = 0; from < splits; ++from) {
-                    float4 v = make_float4(acc[4 * g], acc[4 * g + 1], acc[4 * g + 2], acc[4 * g + 3]);
-                    if (from != split) {
-                        const int place = (from < split ? from : from - 1) * each + g / splits;
-                        v = *reinterpret_cast<const float4*>(smem + (size_t)(place * THREADS + tid) * 16);
+                for (int g = 0; g < GROUPS; ++g) {
+                    if (g % splits != split) continue;
+                    float sum[4];
+                    for (int from = 0; from < splits; ++from) {
+                        float4 v = make_float4(acc[4 * g], acc[4 * g + 1], acc[4 * g + 2], acc[4 * g + 3]);
+                        if (from != split) {
+                            const int place = (from < split ? from : from - 1) * each + g / splits;
+                            v = *reinterpret_cast<const float4*>(smem + (size_t)(place * THREADS + tid) * 16);
+                        }
+                        const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) sum[i] = from ? sum[i] + f[i] : f[i];
                     }
-                    const float f[4] = {v.x, v.y, v.z, v.w};
+                    uint32_t odd = 0;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) sum[i] = from ? sum[i] + f[i] : f[i];
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int t = t0 + 4 * g + i;
-                    if (t >= p.M) continue;
-                    float v = sum[i];
-                    if (!is_finite(v)) v = dot_in_order(p.x + (size_t)t * p.ldx, p.w + (size_t)n * p.ldw, p.K);
-                    if (p.bias) v += bias;
-                    float* o = p.out + (size_t)t * p.ldo + n;
-                    *o = p.accumulate ? *o + v : v;
+                    for (int i = 0; i < 4; ++i) {
+                        const int t = t0 + 4 * g + i;
+                        if (t >= p.M) continue;
+                        float* o = p.out + (size_t)t * p.ldo + n;
+                        const float v = p.bias ? sum[i] + bias : sum[i];
+                        if (is_finite(sum[i]))
+                            *o = p.accumulate ? *o + v : v;
+                        else
+                            odd |= 1u << i;
+                    }
+                    while (odd) {
+                        const int i = __ffs(odd) - 1;
+                        odd &= odd - 1;
+                        write_in_order<false>(p, t0 + 4 * g + i, n);
+                    }
                 }
             }
         }
@@ -441,7 +479,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
 // ------------------------------------------------------------------------------------------------- launching
 template <int NT, bool SWIGLU>
 int launch_split(const SplitParams& p, int clusters, cudaStream_t s) {
-    const size_t smem = 2 * SplitShape<NT>::SLOT + (SWIGLU ? SplitShape<NT>::EXCHANGE : 0) + 1024;
+    const size_t smem = 2 * SplitShape<NT>::SLOT + (SWIGLU ? SP_EXCHANGE : 0) + 1024;
     if (int rc = ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<NT, SWIGLU>, smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * p.splits * clusters);
@@ -469,8 +507,7 @@ int launch_split_of(int nt, const SplitParams& p, int clusters, cudaStream_t s) 
     if (nt == 32) return launch_split<32, SWIGLU>(p, clusters, s);
     if (nt == 64) return launch_split<64, SWIGLU>(p, clusters, s);
     if (nt == 96) return launch_split<96, SWIGLU>(p, clusters, s);
-    if (nt == 128) return launch_split<128, SWIGLU>(p, clusters, s);
-    return launch_split<160, SWIGLU>(p, clusters, s);
+    return launch_split<128, SWIGLU>(p, clusters, s);
 }
 
 // Clusters of so many pairs that the GPU holds at once, a CTA an SM (a cluster keeps to a GPC).
@@ -507,16 +544,17 @@ struct SplitPlan {
 // The cut of the least time, from what a slice was measured to take (us, token tiles of 32 to 160), a tile's end, the launch and a cluster's
 // exchange.
 SplitPlan split_plan(int M, int rows, int K, bool swiglu, int nt_only = 0, int splits_only = 0) {
-    constexpr double SLICE[5] = {2.0, 2.3, 2.5, 3.15, 4.5};
+    constexpr double SLICE[4] = {2.0, 2.3, 2.5, 3.0};
     SplitPlan best = {};
     const int slices = (K + SP_K - 1) / SP_K, n_tiles = (rows + 2 * SP_M - 1) / (2 * SP_M);
-    for (int nt = 32; nt <= 160; nt += 32) {
+    for (int nt = 32; nt <= 128; nt += 32) {
         if (nt_only && nt != nt_only) continue;
         const long long m_tiles = (M + nt - 1) / nt;
         for (int sp = 1; sp <= (swiglu ? 1 : SP_MAX_SPLITS); ++sp) {
             if (splits_only && sp != splits_only) continue;
             const int per = (slices + sp - 1) / sp;
             if (sp > 1 && (per < 4 || (sp - 1) * per >= slices)) continue;
+            if (nt == 128 && per > SP_LEVEL) continue;  // no tensor memory left for the outer sums
             const int at_once = active_clusters(sp);
             const long long tiles = m_tiles * n_tiles, rounds = (tiles + at_once - 1) / at_once;
             const double us = rounds * (per * SLICE[nt / 32 - 1] + (sp > 1 ? 7.0 : 1.0)) + 3.0;
@@ -549,7 +587,7 @@ int ferris_gemm_f32_split(const float* x, const float* w, const float* bias, flo
                      split_plan(M, up_offset > 0 ? 2 * N : N, K, up_offset > 0), s);
 }
 
-// The product on the tensor cores whatever its size, cut as told (token_tile 32 to 160 in steps of 32, splits 1 to 4; 0: by the plan).  Rows aligned as
+// The product on the tensor cores whatever its size, cut as told (token_tile 32 to 128 in steps of 32, splits 1 to 4; 0: by the plan).  Rows aligned as
 // ferris_gemm_f32_takes has it; swiglu: N outputs of 2 N weight rows, gate rows first.
 FERRIS_API int ferris_gemm_f32_split_run(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldx,
                                          int ldw, int ldo, int accumulate, int swiglu, int token_tile, int splits, void* stream) {
@@ -557,7 +595,7 @@ FERRIS_API int ferris_gemm_f32_split_run(const float* x, const float* w, const f
     if (K <= 0 || ldx < K || ldw < K || ldo < N) FERRIS_REFUSE("gemm: K=%d, row strides %d, %d, %d", K, ldx, ldw, ldo);
     if (!ferris_gemm_f32_takes(x, w, out, K, ldx, ldw)) FERRIS_REFUSE("gemm: rows that do not begin on 16 bytes");
     if ((long long)((M + 31) / 32) * ((2LL * N + 255) / 256) >= (1 << 28) || ldx > SP_MAX_LD || ldw > SP_MAX_LD) FERRIS_REFUSE("gemm: %d x %d outputs", M, N);
-    if (token_tile % 32 || token_tile < 0 || token_tile > 160 || splits < 0 || splits > SP_MAX_SPLITS || (swiglu && (splits > 1 || bias || accumulate)))
+    if (token_tile % 32 || token_tile < 0 || token_tile > 128 || splits < 0 || splits > SP_MAX_SPLITS || (swiglu && (splits > 1 || bias || accumulate)))
         FERRIS_REFUSE("gemm: token tile %d, %d splits", token_tile, splits);
     const SplitPlan q = split_plan(M, swiglu ? 2 * N : N, K, swiglu != 0, token_tile, splits);
     if (!q.nt) FERRIS_REFUSE("gemm: %d k's in %d splits", K, splits);

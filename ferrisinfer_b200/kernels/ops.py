@@ -273,7 +273,7 @@ def gemm_f32_plan(tokens: int, outputs: int, k: int, swiglu: bool = False) -> in
 
 
 def gemm_f32_split(x, w, bias, out, accumulate: bool = False, swiglu: bool = False, token_tile: int = 0, splits: int = 0):
-    """The 32-bit product of many tokens on the tensor cores, whatever its size, cut as told: tokens of a tile (32 to 160 in steps of
+    """The 32-bit product of many tokens on the tensor cores, whatever its size, cut as told: tokens of a tile (32 to 128 in steps of
     32) and K splits (1 to 4), 0: by the plan.  ``swiglu``: out = silu(x Wg^T) * (x Wu^T) of w = [Wg; Wu]."""
     M, K, ldx = _rows(x, "gemm input")
     N, K2, ldw = _rows(w, "gemm weight")

@@ -21,7 +21,7 @@ def bound(x, w, K):
     return steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
 
 
-# token tiles of 32 to 160: one token more than a tile, one less, exactly; weight rows around 128 and 256; k's around slices of 64 and
+# token tiles of 32 to 128: one token more than a tile, one less, exactly; weight rows around 128 and 256; k's around slices of 64 and
 # around the 1,024 of the outer sum
 @pytest.mark.parametrize("M, N, K", [(1, 1, 4), (33, 40, 60), (160, 256, 128), (161, 129, 68), (95, 257, 1024), (31, 300, 1092),
                                      (130, 896, 896), (50, 33, 9220)])
@@ -38,7 +38,9 @@ def test_split_products_against_64_bits(M, N, K, device):
                 ops.gemm_f32_split(x, w, None, torch.empty(M, N, device=device), splits=splits)
             continue
         first = None
-        for tile in (0, 32, 64, 96, 128, 160):
+        for tile in (0, 32, 64, 96, 128):
+            if tile == 128 and -(-slices // max(1, splits)) > 20:  # (its outer sums have no room)
+                continue
             out = torch.full((M, N + 3), 7.0, device=device)
             ops.gemm_f32_split(x, w, None, out[:, :N], token_tile=tile, splits=splits)
             assert ((out[:, :N].double() - want).abs() <= limit).all(), (tile, splits)
@@ -67,7 +69,7 @@ def test_split_products_with_swiglu_on_the_way(M, I, K, device):
     gate_up, want = torch.empty(M, 2 * I, device=device), torch.empty(M, I, device=device)
     ops.gemm_f32_split(x, w, None, gate_up, splits=1)
     ops.swiglu(gate_up, want)
-    for tile in (0, 32, 64, 96, 128, 160):
+    for tile in (0, 32, 64, 96, 128):
         out = torch.full((M, I), 7.0, device=device)
         ops.gemm_f32_split(x, w, None, out, swiglu=True, token_tile=tile)
         assert torch.equal(out, want), tile
