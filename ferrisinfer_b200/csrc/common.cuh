@@ -202,7 +202,7 @@ FerrisEpilogueAct ferris_take_epilogue_act();
 // sizes, 512 tokens 3.01 -> 2.93; 64 decoded tokens of 0.5B 1.66 -> 1.64).
 __device__ __forceinline__ float ferris_exp_unit(float v) {
     float r;
-    asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(v * 1.4426950408889634f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v * 1.4426950408889634f));
     return r;
 }
 __device__ __forceinline__ float ferris_rcp_unit(float v) {
@@ -210,8 +210,25 @@ __device__ __forceinline__ float ferris_rcp_unit(float v) {
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
+// xIELU without a branch: lanes on both sides of zero, and the two halves of a branch for every one of an epilogue's columns, cost twice what
+// the products left (up product of 2,048 tokens x 8,192 x 2,048: see gemm_tcgen05.cu).  e^z - 1 - z for z <= 0: above -1/2 its Taylor series,
+// z^2 (1/2! + z / 3! + .. + z^6 / 8!), whose rest is below 4e-8 of it; else the difference of the three numbers, no smaller than a fifth of
+// them.
+__device__ __forceinline__ float ferris_xielu(float z, float a, float b) {
+    const float n = fminf(z, 0.0f), half = 0.5f * z;
+    float s = 1.0f / 40320.0f;
+    s = fmaf(s, n, 1.0f / 5040.0f);
+    s = fmaf(s, n, 1.0f / 720.0f);
+    s = fmaf(s, n, 1.0f / 120.0f);
+    s = fmaf(s, n, 1.0f / 24.0f);
+    s = fmaf(s, n, 1.0f / 6.0f);
+    s = fmaf(s, n, 0.5f);
+    const float near = (n * n) * s, far = (ferris_exp_unit(n) - 1.0f) - n;
+    const float below = fmaf(b, n > -0.5f ? near : far, half), above = fmaf(a * z, z, half);
+    return z > 0.0f ? above : below;
+}
 __device__ __forceinline__ float ferris_epilogue_act(float z, const FerrisEpilogueAct& e) {
-    if (e.kind == 1) return z > 0.0f ? fmaf(e.a * z, z, 0.5f * z) : fmaf(e.b, expm1f(z) - z, 0.5f * z);
+    if (e.kind == 1) return ferris_xielu(z, e.a, e.b);
     if (e.kind == 2) return z / (1.0f + expf(-z));
     if (e.kind == 3) return z > 0.0f ? z * z : 0.0f;
     return z;
