@@ -10,10 +10,15 @@
 // (2-norm, relative, normal numbers; this kernel / the FMA kernels of gemm_f32.cu): K = 64 0.7 / 1.1, 896 0.9 to 1.15 / 1.55, 4,864
 // 1.2 to 1.3 / 1.6, 9,220 1.3 / 1.65, each 1e-7.
 //
-// A cluster of two CTAs (cta_group::2) takes 256 weight rows x NT tokens.  Nothing reads the fp32 operands twice from
-// shared memory: every thread loads runs of 8 k's straight into registers one slice ahead (a warp: 4 rows x 64 k's, whole 128-byte
-// lines), splits them and stores three 16-byte chunks into bf16 tiles in the 128-byte swizzle that the MMA reads; the SAME warps
-// drain the accumulators, because with two slices of 64 k's in shared memory and two accumulators both jobs fit beside the MMAs.
+// A cluster of two CTAs (cta_group::2) takes 256 weight rows x NT tokens.  Nothing reads the fp32 operands from shared memory: sixteen
+// warps load runs of 8 k's straight into registers (a warp: 4 rows x 64 k's, whole 128-byte lines), split them, take the next slice's into
+// the same registers and store three 16-byte chunks into bf16 tiles in the 128-byte swizzle that the MMA reads; one lane issues the
+// MMAs; eight warps add the sums up.  Three slices of 64 k's stand in shared memory, because a slot's way around (split, its arrival at the
+// leader, MMAs, their commit) is longer than any of its parts: with two slots it took 2.45 us a slice at 128 tokens, of which the MMAs
+// are 0.8 and everything else without them 1.65; with three (and the MMAs issued by a warp of their own) 1.8.  Before that: one set of
+// warps that split and drained 4.2, two 3.1, two accumulators in turn 2.45.
+// Measured (us, tokens: 96 / 200 / 777 / 2,048; in brackets the FMA kernels): 1,152 x 896 12 / 17 / 26 / 49 (27 / 29 / 61 / 109), 896 x 896
+// 12 / 16 / 27 / 31 (26 / 28 / 54 / 108), 9,728 x 896 29 / 51 / 105 / 229 (84 / 131 / 351 / 817; 155 TFLOP/s), 896 x 4,864 32 / 37 / 81 / 188 (61 / 79 / 218 / 564).
 //
 // K SPLITS: where tiles are few a cluster of up to four pairs takes one tile, each a run of slices; the sums meet through
 // shared memory and are added in the runs' order.  SwiGLU: a CTA's rows 0..63 are gate rows, 64..127 their up rows.
@@ -26,15 +31,17 @@
 
 namespace {
 
-constexpr int SP_DRAINERS = 8;   // warps that add the accumulators up and write; lane 0 of the leader's first issues the MMAs
-constexpr int SP_SPLITTERS = 16; // warps that load and split the operands
-constexpr int SP_THREADS = (SP_DRAINERS + SP_SPLITTERS) * 32;
-// Registers a thread: 80 at the launch, then so many for either kind of warp, which together are no more.
-constexpr int SP_LAUNCH_REGS = 80, SP_DRAIN_REGS = 128, SP_SPLIT_REGS = 56;
-static_assert(SP_DRAINERS * SP_DRAIN_REGS + SP_SPLITTERS * SP_SPLIT_REGS <= (SP_DRAINERS + SP_SPLITTERS) * SP_LAUNCH_REGS &&
-                  SP_THREADS * SP_LAUNCH_REGS <= 65536 && SP_DRAINERS % 4 == 0 && SP_SPLITTERS % 4 == 0,
+constexpr int SP_DRAINERS = 8;    // warps that add the accumulators up and write
+constexpr int SP_SPLITTERS = 16;  // warps that load and split the operands
+constexpr int SP_ISSUERS = 4;     // and a group of four of which one lane (of the leader) issues the MMAs
+constexpr int SP_THREADS = (SP_DRAINERS + SP_SPLITTERS + SP_ISSUERS) * 32;
+// Registers a thread: 72 at the launch, then so many for either kind of warp, which together are no more.
+constexpr int SP_LAUNCH_REGS = 72, SP_DRAIN_REGS = 128, SP_SPLIT_REGS = 56, SP_ISSUE_REGS = 24;
+static_assert(SP_DRAINERS * SP_DRAIN_REGS + SP_SPLITTERS * SP_SPLIT_REGS + SP_ISSUERS * SP_ISSUE_REGS <= SP_THREADS / 32 * SP_LAUNCH_REGS &&
+                  SP_THREADS * SP_LAUNCH_REGS <= 65536 && SP_DRAINERS % 4 == 0 && SP_SPLITTERS % 4 == 0 && SP_ISSUERS % 4 == 0,
               "the shares come out of the launch's registers, by groups of four warps");
 constexpr int SP_ROWS = SP_SPLITTERS * 4;  // rows that the splitting warps take at a time, eight threads a row
+constexpr int SP_SLOTS = 3;                // slices in shared memory
 constexpr int SP_M = 128;                  // weight rows of a CTA, 256 of a pair
 constexpr int SP_K = 64;                   // k's of a slice: two runs of 32
 constexpr int SP_LEVEL = 20;               // slices whose runs are added up before they join the outer sum
@@ -139,6 +146,9 @@ __device__ __forceinline__ void tmem_store_32x8(uint32_t taddr, const uint32_t* 
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// All of an SM's tensor memory, for both CTAs of a pair.
+__device__ __forceinline__ void take_tensor_memory(uint32_t* dst) { tmem_alloc_pair(dst, 512); }
+
 template <int NT>  // tokens of a tile
 struct SplitShape {
     static constexpr int CW = NT / 2;  // columns of a draining warp
@@ -152,7 +162,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
     using S = SplitShape<NT>;
     constexpr int CW = S::CW;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[2], slot_free[2], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full[SP_SLOTS], slot_free[SP_SLOTS], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -164,15 +174,17 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
     const int total = first < tiles ? (tiles - first + stride - 1) / stride * per_tile : 0;  // slices of this CTA
     const uint16_t both = (uint16_t)(3u << leader);
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&full[i], 2 * SP_SPLITTERS);   // the splitting warps of both CTAs (used in the leader only)
+        for (int i = 0; i < SP_SLOTS; ++i) {
+            mbar_init(&full[i], 2 * SP_SPLITTERS);  // the splitting warps of both CTAs (used in the leader only)
             mbar_init(&slot_free[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], 2 * SP_DRAINERS);  // (the leader's only)
         }
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc_pair(&tmem_base, 512);
+    if (warp == 0) take_tensor_memory(&tmem_base);  // ahead of the dependents: a launch that had it could wait for this one
     tcgen05_fence_before();
     __syncthreads();
     cluster_sync();
@@ -180,8 +192,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
     const uint32_t tmem = tmem_base;
     pdl_launch_dependents();
 
-    int ok = 1;  // 0: a wait ran out; no MMA is issued and nothing waited for any more, every barrier is still met
-    if (warp >= SP_DRAINERS) {
+    int ok = 1;  // 0: a wait ran out; nothing is waited for any more, every barrier is still met
+    if (warp >= SP_DRAINERS && warp < SP_DRAINERS + SP_SPLITTERS) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SP_SPLIT_REGS));
         // -------------------------------------------------------------------------------- operands: fp32 -> three bf16 tiles
         constexpr int WG = SP_M / SP_ROWS, XG = (S::XR + SP_ROWS - 1) / SP_ROWS;  // rows of a thread, SP_ROWS apart
@@ -238,9 +250,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
         if (p.early_weights) pdl_wait();
 #pragma unroll
         for (int j = 0; j < XG; ++j) load_x(j);
+        int s = 0, phase = 1;  // the slot that is filled next, and the phase of its barrier that frees it
         for (int it = 0; it < total; ++it) {
-            uint8_t* slot = smem + (it & 1) * S::SLOT + at0;
-            if (it >= 2 && ok) ok = __all_sync(0xffffffffu, mbar_wait(&slot_free[it & 1], ((it >> 1) - 1) & 1, p.status, 0x73));
+            uint8_t* slot = smem + s * S::SLOT + at0;
+            if (it >= SP_SLOTS && ok) ok = __all_sync(0xffffffffu, mbar_wait(&slot_free[s], phase, p.status, 0x73));
             turn();
             uint4 p1, p2, p3;
             // a run of rows is split and stored, and its registers take the next slice's at once
@@ -265,7 +278,44 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what every lane wrote
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(full_at + 8u * (it & 1));
+            if (lane == 0) mbar_arrive_cluster(full_at + 8u * s);
+            if (++s == SP_SLOTS) s = 0, phase ^= 1;
+        }
+        if (!SWIGLU && splits > 1) {  // (the draining warps' exchange)
+            __syncwarp();
+            cluster_sync();
+            cluster_sync();
+        }
+    } else if (warp >= SP_DRAINERS) {
+        // ---------------------------------------------------------------------------------------- MMAs
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SP_ISSUE_REGS));
+        if (warp == SP_DRAINERS + SP_SPLITTERS && lane == 0 && rank == 0) {
+            // A slice: its two runs of 32 k's into the two accumulators of its set, the smallest products first.  A product waits for the one
+            // before it in the same accumulator, so the runs take turns.
+            const uint32_t idesc = umma_idesc_bf16(2 * SP_M, NT);
+            int s = 0, phase = 0;
+            for (int it = 0; it < total; ++it) {
+                const int set = it & 1;
+                if (!mbar_wait(&full[s], phase, p.status, 0x70)) break;
+                if (it >= 2 && !mbar_wait(&acc_empty[set], ((it >> 1) - 1) & 1, p.status, 0x71)) break;
+                tcgen05_fence_after();
+                constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
+                const uint32_t at = smem_u32(smem + s * S::SLOT), d = tmem + set * 2 * NT;
+                const uint64_t a = umma_desc_k_major_sw128(at), b = umma_desc_k_major_sw128(at + 3 * SP_A_PART);
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint64_t step = (uint64_t)(2 * (2 * h + k));
+                            tcgen05_mma_bf16_pair(d + h * NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
+                                                  b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
+                        }
+                tcgen05_commit_pair(&slot_free[s], both);
+                tcgen05_commit_pair(&acc_full[set], both);
+                if (++s == SP_SLOTS) s = 0, phase ^= 1;
+            }
         }
         if (!SWIGLU && splits > 1) {  // (the draining warps' exchange)
             __syncwarp();
@@ -273,43 +323,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             cluster_sync();
         }
     } else {
-        // ---------------------------------------------------------------------------------------- MMAs, sums, outputs
+        // ---------------------------------------------------------------------------------------- sums, outputs
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SP_DRAIN_REGS));
         const int quarter = warp & 3, wc = warp >> 2;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + wc * CW;
         const uint32_t empty_at = map_to_cta(smem_u32(&acc_empty[0]), leader);
-        // Slice `it`: the two runs of 32 k's into the two accumulators of its set, the smallest products first.  A product waits for the one
-        // before it in the same accumulator (some 190 cycles whatever the width), so the runs take turns.
-        auto issue = [&](int it) {
-            if (warp != 0) return;
-            if (lane == 0 && rank == 0 && it < total && ok) {
-                const int s = it & 1;
-                ok = mbar_wait(&full[s], (it >> 1) & 1, p.status, 0x70) &&
-                     (it < 2 || mbar_wait(&acc_empty[s], ((it >> 1) - 1) & 1, p.status, 0x71));
-                if (ok) {
-                    tcgen05_fence_after();
-                    constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
-                    const uint32_t at = smem_u32(smem + s * S::SLOT), idesc = umma_idesc_bf16(2 * SP_M, NT), d = tmem + s * 2 * NT;
-                    const uint64_t a = umma_desc_k_major_sw128(at), b = umma_desc_k_major_sw128(at + 3 * SP_A_PART);
-#pragma unroll
-                    for (int i = 0; i < 6; ++i)
-#pragma unroll
-                        for (int k = 0; k < 2; ++k)
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const uint64_t step = (uint64_t)(2 * (2 * h + k));
-                                tcgen05_mma_bf16_pair(d + h * NT, a + (uint64_t)(PA[i] * (SP_A_PART >> 4)) + step,
-                                                      b + (uint64_t)(PB[i] * (S::B_PART >> 4)) + step, idesc, (i | k) ? 1u : 0u);
-                            }
-                    tcgen05_commit_pair(&acc_full[s], both);
-                    tcgen05_commit_pair(&slot_free[s], both);
-                }
-            }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-        };
         pdl_wait();  // (an accumulating product reads what the launch before wrote)
-        issue(0);
-        issue(1);
         float acc[CW];
 #pragma unroll
         for (int c = 0; c < CW; ++c) acc[c] = 0.0f;
@@ -336,7 +355,6 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(empty_at + 8u * set);
-            issue(it + 2);
             const bool last = slice + 1 == per_tile;
             if ((slice + 1) % SP_LEVEL == 0 || (last && slice >= SP_LEVEL)) {  // the runs so far join the outer sum
 #pragma unroll
@@ -363,7 +381,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
             const int t0 = (tile % p.m_tiles) * NT + wc * CW, nt = tile / p.m_tiles;
             const int n = SWIGLU ? nt * SP_M + (int)rank * 64 + (quarter & 1) * 32 + lane : nt * 2 * SP_M + (int)rank * SP_M + quarter * 32 + lane;
             // sixteen tokens at a time; those whose sums are not finite are left for the loop behind
-            float* up = reinterpret_cast<float*>(smem + 2 * S::SLOT) + (wc * 2 + (quarter & 1)) * (16 * 32) + lane;
+            float* up = reinterpret_cast<float*>(smem + SP_SLOTS * S::SLOT) + (wc * 2 + (quarter & 1)) * (16 * 32) + lane;
             const int bar = 1 + wc * 2 + (quarter & 1);  // the warp of the gate rows and that of their up rows
             const float bias = !SWIGLU && p.bias && n < p.N ? p.bias[n] : 0.0f;
 #pragma unroll
@@ -479,7 +497,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
 // ------------------------------------------------------------------------------------------------- launching
 template <int NT, bool SWIGLU>
 int launch_split(const SplitParams& p, int clusters, cudaStream_t s) {
-    const size_t smem = 2 * SplitShape<NT>::SLOT + (SWIGLU ? SP_EXCHANGE : 0) + 1024;
+    const size_t smem = SP_SLOTS * SplitShape<NT>::SLOT + (SWIGLU ? SP_EXCHANGE : 0) + 1024;
     if (int rc = ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<NT, SWIGLU>, smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * p.splits * clusters);
@@ -515,7 +533,7 @@ int active_clusters(int pairs) {
     static int known[SP_MAX_SPLITS + 1] = {};
     if (known[pairs] > 0) return known[pairs];
     constexpr int UNKNOWN[SP_MAX_SPLITS + 1] = {0, 74, 32, 20, 12};
-    const size_t smem = 2 * SplitShape<128>::SLOT + 1024;
+    const size_t smem = SP_SLOTS * SplitShape<128>::SLOT + 1024;
     int n = 0;
     if (ferris_allow_dynamic_smem((const void*)gemm_f32_split_kernel<128, false>, smem) == FERRIS_OK) {
         cudaLaunchConfig_t cfg = {};
@@ -544,7 +562,7 @@ struct SplitPlan {
 // The cut of the least time, from what a slice was measured to take (us, token tiles of 32 to 160), a tile's end, the launch and a cluster's
 // exchange.
 SplitPlan split_plan(int M, int rows, int K, bool swiglu, int nt_only = 0, int splits_only = 0) {
-    constexpr double SLICE[4] = {2.0, 2.3, 2.5, 3.0};
+    constexpr double SLICE[4] = {1.3, 1.55, 1.7, 1.8};
     SplitPlan best = {};
     const int slices = (K + SP_K - 1) / SP_K, n_tiles = (rows + 2 * SP_M - 1) / (2 * SP_M);
     for (int nt = 32; nt <= 128; nt += 32) {
@@ -557,7 +575,7 @@ SplitPlan split_plan(int M, int rows, int K, bool swiglu, int nt_only = 0, int s
             if (nt == 128 && per > SP_LEVEL) continue;  // no tensor memory left for the outer sums
             const int at_once = active_clusters(sp);
             const long long tiles = m_tiles * n_tiles, rounds = (tiles + at_once - 1) / at_once;
-            const double us = rounds * (per * SLICE[nt / 32 - 1] + (sp > 1 ? 7.0 : 1.0)) + 3.0;
+            const double us = rounds * (per * SLICE[nt / 32 - 1] + (sp > 1 ? 5.0 : 1.0)) + 3.0;
             if (best.nt && us >= best.us) continue;
             best = {nt, sp, (int)(sp > 1 || tiles < at_once ? tiles : at_once), (int)m_tiles, n_tiles, per, us};
         }
@@ -575,7 +593,7 @@ int run_split(const float* x, const float* w, const float* bias, float* out, int
 }  // namespace
 
 // More than 32 tokens and 150 million multiply-adds.  Up to there every form of the product adds in one order, so that a row's bits do not depend
-// on how many others the step brings; from 33 tokens on this kernel would win there too, by 4 to 6 us of 18 to 27.
+// on how many others the step brings; from 33 tokens on this kernel would win there too, by 5 to 14 us of 18 to 27.
 bool ferris_gemm_f32_split_takes(int M, int rows, int K, int ldx, int ldw) {
     return M > 32 && (long long)M * rows * K >= 150000000LL && (long long)((M + 31) / 32) * ((rows + 255) / 256) < (1 << 28) &&
            ldx <= SP_MAX_LD && ldw <= SP_MAX_LD;
