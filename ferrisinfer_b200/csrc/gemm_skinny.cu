@@ -273,8 +273,19 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
         for (int t = warp; t < p.x_rows; t += SK_WARPS) {
             const float4* row = reinterpret_cast<const float4*>(p.norm_h + (size_t)(t < p.T ? t : 0) * p.K);
             const bool live = t < p.T;
+            auto put = [&](int idx, float4 h, float4 w, float r) {  // columns 4 idx .. 4 idx + 3 of row t
+                uint2 v = make_uint2(0u, 0u);
+                if (live && idx < n4) {
+                    v.x = pack_bf16((h.x * r) * w.x, (h.y * r) * w.y);
+                    v.y = pack_bf16((h.z * r) * w.z, (h.w * r) * w.w);
+                }
+                const int kb = idx >> 4;  // K block of these columns; group kb / nb, line t * nb + kb % nb of its box
+                const int grp = p.nb == 1 ? kb : (int)__umulhi((unsigned)kb, p.nb_magic);  // kb / nb, exact for small kb
+                *reinterpret_cast<uint2*>(x_smem + (size_t)grp * x_box_bytes +
+                                          swizzle128(t * p.nb + (kb - grp * p.nb), (idx >> 1) & 7) + (idx & 1) * 8) = v;
+            };
+            float ss = 0.0f;
             if (tile4 <= 256) {
-                float ss = 0.0f;
                 float4 hv[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) hv[j] = (live && j * 32 + lane < n4) ? row[j * 32 + lane] : zero4;
@@ -284,9 +295,29 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
                 const float r = 1.0f / sqrtf(ss / (float)p.K + p.norm_eps);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    if (j * 32 + lane < tile4) sk_put_row(p, x_smem, x_box_bytes, t, live, j * 32 + lane, hv[j], wv[j], r);
+                    if (j * 32 + lane < tile4) put(j * 32 + lane, hv[j], wv[j], r);
             } else {
-                sk_norm_row(p, x_smem, x_box_bytes, t, lane);
+                for (int base = 0; base < n4 && live; base += 256) {
+                    float4 hv[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) hv[j] = base + j * 32 + lane < n4 ? row[base + j * 32 + lane] : zero4;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) ss += (hv[j].x * hv[j].x + hv[j].y * hv[j].y) + (hv[j].z * hv[j].z + hv[j].w * hv[j].w);
+                }
+                ss = warp_sum(ss);
+                const float r = 1.0f / sqrtf(ss / (float)p.K + p.norm_eps);
+                for (int base = 0; base < tile4; base += 256) {
+                    float4 hv[8], wl[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int idx = base + j * 32 + lane;
+                        hv[j] = (live && idx < n4) ? row[idx] : zero4;
+                        wl[j] = idx < n4 ? w4[idx] : zero4;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (base + j * 32 + lane < tile4) put(base + j * 32 + lane, hv[j], wl[j], r);
+                }
             }
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
