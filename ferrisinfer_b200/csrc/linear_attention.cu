@@ -15,6 +15,7 @@
 // rotated by their positions there, and k scaled (RotaryArgs): what enters the recurrence is then fp32 throughout.
 #include "common.cuh"
 #include "linear_attention.cuh"
+#include "sm100.cuh"
 
 namespace {
 
@@ -281,6 +282,170 @@ __global__ void __launch_bounds__(GN_THREADS) gated_rmsnorm_vec_kernel(const flo
     }
 }
 
+// A step of single tokens: heads of 128, states of many requests.  Nothing but the states' way through the SMs costs time (64 requests,
+// 16 heads of 128 / 128: 67 MB in and out), and the walk above leaves them two dependent look-ups, a trip to memory and a store one after
+// the other in each of 4,096 short blocks.  Here three CTAs an SM take their runs of tiles of 32 columns (16 KB that lie together) through
+// rings of bulk copies: one thread requests tiles and stores the finished ones from where they stand, eight warps (four columns each, a
+// lane four rows) turn them in place; q, k and v of the next tile are on their way meanwhile, and q and k are activated and turned once
+// for a head's tiles.  us, walk / here, requests: 16 15.6 / 16.3,
+// 24 16.8 / 15.7, 32 21.3 / 16.8, 64 38.1 / 28.4 (4.7 TB/s), 128 70.9 / 51.3.  One CTA an SM with a ring of twelve: 51 at 64, the serial work of a tile.
+constexpr int LS_DIM = 128, LS_COLS = 32, LS_WARPS = 8, LS_STAGES = 4, LS_BEHIND = 1, LS_CTAS = 3;
+constexpr int LS_MIN_TILES = 1536;  // fewer: the walk is as fast
+constexpr int LS_TILE = LS_COLS * LS_DIM * 4;
+constexpr int LS_SMEM = LS_STAGES * LS_TILE + 128;
+
+template <typename T>
+__global__ void __launch_bounds__(LS_WARPS * 32 + 32, LS_CTAS) linear_attention_singles_kernel(
+    const T* qkv, int ld, int q_off, int k_off, int v_off, float* out, int ldo, float* state, const float* __restrict__ decay,
+    const int* __restrict__ seq_q_start, const int* __restrict__ seq_state_slot, int seqs, int heads, int vdim, int silu, int write_state,
+    const RotaryArgs rot, int* status) {
+    extern __shared__ uint8_t ls_raw[];
+    __shared__ uint64_t full[LS_STAGES], done[LS_STAGES];
+    __shared__ __align__(16) float qk[2][2][LS_DIM];  // [unit & 1][q, k]
+    __shared__ float vs[2][LS_COLS];
+    uint8_t* ring = ls_raw + ((128u - (smem_u32(ls_raw) & 127u)) & 127u);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int per_head = vdim / LS_COLS, per_seq = heads * per_head;
+    const long long tiles = (long long)seqs * per_seq;
+    const int lo = (int)(tiles * blockIdx.x / gridDim.x), hi = (int)(tiles * (blockIdx.x + 1) / gridDim.x);
+    if (tid == 0) {
+        for (int i = 0; i < LS_STAGES; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&done[i], LS_WARPS);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    pdl_wait();
+    pdl_launch_dependents();
+    // requests with a token of this step only
+    auto next_tile = [&](int t) {
+        while (t < hi) {
+            const int seq = t / per_seq;
+            if (seq_q_start[seq + 1] - seq_q_start[seq] == 1) break;
+            t = (seq + 1) * per_seq;
+        }
+        return t;
+    };
+    auto tile_at = [&](int t) {
+        const int seq = t / per_seq, rest = t - seq * per_seq;
+        return state + ((size_t)seq_state_slot[seq] * per_seq + rest) * (LS_TILE / 4);
+    };
+    if (warp == LS_WARPS) {
+        if (lane != 0) return;
+        int load_t = next_tile(lo), loaded = 0;
+        auto load = [&]() {
+            const int s = loaded % LS_STAGES;
+            mbar_expect_tx(&full[s], LS_TILE);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             smem_u32(ring + s * LS_TILE)),
+                         "l"(tile_at(load_t)), "r"(LS_TILE), "r"(smem_u32(&full[s]))
+                         : "memory");
+            ++loaded;
+            load_t = next_tile(load_t + 1);
+        };
+        while (load_t < hi && loaded < LS_STAGES) load();
+        int i = 0;
+        for (int t = next_tile(lo); t < hi; t = next_tile(t + 1), ++i) {
+            const int s = i % LS_STAGES;
+            if (!mbar_wait(&done[s], (i / LS_STAGES) & 1, status, 0x80)) break;
+            if (write_state) {
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(tile_at(t)), "r"(smem_u32(ring + s * LS_TILE)),
+                             "r"(LS_TILE)
+                             : "memory");
+            }
+            tma_store_commit();
+            // the tile LS_BEHIND before this one has left its stage
+            asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(LS_BEHIND) : "memory");
+            if (i >= LS_BEHIND && load_t < hi) load();
+        }
+        tma_store_wait_all();
+        return;
+    }
+    const int half = rot.positions ? rot.rotary >> 1 : 0;
+    // this thread's share of a tile: an element of q (threads 0-127) or k, and of the first warp's an element of v
+    float raw = 0.0f, raw_v = 0.0f;
+    auto fetch = [&](int t) {
+        const int seq = t / per_seq, rest = t - seq * per_seq, h = rest / per_head, z = rest - h * per_head;
+        const T* row = qkv + (size_t)seq_q_start[seq] * ld;
+        raw = to_float(tid < LS_DIM ? row[q_off + h * LS_DIM + tid] : row[k_off + h * LS_DIM + tid - LS_DIM]);
+        if (tid < LS_COLS) raw_v = to_float(row[v_off + h * vdim + z * LS_COLS + tid]);
+    };
+    int t = next_tile(lo), unit = -1, units = 0;
+    if (t < hi) fetch(t);
+    for (int i = 0; t < hi; ++i) {
+        const int seq = t / per_seq, rest = t - seq * per_seq, h = rest / per_head, z = rest - h * per_head, row = seq_q_start[seq];
+        const int s = i % LS_STAGES;
+        const int after = next_tile(t + 1);
+        if (t / per_head != unit) {
+            unit = t / per_head;
+            ++units;
+            float* mine = &qk[units & 1][tid >> 7][tid & (LS_DIM - 1)];
+            *mine = silu ? silu_f(raw) : raw;
+            if (half > 0 || rot.k_scale != 1.0f) {
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if ((tid & (LS_DIM - 1)) < half) {  // the pair of a frequency, of q or of k
+                    const int f = tid & (LS_DIM - 1), which = tid >> 7;
+                    float sn, cs;
+                    sincosf((float)rot.positions[row] * rot.freq[f], &sn, &cs);
+                    sn *= rot.mag, cs *= rot.mag;
+                    const int iu = rot.interleaved ? 2 * f : f, iv = rot.interleaved ? 2 * f + 1 : f + half;
+                    float* x = qk[units & 1][which];
+                    const float u = x[iu], v = x[iv], factor = which ? rot.k_scale : 1.0f;
+                    x[iu] = (u * cs - v * sn) * factor;
+                    x[iv] = (v * cs + u * sn) * factor;
+                } else if (tid >= LS_DIM && tid - LS_DIM >= 2 * half) {
+                    *mine *= rot.k_scale;
+                }
+            }
+        }
+        if (tid < LS_COLS) vs[i & 1][tid] = silu ? silu_f(raw_v) : raw_v;
+        if (after < hi) fetch(after);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const float4 k4 = *reinterpret_cast<const float4*>(&qk[units & 1][1][4 * lane]);
+        const float4 q4 = *reinterpret_cast<const float4*>(&qk[units & 1][0][4 * lane]);
+        const float lam = decay[h];
+        float4* S = reinterpret_cast<float4*>(ring + s * LS_TILE) + warp * 4 * (LS_DIM / 4) + lane;
+        mbar_wait(&full[s], (i / LS_STAGES) & 1, status, 0x81);
+        float o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float v = vs[i & 1][warp * 4 + c];
+            float4 x = S[c * (LS_DIM / 4)];
+            x.x = fmaf(k4.x, v, lam * x.x), x.y = fmaf(k4.y, v, lam * x.y), x.z = fmaf(k4.z, v, lam * x.z), x.w = fmaf(k4.w, v, lam * x.w);
+            S[c * (LS_DIM / 4)] = x;
+            o[c] = fmaf(x.w, q4.w, fmaf(x.z, q4.z, fmaf(x.y, q4.y, x.x * q4.x)));
+        }
+        fence_proxy_async();  // the copy out reads what every lane wrote
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&done[s]);
+        // four sums over the lanes with six shuffles: a lane hands half of its sums to its partner and keeps the other half
+        const bool h1 = lane & 16, h2 = lane & 8;
+        float a[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) a[c] = (h1 ? o[c + 2] : o[c]) + __shfl_xor_sync(0xffffffffu, h1 ? o[c] : o[c + 2], 16);
+        float sum = (h2 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, h2 ? a[0] : a[1], 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        if ((lane & 7) == 0)
+            out[(size_t)row * ldo + (size_t)h * vdim + z * LS_COLS + warp * 4 + ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)] = sum;
+        t = after;
+    }
+}
+
+template <typename T>
+int launch_singles(const void* qkv, int ld, int q_off, int k_off, int v_off, float* out, int ldo, float* state, const float* decay,
+                   const int* seq_q_start, const int* seq_state_slot, int seqs, int heads, int vdim, int silu, int write_state,
+                   const RotaryArgs rot, cudaStream_t s) {
+    if (int rc = ferris_allow_dynamic_smem((const void*)linear_attention_singles_kernel<T>, LS_SMEM)) return rc;
+    const long long tiles = (long long)seqs * heads * (vdim / LS_COLS);
+    ferris_launch(linear_attention_singles_kernel<T>, dim3((unsigned)(tiles < 148 * LS_CTAS ? tiles : 148 * LS_CTAS)), dim3(LS_WARPS * 32 + 32),
+                  LS_SMEM, s, (const T*)qkv, ld, q_off, k_off, v_off, out, ldo, state, decay, seq_q_start, seq_state_slot, seqs, heads, vdim,
+                  silu, write_state, rot, ferris_status_ptr());
+    FERRIS_LAUNCH_CHECK();
+}
+
 template <typename T, int MODE>
 void launch_scan_mode(const void* qkv, int ld, int q_off, int k_off, int v_off, float* out, int ldo, float* state,
                       float* scratch, const float* decay, const int* seq_q_start, const int* seq_state_slot, int seqs,
@@ -308,6 +473,11 @@ int launch_scan(const void* qkv, int ld, int q_off, int k_off, int v_off, float*
                 float* scratch, const float* decay, const int* seq_q_start, const int* seq_state_slot, int seqs,
                 int heads, int dim, int vdim, int silu, int write_state, int seg_len, int segs_max, int most, const RotaryArgs rot,
                 cudaStream_t s) {
+    const long long singles = (long long)seqs * heads * (vdim / LS_COLS);
+    if (segs_max <= 1 && most == 1 && dim == LS_DIM && vdim % LS_COLS == 0 && ((uintptr_t)state & 15) == 0 && singles >= LS_MIN_TILES &&
+        singles < (1 << 30))
+        return launch_singles<T>(qkv, ld, q_off, k_off, v_off, out, ldo, state, decay, seq_q_start, seq_state_slot, seqs, heads, vdim, silu,
+                                 write_state, rot, s);
     if (segs_max <= 1) {
         launch_scan_mode<T, 0>(qkv, ld, q_off, k_off, v_off, out, ldo, state, scratch, decay, seq_q_start, seq_state_slot,
                                seqs, heads, dim, vdim, silu, write_state, seg_len, 1, most, rot, s);

@@ -1306,8 +1306,8 @@ def linear_attention(qkv: torch.Tensor, offsets: tuple, out: torch.Tensor, state
                                        _ptr(decay), _ptr(ctx.seq_q_start), _ptr(ctx.seq_state_slot), _c_int(ctx.num_seqs),
                                        _c_int(heads), _c_int(dim), _c_int(vdim), _c_int(1 if silu else 0),
                                        _c_int(1 if write_state else 0), _c_int(seg), _c_int(segs_max), _ptr(scratch),
-                                       *_rotary_args(rotary, ctx, dim, qkv.device), _c_float(k_scale), _c_int(0x7FFFFFFF),
-                                       _stream()),
+                                       *_rotary_args(rotary, ctx, dim, qkv.device), _c_float(k_scale),
+                                       _c_int(1 if longest <= 1 else 0x7FFFFFFF), _stream()),
         "linear attention", 1 if segs_max == 1 else 3,
     )
 
