@@ -196,18 +196,10 @@ struct FerrisEpilogueAct {
 };
 FerrisEpilogueAct ferris_take_epilogue_act();
 
-// e^v and 1 / v for SwiGLU in the epilogues of the tensor-core products, whose results are rounded to bf16: the exponential and reciprocal
-// units, 2^-22 and 2^-23 relative (and |v| 2^-24 for the exponent's own rounding).  The full functions are some twenty instructions
-// more an output, which the epilogue of a gate / up product with a short K does not hide (0.5B sizes, 2,048 tokens: a step 2.81 -> 2.69 ms; 1.5B
-// sizes, 512 tokens 3.01 -> 2.93; 64 decoded tokens of 0.5B 1.66 -> 1.64).
+// e^v by the exponential unit: 2^-22 relative, and |v| 2^-24 for the exponent's own rounding.
 __device__ __forceinline__ float ferris_exp_unit(float v) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v * 1.4426950408889634f));
-    return r;
-}
-__device__ __forceinline__ float ferris_rcp_unit(float v) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
 // xIELU without a branch: lanes on both sides of zero, and the two halves of a branch for every one of an epilogue's columns, cost twice what

@@ -85,7 +85,7 @@ struct Params {
     int* status;
 };
 
-__device__ __forceinline__ float silu_mul(float g, float u) { return u * (g * ferris_rcp_unit(1.0f + ferris_exp_unit(-g))); }
+__device__ __forceinline__ float silu_mul(float g, float u) { return u * (g * (1.0f / (1.0f + expf(-g)))); }
 
 // a: the product (the gate's in SwiGLU mode), b: the up product, bias_v: bias[n] or 0.
 template <int MODE>
