@@ -286,9 +286,10 @@ __global__ void __launch_bounds__(GN_THREADS) gated_rmsnorm_vec_kernel(const flo
 // 16 heads of 128 / 128: 67 MB in and out), and the walk above leaves them two dependent look-ups, a trip to memory and a store one after
 // the other in each of 4,096 short blocks.  Here three CTAs an SM take their runs of tiles of 32 columns (16 KB that lie together) through
 // rings of bulk copies: one thread requests tiles and stores the finished ones from where they stand, eight warps (four columns each, a
-// lane four rows) turn them in place; q, k and v of the next tile are on their way meanwhile, and q and k are activated and turned once
-// for a head's tiles.  us, walk / here, requests: 16 15.6 / 16.3,
-// 24 16.8 / 15.7, 32 21.3 / 16.8, 64 38.1 / 28.4 (4.7 TB/s), 128 70.9 / 51.3.  One CTA an SM with a ring of twelve: 51 at 64, the serial work of a tile.
+// lane the rows and the order of sums that it has in the walk, so that an output's bits do not depend on how many requests a step holds)
+// turn them in place; q, k and v of the next tile are on their way meanwhile, and q and k are activated and turned once for a head's tiles.
+// us, walk / here, requests: 16 15.9 / 15.8, 24 18.0 / 15.5, 32 21.6 / 16.7, 64 37.9 / 28.6 (4.7 TB/s), 128 71.1 / 51.4; with four rows that lie
+// together, one load a column, 28.2 and 50.7.  One CTA an SM with a ring of twelve: 51 at 64, the serial work of a tile.
 constexpr int LS_DIM = 128, LS_COLS = 32, LS_WARPS = 8, LS_STAGES = 4, LS_BEHIND = 1, LS_CTAS = 3;
 constexpr int LS_MIN_TILES = 1536;  // fewer: the walk is as fast
 constexpr int LS_TILE = LS_COLS * LS_DIM * 4;
@@ -402,19 +403,24 @@ __global__ void __launch_bounds__(LS_WARPS * 32 + 32, LS_CTAS) linear_attention_
         if (tid < LS_COLS) vs[i & 1][tid] = silu ? silu_f(raw_v) : raw_v;
         if (after < hi) fetch(after);
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        const float4 k4 = *reinterpret_cast<const float4*>(&qk[units & 1][1][4 * lane]);
-        const float4 q4 = *reinterpret_cast<const float4*>(&qk[units & 1][0][4 * lane]);
+        float kk[LS_DIM / 32], qq[LS_DIM / 32];  // rows lane, lane + 32, .. as the walk has them: the same sums in the same order
+#pragma unroll
+        for (int r = 0; r < LS_DIM / 32; ++r) kk[r] = qk[units & 1][1][lane + 32 * r], qq[r] = qk[units & 1][0][lane + 32 * r];
         const float lam = decay[h];
-        float4* S = reinterpret_cast<float4*>(ring + s * LS_TILE) + warp * 4 * (LS_DIM / 4) + lane;
+        float* S = reinterpret_cast<float*>(ring + s * LS_TILE) + warp * 4 * LS_DIM + lane;
         mbar_wait(&full[s], (i / LS_STAGES) & 1, status, 0x81);
         float o[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const float v = vs[i & 1][warp * 4 + c];
-            float4 x = S[c * (LS_DIM / 4)];
-            x.x = fmaf(k4.x, v, lam * x.x), x.y = fmaf(k4.y, v, lam * x.y), x.z = fmaf(k4.z, v, lam * x.z), x.w = fmaf(k4.w, v, lam * x.w);
-            S[c * (LS_DIM / 4)] = x;
-            o[c] = fmaf(x.w, q4.w, fmaf(x.z, q4.z, fmaf(x.y, q4.y, x.x * q4.x)));
+            float acc = 0.0f;
+#pragma unroll
+            for (int r = 0; r < LS_DIM / 32; ++r) {
+                const float x = fmaf(kk[r], v, lam * S[c * LS_DIM + 32 * r]);
+                S[c * LS_DIM + 32 * r] = x;
+                acc = fmaf(x, qq[r], acc);
+            }
+            o[c] = acc;
         }
         fence_proxy_async();  // the copy out reads what every lane wrote
         __syncwarp();
