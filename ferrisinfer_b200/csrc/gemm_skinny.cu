@@ -43,6 +43,8 @@ constexpr int SK_MAX_ROWS = 16 * SK_MAX_MT;
 constexpr int SK_MAX_STAGES = 96;
 constexpr int SK_MAX_TOKENS = 16;
 constexpr int SK_PASS_SMEM = 224 * 1024;          // of a CTA that works in passes (beside 1 KB of alignment and its barriers)
+constexpr int SK_PASS_STAGES = 16;                // at most
+constexpr size_t SK_PASS_RING = 108 * 1024;       // of it the weights on their way, at least
 
 enum SkMode { SK_STORE_BF16 = 0, SK_STORE_F32 = 1, SK_ACCUM_F32 = 2, SK_SWIGLU_BF16 = 3 };
 
@@ -64,6 +66,7 @@ struct SkParams {
     int stages;    // groups of weights that shared memory holds at once
     int boxes_3d;  // the copies use the 3-D maps (K a multiple of 64); else nb == 1 and the 2-D maps
     int x_in_stages;  // the step's rows travel with the weights, a box per stage, instead of standing whole beside them
+    int run;       // passes: warp (kb / run) % 8 takes K block kb
     int up_row_offset;
     int mode;
     int* status;
@@ -442,18 +445,20 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
 // rows on rows 0-7 of the MMA's tile and their up rows on rows 8-15, so that a thread holds both sums of an output.  A slab of
 // 2 x 64 rows at once leaves a copy one K block (128 bytes) of each row, which comes out of HBM at 4.2 TB/s, and CTAs of 64 outputs two
 // rounds with a gap between; sixteen rows at once let a copy bring nine K blocks of them, and the ring runs on from pass to pass,
-// so that the copies never stop.  The step's rows are formed or brought in once for all passes.  Bound by HBM (figures: sk_passes).
+// so that the copies never stop.  The step's rows are formed or brought in once for all passes.  Every warp takes its K blocks out of
+// every stage, namely those that it has in the kernel above, so that the sums are that kernel's to the bit.  Bound by HBM (figures:
+// sk_passes).
 template <int NT, bool ACT = false>
 __global__ void __launch_bounds__(SK_THREADS, 1)
     gemm_skinny_passes_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SkParams p) {
     FERRIS_TL_ENTRY();
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[SK_WARPS], empty[SK_WARPS], full_x;
+    __shared__ uint64_t full[SK_PASS_STAGES], empty[SK_PASS_STAGES], full_x;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int box_bytes = 8 * p.nb * 128, stage_bytes = 2 * box_bytes;  // eight gate rows, eight up rows; a stage for every warp
+    const int box_bytes = 8 * p.nb * 128, stage_bytes = 2 * box_bytes;  // eight gate rows, eight up rows
     const int x_box_bytes = p.x_rows * p.nb * 128;
-    uint8_t* x_smem = smem + (size_t)SK_WARPS * stage_bytes;
+    uint8_t* x_smem = smem + (size_t)p.stages * stage_bytes;
     float* red = reinterpret_cast<float*>(x_smem + (size_t)p.groups * x_box_bytes);  // [pass & 1][warp][NT * 4][lane]
     const int all = (p.N + 7) / 8;  // passes of the product, dealt to the CTAs in turn
     const int passes = ((int)blockIdx.x < all) ? (all - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -462,9 +467,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     if (threadIdx.x == 0) {
         tma_prefetch_descriptor(&map_w);
         if (!p.norm_h) tma_prefetch_descriptor(&map_x);
-        for (int s = 0; s < SK_WARPS; ++s) {
+        for (int s = 0; s < p.stages; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
+            mbar_init(&empty[s], SK_WARPS);
         }
         mbar_init(&full_x, 1);
         mbar_fence_init();
@@ -473,18 +478,19 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     pdl_launch_dependents();
 
     if (warp == SK_WARPS) {
-        int pass = 0, g = 0;  // of the group that is requested next
-        auto request = [&](int it) {
-            const int s = it % SK_WARPS, n0 = first_row(pass);
+        int pass = 0, g = 0, s = 0, phase = 1;  // of the group that is requested next; the phase that frees its stage
+        auto request = [&]() {
+            const int n0 = first_row(pass);
             uint8_t* st = smem + (size_t)s * stage_bytes;
             mbar_expect_tx(&full[s], stage_bytes);
             tma_load_3d(st, &map_w, 0, g * p.nb, n0, &full[s]);
             tma_load_3d(st + box_bytes, &map_w, 0, g * p.nb, p.up_row_offset + n0, &full[s]);
             if (++g == p.groups) g = 0, ++pass;
+            if (++s == p.stages) s = 0, phase ^= 1;
         };
-        const int first = min(total, SK_WARPS);
+        const int first = min(total, p.stages);
         if (lane == 0)
-            for (int it = 0; it < first; ++it) request(it);  // a model's weights: ahead of the wait
+            for (int it = 0; it < first; ++it) request();  // a model's weights: ahead of the wait
         if (!p.norm_h) {
             pdl_wait();
             if (lane == 0) mbar_expect_tx(&full_x, p.groups * x_box_bytes);
@@ -493,8 +499,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
         }
         if (lane == 0)
             for (int it = first; it < total; ++it) {
-                if (!mbar_wait(&empty[it % SK_WARPS], ((it / SK_WARPS) - 1) & 1, p.status, 43)) break;
-                request(it);
+                if (!mbar_wait(&empty[s], phase, p.status, 43)) break;
+                request();
             }
         return;
     }
@@ -511,10 +517,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
         mbar_wait(&full_x, 0, p.status, 42);
     }
     const int mi = lane >> 3, r8 = lane & 7;
-    const uint32_t x_base = smem_u32(x_smem), st = smem_u32(smem + (size_t)warp * stage_bytes);
-    // A operands: matrices (gate rows | up rows) x (columns 0-7 | 8-15 of the K step)
-    const uint32_t wg = st + (mi & 1) * box_bytes;
-    int it = warp, phase = 0;  // this warp's next group and its stage's phase
+    const uint32_t x_base = smem_u32(x_smem), st0 = smem_u32(smem) + (mi & 1) * box_bytes;
+    int s = 0, phase = 0;  // the stage of the next group and its phase
     bool ok = true;
     for (int pass = 0; pass < passes; ++pass) {
         float acc[NT][4];
@@ -522,13 +526,13 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[nt][j] = 0.0f;
-        const int g0 = pass * p.groups;
-        for (; it < g0 + p.groups; it += SK_WARPS, phase ^= 1) {
-            if (ok) ok = mbar_wait(&full[warp], phase, p.status, 44);
-            const int g = it - g0;
-            const uint32_t xg = x_base + g * x_box_bytes;
-            const int blocks = min(p.nb, p.kblocks - g * p.nb);
-            for (int kbi = 0; kbi < blocks; ++kbi) {
+        int kb = warp * p.run, left = p.run;  // this warp's next K block, and how many of its run there are from there on
+        for (int g = 0; g < p.groups; ++g) {
+            if (ok) ok = mbar_wait(&full[s], phase, p.status, 44);
+            // A operands: matrices (gate rows | up rows) x (columns 0-7 | 8-15 of the K step)
+            const uint32_t wg = st0 + s * stage_bytes, xg = x_base + g * x_box_bytes;
+            for (const int first = g * p.nb, end = min(first + p.nb, p.kblocks); kb < end;) {
+                const int kbi = kb - first;
                 uint32_t b[4][NT][2], af[4][4];
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
@@ -547,9 +551,12 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
                 for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[nt], af[ks], b[ks][nt][0], b[ks][nt][1]);
+                ++kb;
+                if (--left == 0) kb += (SK_WARPS - 1) * p.run, left = p.run;
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[warp]);
+            if (lane == 0) mbar_arrive(&empty[s]);
+            if (++s == p.stages) s = 0, phase ^= 1;
         }
         // the warps' sums, added in their order
         float* mine = red + (size_t)(pass & 1) * (SK_WARPS * NT * 4 * 32);
@@ -593,6 +600,7 @@ struct SkPlan {
     int rows, box_rows, x_rows, mt, ctas, kblocks, nb, groups, stages;
     size_t smem;
     int x_in_stages;
+    int run;  // of a plan in passes
 };
 
 // Shared memory of one CTA: the step's rows whole, the weight stages beside them; a slab that does not fit streams
@@ -674,35 +682,44 @@ bool sk_plan(int T, int N, int K, int accs, bool rows_by_tma, SkPlan* out) {
     size_t smem = best_in_stages ? (size_t)stages * (accs * box_rows + x_rows) * nb * 128
                                  : (size_t)stages * accs * box_rows * nb * 128 + (size_t)groups * x_rows * nb * 128;
     if (smem < red_bytes) smem = red_bytes;
-    *out = {rows, box_rows, x_rows, mt, ctas, kblocks, nb, groups, stages, smem + 1024, best_in_stages};
+    *out = {rows, box_rows, x_rows, mt, ctas, kblocks, nb, groups, stages, smem + 1024, best_in_stages, 0};
     return true;
 }
 
-// SwiGLU in passes of eight outputs: where the slab does not stand whole in shared memory, and copies of nine K blocks (or seven, where the
-// step's rows leave no more) fit beside the rows.  Fewer blocks a copy lose what the passes gain; more stages than one a warp bring
-// nothing (the others' copies are under way while a warp works on its own).  Measured (us a launch, weights from HBM, 1 / 8 / 16 tokens,
-// before and in passes of copies of nine): 2 x 18,944 x 3,584 56.7 / 57.1 / 59.4 -> 41.2 / 41.2 (6.6 TB/s) / as before, eight tokens at
-// seven blocks 44.6; 2 x 8,960 x 1,536 13.2 / 13.4 / 14.5 -> 11.8 / 11.5 / 12.4, at three 16.4; 2 x 11,008 x 4,096 61 / 62 / 64 -> 30.5 / 30.5 / as before, at
-// three blocks 64.
+// SwiGLU in passes of eight outputs: where the slab does not stand whole in shared memory, and a ring of 108 KB fits beside the step's
+// rows.  Copies of as many K blocks as leave the fewest groups: a group costs every warp a wait and an arrival (copies of nine blocks
+// throughout: 2 x 18,944 x 3,584 43.2 us, as below 40.6).  Not for rows of less than 24 K blocks, unless a CTA's outputs would take
+// it two rounds and a row has 16.  Measured (us a launch, weights from HBM, rows in bf16 of 1 / 8 / 16 tokens, in one slab and in
+// passes): 2 x 18,944 x 3,584 56.7 / 57.4 / 59.5 -> 40.5 / 40.6 (6.7 TB/s) / as before; 2 x 8,960 x 1,536 13.4 / 13.6 / 14.6 -> 12.2 / 12.1 / 12.5;
+// 2 x 11,008 x 4,096 61.2 / 61.8 / 64.1 -> 29.0 / 28.7 / as before; 2 x 12,000 x 1,280 20.4 / 20.5 / 22.4 -> 14.8 / 14.4 / 15.8; 2 x 18,000 x 1,152 20.5 / 21.1 / 23.0 ->
+// 20.3 / 20.0 / 21.1; but 2 x 9,472 x 1,408 12.5 / 12.7 / 13.7 -> 12.9 / 12.8 / 13.5, x 1,024 11.6 / 11.5 / 11.4 -> 12.6 / 12.2 / 12.3.
+// One warp taking all of a stage, so that its warps share no stage, spares waits (at 8,960 x 1,536 11.4), but adds the products up in another order.
 bool sk_passes(int T, int N, int K, const SkPlan& whole, SkPlan* out) {
-    if ((K & 63) || whole.groups <= whole.stages) return false;
-    const int x_rows = T > 8 ? 16 : 8, nt = T > 8 ? 2 : 1, kblocks = K / SK_BLOCK_K;
+    const int kblocks = K / SK_BLOCK_K, sms = sk_sm_count();
+    if ((K & 63) || whole.groups <= whole.stages || kblocks < (whole.ctas > sms ? 16 : 24)) return false;
+    const int x_rows = T > 8 ? 16 : 8, nt = T > 8 ? 2 : 1;
     const size_t red = (size_t)2 * SK_WARPS * nt * 4 * 32 * 4;
-    for (int nb = 9; nb >= 7; nb -= 2) {
+    SkPlan q = whole;
+    q.run = 0;
+    for (int nb = 7; nb <= 15; nb += 2) {  // (odd: see sk_plan)
         const int groups = (kblocks + nb - 1) / nb;
-        const size_t smem = (size_t)groups * x_rows * nb * 128 + (size_t)SK_WARPS * 16 * nb * 128 + red;
-        if (nb > kblocks || smem > SK_PASS_SMEM) continue;
-        SkPlan q = whole;
-        q.nb = nb, q.groups = groups, q.stages = SK_WARPS, q.x_rows = x_rows, q.x_in_stages = 0;
-        q.smem = smem + 1024;
-        q.rows = q.box_rows = 8;
-        q.mt = 1;
-        const int sms = sk_sm_count(), all = (N + 7) / 8;
-        q.ctas = all < sms ? all : sms;
-        *out = q;
-        return true;
+        const size_t stage = (size_t)16 * nb * 128, fixed = (size_t)groups * x_rows * nb * 128 + red;
+        if (fixed + SK_PASS_RING > SK_PASS_SMEM || (q.run && groups >= q.groups)) continue;
+        int stages = (int)((SK_PASS_SMEM - fixed) / stage);
+        if (stages > SK_PASS_STAGES) stages = SK_PASS_STAGES;
+        if (stages * stage < SK_PASS_RING) continue;
+        q.run = whole.nb;
+        q.nb = nb, q.groups = groups, q.stages = stages;
+        q.smem = fixed + stages * stage + 1024;
     }
-    return false;
+    if (!q.run) return false;
+    q.x_rows = x_rows, q.x_in_stages = 0;
+    q.rows = q.box_rows = 8;
+    q.mt = 1;
+    const int all = (N + 7) / 8;
+    q.ctas = all < sms ? all : sms;
+    *out = q;
+    return true;
 }
 
 template <int NT, bool ACT = false>
@@ -751,6 +768,19 @@ FERRIS_API int ferris_set_gemm_skinny(int on) {
 FERRIS_API int ferris_gemm_skinny_takes(int T, int N, int K, int accumulators, int rows_by_tma) {
     SkPlan plan;
     return (ferris_gemm_skinny_enabled() && sk_plan(T, N, K, accumulators == 2 ? 2 : 1, rows_by_tma != 0, &plan)) ? 1 : 0;
+}
+
+// How a product is cut: plan = {whether in passes, K blocks a copy brings, consecutive K blocks that a warp adds up (run i of a row is warp
+// i % 8's, and the warps' sums are added in their order), stages, shared memory}.
+FERRIS_API int ferris_gemm_skinny_plan(int T, int N, int K, int accumulators, int rows_by_tma, int* plan) {
+    SkPlan whole, q;
+    if (!sk_plan(T, N, K, accumulators == 2 ? 2 : 1, rows_by_tma != 0, &whole))
+        FERRIS_REFUSE("skinny gemm: %d tokens x %d outputs x K=%d is not a shape it takes", T, N, K);
+    const bool passes = accumulators == 2 && sk_passes(T, N, K, whole, &q);
+    if (!passes) q = whole;
+    const int of[5] = {passes ? 1 : 0, q.nb, whole.nb, q.stages, (int)q.smem};
+    for (int i = 0; i < 5; ++i) plan[i] = of[i];
+    return FERRIS_OK;
 }
 
 // x: bf16 [T, K] rows ldx apart (16-byte aligned rows), or null with norm_h / norm_w / norm_eps: the rows are the RMSNorm of the fp32 rows
@@ -816,6 +846,7 @@ FERRIS_API int ferris_gemm_skinny(const void* x, int ldx, const float* norm_h, c
     p.stages = plan.stages;
     p.boxes_3d = boxes_3d ? 1 : 0;
     p.x_in_stages = plan.x_in_stages;
+    p.run = plan.run;
     p.up_row_offset = up_row_offset;
     p.mode = mode;
     p.status = ferris_status_ptr();

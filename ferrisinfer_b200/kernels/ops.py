@@ -537,6 +537,16 @@ def _skinny_takes(x, w, out, accs: int) -> bool:
     return takes
 
 
+def gemm_skinny_plan(tokens: int, outputs: int, k: int, swiglu: bool = False, formed: bool = False) -> dict:
+    """How the kernel for few tokens cuts a product (``formed``: of a LazyRMSNorm): whether its outputs go through in passes, the K
+    blocks of 64 that a copy brings, the consecutive ones that a warp adds up (run i of a row is warp i % 8's; the warps' sums are added
+    in their order), the copies under way at once, the shared memory of a CTA."""
+    plan = (ctypes.c_int * 5)()
+    _check(_lib().ferris_gemm_skinny_plan(_c_int(tokens), _c_int(outputs), _c_int(k), _c_int(2 if swiglu else 1),
+                                          _c_int(0 if formed else 1), plan), "skinny gemm", 0)
+    return dict(passes=bool(plan[0]), blocks=plan[1], run=plan[2], stages=plan[3], smem=plan[4])
+
+
 def gemm_skinny(x, w, bias, out, mode: int, up_row_offset: int = 0):
     """out (+)= x w^T (+ bias) for at most 16 tokens; ``x`` a bf16 tensor or a LazyRMSNorm (formed in the kernel).
     Modes as gemm_tcgen05."""

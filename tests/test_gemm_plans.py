@@ -21,3 +21,15 @@ def test_swiglu_rides_along_where_the_rows_kernel_takes_both_products():
         for M in (1, 4, 8, 12, 16):
             assert (ops.gemm_f32_plan(M, I, K, swiglu=True) > 0) == (ops.gemm_f32_plan(M, 2 * I, K) > 0), (I, K, M)
         assert ops.gemm_f32_plan(33, I, K, swiglu=True) == 0
+
+
+@pytest.mark.parametrize("T, I, K, blocks", [
+    (8, 18944, 3584, 15), (16, 18944, 3584, 0), (8, 8960, 1536, 13), (16, 8960, 1536, 13), (1, 9001, 1536, 13), (8, 11008, 4096, 13),
+    (9, 11008, 4096, 0), (8, 5632, 2048, 11), (16, 13824, 2560, 11), (8, 4864, 896, 0), (8, 9472, 1408, 0), (8, 9536, 1408, 11), (8, 18000, 896, 0),
+    (8, 18000, 1024, 9)])
+def test_gate_and_up_products_of_few_tokens_that_go_through_in_passes(T, I, K, blocks):
+    """Where the weights of a CTA do not stand whole in shared memory and enough of them fit beside the step's rows (the measured times stand
+    beside the rule); 0: the other kernel's."""
+    plan = ops.gemm_skinny_plan(T, I, K, swiglu=True)
+    assert plan["passes"] == (blocks > 0) and (not blocks or plan["blocks"] == blocks)
+    assert not ops.gemm_skinny_plan(T, I, K)["passes"]
