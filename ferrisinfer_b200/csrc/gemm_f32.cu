@@ -450,7 +450,8 @@ FERRIS_API int ferris_gemm_f32_swiglu_takes(const void* x, const void* w, int M,
     if (M <= 0 || N <= 0 || N > (1 << 30) || !ferris_gemm_f32_takes(x, w, nullptr, K, ldx, ldw)) return 0;
     return M <= SWIGLU_MAX_TOKENS ? rows_take(M, 2 * N, K, 2 * RS, q) : ferris_gemm_f32_split_takes(M, 2 * N, K, ldx, ldw);
 }
-// out[t, n] = silu(x[t] . w[n]) (x[t] . w[N + n]), fp32 throughout, with the sums of every other form of the product.
+// out[t, n] = silu(x[t] . w[n]) (x[t] . w[N + n]), fp32 throughout, with the sums of the plain product (on the tensor cores: of one without K
+// splits, which the 2 N rows have where there are many of them).
 // early_weights: no launch that may still run writes w.
 FERRIS_API int ferris_gemm_f32_swiglu(const float* x, const float* w, float* out, int M, int N, int K, int ldx, int ldw, int ldo,
                                       int early_weights, void* stream) {

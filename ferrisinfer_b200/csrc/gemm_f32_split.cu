@@ -17,10 +17,11 @@
 // leader, MMAs, their commit) is longer than any of its parts: with two slots it took 2.45 us a slice at 128 tokens, of which the MMAs
 // are 0.8 and everything else without them 1.65; with three (and the MMAs issued by a warp of their own) 1.8.  Before that: one set of
 // warps that split and drained 4.2, two 3.1, two accumulators in turn 2.45.
-// Measured (us, tokens: 96 / 200 / 777 / 2,048; in brackets the FMA kernels): 1,152 x 896 12 / 17 / 26 / 49 (27 / 29 / 61 / 109), 896 x 896
-// 12 / 16 / 27 / 31 (26 / 28 / 54 / 108), 9,728 x 896 29 / 51 / 105 / 229 (84 / 131 / 351 / 817; 155 TFLOP/s), 896 x 4,864 32 / 37 / 81 / 188 (61 / 79 / 218 / 564).
+// Measured (us, tokens: 96 / 200 / 777 / 2,048; in brackets the FMA kernels): 9,728 x 896 29 / 51 / 105 / 229 (84 / 131 / 351 / 817; 155
+// TFLOP/s), 896 x 4,864 32 / 37 / 80 / 199 (61 / 79 / 218 / 564); 200 / 777 / 2,048: 1,152 x 896 24 / 26 / 50 (29 / 61 / 109), 896 x 896 24 / 26 / 32 (28 / 54 /
+// 108).
 //
-// K SPLITS: where tiles are few a cluster of up to four pairs takes one tile, each a run of slices; the sums meet through
+// K SPLITS: where rows are long and few a cluster of up to four pairs takes one tile, each a run of slices; the sums meet through
 // shared memory and are added in the runs' order.  SwiGLU: a CTA's rows 0..63 are gate rows, 64..127 their up rows.
 //
 // Infinities and overflow: a part of an infinity times a part that is zero is not a number, so a result that is not finite is
@@ -559,26 +560,31 @@ struct SplitPlan {
     int nt, splits, clusters, m_tiles, n_tiles, slices_per;
     double us;
 };
-// The cut of the least time, from what a slice was measured to take (us, token tiles of 32 to 160), a tile's end, the launch and a cluster's
-// exchange.
+// K splits regroup an output's sum, so they are chosen without a look at the number of tokens: a row's bits do not depend on what else is in
+// the step.  Long rows and few of them gain from splits where tokens are few too, and lose the less by them where tokens are many; with
+// many weight rows there are tiles enough.  Against the splits that are best for each of up to ten numbers of tokens from 48 to 4,096 (times the
+// time on average, at worst): 896 x 896 and 1,152 x 896 1.09 and 1.10, 1.7 (192 tokens 24 us instead of 14; FMAs 29); 896 x 4,864 1.07, 1.40;
+// 1,536 x 1,536 1.10, 1.39; 1,536 x 8,960 1.17, 1.46; 2,048 x 2,048 1.13, 1.47; 3,584 x 3,584 1.08, 1.31; 3,584 x 18,944 1.10, 1.23; 9,728 x 896 none.
+int split_count(int slices, int n_tiles) {
+    if (n_tiles >= 20 || slices < 24) return 1;
+    if (slices < 48) return 2;
+    return slices >= 72 && n_tiles <= 8 ? 4 : 3;
+}
+// The cut of a product: its splits, and the token tile of the least time, from what a slice was measured to take (us, token tiles of 32 to
+// 128), a tile's end, the launch and a cluster's exchange.
 SplitPlan split_plan(int M, int rows, int K, bool swiglu, int nt_only = 0, int splits_only = 0) {
     constexpr double SLICE[4] = {1.3, 1.55, 1.7, 1.8};
     SplitPlan best = {};
     const int slices = (K + SP_K - 1) / SP_K, n_tiles = (rows + 2 * SP_M - 1) / (2 * SP_M);
+    const int sp = splits_only ? splits_only : swiglu ? 1 : split_count(slices, n_tiles), per = (slices + sp - 1) / sp;
+    if (sp > 1 && (per < 4 || (sp - 1) * per >= slices)) return best;
+    const int at_once = active_clusters(sp);
     for (int nt = 32; nt <= 128; nt += 32) {
-        if (nt_only && nt != nt_only) continue;
-        const long long m_tiles = (M + nt - 1) / nt;
-        for (int sp = 1; sp <= (swiglu ? 1 : SP_MAX_SPLITS); ++sp) {
-            if (splits_only && sp != splits_only) continue;
-            const int per = (slices + sp - 1) / sp;
-            if (sp > 1 && (per < 4 || (sp - 1) * per >= slices)) continue;
-            if (nt == 128 && per > SP_LEVEL) continue;  // no tensor memory left for the outer sums
-            const int at_once = active_clusters(sp);
-            const long long tiles = m_tiles * n_tiles, rounds = (tiles + at_once - 1) / at_once;
-            const double us = rounds * (per * SLICE[nt / 32 - 1] + (sp > 1 ? 5.0 : 1.0)) + 3.0;
-            if (best.nt && us >= best.us) continue;
-            best = {nt, sp, (int)(sp > 1 || tiles < at_once ? tiles : at_once), (int)m_tiles, n_tiles, per, us};
-        }
+        if ((nt_only && nt != nt_only) || (nt == 128 && per > SP_LEVEL)) continue;  // (128: no tensor memory left for the outer sums)
+        const long long m_tiles = (M + nt - 1) / nt, tiles = m_tiles * n_tiles, rounds = (tiles + at_once - 1) / at_once;
+        const double us = rounds * (per * SLICE[nt / 32 - 1] + (sp > 1 ? 5.0 : 1.0)) + 3.0;
+        if (best.nt && us >= best.us) continue;
+        best = {nt, sp, (int)(sp > 1 || tiles < at_once ? tiles : at_once), (int)m_tiles, n_tiles, per, us};
     }
     return best;
 }
@@ -592,8 +598,9 @@ int run_split(const float* x, const float* w, const float* bias, float* out, int
 
 }  // namespace
 
-// More than 32 tokens and 150 million multiply-adds.  Up to there every form of the product adds in one order, so that a row's bits do not depend
-// on how many others the step brings; from 33 tokens on this kernel would win there too, by 5 to 14 us of 18 to 27.
+// More than 32 tokens and 150 million multiply-adds.  Up to there every form of the product adds in one order, and a row's bits do not depend
+// on how many others the step brings, nor do they beyond (split_count): only on which side of the line the product lies.  From 33 tokens on this
+// kernel would win below it too, by 5 to 14 us of 18 to 27, with other bits for the products of short steps.
 bool ferris_gemm_f32_split_takes(int M, int rows, int K, int ldx, int ldw) {
     return M > 32 && (long long)M * rows * K >= 150000000LL && (long long)((M + 31) / 32) * ((rows + 255) / 256) < (1 << 28) &&
            ldx <= SP_MAX_LD && ldw <= SP_MAX_LD;

@@ -1,7 +1,8 @@
 // Plain matrix product on the CUDA cores: out[t, n] = sum_k x[t, k] * w[n, k] (+ bias[n]).
 // Every product and sum is an fp32 FMA (no tensor cores, no TF32, no reduced-precision staging),
 // and each output is summed in one order whatever the number of rows (even and odd k's ascending within
-// runs, the runs within parts and the parts in ascending order: gemm_f32.cuh), so a row's result does not depend on what else is in the batch.
+// runs, the runs within parts and the parts in ascending order: gemm_f32.cuh), so a row's result does not depend on what else is in the batch
+// (32-bit rows that are aligned have another order from 33 rows and 150 million multiply-adds on: gemm_f32_split.cu).
 // This is the checked fallback for shapes that the tensor-core kernels refuse, and for 32-bit rows that the
 // kernels of gemm_f32.cu do not take (K or strides that are no multiples of four); it sums in the order of theirs.
 //

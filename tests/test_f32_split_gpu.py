@@ -123,6 +123,21 @@ def test_long_products_go_to_the_tensor_cores_by_their_size(device):
     assert ops.launch_count() - before == 1 and torch.equal(act, one)
     assert ops.kernel_status() == 0
 
+# weights for which other K splits are the fastest from size to size, and K's that are no whole slices
+@pytest.mark.parametrize("N, K, sizes", [(896, 896, (188, 300, 512, 777, 1500, 2048)), (1152, 896, (160, 333, 640, 2048)),
+                                         (896, 4864, (40, 64, 100, 300, 777, 2048)), (1500, 2052, (64, 400, 1500)), (256, 1024, (600, 3000))])
+def test_a_row_has_the_same_bits_in_every_step_on_the_tensor_cores(N, K, sizes, device):
+    from ferrisinfer_b200.kernels import ops
+
+    x, w, first = rnd((max(sizes), K), F32, device, 41), rnd((N, K), F32, device, 42, 0.1), None
+    for M in sizes:
+        assert M * N * K >= 150e6
+        out = torch.empty(M, N, device=device)
+        ops.gemm(x[:M], w, None, out)
+        first = out if first is None else first
+        assert torch.equal(out[:sizes[0]], first), M
+    assert ops.kernel_status() == 0
+
 
 # ------------------------------------------------------------------------------------------------------------------ attention
 @pytest.mark.parametrize("window", [0, 50])
