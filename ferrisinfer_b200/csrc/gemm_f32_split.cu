@@ -1,13 +1,15 @@
 // The 32-bit path's products of many tokens on the tensor cores: out[t, n] (+)= sum_k x[t, k] * w[n, k] (+ bias[n]) with operands and
 // sums of 32 bits.
 //
-// Every operand is written as the sum of three bf16 numbers, v = v1 + v2 + v3 (each the rest rounded to nearest; the third is
-// exact, so 24 bits of significand are kept whole), and a product is the six of their nine products that reach into 32 bits:
-// x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1; what is left out is below 2^-26 of |x w|, under half of an fp32 rounding.  The products
+// Every operand, times 2^40, is written as the sum of three bf16 numbers, v = v1 + v2 + v3 (each the rest rounded to nearest; the third
+// is exact), so that every fp32 number below 2^88 keeps all its bits, the smallest subnormal ones too (bf16 ends at 2^-133: without the
+// factor a number of 2^-120 would keep 14 bits).  Sums come back times 2^-80; an operand from 2^88 on or a sum from 2^48 on is no longer
+// finite there (see below).  A product is the six of their nine products that reach into 32 bits: x1 w1, x1 w2, x2 w1, x2 w2, x1 w3,
+// x3 w1.  What is left out, x2 w3 + x3 w2 + x3 w3, is at most 2^-24 of |x w| and some 2^-27 of it on average.  The products
 // themselves are exact.  The tensor core's own additions cut off instead of rounding, so a sum stays there for 32 k's only, the
 // small products first (the cuts then fall on sums a 256th as large) and the two steps of large ones last; after that it is
 // added to sums in registers, rounded to nearest, and these every 1,024 k's to a sum of their own.  Error against 64 bits
-// (2-norm, relative, normal numbers; this kernel / the FMA kernels of gemm_f32.cu): K = 64 0.7 / 1.1, 896 0.9 to 1.15 / 1.55, 4,864
+// (2-norm, relative; this kernel / the FMA kernels of gemm_f32.cu): K = 64 0.7 / 1.1, 896 0.9 to 1.15 / 1.55, 4,864
 // 1.2 to 1.3 / 1.6, 9,220 1.3 / 1.65, each 1e-7.
 //
 // A cluster of two CTAs (cta_group::2) takes 256 weight rows x NT tokens.  Nothing reads the fp32 operands from shared memory: sixteen
@@ -50,6 +52,7 @@ constexpr int SP_MAX_SPLITS = 4;
 constexpr int SP_MAX_LD = 1 << 24;         // elements between rows (offsets of a thread's rows are 32-bit numbers)
 constexpr int SP_EXCHANGE = 4 * 16 * 32 * 4;  // SwiGLU: sums of up rows on their way, of sixteen tokens for each pair of warps
 constexpr int SP_A_PART = SP_M * 128;      // bytes of one part of a slice of the weights
+constexpr float SP_UP = 0x1p40f, SP_DOWN = 0x1p-80f;  // operands are split times 2^40, sums come back times 2^-80
 
 struct SplitParams {
     const float* x;
@@ -69,6 +72,11 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
     return reinterpret_cast<float2&>(r);
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return reinterpret_cast<float2&>(r);
+}
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     const float2 minus = make_float2(-1.0f, -1.0f);  // (a - b in one rounding: -b is exact)
     unsigned long long r;
@@ -79,10 +87,12 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     return reinterpret_cast<float2&>(r);
 }
 
-// Eight fp32 values as three runs of eight bf16: the value rounded, the rest rounded, what then is left.
+// Eight fp32 values times SP_UP as three runs of eight bf16: the value rounded, the rest rounded, what then is left.
 __device__ __forceinline__ float2 unpack2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 __device__ __forceinline__ void split8(const float4 a, const float4 b, uint4& p1, uint4& p2, uint4& p3) {
-    const float2 v[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
+    const float2 up = make_float2(SP_UP, SP_UP);
+    const float2 v[4] = {mul2(make_float2(a.x, a.y), up), mul2(make_float2(a.z, a.w), up), mul2(make_float2(b.x, b.y), up),
+                         mul2(make_float2(b.z, b.w), up)};
     uint32_t o1[4], o2[4], o3[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -400,10 +410,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
 #pragma unroll
                     for (int c = 0; c < 16; ++c) {
                         if (t0 + c0 + c >= p.M) continue;
-                        const float v = acc[c0 + c];
+                        const float v = acc[c0 + c] * SP_DOWN;
                         float* at = o + (size_t)c * p.ldo;
                         if (SWIGLU) {
-                            const float u = up[c * 32];
+                            const float u = up[c * 32] * SP_DOWN;
                             if (is_finite(v) && is_finite(u))
                                 *at = u * (v * (1.0f / (1.0f + expf(-v))));
                             else
@@ -470,8 +480,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_f32_split_kernel(const Spl
                         const int t = t0 + 4 * g + i;
                         if (t >= p.M) continue;
                         float* o = p.out + (size_t)t * p.ldo + n;
-                        const float v = p.bias ? sum[i] + bias : sum[i];
-                        if (is_finite(sum[i]))
+                        const float dot = sum[i] * SP_DOWN, v = p.bias ? dot + bias : dot;
+                        if (is_finite(dot))
                             *o = p.accumulate ? *o + v : v;
                         else
                             odd |= 1u << i;

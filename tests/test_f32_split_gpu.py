@@ -138,6 +138,37 @@ def test_a_row_has_the_same_bits_in_every_step_on_the_tensor_cores(N, K, sizes, 
         assert torch.equal(out[:sizes[0]], first), M
     assert ops.kernel_status() == 0
 
+def some(shape, device, seed, scale=1.0):
+    """Normal numbers without the smallest ones (products with powers of two down to 2^-116 stay exact)."""
+    v = rnd(shape, F32, device, seed, scale)
+    return torch.where(v.abs() < 2.0 ** -10, torch.zeros_like(v), v)
+
+
+@pytest.mark.parametrize("M, N, K, splits", [(64, 300, 200, 1), (96, 256, 1028, 2), (130, 129, 1300, 0)])
+def test_split_products_of_the_smallest_and_of_large_numbers(M, N, K, splits, device):
+    """Parts of a number of any size keep all its bits: operands times powers of two give the result times both."""
+    from ferrisinfer_b200.kernels import ops
+
+    x, w = some((M, K), device, 71), some((N, K), device, 72, 0.1)
+    want = torch.empty(M, N, device=device)
+    ops.gemm_f32_split(x, w, None, want, splits=splits)
+    for i, j in ((-115, 20), (-112, 80), (60, -110), (-60, 70), (39, 0)):
+        out = torch.empty(M, N, device=device)
+        ops.gemm_f32_split(x * 2.0 ** i, w * 2.0 ** j, None, out, splits=splits)
+        assert torch.equal(out, want * 2.0 ** (i + j)), (i, j)
+    act, one = torch.empty(M, N // 2, device=device), torch.empty(M, N // 2, device=device)
+    ops.gemm_f32_split(x, w[:N // 2 * 2], None, act, swiglu=True)
+    ops.gemm_f32_split(x * 2.0 ** -85, w[:N // 2 * 2] * 2.0 ** 85, None, one, swiglu=True)
+    assert torch.equal(act, one)
+    # subnormal operands (fewer bits, all of them kept); subnormal results; sums and operands beyond the split's range, which FMAs form
+    for i, j in ((-140, 60), (100, -145), (-70, -70), (30, 30), (100, -40)):
+        a, b, out = x * 2.0 ** i, w * 2.0 ** j, torch.empty(M, N, device=device)
+        ops.gemm_f32_split(a, b, None, out, splits=splits)
+        limit = (128 + K / 1024 + 8 + 3) * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())  # (of either form; see bound)
+        # (a chain of subnormal sums: half a unit of the last place for each of its products)
+        assert ((out.double() - a.double() @ b.double().t()).abs() <= limit + K * 2.0 ** -150).all(), (i, j)
+    assert ops.kernel_status() == 0
+
 
 # ------------------------------------------------------------------------------------------------------------------ attention
 @pytest.mark.parametrize("window", [0, 50])
