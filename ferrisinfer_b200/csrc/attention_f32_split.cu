@@ -1,7 +1,8 @@
 // Attention of prompts on the 32-bit path, heads of 64: products on tensor cores with operands and sums of 32 bits.
 //
-// Every operand (queries, keys, softmax weights, values) is the sum of three bf16 numbers, v = v1 + v2 + v3 (each the rest rounded to
-// nearest, the third exact), and a product the six of their products that reach into 32 bits; what is left out is below 2^-26 of it.
+// Every operand (queries, keys, softmax weights, values), times 2^40, is the sum of three bf16 numbers, v = v1 + v2 + v3 (each the rest
+// rounded to nearest, the third exact: also for the smallest subnormal numbers), and a product the six of their products that reach into
+// 32 bits; what is left out is at most 2^-24 of it and some 2^-27 on average.
 // The tensor core's additions cut off, so the four steps of large products (v1 v1) of a tile have an accumulator of their own, the
 // twenty of small ones another, and a tile's weighted values join the output by rounded fp32 additions.  Softmax in fp32.
 // Error against 64 bits (2-norm, relative, 1e-7; here / the FMA kernel): 777 tokens 1.4 / 3.0, 2,048 1.6 / 4.0, 512 behind 4,096 keys 2.8 / 12.
@@ -14,7 +15,8 @@
 // 14 heads over 2 (us, before / here): 777 tokens 122 / 84, 2,048 335 / 212, 512 behind 4,096 keys 521 / 365, 31 single tokens beside 481 of a
 // prompt 536 / 174 (a block a request; with a block's requests one after the other 989), 16 to 130 tokens the same 18 to 20.
 //
-// A row whose output is not finite (an infinity times a part of zero) is formed again key by key with FMAs.
+// A row whose output is not finite (an infinity times a part of zero, an operand from 2^88 on, sums from 2^48 on), or that has a score of
+// minus infinity, is formed again key by key with FMAs.
 #include <math.h>
 
 #include "attention_f32_split.cuh"
@@ -29,6 +31,7 @@ constexpr int AF_PITCH = (AF_D + 8) * 2;        // bytes of a row of parts
 constexpr int AF_PART = AF_KEYS * AF_PITCH;
 constexpr int AF_RAW = AF_KEYS * AF_D * 4;      // bytes of a tile's keys as they come
 constexpr int AF_SMEM = 6 * AF_PART + 2 * AF_RAW;
+constexpr float AF_UP = 0x1p40f, AF_DOWN = 0x1p-80f;  // operands are split times 2^40, their products come back times 2^-80
 
 struct SplitAttArgs {
     const float* q;
@@ -42,8 +45,9 @@ struct SplitAttArgs {
     float scale;
 };
 
-// Two values as three packed pairs of bf16.
+// Two values, times AF_UP, as three packed pairs of bf16.
 __device__ __forceinline__ void split2(float lo, float hi, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    lo *= AF_UP, hi *= AF_UP;
     p1 = pack_bf16(lo, hi);
     lo -= __uint_as_float(p1 << 16), hi -= __uint_as_float(p1 & 0xffff0000u);
     p2 = pack_bf16(lo, hi);
@@ -168,6 +172,7 @@ __global__ void __launch_bounds__(AF_THREADS, 2) prefill_attention_f32_kernel(co
     };
 
     float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+    bool over[2] = {false, false};  // whether a score beyond the range came out as minus infinity (any other makes the row's sums not finite)
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
@@ -229,7 +234,9 @@ __global__ void __launch_bounds__(AF_THREADS, 2) prefill_attention_f32_kernel(co
                 for (int e = 0; e < 2; ++e) {
                     const int j = j0 + 8 * n + 2 * (lane & 3) + e;
                     float& v = s[n][2 * a + e];
-                    v = j >= lo && j <= hi ? (v + low[n][2 * a + e]) * p.scale : -INFINITY;
+                    const bool seen = j >= lo && j <= hi;
+                    v = seen ? (v + low[n][2 * a + e]) * AF_DOWN * p.scale : -INFINITY;
+                    over[a] |= seen && v == -INFINITY;
                     best = fmaxf(best, v);
                 }
             best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 1));
@@ -288,14 +295,14 @@ __global__ void __launch_bounds__(AF_THREADS, 2) prefill_attention_f32_kernel(co
         const int r = warp * 16 + (lane >> 2) + 8 * a;
         const bool there = rt[a] < t_end;
         const int head = hk * g + (there ? r % g : 0);
-        bool odd = false;
+        bool odd = there && over[a];
         if (there) {
             float* row = p.out + (size_t)rt[a] * p.ldo + (size_t)head * AF_D;
 #pragma unroll
             for (int n = 0; n < 8; ++n)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const float v = o[n][2 * a + e] / l[a];
+                    const float v = o[n][2 * a + e] / l[a] * AF_DOWN;
                     odd |= !(fabsf(v) <= 3.402823466e38f);
                     row[8 * n + 2 * (lane & 3) + e] = v;
                 }

@@ -218,3 +218,28 @@ def test_split_attention_of_infinities(device):
     ops.paged_attention_simt(qkv, want, *args, max_q_len=1)
     assert torch.allclose(out, want, rtol=1e-4, atol=2e-5, equal_nan=True)
     assert not torch.isfinite(out).all() and torch.isfinite(out[:32]).all()
+
+
+def test_split_attention_of_the_smallest_and_of_large_numbers(device):
+    """Queries, keys and values times powers of two, and the scale that takes the first two back: the same bits; scores beyond the
+    split's range: FMAs."""
+    from ferrisinfer_b200.kernels import ops
+
+    case = AttentionCase(device, F32, 14, 2, 64, 16, [(150, 150), (40, 20)], seed=9)
+    qkv, k, v, tables, ctx, T = case.device_inputs()
+    qkv, k, v = (torch.where(t.abs() < 2.0 ** -10, torch.zeros_like(t), t) for t in (qkv, k, v))
+
+    def attend(i, j, n):
+        out = torch.empty(T, 14 * 64, device=device)
+        ops.paged_attention_simt(qkv * 2.0 ** i, out, k * 2.0 ** j, v * 2.0 ** n, tables, ctx.token_seq, ctx.positions, 14, 2, 64, 0,
+                                 0.125 * 2.0 ** -(i + j), max_q_len=150)
+        return out * 2.0 ** -n
+
+    want = attend(0, 0, 0)
+    large = want.abs() > 2.0 ** -14  # (that stay normal numbers)
+    for i, j, n in ((-115, 80, 0), (70, -112, 0), (0, 0, -108), (-40, -30, 30)):
+        got = attend(i, j, n)
+        assert torch.equal(got[large], want[large]), (i, j, n)
+    for i, j, n in ((30, 30, 0), (100, -100, 0), (0, 0, 100), (60, 50, 60)):
+        got = attend(i, j, n)
+        assert (got - want).norm() <= 2e-6 * want.norm(), (i, j, n)
