@@ -82,6 +82,11 @@ __device__ __noinline__ void row_by_keys(const SplitAttArgs& p, int t, int head,
     const int lane = threadIdx.x & 31, seq = p.token_seq[t], P = p.positions[t];
     const float* q = p.q + (size_t)t * p.ldq + (size_t)head * AF_D;
     const float q0 = q[lane], q1 = q[lane + 32];
+    float* o = p.out + (size_t)t * p.ldo + (size_t)head * AF_D;
+    if (__any_sync(0xffffffffu, q0 != q0 || q1 != q1)) {  // whatever the keys are
+        o[lane] = o[lane + 32] = __int_as_float(0x7fffffff);
+        return;
+    }
     float m = -INFINITY, l = 0.0f, a0 = 0.0f, a1 = 0.0f;
     for (int j = first_key(P, p.window); j <= P; ++j) {
         const float* k = cache_row(p, p.k_cache, seq, hk, j);
@@ -95,7 +100,6 @@ __device__ __noinline__ void row_by_keys(const SplitAttArgs& p, int t, int head,
         a1 = fmaf(w, v[lane + 32], a1 * alpha);
         m = m_new;
     }
-    float* o = p.out + (size_t)t * p.ldo + (size_t)head * AF_D;
     o[lane] = a0 / l;
     o[lane + 32] = a1 / l;
 }

@@ -243,3 +243,33 @@ def test_split_attention_of_the_smallest_and_of_large_numbers(device):
     for i, j, n in ((30, 30, 0), (100, -100, 0), (0, 0, 100), (60, 50, 60)):
         got = attend(i, j, n)
         assert (got - want).norm() <= 2e-6 * want.norm(), (i, j, n)
+
+
+def test_numbers_that_are_none_do_not_hold_a_prompt_up(device):
+    """Rows of a NaN are not formed again number by number."""
+    from ferrisinfer_b200.kernels import ops
+
+    def took(run):
+        times = []
+        for _ in range(4):
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            events[0].record()
+            run()
+            events[1].record()
+            torch.cuda.synchronize()
+            times.append(events[0].elapsed_time(events[1]))
+        return min(times[1:])
+
+    w, out = rnd((2432, 896), F32, device, 81, 0.1), torch.empty(400, 2432, device=device)
+    x = rnd((400, 896), F32, device, 82)
+    case = AttentionCase(device, F32, 14, 2, 64, 16, [(400, 400)], seed=10)
+    qkv, k, v, tables, ctx, T = case.device_inputs()
+    att = torch.empty(T, 14 * 64, device=device)
+    product = lambda: ops.gemm(x, w, None, out)
+    attention = lambda: ops.paged_attention_simt(qkv, att, k, v, tables, ctx.token_seq, ctx.positions, 14, 2, 64, 0, 0.125, max_q_len=400)
+    before = took(product), took(attention)
+    x[:], qkv[:] = math.nan, math.nan
+    after = took(product), took(attention)
+    assert out.isnan().all() and att.isnan().all()
+    # (measured: some four times and the same; number by number some 200 and 70 times)
+    assert after[0] < 20 * before[0] and after[1] < 20 * before[1], (before, after)
