@@ -42,7 +42,7 @@ constexpr int SK_MAX_MT = 4;                      // 16-row tiles of a slab (per
 constexpr int SK_MAX_ROWS = 16 * SK_MAX_MT;
 constexpr int SK_MAX_STAGES = 96;
 constexpr int SK_MAX_TOKENS = 16;
-constexpr int SK_PASS_SMEM = 224 * 1024;          // of a CTA that works in passes (beside 1 KB of alignment and its barriers)
+constexpr size_t SK_PASS_SMEM = 224 * 1024;       // of a CTA that works in passes (beside 1 KB of alignment and its barriers)
 constexpr int SK_PASS_STAGES = 16;                // at most
 constexpr size_t SK_PASS_RING = 108 * 1024;       // of it the weights on their way, at least
 
@@ -624,6 +624,8 @@ int sk_smem_budget() {
     }
     return g_sk_budget;
 }
+// What passes take of it: 4 KB more than the default, or no more than was asked for.
+size_t sk_pass_smem() { return sk_smem_budget() < 220 * 1024 ? (size_t)sk_smem_budget() : SK_PASS_SMEM; }
 
 // rows_by_tma: the step's rows exist as bf16 (not formed by the kernel as a norm), so they may travel with the weights.
 bool sk_plan(int T, int N, int K, int accs, bool rows_by_tma, SkPlan* out) {
@@ -698,14 +700,14 @@ bool sk_passes(int T, int N, int K, const SkPlan& whole, SkPlan* out) {
     const int kblocks = K / SK_BLOCK_K, sms = sk_sm_count();
     if ((K & 63) || whole.groups <= whole.stages || kblocks < (whole.ctas > sms ? 16 : 24)) return false;
     const int x_rows = T > 8 ? 16 : 8, nt = T > 8 ? 2 : 1;
-    const size_t red = (size_t)2 * SK_WARPS * nt * 4 * 32 * 4;
+    const size_t red = (size_t)2 * SK_WARPS * nt * 4 * 32 * 4, most = sk_pass_smem();
     SkPlan q = whole;
     q.run = 0;
     for (int nb = 7; nb <= 15; nb += 2) {  // (odd: see sk_plan)
         const int groups = (kblocks + nb - 1) / nb;
         const size_t stage = (size_t)16 * nb * 128, fixed = (size_t)groups * x_rows * nb * 128 + red;
-        if (fixed + SK_PASS_RING > SK_PASS_SMEM || (q.run && groups >= q.groups)) continue;
-        int stages = (int)((SK_PASS_SMEM - fixed) / stage);
+        if (fixed + SK_PASS_RING > most || (q.run && groups >= q.groups)) continue;
+        int stages = (int)((most - fixed) / stage);
         if (stages > SK_PASS_STAGES) stages = SK_PASS_STAGES;
         if (stages * stage < SK_PASS_RING) continue;
         q.run = whole.nb;

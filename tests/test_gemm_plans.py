@@ -1,5 +1,9 @@
 """How products are divided among kernels; plans are made on the host."""
 
+import os
+import subprocess
+import sys
+
 import pytest
 
 from ferrisinfer_b200.kernels import ops
@@ -33,3 +37,13 @@ def test_gate_and_up_products_of_few_tokens_that_go_through_in_passes(T, I, K, b
     plan = ops.gemm_skinny_plan(T, I, K, swiglu=True)
     assert plan["passes"] == (blocks > 0) and (not blocks or plan["blocks"] == blocks)
     assert not ops.gemm_skinny_plan(T, I, K)["passes"]
+
+
+@pytest.mark.parametrize("kb", [60, 128, 160, 200, 219])
+def test_passes_keep_to_the_shared_memory_that_was_asked_for(kb):
+    code = ("from ferrisinfer_b200.kernels import ops\n"
+            "for T, I, K in ((1, 8960, 1536), (16, 8960, 1536), (8, 18944, 3584), (8, 18000, 1024), (8, 4864, 896)):\n"
+            "    plan = ops.gemm_skinny_plan(T, I, K, swiglu=True)\n"
+            f"    assert not plan['passes'] or plan['smem'] <= {kb} * 1024 + 1024, (T, I, K, plan)\n")
+    subprocess.run([sys.executable, "-c", code], check=True, env={**os.environ, "FERRIS_SKINNY_SMEM_KB": str(kb)},
+                   cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
