@@ -28,6 +28,8 @@
 //
 // Infinities and overflow: a part of an infinity times a part that is zero is not a number, so a result that is not finite is
 // formed again with FMAs in the order of gemm_f32.cuh.
+#include <atomic>
+
 #include "common.cuh"
 #include "gemm_f32.cuh"
 #include "sm100.cuh"
@@ -555,10 +557,16 @@ int launch_split_of(int nt, const SplitParams& p, int clusters, cudaStream_t s) 
     return launch_split<128, SWIGLU>(p, clusters, s);
 }
 
-// Clusters of so many pairs that the GPU holds at once, a CTA an SM (a cluster keeps to a GPC).
+// Clusters of so many pairs that the current GPU holds at once, a CTA an SM (a cluster keeps to a GPC); asked for once on each GPU, and where
+// two threads ask at once they write the same.
 int active_clusters(int pairs) {
-    static int known[SP_MAX_SPLITS + 1] = {};
-    if (known[pairs] > 0) return known[pairs];
+    constexpr int DEVICES = 16;
+    static std::atomic<int> known[DEVICES][SP_MAX_SPLITS + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError(), dev = DEVICES;
+    const bool keep = dev >= 0 && dev < DEVICES;
+    if (keep)
+        if (const int n = known[dev][pairs].load(std::memory_order_relaxed)) return n;
     constexpr int UNKNOWN[SP_MAX_SPLITS + 1] = {0, 74, 32, 20, 12};
     const size_t smem = SP_SLOTS * SplitShape<128>::SLOT + 1024;
     int n = 0;
@@ -579,7 +587,9 @@ int active_clusters(int pairs) {
             n = 0;
         }
     }
-    return known[pairs] = n > 0 ? n : UNKNOWN[pairs];
+    if (n <= 0) n = UNKNOWN[pairs];
+    if (keep) known[dev][pairs].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 struct SplitPlan {
