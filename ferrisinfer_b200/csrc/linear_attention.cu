@@ -446,7 +446,8 @@ int launch_singles(const void* qkv, int ld, int q_off, int k_off, int v_off, flo
                    const RotaryArgs rot, cudaStream_t s) {
     if (int rc = ferris_allow_dynamic_smem((const void*)linear_attention_singles_kernel<T>, LS_SMEM)) return rc;
     const long long tiles = (long long)seqs * heads * (vdim / LS_COLS);
-    ferris_launch(linear_attention_singles_kernel<T>, dim3((unsigned)(tiles < 148 * LS_CTAS ? tiles : 148 * LS_CTAS)), dim3(LS_WARPS * 32 + 32),
+    const int sms = ferris_sm_count(), most = (sms > 0 ? sms : 148) * LS_CTAS;
+    ferris_launch(linear_attention_singles_kernel<T>, dim3((unsigned)(tiles < most ? tiles : most)), dim3(LS_WARPS * 32 + 32),
                   LS_SMEM, s, (const T*)qkv, ld, q_off, k_off, v_off, out, ldo, state, decay, seq_q_start, seq_state_slot, seqs, heads, vdim,
                   silu, write_state, rot, ferris_status_ptr());
     FERRIS_LAUNCH_CHECK();
