@@ -18,10 +18,10 @@
 #define FERRIS_BF16 1
 
 void ferris_set_error(const char* fmt, ...);
+FERRIS_API int ferris_sm_count();  // of the current GPU; below zero: unknown
 
 // Allow `fn` (a kernel) `bytes` of dynamic shared memory on the current device; the driver is asked only when the
 // size grows.  Returns FERRIS_OK or a cudaError_t (text in ferris_last_error()).
-FERRIS_API int ferris_sm_count();  // of the current GPU; below zero: unknown
 int ferris_allow_dynamic_smem(const void* fn, size_t bytes);
 
 #define FERRIS_REFUSE(...)            \

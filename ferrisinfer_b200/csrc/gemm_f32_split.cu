@@ -8,7 +8,7 @@
 // x3 w1.  What is left out, x2 w3 + x3 w2 + x3 w3, is at most 2^-24 of |x w| and some 2^-27 of it on average.  The products
 // themselves are exact.  The tensor core's own additions cut off instead of rounding, so a sum stays there for 32 k's only, the
 // small products first (the cuts then fall on sums a 256th as large) and the two steps of large ones last; after that it is
-// added to sums in registers, rounded to nearest, and these every 1,024 k's to a sum of their own.  Error against 64 bits
+// added to sums in registers, rounded to nearest, and these every 1,280 k's to a sum of their own.  Error against 64 bits
 // (2-norm, relative; this kernel / the FMA kernels of gemm_f32.cu): K = 64 0.7 / 1.1, 896 0.9 to 1.15 / 1.55, 4,864
 // 1.2 to 1.3 / 1.6, 9,220 1.3 / 1.65, each 1e-7.
 //

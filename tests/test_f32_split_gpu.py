@@ -15,15 +15,15 @@ F32 = torch.float32
 
 def bound(x, w, K):
     """|error| of a product: in a run of 32 k's two additions of large products cut off (2^-23 each) and the 32 large products, laid
-    out at the largest one's exponent before they are added, may lose 2^-23 each; the rest is added in rounded fp32: at most 32
-    runs to a sum, the sums of 1,024 k's, at most four splits, the bias.  The small products and what is left out: 2^-24."""
-    steps = 2 * (2 + 32) + min(32, K / 32 + 1) + K / 1024 + 1 + 4 + 1 + 1
+    out at the largest one's exponent before they are added, may lose 2^-23 each; the rest is added in rounded fp32: at most 40
+    runs to a sum, the sums of 1,280 k's, at most four splits, the bias.  The small products 2^-24, what is left out as much."""
+    steps = 2 * (2 + 32) + min(40, K / 32 + 1) + K / 1280 + 1 + 4 + 1 + 2
     return steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
 
 
 # token tiles of 32 to 128: one token more than a tile, one less, exactly; weight rows around 128 and 256; k's around slices of 64 and
-# around the 1,024 of the outer sum
-@pytest.mark.parametrize("M, N, K", [(1, 1, 4), (33, 40, 60), (160, 256, 128), (161, 129, 68), (95, 257, 1024), (31, 300, 1092),
+# around the 1,280 and 2,560 of the outer sum
+@pytest.mark.parametrize("M, N, K", [(1, 1, 4), (33, 40, 60), (160, 256, 128), (161, 129, 68), (95, 257, 1024), (31, 300, 1092), (130, 129, 1280), (70, 300, 1284), (64, 40, 2560), (33, 130, 2564),
                                      (130, 896, 896), (50, 33, 9220)])
 def test_split_products_against_64_bits(M, N, K, device):
     from ferrisinfer_b200.kernels import ops
@@ -73,6 +73,36 @@ def test_split_products_with_swiglu_on_the_way(M, I, K, device):
         out = torch.full((M, I), 7.0, device=device)
         ops.gemm_f32_split(x, w, None, out, swiglu=True, token_tile=tile)
         assert torch.equal(out, want), tile
+    assert ops.kernel_status() == 0
+
+
+# more tiles than clusters that the GPU holds (74 pairs), so that a cluster's outer sums begin anew
+@pytest.mark.parametrize("K", [1280, 1284, 2564])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_split_products_of_many_tiles_and_long_rows(swiglu, K, device):
+    from ferrisinfer_b200.kernels import ops
+
+    M, N = 2100, 300
+    x, w = rnd((M, K), F32, device, 51), rnd((2 * N if swiglu else N, K), F32, device, 52, 0.1)
+    y, limit = x.double() @ w.double().t(), bound(x, w, K)
+    first = None
+    for tile in (32, 64, 96, 128):
+        if tile == 128 and K > 1280:
+            with pytest.raises(Exception, match="splits"):
+                ops.gemm_f32_split(x, w, None, torch.empty(M, N, device=device), swiglu=swiglu, token_tile=tile, splits=1)
+            continue
+        out = torch.empty(M, N, device=device)
+        ops.gemm_f32_split(x, w, None, out, swiglu=swiglu, token_tile=tile, splits=1)
+        first = out if first is None else first
+        assert torch.equal(out, first), tile
+    if not swiglu:
+        assert ((first.double() - y).abs() <= limit).all()
+    else:
+        plain, want = torch.empty(M, 2 * N, device=device), torch.empty(M, N, device=device)
+        ops.gemm_f32_split(x, w, None, plain, splits=1)
+        assert ((plain.double() - y).abs() <= limit).all()
+        ops.swiglu(plain, want)
+        assert torch.equal(first, want)
     assert ops.kernel_status() == 0
 
 
