@@ -10,10 +10,12 @@
 // A block takes 64 query rows (the g query heads of one kv head for floor(64 / g) consecutive tokens of a request), a warp 16 of
 // them, and walks the keys in tiles of 64: each warp brings 16 keys and values of the next tile in by cp.async while this one is
 // multiplied, splits them once for all warps and stores the parts in rows of 144 bytes, from which ldmatrix reads without conflicts.
-// Queries stay split in registers, weights are split where the scores lie.  Bound by mma.sync (384 of 16 x 8 x 16 a warp and tile, one in
-// five cycles an SM); before, FMAs bound by what shared memory returns to the lanes (attention_simt.cu, which takes every other form).
-// 14 heads over 2 (us, before / here): 777 tokens 122 / 84, 2,048 335 / 212, 512 behind 4,096 keys 521 / 365, 31 single tokens beside 481 of a
-// prompt 536 / 174 (a block a request; with a block's requests one after the other 989), 16 to 130 tokens the same 18 to 20.
+// Queries stay split in registers, weights are split where the scores lie.  Bound by the chain of a block's tiles at two blocks of four
+// warps an SM: 2,048 tokens keep the tensor pipe busy 41 % of the time; 777 tokens, whose 174 blocks leave most SMs one, 14 %, and last as
+// long as the block that walks 13 tiles (4 x 384 products of 16 x 8 x 16 each, which the pipe alone would take in some 52 us).  Before, FMAs
+// bound by what shared memory returns to the lanes (attention_simt.cu, which takes every other form).  14 heads over 2 (us, before /
+// here): 777 tokens 123 / 83, 2,048 339 / 213, 512 behind 4,096 keys 521 / 367, 31 single tokens beside 481 of a prompt 456 / 149 (a block a
+// request; with a block's requests one after the other much longer), 4 prompts of 96 21 / 20.
 //
 // A row whose output is not finite (an infinity times a part of zero, an operand from 2^88 on, sums from 2^48 on), or that has a score of
 // minus infinity, is formed again key by key with FMAs.

@@ -533,8 +533,9 @@ void launch_lanes(const void* q, int ldq, void* out, int ldo, const void* k_cach
 // kernel above's.
 // Bound by what shared memory returns to the lanes: 16 bytes a lane take four cycles of an SM a warp, and eight FMAs go with each.
 // Four blocks share an SM, so that the rows of one come in while others compute; blocks with the most keys begin first.
-// A prompt of 777 tokens, 14 heads of 64 over 2, fp32 (plain scores of such heads are attention_f32_split.cu's): 110 us, 137 with the head size known at run time only (the instructions),
-// 193 with blocks of 64 rows, tiles of 32 keys and two rows a lane.
+// A prompt of 777 tokens, 14 heads of 64 over 2, fp32 (plain scores of such heads are attention_f32_split.cu's): 123 us; in one earlier
+// comparison 110, 137 with the head size known at run time only (the instructions), 193 with blocks of 64 rows, tiles of 32 keys and two rows
+// a lane.
 // ---------------------------------------------------------------------------------------------
 constexpr int TL_KEYS = 64;
 
