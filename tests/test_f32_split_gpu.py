@@ -134,6 +134,28 @@ def test_split_products_of_infinities_and_of_the_largest_numbers(device):
         assert torch.allclose(out[t], want[0], rtol=1e-4, atol=1e-4, equal_nan=True), t
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3, 4])
+def test_infinities_among_k_splits(splits, device):
+    """Whichever pair of a cluster owns an output, with a bias and a sum to add to: the FMA kernel's result; a row of a NaN is NaN, and
+    the rows and columns beside are left alone."""
+    from ferrisinfer_b200.kernels import ops
+
+    M, N, K = 70, 300, 1028
+    x, w, bias, acc = rnd((M, K), F32, device, 91), rnd((N, K), F32, device, 92, 0.1), rnd((N,), F32, device, 93), rnd((M, N), F32, device, 94)
+    x[2, 1000], x[33, 5], x[69, 700], x[64, 64] = math.inf, math.nan, -math.inf, 3e38
+    w[140, 300], w[299, 1027] = math.inf, -math.inf
+    x[10, 300] = 0.0  # infinity times zero
+    out, want = acc.clone(), acc.clone()
+    ops.gemm_f32_split(x, w, bias, out, accumulate=True, splits=splits)
+    for t in range(0, M, 7):  # (few rows: the FMA kernels)
+        ops.gemm_simt(x[t:t + 7], w, bias, want[t:t + 7], accumulate=True)
+    assert out[33].isnan().all() and out[10, 140].isnan() and torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    assert torch.isfinite(out).sum() > 60 * 290
+    ok = torch.isfinite(want)
+    assert torch.allclose(out[ok], want[ok], rtol=1e-5, atol=2e-5)
+    assert ops.kernel_status() == 0
+
+
 def test_long_products_go_to_the_tensor_cores_by_their_size(device):
     """``gemm`` of a long step: the split product's bits; the weight may be what the launch before writes; SwiGLU in one launch."""
     from ferrisinfer_b200.kernels import ops
